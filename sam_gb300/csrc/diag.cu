@@ -200,7 +200,7 @@ __global__ void k_sum_finish(const double* part, int np, double* out) {
 // Spectral derivative of a real (Nx, Ny) plane along x (dir 0) or y (dir 1).
 // Two real lines share one complex transform; kx (or ky) <= k_max keep i k,
 // everything else (the mean and the truncated band) is zeroed.
-__global__ void k_deriv(Grid g, int dir, const FftPlan* __restrict__ gpl, const double2* __restrict__ gtw,
+__global__ void k_deriv(Grid g, int dir, const FftPlan* __restrict__ gpl, const fxw* __restrict__ gtw,
                         const double* __restrict__ u, double* __restrict__ du, int pairs_per_cta) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ FftPlan pl;
@@ -208,8 +208,8 @@ __global__ void k_deriv(Grid g, int dir, const FftPlan* __restrict__ gpl, const 
   __syncthreads();
   const int n = pl.n;
   const int ld = line_stride(n);
-  double2* s_tw = reinterpret_cast<double2*>(smem_raw);
-  double2* s_ln = s_tw + pl.tw_total;
+  fxw* s_tw = reinterpret_cast<fxw*>(smem_raw);
+  double2* s_ln = reinterpret_cast<double2*>(s_tw + pl.tw_total);
   for (int e = threadIdx.x; e < pl.tw_total; e += blockDim.x) s_tw[e] = gtw[e];
   const int nrows = dir == 0 ? g.ny : g.nx;  // lines along the derivative direction
   const long long sline = dir == 0 ? g.nx : 1;
@@ -396,7 +396,7 @@ void diag_cl_energy(const DiagArgs& d, const void* u, double* scratch, double* h
   cudaMemcpyAsync(host_out, out, sizeof(double), cudaMemcpyDeviceToHost, s);
 }
 
-void diag_deriv(const Grid& g, int dir, const FftPlan* dplan, const double2* tw, const FftPlan& hplan, const double* u,
+void diag_deriv(const Grid& g, int dir, const FftPlan* dplan, const fxw* tw, const FftPlan& hplan, const double* u,
                 double* du, cudaStream_t s) {
   const int n = hplan.n;
   const int ld = line_stride(n);

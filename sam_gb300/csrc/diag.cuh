@@ -19,6 +19,6 @@ double diag_fp64_peak(cudaStream_t s);
 void diag_spectra(const DiagArgs& d, const void* u, const void* r, double* scratch, double* host_out, cudaStream_t s);
 void diag_div_check(const DiagArgs& d, const void* u, double* scratch, double* host_out, cudaStream_t s);
 void diag_cl_energy(const DiagArgs& d, const void* u, double* scratch, double* host_out, cudaStream_t s);
-void diag_deriv(const Grid& g, int dir, const FftPlan* dplan, const double2* tw, const FftPlan& hplan, const double* u,
+void diag_deriv(const Grid& g, int dir, const FftPlan* dplan, const fxw* tw, const FftPlan& hplan, const double* u,
                 double* du, cudaStream_t s);
 }  // namespace samgpu

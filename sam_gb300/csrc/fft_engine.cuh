@@ -14,7 +14,10 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "ddfloat.cuh"
+#include "fx64.cuh"
 
 namespace samgpu {
 
@@ -23,6 +26,13 @@ template <> struct Cx<double> { using type = double2; };
 template <> struct Cx<float> { using type = float2; };
 template <> struct Cx<dd> { using type = ddc; };
 template <typename T> using cx_t = typename Cx<T>::type;
+
+// Type of a transform's twiddles: fixed point for the FP64 form's lines
+// (fx64.cuh), else the lines' own type.
+template <typename C> struct TwOf { using type = C; };
+template <> struct TwOf<double2> { using type = fxw; };
+template <typename T> using tw_t = typename TwOf<cx_t<T>>::type;
+static_assert(sizeof(fxw) == sizeof(double2), "a twiddle table's entries have one size");
 
 template <typename C> __device__ __forceinline__ C mk(decltype(C::x) a, decltype(C::x) b) { C r; r.x = a; r.y = b; return r; }
 
@@ -160,6 +170,20 @@ template <int SIGN, typename C> __device__ __forceinline__ C cmul_si(C a) {
   if (SIGN < 0) return mk<C>(a.y, -a.x);
   return mk<C>(-a.y, a.x);
 }
+
+// Code paths of the line transforms: kFftAny picks at run time (the plan's
+// length); kFft256 compiles only the 16 x 16 register path (n = 256) and
+// kFftGeneric only the Stockham stages with the radix chosen at run time;
+// PATH = n (32, 64, 96, 128, 256, 512) compiles the Stockham stages of that length
+// with their radices fixed at compile time.  A kernel built for one length
+// thus carries no registers for another path.
+// The FP64 form's lines run in fixed point (fx64.cuh) up to kFxMaxLine points
+// and in FP64 arithmetic beyond (kFftLong): the fixed-point roundings grow as
+// sqrt(n) against the line's norm and pass FP64's own near n = 1000 (2.1
+// against 1.9 in units of 2^-53 for white lines at 1024, 0.9 against 1.8 at
+// 512, 0.55 against 1.6 at 256).
+constexpr int kFftAny = 0, kFft256 = 1, kFftGeneric = 2, kFftLong = 3;
+constexpr int kFxMaxLine = 512;
 
 struct FftStage {
   int p;       // radix
@@ -412,6 +436,79 @@ __device__ __forceinline__ void fft_stage(C* line, const C* __restrict__ tw, con
   team_sync(TW);
 }
 
+// The same stage of an FP64 line in fixed point (fx64.cuh).  The first stage
+// (FIRST, l = 1: no twiddles) reads doubles through load and fixes the line's
+// scale, which it leaves in sc; the others read the line's integers.  The
+// last stage writes doubles, the others integers.
+template <int P, int SIGN, bool FIRST, typename Ld>
+__device__ __forceinline__ void fx_stage(double2* line, const fxw* __restrict__ tw, const FftStage& s, int n, int tl,
+                                         int TW, Ld load, FxScale& sc, bool last) {
+  constexpr int MAXB = Emax<double2>::value / P;
+  const int nb = n / P;
+  fxc a[MAXB][P];
+  int ds[MAXB];  // where the butterfly's outputs start
+  if constexpr (FIRST) {
+    double2 v[MAXB][P];
+#pragma unroll
+    for (int i = 0; i < MAXB; ++i) {
+      const int b = tl + i * TW;
+      ds[i] = b;
+#pragma unroll
+      for (int q = 0; q < P; ++q) v[i][q] = make_double2(0.0, 0.0);
+      if (b < nb) {
+#pragma unroll
+        for (int q = 0; q < P; ++q) v[i][q] = load(b + s.m * q);
+      }
+    }
+    sc = fx_begin<MAXB * P>(&v[0][0], &a[0][0], TW);
+  } else {
+    const fxc* fl = reinterpret_cast<const fxc*>(line);
+#pragma unroll
+    for (int i = 0; i < MAXB; ++i) {
+      const int b = tl + i * TW;
+      ds[i] = 0;
+      if (b < nb) {
+        const int f = div_m(b, s);
+        const int src = b + f * s.m * (P - 1);
+        ds[i] = b;
+        const fxw* w = tw + s.tw_off + f * (P - 1);
+        a[i][0] = fl[sidx(src)];
+#pragma unroll
+        for (int q = 1; q < P; ++q) a[i][q] = ctw<SIGN>(fl[sidx(src + s.m * q)], w[q - 1]);
+      }
+    }
+  }
+  team_sync(TW);
+  const int os = s.l * s.m;
+#pragma unroll
+  for (int i = 0; i < MAXB; ++i) {
+    const int b = tl + i * TW;
+    if (b < nb) {
+      dftp<P, SIGN>(a[i]);
+      if (last) {
+#pragma unroll
+        for (int q = 0; q < P; ++q) line[sidx(ds[i] + q * os)] = fx_out(a[i][q], sc);
+      } else {
+        fxc* fl = reinterpret_cast<fxc*>(line);
+#pragma unroll
+        for (int q = 0; q < P; ++q) fl[sidx(ds[i] + q * os)] = a[i][q];
+      }
+    }
+  }
+  team_sync(TW);
+}
+template <int SIGN, bool FIRST, typename Ld>
+__device__ __forceinline__ void fx_stage_p(double2* line, const fxw* __restrict__ tw, const FftStage& st, int n, int tl,
+                                           int TW, Ld load, FxScale& sc, bool last) {
+  switch (st.p) {
+    case 8: fx_stage<8, SIGN, FIRST>(line, tw, st, n, tl, TW, load, sc, last); break;
+    case 4: fx_stage<4, SIGN, FIRST>(line, tw, st, n, tl, TW, load, sc, last); break;
+    case 2: fx_stage<2, SIGN, FIRST>(line, tw, st, n, tl, TW, load, sc, last); break;
+    case 3: fx_stage<3, SIGN, FIRST>(line, tw, st, n, tl, TW, load, sc, last); break;
+    default: fx_stage<5, SIGN, FIRST>(line, tw, st, n, tl, TW, load, sc, last); break;
+  }
+}
+
 // Full transform of one line (all threads of the team call this together;
 // a team with no line passes active=false and still synchronises).
 template <int SIGN, typename C, typename Ld>
@@ -426,26 +523,31 @@ __device__ __forceinline__ void fft_stage_p(C* line, const C* __restrict__ tw, c
   }
 }
 
-// Full transform of one line (all threads of the team call this together;
-// a team with no line passes active=false and still synchronises).
-template <int SIGN, typename C>
-__device__ __forceinline__ void fft_line(C* line, const C* __restrict__ tw, const FftPlan& pl, int tl, bool active) {
+// Full transform of one line, the first stage reading its inputs through
+// first(idx), so a caller can form the line on the fly (e.g. the product of
+// two other lines).  All threads of the team call this together; a team with
+// no line passes active=false and still synchronises.
+template <int SIGN, int PATH, typename C, typename First>
+__device__ __forceinline__ void fft_line_from(C* line, const typename TwOf<C>::type* __restrict__ tw, const FftPlan& pl,
+                                              int tl, bool active, First first) {
   const int n = pl.n;
   const int TW = team_of<C>(pl);
   const int tla = active ? tl : (1 << 20);  // inactive lanes own no butterfly
-  for (int s = 0; s < pl.nst; ++s) fft_stage_p<SIGN>(line, tw, pl.st[s], n, tla, TW, LineLoad<C>{line});
-}
-
-// As fft_line, but the first stage reads its inputs through first(idx), so a
-// caller can form the line on the fly (e.g. the product of two other lines).
-template <int SIGN, typename C, typename First>
-__device__ __forceinline__ void fft_line_from(C* line, const C* __restrict__ tw, const FftPlan& pl, int tl,
-                                              bool active, First first) {
-  const int n = pl.n;
-  const int TW = team_of<C>(pl);
-  const int tla = active ? tl : (1 << 20);
-  fft_stage_p<SIGN>(line, tw, pl.st[0], n, tla, TW, first);
-  for (int s = 1; s < pl.nst; ++s) fft_stage_p<SIGN>(line, tw, pl.st[s], n, tla, TW, LineLoad<C>{line});
+  if constexpr (std::is_same<C, double2>::value && PATH != kFftLong) {
+    if (PATH != kFftAny || n <= kFxMaxLine) {
+      FxScale sc;
+      fx_stage_p<SIGN, true>(line, tw, pl.st[0], n, tla, TW, first, sc, pl.nst == 1);
+      for (int s = 1; s < pl.nst; ++s)
+        fx_stage_p<SIGN, false>(line, tw, pl.st[s], n, tla, TW, LineLoad<C>{line}, sc, s + 1 == pl.nst);
+      return;
+    }
+  }
+  if constexpr (!std::is_same<C, double2>::value || PATH == kFftLong || PATH == kFftAny) {
+    // (a table of a length above kFxMaxLine holds FP64 twiddles)
+    const C* w = reinterpret_cast<const C*>(tw);
+    fft_stage_p<SIGN>(line, w, pl.st[0], n, tla, TW, first);
+    for (int s = 1; s < pl.nst; ++s) fft_stage_p<SIGN>(line, w, pl.st[s], n, tla, TW, LineLoad<C>{line});
+  }
 }
 
 // n = 256 as 16 x 16 in registers: a team of 16 threads per line, two lines
@@ -493,13 +595,56 @@ __device__ __forceinline__ void fft256_lines(C* base, int ld, int nlines, const 
   }
 }
 
-// Code paths of the line transforms: kFftAny picks at run time (the plan's
-// length); kFft256 compiles only the 16 x 16 register path (n = 256) and
-// kFftGeneric only the Stockham stages with the radix chosen at run time;
-// PATH = n (32, 64, 96, 128, 256, 512) compiles the Stockham stages of that length
-// with their radices fixed at compile time.  A kernel built for one length
-// thus carries no registers for another path.
-constexpr int kFftAny = 0, kFft256 = 1, kFftGeneric = 2;
+// The same for FP64 lines in fixed point: 16 of the line's doubles become
+// integers in each thread once the team has agreed on the line's scale, and
+// the second stage's results become doubles on their way to shared memory.
+template <int SIGN, typename First>
+__device__ __forceinline__ void fft256_lines(double2* base, int ld, int nlines, const fxw* __restrict__ tw,
+                                             const FftPlan& pl, First first) {
+  const int team = threadIdx.x >> 4;
+  const int k = threadIdx.x & 15;
+  const int nteams = blockDim.x >> 4;
+  const int rounds = (nlines + nteams - 1) / nteams;
+  const fxw* w = tw + pl.tw16_off + k;  // w[16 q] = w_256^{k q}
+  for (int r = 0; r < rounds; ++r) {
+    const int L = r * nteams + team;
+    const bool active = L < nlines;
+    double2* line = base + (active ? L : 0) * ld;
+    fxc* fl = reinterpret_cast<fxc*>(line);
+    fxc a[16];
+    FxScale sc;
+    {
+      double2 v[16];
+#pragma unroll
+      for (int q = 0; q < 16; ++q) v[q] = make_double2(0.0, 0.0);
+      if (active) {
+        const auto ld0 = first(L);
+#pragma unroll
+        for (int q = 0; q < 16; ++q) v[q] = ld0(k + 16 * q);
+      }
+      sc = fx_begin<16>(v, a, 16);
+    }
+    dft16<SIGN>(a);
+    __syncwarp();
+    if (active) {
+#pragma unroll
+      for (int s = 0; s < 16; ++s) fl[sidx(16 * s + k)] = a[s];
+    }
+    __syncwarp();
+    if (active) {
+      a[0] = fl[sidx(16 * k)];
+#pragma unroll
+      for (int q = 1; q < 16; ++q) a[q] = ctw<SIGN>(fl[sidx(16 * k + q)], w[16 * q]);
+      dft16<SIGN>(a);
+    }
+    __syncwarp();
+    if (active) {
+#pragma unroll
+      for (int s = 0; s < 16; ++s) line[sidx(k + 16 * s)] = fx_out(a[s], sc);
+    }
+    __syncwarp();
+  }
+}
 
 // The s-th radix of the plan for length n (build_plan's order: 8s, then 4,
 // 2, 3, 5) and the number of stages, at compile time.
@@ -529,47 +674,28 @@ template <int PATH> __device__ __forceinline__ int tw_load(const FftPlan& pl) {
 
 // Stages S.. of a compile-time length N on one line; stage 0 reads through first.
 template <int SIGN, int N, int S, typename C, typename First>
-__device__ __forceinline__ void fft_ct_stages(C* line, const C* __restrict__ tw, const FftPlan& pl, int tl, int TW,
-                                              First first) {
+__device__ __forceinline__ void fft_ct_stages(C* line, const typename TwOf<C>::type* __restrict__ tw, const FftPlan& pl,
+                                              int tl, int TW, First first, FxScale sc = FxScale{}) {
   if constexpr (S < ct_nst(N)) {
-    if constexpr (S == 0) fft_stage<ct_radix(N, 0), SIGN>(line, tw, pl.st[0], N, tl, TW, first);
-    else fft_stage<ct_radix(N, S), SIGN>(line, tw, pl.st[S], N, tl, TW, LineLoad<C>{line});
-    fft_ct_stages<SIGN, N, S + 1>(line, tw, pl, tl, TW, first);
+    if constexpr (std::is_same<C, double2>::value) {
+      if constexpr (S == 0) fx_stage<ct_radix(N, 0), SIGN, true>(line, tw, pl.st[0], N, tl, TW, first, sc, ct_nst(N) == 1);
+      else fx_stage<ct_radix(N, S), SIGN, false>(line, tw, pl.st[S], N, tl, TW, LineLoad<C>{line}, sc, S + 1 == ct_nst(N));
+    } else {
+      if constexpr (S == 0) fft_stage<ct_radix(N, 0), SIGN>(line, tw, pl.st[0], N, tl, TW, first);
+      else fft_stage<ct_radix(N, S), SIGN>(line, tw, pl.st[S], N, tl, TW, LineLoad<C>{line});
+    }
+    fft_ct_stages<SIGN, N, S + 1>(line, tw, pl, tl, TW, first, sc);
   }
 }
 
 // Transform `nlines` lines of a CTA's shared-memory tile.  Line L starts at
-// base + L*ld.  Every thread of the CTA must call this with the same plan.
-template <int SIGN, int PATH = kFftAny, typename C>
-__device__ __forceinline__ void fft_lines(C* base, int ld, int nlines, const C* __restrict__ tw, const FftPlan& pl) {
-  if (pl.n == 1) return;
-  if (PATH == kFft256 || (PATH == kFftAny && pl.tw16_off >= 0)) {
-    fft256_lines<SIGN>(base, ld, nlines, tw, pl, [&](int L) { return LineLoad<C>{base + L * ld}; });
-    return;
-  }
-  if (PATH == kFft256) return;
-  const int TW = team_of<C>(pl);
-  const int nteams = blockDim.x / TW;
-  const int team = threadIdx.x / TW;
-  const int tl = threadIdx.x - team * TW;
-  const int rounds = (nlines + nteams - 1) / nteams;
-  for (int r = 0; r < rounds; ++r) {
-    const int L = r * nteams + team;
-    const bool active = L < nlines;
-    if constexpr (ct_length(PATH)) {
-      C* line = base + (active ? L : 0) * ld;
-      fft_ct_stages<SIGN, PATH, 0>(line, tw, pl, active ? tl : (1 << 20), TW, LineLoad<C>{line});
-    } else {
-      fft_line<SIGN>(base + (active ? L : 0) * ld, tw, pl, tl, active);
-    }
-  }
-}
-
-// As fft_lines, with the first stage of line L reading through the loader
-// first(L) returns (a functor idx -> value).  A length-1 transform is the
-// identity: the inputs are only copied into place.
+// base + L*ld; its first stage reads through the loader first(L) returns (a
+// functor idx -> value).  Every thread of the CTA must call this with the
+// same plan.  A length-1 transform is the identity: the inputs are only
+// copied into place.
 template <int SIGN, int PATH = kFftAny, typename C, typename First>
-__device__ __forceinline__ void fft_lines_from(C* base, int ld, int nlines, const C* __restrict__ tw,
+__device__ __forceinline__ void fft_lines_from(C* base, int ld, int nlines,
+                                               const typename TwOf<C>::type* __restrict__ tw,
                                                const FftPlan& pl, First first) {
   if (pl.n == 1 || pl.nst == 0) {
     for (int L = threadIdx.x; L < nlines; L += blockDim.x) base[L * ld] = first(L)(0);
@@ -592,9 +718,17 @@ __device__ __forceinline__ void fft_lines_from(C* base, int ld, int nlines, cons
     if constexpr (ct_length(PATH)) {
       fft_ct_stages<SIGN, PATH, 0>(base + Lc * ld, tw, pl, active ? tl : (1 << 20), TW, first(Lc));
     } else {
-      fft_line_from<SIGN>(base + Lc * ld, tw, pl, tl, active, first(Lc));
+      fft_line_from<SIGN, PATH>(base + Lc * ld, tw, pl, tl, active, first(Lc));
     }
   }
+}
+
+// As fft_lines_from on lines already in place.
+template <int SIGN, int PATH = kFftAny, typename C>
+__device__ __forceinline__ void fft_lines(C* base, int ld, int nlines, const typename TwOf<C>::type* __restrict__ tw,
+                                          const FftPlan& pl) {
+  if (pl.n == 1) return;
+  fft_lines_from<SIGN, PATH>(base, ld, nlines, tw, pl, [&](int L) { return LineLoad<C>{base + L * ld}; });
 }
 
 // Copy a plan from global memory into shared memory (call before a barrier).

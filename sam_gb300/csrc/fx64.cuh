@@ -1,0 +1,318 @@
+// Fixed-point arithmetic of the FP64 line transforms.
+//
+// GB300 issues one FP64 instruction per 64 cycles and SM sub-partition, a
+// 64-bit integer sum in 2 and a 32 x 32 -> 64-bit multiply-add in about 5
+// (measured).  The transforms of the FP64 form therefore run in 64-bit fixed
+// point on the integer pipes: a line's doubles become integers under one
+// scale for the whole line, every butterfly sum is exact, every twiddle
+// product is rounded once at the line's last bit, and the results are
+// converted back to doubles.
+//
+// Scale: with L1 = sum (|re| + |im|) over the line, every partial sum and
+// every result of a discrete Fourier transform is at most L1 in modulus, so
+// the line is scaled to L1 < 2^62 and nothing can overflow.  A unit in the
+// last place is then at most 2^-61 L1 <= 2^-61 sqrt(2 n) |x|_2: about 2^-57
+// of the line's norm at n = 256, which leaves room for the roundings of the
+// twiddle products below the 2^-53 of FP64 arithmetic
+// (tests/test_gpu_fixed_point.py compares both with extended precision).
+//
+// Exceptional lines: a line holding an infinity or a NaN gives NaN
+// throughout; lines whose largest value is so small or so large that the
+// exponent arithmetic could leave the normal range take a slower exact path.
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace samgpu {
+
+__device__ __forceinline__ void team_sync(int TW);
+
+// complex fixed-point value (units of the line's last place)
+struct __align__(16) fxc {
+  long long x, y;
+};
+
+// twiddle in units of 2^-62, each part split as h * 2^32 + l with l signed
+struct __align__(16) fxw {
+  int xh, xl, yh, yl;
+};
+
+__device__ __forceinline__ fxc cadd(fxc a, fxc b) { return fxc{a.x + b.x, a.y + b.y}; }
+__device__ __forceinline__ fxc csub(fxc a, fxc b) { return fxc{a.x - b.x, a.y - b.y}; }
+
+// h * 2^32 + l = v with l signed
+struct FxSplit {
+  int h, l;
+};
+__device__ __forceinline__ FxSplit fx_split(long long v) {
+  return FxSplit{(int)((v + 0x80000000ll) >> 32), (int)v};
+}
+__host__ __device__ constexpr FxSplit fx_const(long long v) {
+  return FxSplit{(int)((v + 0x80000000ll) >> 32), (int)(uint32_t)(v & 0xffffffffll)};
+}
+__device__ __forceinline__ long long fx_mad(int a, int b, long long c) { return (long long)a * b + c; }
+
+// (A 2^32 + C) >> 30 for A the sum of the high products and C the cross terms
+__device__ __forceinline__ long long fx_join(long long A, uint32_t clo) {
+  const uint32_t lo = __funnelshift_l(clo, (uint32_t)A, 2);
+  const uint32_t hi = __funnelshift_l((uint32_t)A, (uint32_t)(A >> 32), 2);
+  return (long long)(((uint64_t)hi << 32) | lo);
+}
+// a * w, w in units of 2^-62, |w| <= 1: rounded to the nearest unit (the low
+// halves' product, below 2^-32 of a unit, is left out)
+__device__ __forceinline__ long long fx_mul(FxSplit a, FxSplit w) {
+  const long long c = fx_mad(a.l, w.h, fx_mad(a.h, w.l, 1ll << 29));
+  return fx_join(fx_mad(a.h, w.h, c >> 32), (uint32_t)c);
+}
+// a * u + b * v, rounded once.  |a|, |b| < 2^62 with a^2 + b^2 < 2^124 and
+// u^2 + v^2 <= 1 (or |a| + |b| < 2^62 and |u| + |v| < 1.6) keep the cross
+// terms below 2^63.
+__device__ __forceinline__ long long fx_dot(FxSplit a, FxSplit b, FxSplit u, FxSplit v) {
+  const long long c = fx_mad(b.l, v.h, fx_mad(b.h, v.l, fx_mad(a.l, u.h, fx_mad(a.h, u.l, 1ll << 29))));
+  return fx_join(fx_mad(b.h, v.h, fx_mad(a.h, u.h, c >> 32)), (uint32_t)c);
+}
+__device__ __forceinline__ FxSplit fx_neg(FxSplit w) { return FxSplit{-w.h, -w.l}; }
+
+// a * w (SIGN = -1) or a * conj(w) (SIGN = +1)
+template <int SIGN> __device__ __forceinline__ fxc ctw(fxc a, fxw w) {
+  const FxSplit x = fx_split(a.x), y = fx_split(a.y), u{w.xh, w.xl}, v{w.yh, w.yl}, nv = fx_neg(v);
+  if (SIGN < 0) return fxc{fx_dot(x, y, u, nv), fx_dot(x, y, v, u)};
+  return fxc{fx_dot(x, y, u, v), fx_dot(x, y, nv, u)};
+}
+// a * (cr + i ci) for constants
+__device__ __forceinline__ fxc fx_rot(fxc a, FxSplit cr, FxSplit ci) {
+  const FxSplit x = fx_split(a.x), y = fx_split(a.y);
+  return fxc{fx_dot(x, y, cr, fx_neg(ci)), fx_dot(x, y, ci, cr)};
+}
+template <int SIGN> __device__ __forceinline__ fxc cmul_si(fxc a) {
+  return SIGN < 0 ? fxc{a.y, -a.x} : fxc{-a.y, a.x};
+}
+// v / 2, ties to even
+__device__ __forceinline__ long long fx_half(long long v) { return (v + ((v >> 1) & 1)) >> 1; }
+__device__ __forceinline__ long long fx_quarter(long long v) { return (v + 1 + ((v >> 2) & 1)) >> 2; }
+
+// constants in units of 2^-62, rounded from extended precision
+constexpr long long kFxH = 3260954456333195553ll;    // sqrt(2)/2
+constexpr long long kFxC1 = 4260642322793532497ll;   // cos(pi/8)
+constexpr long long kFxS1 = 1764815834521887442ll;   // sin(pi/8)
+constexpr long long kFxS3 = 3993837246235628775ll;   // sin(2 pi/3)
+constexpr long long kFxR5 = 2578010857022246787ll;   // sqrt(5)/4
+constexpr long long kFxS51 = 4385974038932618941ll;  // sin(2 pi/5)
+constexpr long long kFxS52 = 2710681029835013083ll;  // sin(4 pi/5)
+
+template <int SIGN> __device__ __forceinline__ void dft8(fxc* a) {
+  const FxSplit h = fx_const(kFxH);
+  fxc b[8];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    b[q] = cadd(a[q], a[q + 4]);
+    b[q + 4] = csub(a[q], a[q + 4]);
+  }
+  b[6] = cmul_si<SIGN>(b[6]);
+  {
+    // h (1 + SIGN i) and h (-1 + SIGN i)
+    const long long p = b[5].x + b[5].y, m = b[5].x - b[5].y;
+    b[5] = SIGN < 0 ? fxc{fx_mul(fx_split(p), h), fx_mul(fx_split(-m), h)}
+                    : fxc{fx_mul(fx_split(m), h), fx_mul(fx_split(p), h)};
+    const long long p7 = b[7].x + b[7].y, m7 = b[7].x - b[7].y;
+    b[7] = SIGN < 0 ? fxc{fx_mul(fx_split(-m7), h), fx_mul(fx_split(-p7), h)}
+                    : fxc{fx_mul(fx_split(-p7), h), fx_mul(fx_split(m7), h)};
+  }
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const fxc t0 = cadd(b[4 * e], b[4 * e + 2]), t1 = csub(b[4 * e], b[4 * e + 2]);
+    const fxc t2 = cadd(b[4 * e + 1], b[4 * e + 3]), t3 = cmul_si<SIGN>(csub(b[4 * e + 1], b[4 * e + 3]));
+    a[e] = cadd(t0, t2);
+    a[4 + e] = csub(t0, t2);
+    a[2 + e] = cadd(t1, t3);
+    a[6 + e] = csub(t1, t3);
+  }
+}
+
+template <int SIGN> __device__ __forceinline__ void dft3(fxc* a) {
+  const FxSplit s = fx_const(SIGN * kFxS3);
+  const fxc t = cadd(a[1], a[2]), d = csub(a[1], a[2]);
+  const fxc m{a[0].x - fx_half(t.x), a[0].y - fx_half(t.y)};
+  const fxc r{-fx_mul(fx_split(d.y), s), fx_mul(fx_split(d.x), s)};
+  a[0] = cadd(a[0], t);
+  a[1] = cadd(m, r);
+  a[2] = csub(m, r);
+}
+
+// cos(2 pi/5), cos(4 pi/5) = -1/4 +- sqrt(5)/4
+template <int SIGN> __device__ __forceinline__ void dft5(fxc* a) {
+  const FxSplit r5 = fx_const(kFxR5), s1 = fx_const(SIGN * kFxS51), s2 = fx_const(SIGN * kFxS52);
+  const fxc t1 = cadd(a[1], a[4]), d1 = csub(a[1], a[4]);
+  const fxc t2 = cadd(a[2], a[3]), d2 = csub(a[2], a[3]);
+  const fxc t = cadd(t1, t2), dt = csub(t1, t2);
+  const fxc m{a[0].x - fx_quarter(t.x), a[0].y - fx_quarter(t.y)};
+  const fxc c{fx_mul(fx_split(dt.x), r5), fx_mul(fx_split(dt.y), r5)};
+  const fxc m1 = cadd(m, c), m2 = csub(m, c);
+  const FxSplit x1 = fx_split(d1.x), y1 = fx_split(d1.y), x2 = fx_split(d2.x), y2 = fx_split(d2.y);
+  const FxSplit ns1 = fx_neg(s1);
+  const fxc n1{-fx_dot(y1, y2, s1, s2), fx_dot(x1, x2, s1, s2)};
+  const fxc n2{-fx_dot(y1, y2, s2, ns1), fx_dot(x1, x2, s2, ns1)};
+  a[0] = cadd(a[0], t);
+  a[1] = cadd(m1, n1);
+  a[4] = csub(m1, n1);
+  a[2] = cadd(m2, n2);
+  a[3] = csub(m2, n2);
+}
+
+// dft16 of fft_engine.cuh (4 x 4) with the rotations by odd multiples of
+// pi/4 as a sum, a difference and two products
+template <int SIGN> __device__ __forceinline__ void fx_dft4(fxc& a, fxc& b, fxc& c, fxc& d) {
+  const fxc t0 = cadd(a, c), t1 = csub(a, c), t2 = cadd(b, d), t3 = cmul_si<SIGN>(csub(b, d));
+  a = cadd(t0, t2);
+  c = csub(t0, t2);
+  b = cadd(t1, t3);
+  d = csub(t1, t3);
+}
+template <int SIGN> __device__ __forceinline__ void dft16(fxc* a) {
+  const FxSplit h = fx_const(kFxH);
+#pragma unroll
+  for (int n2 = 0; n2 < 4; ++n2) fx_dft4<SIGN>(a[n2], a[4 + n2], a[8 + n2], a[12 + n2]);
+  // a[4 k1 + n2] *= w16^{n2 k1}
+  auto rot = [&](fxc& v, long long cr, long long ci) { v = fx_rot(v, fx_const(cr), fx_const(SIGN * ci)); };
+  auto rot45 = [&](fxc& v) {  // h (1 + SIGN i)
+    const long long p = v.x + v.y, m = v.x - v.y;
+    v = SIGN < 0 ? fxc{fx_mul(fx_split(p), h), fx_mul(fx_split(-m), h)}
+                 : fxc{fx_mul(fx_split(m), h), fx_mul(fx_split(p), h)};
+  };
+  auto rot135 = [&](fxc& v) {  // h (-1 + SIGN i)
+    const long long p = v.x + v.y, m = v.x - v.y;
+    v = SIGN < 0 ? fxc{fx_mul(fx_split(-m), h), fx_mul(fx_split(-p), h)}
+                 : fxc{fx_mul(fx_split(-p), h), fx_mul(fx_split(m), h)};
+  };
+  rot(a[4 + 1], kFxC1, kFxS1);
+  rot45(a[8 + 1]);
+  rot(a[12 + 1], kFxS1, kFxC1);
+  rot45(a[4 + 2]);
+  a[8 + 2] = cmul_si<SIGN>(a[8 + 2]);
+  rot135(a[12 + 2]);
+  rot(a[4 + 3], kFxS1, kFxC1);
+  rot135(a[8 + 3]);
+  rot(a[12 + 3], -kFxC1, -kFxS1);
+#pragma unroll
+  for (int k1 = 0; k1 < 4; ++k1) fx_dft4<SIGN>(a[4 * k1], a[4 * k1 + 1], a[4 * k1 + 2], a[4 * k1 + 3]);
+  // a[4 k1 + k2] holds output k1 + 4 k2
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = i + 1; j < 4; ++j) {
+      const fxc t = a[4 * i + j];
+      a[4 * i + j] = a[4 * j + i];
+      a[4 * j + i] = t;
+    }
+}
+
+// ---------------------------------------------------------------- conversions
+// The scale of a line: value = integer * 2^ex.
+struct FxScale {
+  int ex;
+  int kind;  // kFxPlain, or one of the exceptional lines
+};
+constexpr int kFxPlain = 0;  // every result's exponent stays in the normal range
+constexpr int kFxEdge = 1;   // it may not: results go through ldexp
+constexpr int kFxNaN = 2;    // the line holds an infinity or a NaN
+// lines whose largest value has a biased exponent below kFxTiny are lifted by
+// 2^kFxLift before the conversion (subnormals become normal numbers)
+constexpr int kFxTiny = 80, kFxLift = 256;
+
+// Reduction over the TW threads of a team (all threads of the CTA call it);
+// teams wider than a warp go through shared memory.
+template <typename V, typename Op> __device__ __forceinline__ V team_reduce(V v, int TW, Op op) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    if (o < TW) v = op(v, __shfl_xor_sync(0xffffffffu, v, o));
+  if (TW > 32) {
+    __shared__ V s_red[32];
+    const int w = threadIdx.x >> 5, nw = TW >> 5, w0 = w & ~(nw - 1);
+    if ((threadIdx.x & 31) == 0) s_red[w] = v;
+    team_sync(TW);
+    v = s_red[w0];
+    for (int i = 1; i < nw; ++i) v = op(v, s_red[w0 + i]);
+    team_sync(TW);
+  }
+  return v;
+}
+
+// largest |high word| of a thread's N values
+template <int N> __device__ __forceinline__ uint32_t fx_max_hi(const double2* v) {
+  uint32_t hm = 0;
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    hm = max(hm, max((uint32_t)__double2hiint(v[i].x) & 0x7fffffffu, (uint32_t)__double2hiint(v[i].y) & 0x7fffffffu));
+  return hm;
+}
+// sum of |v| / 2^(E - 1023) over a thread's N values from their leading 20
+// bits: the high word less the exponent E, shifted into an FP32 pattern
+template <int N> __device__ __forceinline__ float fx_l1(const double2* v, int E) {
+  const int base = (E - 127) * (1 << 20);
+  float s = 0.f, t = 0.f;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    s += __int_as_float(max((__double2hiint(v[i].x) & 0x7fffffff) - base, 0) << 3);
+    t += __int_as_float(max((__double2hiint(v[i].y) & 0x7fffffff) - base, 0) << 3);
+  }
+  return s + t;
+}
+// the double's mantissa as an integer with its leading bit at 62, shifted
+// down by dsh less its biased exponent (truncated: only values too small for
+// their last bits to reach the line's last place lose any)
+__device__ __forceinline__ long long fx_from(double d, int dsh) {
+  const uint32_t hi = (uint32_t)__double2hiint(d), lo = (uint32_t)__double2loint(d);
+  const int sh = dsh - (int)((hi >> 20) & 0x7ffu);
+  const uint32_t mh = (__funnelshift_l(lo, hi, 10) & 0x3fffffffu) | 0x40000000u, ml = lo << 10;
+  uint64_t m = ((uint64_t)mh << 32) | ml;
+  asm("shr.u64 %0, %0, %1;" : "+l"(m) : "r"(sh));  // (shifts past 63 give 0)
+  const long long s = (long long)((int)hi >> 31);
+  return ((long long)m ^ s) - s;
+}
+// The N values of each thread of a team to the line's fixed-point integers.
+template <int N> __device__ __forceinline__ FxScale fx_begin(double2* v, fxc* a, int TW) {
+  const auto umax = [](uint32_t x, uint32_t y) { return max(x, y); };
+  uint32_t hm = team_reduce(fx_max_hi<N>(v), TW, umax);
+  FxScale sc{0, kFxPlain};
+  int lift = 0;
+  if (hm < ((uint32_t)kFxTiny << 20) && hm > 0) {
+    lift = kFxLift;
+    const double f = __hiloint2double((1023 + kFxLift) << 20, 0);
+    hm = 0;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      v[i].x *= f;
+      v[i].y *= f;
+    }
+    hm = fx_max_hi<N>(v);
+  }
+  if (__any_sync(0xffffffffu, lift)) hm = team_reduce(hm, TW, umax);
+  const int E = (int)(hm >> 20);
+  const float l1 = team_reduce(fx_l1<N>(v, E), TW, [](float x, float y) { return x + y; });
+  // L1 < 2^(E - 1023 + g) with room for the sum's own rounding
+  int g = (__float_as_int(l1 * 1.0001f) >> 23) - 126;
+  if (E == 0) g = 128;  // a line of zeros
+  if (E == 0x7ff) sc.kind = kFxNaN;
+  else if (lift || E + g > 2040) sc.kind = kFxEdge;
+  sc.ex = E - 1023 - 62 + g - lift;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const double2 d = v[i];
+    a[i].x = fx_from(d.x, E + g);
+    a[i].y = fx_from(d.y, E + g);
+  }
+  return sc;
+}
+// integer * 2^ex, rounded to nearest (kFxPlain: the exponent added in place)
+__device__ __forceinline__ double fx_to(long long v, int ex) {
+  const double r = __ll2double_rn(v);
+  const int hi = __double2hiint(r);
+  return __hiloint2double(hi ? hi + ex * (1 << 20) : 0, __double2loint(r));
+}
+__device__ __forceinline__ double2 fx_out(fxc v, FxScale sc) {
+  if (sc.kind == kFxPlain) return make_double2(fx_to(v.x, sc.ex), fx_to(v.y, sc.ex));
+  if (sc.kind == kFxNaN) return make_double2(__hiloint2double(0x7ff80000, 0), __hiloint2double(0x7ff80000, 0));
+  return make_double2(ldexp(__ll2double_rn(v.x), sc.ex), ldexp(__ll2double_rn(v.y), sc.ex));
+}
+
+}  // namespace samgpu

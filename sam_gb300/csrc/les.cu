@@ -214,7 +214,7 @@ __global__ void k_dm_vt(const double* __restrict__ q, const double* __restrict__
 // ---- get_mean.f:8-56 (i_symm = 0) on the kx = ky = 0 column.  One CTA;
 // line 0 of the shared tile holds the synthesis, line 1 the linear profile.
 __global__ void k_get_mean(double2* __restrict__ col, int mz, int kz, int nz, int i_remove,
-                           const FftPlan* __restrict__ gpl, const double2* __restrict__ gtw,
+                           const FftPlan* __restrict__ gpl, const fxw* __restrict__ gtw,
                            double* __restrict__ u_mean, double* __restrict__ jump_out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ FftPlan pl;
@@ -222,8 +222,8 @@ __global__ void k_get_mean(double2* __restrict__ col, int mz, int kz, int nz, in
   load_plan(&pl, gpl);
   __syncthreads();
   const int ld = line_stride(nz);
-  double2* s_tw = reinterpret_cast<double2*>(smem_raw);
-  double2* ln = s_tw + pl.tw_total;
+  fxw* s_tw = reinterpret_cast<fxw*>(smem_raw);
+  double2* ln = reinterpret_cast<double2*>(s_tw + pl.tw_total);
   for (int e = threadIdx.x; e < pl.tw_total; e += blockDim.x) s_tw[e] = gtw[e];
   const double nz_inv = 1.0 / nz;
   for (int pass = 0; pass < 2; ++pass) {
@@ -422,7 +422,7 @@ template void les_box_filter<float>(const float*, int, int, int, int, int, doubl
 template void les_to_double<double>(const double*, double*, long long, cudaStream_t);
 template void les_to_double<float>(const float*, double*, long long, cudaStream_t);
 
-void les_get_mean(double2* col, int mz, int kz, int nz, int i_remove, const FftPlan* dplan, const double2* tw,
+void les_get_mean(double2* col, int mz, int kz, int nz, int i_remove, const FftPlan* dplan, const fxw* tw,
                   const FftPlan& hplan, double* u_mean, double* jump, cudaStream_t s) {
   const int ld = line_stride(nz);
   const size_t sm = sizeof(double2) * ((size_t)hplan.tw_total + (size_t)ld) + 16;

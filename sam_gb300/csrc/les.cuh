@@ -23,6 +23,6 @@ template <typename T>
 void les_box_filter(const T* ph, int lu, int nx, int ny, int nz, int f, double* out, cudaStream_t s);
 template <typename T>
 void les_to_double(const T* a, double* b, long long n, cudaStream_t s);
-void les_get_mean(double2* col, int mz, int kz, int nz, int i_remove, const FftPlan* dplan, const double2* tw,
+void les_get_mean(double2* col, int mz, int kz, int nz, int i_remove, const FftPlan* dplan, const fxw* tw,
                   const FftPlan& hplan, double* u_mean, double* jump, cudaStream_t s);
 }  // namespace samgpu

@@ -14,7 +14,7 @@ struct ZInvArgs {
   int sched;
   const cx_t<T>* in;   // rows of Nz_min modes
   cx_t<T>* out;        // A(n, z, kx, ky)
-  const cx_t<T>* tw;   // twiddles of the Nz plan
+  const tw_t<T>* tw;   // twiddles of the Nz plan
   int nvar, ty, ld;
   // derive = 1: fields n >= Lu of the launch are the subgrid gradient fields
   // m = n - Lu formed from the velocity (and T) rows while loading: S_ab for
@@ -32,7 +32,7 @@ struct YInvArgs {
   int sched;
   const cx_t<T>* in;  // rows (one per kx) of Ny_min modes or Ny values
   cx_t<T>* out;       // B(n, z, y, kx)
-  const cx_t<T>* tw;
+  const tw_t<T>* tw;
   int nvar, tx, ld, in_full;
   long long in_kx, in_z, in_n;
   long long out_y, out_z, out_n;
@@ -56,7 +56,7 @@ struct XPassArgs {
   cx_t<T>* out;        // out_mode 1/2: C(m, z, kx, y)
   T* out_phys;         // out_mode 0: P(n, z, y, x)
   double* partials;    // vel_max partials (nblocks, lu, 4) or null
-  const cx_t<T>* tw;
+  const tw_t<T>* tw;
   // group: product lines transformed per round of out_mode 2 (a multiple of
   // the CTA's teams where it exceeds them), any split of the Lr * Y/2 lines
   int in_mode, out_mode, nin, yt, group, ld;
@@ -95,7 +95,7 @@ struct YFwdArgs {
   int sched;
   const cx_t<T>* in;  // C(m, z, kx, y)
   cx_t<T>* out;       // D(m, kx, ky, z)
-  const cx_t<T>* tw;
+  const tw_t<T>* tw;
   int nvar, tz, ld;
   long long in_kx, in_z, in_n;
   long long out_ky, out_kx, out_n;
@@ -108,7 +108,7 @@ struct ZFwdArgs {
   // compile-time Stockham stages (radix 8, 8, 4); chosen by the autotuner
   int sched;
   cx_t<T>* in;  // D(m, kx, ky, z); mode 0 writes the result back here
-  const cx_t<T>* tw;
+  const tw_t<T>* tw;
   int mode, nf, ty, ld;
   long long in_ky, in_kx, in_n;
   // mode 1 (rhs): r out and u_sav in

@@ -29,7 +29,7 @@
 namespace samgpu {
 
 template <typename T>
-__device__ __forceinline__ void load_twiddles(cx_t<T>* s_tw, const cx_t<T>* __restrict__ g_tw, int n) {
+__device__ __forceinline__ void load_twiddles(tw_t<T>* s_tw, const tw_t<T>* __restrict__ g_tw, int n) {
   for (int i = threadIdx.x; i < n; i += blockDim.x) s_tw[i] = g_tw[i];
 }
 
@@ -53,7 +53,7 @@ template <typename T, int K, int PATH = kFft256> struct MinBlocks {
       PATH == kFftGeneric ? (K == kPassX ? 1 : 2) : (K == kPassZFwd ? 2 : (K == kPassX ? 3 : (PATH == kFft256 ? (K == kPassYInv ? 5 : 4) : 3)));
 };
 template <int K, int PATH> struct MinBlocks<double, K, PATH> {
-  static constexpr int value = PATH == kFftGeneric ? 1 : 2;
+  static constexpr int value = PATH == kFftGeneric || PATH == kFftLong ? 1 : 2;
 };
 // double-float pairs: the 16 x 16 register path holds 16 complex pairs (64
 // registers) per thread, as in FP64
@@ -173,8 +173,8 @@ __device__ __forceinline__ void z_inv_body(const ZInvArgs<T>& a, const FftPlan* 
   __shared__ FftPlan pl;
   load_plan(&pl, gpl);
   __syncthreads();
-  C* s_tw = reinterpret_cast<C*>(smem_raw);
-  C* s_ln = s_tw + tw_load<PATH>(pl);
+  tw_t<T>* s_tw = reinterpret_cast<tw_t<T>*>(smem_raw);
+  C* s_ln = reinterpret_cast<C*>(s_tw + tw_load<PATH>(pl));
   const int nz = a.g.nz, mz = a.g.mz, km = a.g.kz, my = a.g.my;
   const int ld = a.ld;
   const int nty = (my + a.ty - 1) / a.ty;
@@ -266,8 +266,8 @@ __device__ __forceinline__ void y_inv_body(const YInvArgs<T>& a, const FftPlan* 
   __shared__ FftPlan pl;
   load_plan(&pl, gpl);
   __syncthreads();
-  C* s_tw = reinterpret_cast<C*>(smem_raw);
-  C* s_ln = s_tw + tw_load<PATH>(pl);
+  tw_t<T>* s_tw = reinterpret_cast<tw_t<T>*>(smem_raw);
+  C* s_ln = reinterpret_cast<C*>(s_tw + tw_load<PATH>(pl));
   const int ny = a.g.ny, my = a.g.my, km = a.g.ky, mx = a.g.mx;
   const int ld = a.ld;
   const int ntx = (mx + a.tx - 1) / a.tx;
@@ -497,8 +497,8 @@ __device__ __forceinline__ void x_pass_body(const XPassArgs<T>& a, const FftPlan
   __shared__ FftPlan pl;
   load_plan(&pl, gpl);
   __syncthreads();
-  C* s_tw = reinterpret_cast<C*>(smem_raw);
-  C* s_in = s_tw + tw_load<PATH>(pl);                  // nin * yp lines
+  tw_t<T>* s_tw = reinterpret_cast<tw_t<T>*>(smem_raw);
+  C* s_in = reinterpret_cast<C*>(s_tw + tw_load<PATH>(pl));           // nin * yp lines
   const int nx = a.g.nx, ny = a.g.ny, kmx = a.g.kx, mx = a.g.mx;
   const int Y = a.yt, yp = Y / 2, ld = a.ld;
   const int nin = a.nin;
@@ -1193,8 +1193,8 @@ __device__ __forceinline__ void y_fwd_body(const YFwdArgs<T>& a, const FftPlan* 
   __shared__ FftPlan pl;
   load_plan(&pl, gpl);
   __syncthreads();
-  C* s_tw = reinterpret_cast<C*>(smem_raw);
-  C* s_ln = s_tw + tw_load<PATH>(pl);
+  tw_t<T>* s_tw = reinterpret_cast<tw_t<T>*>(smem_raw);
+  C* s_ln = reinterpret_cast<C*>(s_tw + tw_load<PATH>(pl));
   const int ny = a.g.ny, my = a.g.my, km = a.g.ky, nz = a.g.nz;
   const int ld = a.ld;
   const int ntz = (nz + a.tz - 1) / a.tz;
@@ -1386,8 +1386,8 @@ __device__ __forceinline__ void z_fwd_body(const ZFwdArgs<T>& a, const FftPlan* 
   __shared__ FftPlan pl;
   load_plan(&pl, gpl);
   __syncthreads();
-  C* s_tw = reinterpret_cast<C*>(smem_raw);
-  C* s_ln = s_tw + tw_load<PATH>(pl);
+  tw_t<T>* s_tw = reinterpret_cast<tw_t<T>*>(smem_raw);
+  C* s_ln = reinterpret_cast<C*>(s_tw + tw_load<PATH>(pl));
   const Grid& g = a.g;
   const int nz = g.nz, mz = g.mz, km = g.kz, my = g.my;
   const int ld = a.ld, nf = a.nf;
@@ -1634,41 +1634,48 @@ __device__ __forceinline__ void vel_max_finish_body(const double* __restrict__ p
 }
 
 // ------------------------------------------------------------------ launchers
+// Calls f with the code path (an integral constant) that lines of length n
+// take in precision T; sched = 1 is the Stockham schedule of length 256.
+template <typename T, typename F> void with_path(int n, int sched, F f) {
+  using std::integral_constant;
+  switch (n) {
+    case 256:
+      if (sched == 1) f(integral_constant<int, 256>());
+      else f(integral_constant<int, kFft256>());
+      return;
+    case 32: f(integral_constant<int, 32>()); return;
+    case 64: f(integral_constant<int, 64>()); return;
+    case 96: f(integral_constant<int, 96>()); return;
+    case 128: f(integral_constant<int, 128>()); return;
+    case 512: f(integral_constant<int, 512>()); return;
+  }
+  if constexpr (std::is_same<T, double>::value) {
+    if (n > kFxMaxLine) {
+      f(integral_constant<int, kFftLong>());
+      return;
+    }
+  }
+  f(integral_constant<int, kFftGeneric>());
+}
+// Calls f with every code path of precision T.
+template <typename T, typename F> void each_path(F f) {
+  for (int n : {32, 64, 96, 128, 256, 512, 17, kFxMaxLine + 1}) with_path<T>(n, 0, f);
+  with_path<T>(256, 1, f);
+}
+
 template <typename T>
 void launch_z_inv(const ZInvArgs<T>& a0, const FftPlan* pl, size_t smem, cudaStream_t s) {
-  ZInvArgs<T> a = a0;
-  const int nty = (a.g.my + a.ty - 1) / a.ty;
-  const int grid = a.nvar * a.g.mx * nty;
-  switch (a.g.nz) {
-    case 256:
-      if (a.sched) k_z_inv<T, 256><<<grid, kThreads, smem, s>>>(a, pl);
-      else k_z_inv<T, kFft256><<<grid, kThreads, smem, s>>>(a, pl);
-      break;
-    case 32: k_z_inv<T, 32><<<grid, kThreads, smem, s>>>(a, pl); break;
-    case 64: k_z_inv<T, 64><<<grid, kThreads, smem, s>>>(a, pl); break;
-    case 128: k_z_inv<T, 128><<<grid, kThreads, smem, s>>>(a, pl); break;
-    case 512: k_z_inv<T, 512><<<grid, kThreads, smem, s>>>(a, pl); break;
-    case 96: k_z_inv<T, 96><<<grid, kThreads, smem, s>>>(a, pl); break;
-    default: k_z_inv<T, kFftGeneric><<<grid, kThreads, smem, s>>>(a, pl);
-  }
+  const ZInvArgs<T> a = a0;
+  const int grid = a.nvar * a.g.mx * ((a.g.my + a.ty - 1) / a.ty);
+  with_path<T>(a.g.nz, a.sched,
+               [&](auto p) { k_z_inv<T, decltype(p)::value><<<grid, kThreads, smem, s>>>(a, pl); });
 }
 template <typename T>
 void launch_y_inv(const YInvArgs<T>& a0, const FftPlan* pl, size_t smem, cudaStream_t s) {
-  YInvArgs<T> a = a0;
-  const int ntx = (a.g.mx + a.tx - 1) / a.tx;
-  const int grid = a.nvar * a.g.nz * ntx;
-  switch (a.g.ny) {
-    case 256:
-      if (a.sched) k_y_inv<T, 256><<<grid, kThreads, smem, s>>>(a, pl);
-      else k_y_inv<T, kFft256><<<grid, kThreads, smem, s>>>(a, pl);
-      break;
-    case 32: k_y_inv<T, 32><<<grid, kThreads, smem, s>>>(a, pl); break;
-    case 64: k_y_inv<T, 64><<<grid, kThreads, smem, s>>>(a, pl); break;
-    case 128: k_y_inv<T, 128><<<grid, kThreads, smem, s>>>(a, pl); break;
-    case 512: k_y_inv<T, 512><<<grid, kThreads, smem, s>>>(a, pl); break;
-    case 96: k_y_inv<T, 96><<<grid, kThreads, smem, s>>>(a, pl); break;
-    default: k_y_inv<T, kFftGeneric><<<grid, kThreads, smem, s>>>(a, pl);
-  }
+  const YInvArgs<T> a = a0;
+  const int grid = a.nvar * a.g.nz * ((a.g.mx + a.tx - 1) / a.tx);
+  with_path<T>(a.g.ny, a.sched,
+               [&](auto p) { k_y_inv<T, decltype(p)::value><<<grid, kThreads, smem, s>>>(a, pl); });
 }
 template <typename T>
 int x_pass_blocks(const XPassArgs<T>& a) {
@@ -1699,64 +1706,31 @@ ZFwdArgs<T> prep_z_fwd(const ZFwdArgs<T>& a0) {
 template <typename T>
 void launch_x_pass(const XPassArgs<T>& a0, const FftPlan* pl, size_t smem, cudaStream_t s) {
   const XPassArgs<T> a = prep_x_pass(a0);
-  switch (a.g.nx) {
-    case 256:
-      if (a.sched == 1) {
-        k_x_pass<T, 256><<<x_pass_blocks(a), x_threads(sizeof(T), false), smem, s>>>(a, pl);
-        break;
-      }
-      if constexpr (std::is_same<T, float>::value) {
-        const size_t fsm = x_f256_smem(a.nin * (a.yt / 2));
-        if (x_f256_applies(a) && fsm <= (size_t)smem_optin()) {
-          k_x_pass_f256<><<<x_pass_blocks(a), kXf256Threads, fsm, s>>>(a);
-          break;
-        }
-      }
-      k_x_pass<T, kFft256><<<x_pass_blocks(a), x_threads(sizeof(T), true), smem, s>>>(a, pl);
-      break;
-    case 32: k_x_pass<T, 32><<<x_pass_blocks(a), kThreads, smem, s>>>(a, pl); break;
-    case 64: k_x_pass<T, 64><<<x_pass_blocks(a), kThreads, smem, s>>>(a, pl); break;
-    case 128: k_x_pass<T, 128><<<x_pass_blocks(a), kThreads, smem, s>>>(a, pl); break;
-    case 512: k_x_pass<T, 512><<<x_pass_blocks(a), kThreads, smem, s>>>(a, pl); break;
-    case 96: k_x_pass<T, 96><<<x_pass_blocks(a), kThreads, smem, s>>>(a, pl); break;
-    default: k_x_pass<T, kFftGeneric><<<x_pass_blocks(a), kThreads, smem, s>>>(a, pl);
+  if constexpr (std::is_same<T, float>::value) {
+    const size_t fsm = x_f256_smem(a.nin * (a.yt / 2));
+    if (x_f256_applies(a) && fsm <= (size_t)smem_optin()) {
+      k_x_pass_f256<><<<x_pass_blocks(a), kXf256Threads, fsm, s>>>(a);
+      return;
+    }
   }
+  with_path<T>(a.g.nx, a.sched, [&](auto p) {
+    constexpr int PATH = decltype(p)::value;
+    k_x_pass<T, PATH><<<x_pass_blocks(a), x_threads(sizeof(T), PATH == kFft256), smem, s>>>(a, pl);
+  });
 }
 template <typename T>
 void launch_y_fwd(const YFwdArgs<T>& a0, const FftPlan* pl, size_t smem, cudaStream_t s) {
-  YFwdArgs<T> a = a0;
-  const int ntz = (a.g.nz + a.tz - 1) / a.tz;
-  const int grid = a.nvar * a.g.mx * ntz;
-  switch (a.g.ny) {
-    case 256:
-      if (a.sched) k_y_fwd<T, 256><<<grid, kThreads, smem, s>>>(a, pl);
-      else k_y_fwd<T, kFft256><<<grid, kThreads, smem, s>>>(a, pl);
-      break;
-    case 32: k_y_fwd<T, 32><<<grid, kThreads, smem, s>>>(a, pl); break;
-    case 64: k_y_fwd<T, 64><<<grid, kThreads, smem, s>>>(a, pl); break;
-    case 128: k_y_fwd<T, 128><<<grid, kThreads, smem, s>>>(a, pl); break;
-    case 512: k_y_fwd<T, 512><<<grid, kThreads, smem, s>>>(a, pl); break;
-    case 96: k_y_fwd<T, 96><<<grid, kThreads, smem, s>>>(a, pl); break;
-    default: k_y_fwd<T, kFftGeneric><<<grid, kThreads, smem, s>>>(a, pl);
-  }
+  const YFwdArgs<T> a = a0;
+  const int grid = a.nvar * a.g.mx * ((a.g.nz + a.tz - 1) / a.tz);
+  with_path<T>(a.g.ny, a.sched,
+               [&](auto p) { k_y_fwd<T, decltype(p)::value><<<grid, kThreads, smem, s>>>(a, pl); });
 }
 template <typename T>
 void launch_z_fwd(const ZFwdArgs<T>& a0, const FftPlan* pl, size_t smem, cudaStream_t s) {
   const ZFwdArgs<T> a = prep_z_fwd(a0);
-  const int nty = (a.g.my + a.ty - 1) / a.ty;
-  const int grid = a.g.mx * nty;
-  switch (a.g.nz) {
-    case 256:
-      if (a.sched) k_z_fwd<T, 256><<<grid, kThreads, smem, s>>>(a, pl);
-      else k_z_fwd<T, kFft256><<<grid, kThreads, smem, s>>>(a, pl);
-      break;
-    case 32: k_z_fwd<T, 32><<<grid, kThreads, smem, s>>>(a, pl); break;
-    case 64: k_z_fwd<T, 64><<<grid, kThreads, smem, s>>>(a, pl); break;
-    case 128: k_z_fwd<T, 128><<<grid, kThreads, smem, s>>>(a, pl); break;
-    case 512: k_z_fwd<T, 512><<<grid, kThreads, smem, s>>>(a, pl); break;
-    case 96: k_z_fwd<T, 96><<<grid, kThreads, smem, s>>>(a, pl); break;
-    default: k_z_fwd<T, kFftGeneric><<<grid, kThreads, smem, s>>>(a, pl);
-  }
+  const int grid = a.g.mx * ((a.g.my + a.ty - 1) / a.ty);
+  with_path<T>(a.g.nz, a.sched,
+               [&](auto p) { k_z_fwd<T, decltype(p)::value><<<grid, kThreads, smem, s>>>(a, pl); });
 }
 static inline void allow_dynamic_smem(const void* fn, int optin) {
   cudaFuncAttributes at;
@@ -1769,59 +1743,24 @@ static inline void allow_dynamic_smem(const void* fn, int optin) {
 // group of passes (each group is instantiated in its own translation unit).
 template <typename T>
 void smem_limits_zinv(int optin) {
-  allow_dynamic_smem((const void*)k_z_inv<T, kFft256>, optin);
-  allow_dynamic_smem((const void*)k_z_inv<T, kFftGeneric>, optin);
-  allow_dynamic_smem((const void*)k_z_inv<T, 32>, optin);
-  allow_dynamic_smem((const void*)k_z_inv<T, 64>, optin);
-  allow_dynamic_smem((const void*)k_z_inv<T, 128>, optin);
-  allow_dynamic_smem((const void*)k_z_inv<T, 512>, optin);
-  allow_dynamic_smem((const void*)k_z_inv<T, 96>, optin);
-  allow_dynamic_smem((const void*)k_z_inv<T, 256>, optin);
+  each_path<T>([&](auto p) { allow_dynamic_smem((const void*)k_z_inv<T, decltype(p)::value>, optin); });
 }
 template <typename T>
 void smem_limits_yinv(int optin) {
-  allow_dynamic_smem((const void*)k_y_inv<T, kFft256>, optin);
-  allow_dynamic_smem((const void*)k_y_inv<T, kFftGeneric>, optin);
-  allow_dynamic_smem((const void*)k_y_inv<T, 32>, optin);
-  allow_dynamic_smem((const void*)k_y_inv<T, 64>, optin);
-  allow_dynamic_smem((const void*)k_y_inv<T, 128>, optin);
-  allow_dynamic_smem((const void*)k_y_inv<T, 512>, optin);
-  allow_dynamic_smem((const void*)k_y_inv<T, 96>, optin);
-  allow_dynamic_smem((const void*)k_y_inv<T, 256>, optin);
+  each_path<T>([&](auto p) { allow_dynamic_smem((const void*)k_y_inv<T, decltype(p)::value>, optin); });
 }
 template <typename T>
 void smem_limits_x(int optin) {
   if constexpr (std::is_same<T, float>::value) allow_dynamic_smem((const void*)k_x_pass_f256<>, optin);
-  allow_dynamic_smem((const void*)k_x_pass<T, kFft256>, optin);
-  allow_dynamic_smem((const void*)k_x_pass<T, kFftGeneric>, optin);
-  allow_dynamic_smem((const void*)k_x_pass<T, 32>, optin);
-  allow_dynamic_smem((const void*)k_x_pass<T, 64>, optin);
-  allow_dynamic_smem((const void*)k_x_pass<T, 128>, optin);
-  allow_dynamic_smem((const void*)k_x_pass<T, 512>, optin);
-  allow_dynamic_smem((const void*)k_x_pass<T, 96>, optin);
-  allow_dynamic_smem((const void*)k_x_pass<T, 256>, optin);
+  each_path<T>([&](auto p) { allow_dynamic_smem((const void*)k_x_pass<T, decltype(p)::value>, optin); });
 }
 template <typename T>
 void smem_limits_yfwd(int optin) {
-  allow_dynamic_smem((const void*)k_y_fwd<T, kFft256>, optin);
-  allow_dynamic_smem((const void*)k_y_fwd<T, kFftGeneric>, optin);
-  allow_dynamic_smem((const void*)k_y_fwd<T, 32>, optin);
-  allow_dynamic_smem((const void*)k_y_fwd<T, 64>, optin);
-  allow_dynamic_smem((const void*)k_y_fwd<T, 128>, optin);
-  allow_dynamic_smem((const void*)k_y_fwd<T, 512>, optin);
-  allow_dynamic_smem((const void*)k_y_fwd<T, 96>, optin);
-  allow_dynamic_smem((const void*)k_y_fwd<T, 256>, optin);
+  each_path<T>([&](auto p) { allow_dynamic_smem((const void*)k_y_fwd<T, decltype(p)::value>, optin); });
 }
 template <typename T>
 void smem_limits_zfwd(int optin) {
-  allow_dynamic_smem((const void*)k_z_fwd<T, kFft256>, optin);
-  allow_dynamic_smem((const void*)k_z_fwd<T, kFftGeneric>, optin);
-  allow_dynamic_smem((const void*)k_z_fwd<T, 32>, optin);
-  allow_dynamic_smem((const void*)k_z_fwd<T, 64>, optin);
-  allow_dynamic_smem((const void*)k_z_fwd<T, 128>, optin);
-  allow_dynamic_smem((const void*)k_z_fwd<T, 512>, optin);
-  allow_dynamic_smem((const void*)k_z_fwd<T, 96>, optin);
-  allow_dynamic_smem((const void*)k_z_fwd<T, 256>, optin);
+  each_path<T>([&](auto p) { allow_dynamic_smem((const void*)k_z_fwd<T, decltype(p)::value>, optin); });
 }
 
 #define SAMGPU_INST_ZINV(T)                                                                   \

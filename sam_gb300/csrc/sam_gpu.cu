@@ -49,7 +49,7 @@ int set_error(int code, const char* msg) { return fail(code, "%s", msg); }
 struct Plan {
   FftPlan h{};
   FftPlan* d = nullptr;
-  double2* tw64 = nullptr;
+  fxw* tw64 = nullptr;
   float2* tw32 = nullptr;
   ddc* twdd = nullptr;
 };
@@ -58,6 +58,29 @@ struct Plan {
 static dd dd_of(long double v) {
   const float h = (float)v;
   return dd(h, (float)(v - (long double)h));
+}
+
+// exp(-i a) = (c, sn) as the FP64 form's fixed-point twiddle, in units of
+// 2^-62; a low half of exactly -2^31 (whose negation does not fit) is moved
+// by one unit
+static fxw fxw_of(int n, long double c, long double sn) {
+  if (n > kFxMaxLine) {
+    // the table of a length whose lines run in FP64 arithmetic
+    const double2 d = make_double2((double)c, (double)sn);
+    fxw w;
+    memcpy(&w, &d, sizeof(w));
+    return w;
+  }
+  auto part = [](long double v, int& h, int& l) {
+    long long q = llroundl(v * 4611686018427387904.0L);
+    if ((uint32_t)q == 0x80000000u) ++q;
+    h = (int)((q + 0x80000000ll) >> 32);
+    l = (int)(uint32_t)q;
+  };
+  fxw w;
+  part(c, w.xh, w.xl);
+  part(sn, w.yh, w.yl);
+  return w;
 }
 
 // Radices 8, 4, 2, 3, 5 in that order; twiddles w_{l p}^{f q} = exp(-2 pi i
@@ -92,7 +115,7 @@ static int build_plan(int n, Plan& P) {
   pl.team = team_for(8);
   pl.team_sp = team_for(8);
   if (pl.team > kThreads) return fail(SAM_GPU_EINVAL, "FFT length %d needs too wide a team", n);
-  std::vector<double2> t64;
+  std::vector<fxw> t64;
   std::vector<float2> t32;
   std::vector<ddc> tdd;
   int l = 1, off = 0;
@@ -107,7 +130,7 @@ static int build_plan(int n, Plan& P) {
       for (int f = 0; f < 16; ++f) {
         const long double a = two_pi * (long double)((f * q) % 256) / 256.0L;
         const long double c = cosl(a), sn = -sinl(a);
-        t64.push_back(make_double2((double)c, (double)sn));
+        t64.push_back(fxw_of(n, c, sn));
         t32.push_back(make_float2((float)c, (float)sn));
         tdd.push_back(ddc{dd_of(c), dd_of(sn)});
       }
@@ -126,7 +149,7 @@ static int build_plan(int n, Plan& P) {
         const long e = ((long)f * q) % ((long)l * p);
         const long double a = two_pi * (long double)e / (long double)(l * p);
         const long double c = cosl(a), sn = -sinl(a);
-        t64.push_back(make_double2((double)c, (double)sn));
+        t64.push_back(fxw_of(n, c, sn));
         t32.push_back(make_float2((float)c, (float)sn));
         tdd.push_back(ddc{dd_of(c), dd_of(sn)});
       }
@@ -136,14 +159,14 @@ static int build_plan(int n, Plan& P) {
   pl.tw_total = off;
   pl.tw_pass = n == 256 ? 256 : off;
   if (t64.empty()) {
-    t64.push_back(make_double2(1, 0));
+    t64.push_back(fxw_of(n, 1, 0));
     t32.push_back(make_float2(1, 0));
     tdd.push_back(ddc{dd(1), dd(0)});
   }
   CK(cudaMalloc(&P.d, sizeof(FftPlan)));
   CK(cudaMemcpy(P.d, &pl, sizeof(FftPlan), cudaMemcpyHostToDevice));
-  CK(cudaMalloc(&P.tw64, sizeof(double2) * t64.size()));
-  CK(cudaMemcpy(P.tw64, t64.data(), sizeof(double2) * t64.size(), cudaMemcpyHostToDevice));
+  CK(cudaMalloc(&P.tw64, sizeof(fxw) * t64.size()));
+  CK(cudaMemcpy(P.tw64, t64.data(), sizeof(fxw) * t64.size(), cudaMemcpyHostToDevice));
   CK(cudaMalloc(&P.tw32, sizeof(float2) * t32.size()));
   CK(cudaMemcpy(P.tw32, t32.data(), sizeof(float2) * t32.size(), cudaMemcpyHostToDevice));
   CK(cudaMalloc(&P.twdd, sizeof(ddc) * tdd.size()));
@@ -156,8 +179,8 @@ static void free_plan(Plan& P) {
   P.d = nullptr; P.tw64 = nullptr; P.tw32 = nullptr; P.twdd = nullptr;
 }
 
-template <typename T> const cx_t<T>* tw_of(const Plan& P);
-template <> const double2* tw_of<double>(const Plan& P) { return P.tw64; }
+template <typename T> const tw_t<T>* tw_of(const Plan& P);
+template <> const fxw* tw_of<double>(const Plan& P) { return P.tw64; }
 template <> const float2* tw_of<float>(const Plan& P) { return P.tw32; }
 template <> const ddc* tw_of<dd>(const Plan& P) { return P.twdd; }
 

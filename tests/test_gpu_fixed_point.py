@@ -1,0 +1,123 @@
+"""Accuracy and exceptional lines of the FP64 form's line transforms, which run
+in 64-bit fixed point (sam_gb300/csrc/fx64.cuh), against extended precision.
+
+Bar: the relative error of a line in the 2-norm, rms over the lines, within
+0.8 sqrt(log2 n) 2^-53 (and at least 2^-53): the error model of an FP64
+radix-2 transform, whose log2 n levels each round every value once by 0.4 to
+0.8 units of 2^-53 in the rms."""
+import numpy as np
+import pytest
+
+from sam_gb300 import SamGpu
+
+pytestmark = pytest.mark.gpu
+
+LENGTHS = [2, 3, 4, 5, 6, 8, 9, 15, 16, 25, 30, 32, 45, 48, 64, 81, 96, 125, 128, 135, 162, 200, 243, 256, 320, 500, 512,
+           540, 1024]
+
+
+def lines(kind, n, m, rng):
+    z = rng.standard_normal((n, m)) + 1j * rng.standard_normal((n, m))
+    k = np.minimum(np.arange(n), n - np.arange(n))[:, None]
+    if kind == "steep":
+        return z * (1.0 + k) ** (-5 / 3)
+    if kind == "smooth":
+        return z * np.exp(-0.3 * k)
+    if kind == "single":
+        return z * (k == (1 if n >= 4 else 0))
+    if kind == "range":
+        return z * 10.0 ** rng.uniform(-30, 0, (n, m))
+    return z
+
+
+def solver(n):
+    return SamGpu(nx=4, ny=16, nz=n, n_dealias=0)
+
+
+def stored(g, full):
+    """The stored z modes 0 .. k, -k .. -1 of full lines (n, m) as u(Nze, Ny_min, Nx_min, 1)."""
+    n, km = g.nz, (g.nz_min - 1) // 2
+    u = np.zeros((n, g.ny_min, g.nx_min, 1), dtype=np.complex128, order="F")
+    keep = np.concatenate([full[:km + 1], full[n - km:]], 0) if km else full[:1]
+    u[:g.nz_min, :, :, 0] = keep.reshape(g.nz_min, g.ny_min, g.nx_min)
+    return u
+
+
+def padded(g, u):
+    n, km = g.nz, (g.nz_min - 1) // 2
+    x = np.zeros((n,) + u.shape[1:3], dtype=np.clongdouble)
+    x[:km + 1] = u[:km + 1, :, :, 0]
+    if km:
+        x[n - km:] = u[km + 1:2 * km + 1, :, :, 0]
+    return x
+
+
+def inverse(g, u):
+    return np.moveaxis(g.z_trans_b(u, 1)[..., 0], 2, 0)
+
+
+def line_errors(got, ref):
+    scale = np.sqrt((np.abs(ref) ** 2).sum(0))
+    return np.sqrt((np.abs(got - ref) ** 2).sum(0))[scale > 0] / scale[scale > 0]
+
+
+def bar(n):
+    return 2.0 ** -53 * max(1.0, 0.8 * np.sqrt(np.log2(n)))
+
+
+@pytest.mark.parametrize("n", LENGTHS)
+def test_transforms_against_extended_precision(gpu_lib, n):
+    g = solver(n)
+    rng = np.random.default_rng(n)
+    m = g.ny_min * g.nx_min
+    for kind in ("white", "steep", "smooth", "single", "range"):
+        u = stored(g, lines(kind, n, m, rng))
+        ref = np.fft.ifft(padded(g, u), axis=0, norm="forward")
+        err = line_errors(inverse(g, u), ref)
+        assert np.sqrt((err ** 2).mean()) < bar(n), (kind, "inverse")
+        f = np.zeros((n, g.ny_min, g.nx_min, 1), dtype=np.complex128, order="F")
+        f[..., 0] = lines(kind, n, m, rng).reshape(n, g.ny_min, g.nx_min)
+        full = np.fft.fft(f[..., 0].astype(np.clongdouble), axis=0, norm="forward")
+        km = (g.nz_min - 1) // 2
+        ref = np.concatenate([full[:km + 1], full[n - km:]], 0) if km else full[:1]
+        norm = np.sqrt((np.abs(full) ** 2).sum(0))
+        got = g.z_trans_f(f.copy(order="F"), 1)[:g.nz_min, ..., 0]
+        err = np.sqrt((np.abs(got - ref) ** 2).sum(0)) / norm
+        assert np.sqrt((err ** 2).mean()) < bar(n), (kind, "forward")
+    g.close()
+
+
+@pytest.mark.parametrize("n", [30, 64, 243, 256, 512])
+def test_scaling_by_powers_of_two_is_exact(gpu_lib, n):
+    """One scale per line: a line times 2^k gives the same integers, so the
+    results are the same times 2^k, down to and including lines of subnormals
+    and up to the largest numbers."""
+    g = solver(n)
+    u = stored(g, lines("smooth", n, g.ny_min * g.nx_min, np.random.default_rng(1)))
+    ref = inverse(g, u)
+    for k in (-900, -500, -1, 3, 500, 900, 1005):
+        assert np.array_equal(inverse(g, u * 2.0 ** k), ref * 2.0 ** k), k
+    tiny = inverse(g, u * 2.0 ** -1030)
+    assert np.abs(tiny - ref * 2.0 ** -1030).max() <= n * 2.0 ** -1074  # inputs and results rounded to subnormals
+    # results beyond the largest number are infinities, as in FP64
+    assert not np.isfinite(inverse(g, np.where(u != 0, 1.0, 0.0) * 1.7e308)).all()
+    g.close()
+
+
+@pytest.mark.parametrize("n", [30, 64, 256, 512])
+def test_exceptional_lines(gpu_lib, n):
+    """Zeros stay zeros; an infinity or a NaN spoils its own line and no other."""
+    g = solver(n)
+    u = stored(g, lines("white", n, g.ny_min * g.nx_min, np.random.default_rng(2)))
+    u[:, 1, 0, 0] = 0.0
+    ref = inverse(g, u)
+    assert not ref[:, 1, 0].any()
+    for bad in (np.inf, -np.inf, np.nan):
+        v = u.copy(order="F")
+        v[2, 0, 0, 0] = complex(1.0, bad)
+        got = inverse(g, v)
+        line = got[:, 0, 0]
+        assert not (np.isfinite(line.real) | np.isfinite(line.imag)).any()
+        got[:, 0, 0] = ref[:, 0, 0]
+        assert np.array_equal(got, ref)
+    g.close()
