@@ -184,6 +184,7 @@ template <int SIGN, typename C> __device__ __forceinline__ C cmul_si(C a) {
 // 512, 0.55 against 1.6 at 256).
 constexpr int kFftAny = 0, kFft256 = 1, kFftGeneric = 2, kFftLong = 3;
 constexpr int kFxMaxLine = 512;
+template <typename C, int PATH> inline constexpr bool kIsFx = std::is_same<C, double2>::value && PATH != kFftLong;
 
 struct FftStage {
   int p;       // radix
@@ -436,13 +437,39 @@ __device__ __forceinline__ void fft_stage(C* line, const C* __restrict__ tw, con
   team_sync(TW);
 }
 
+// What becomes of the results of a fixed-point line: element idx, an integer
+// of scale sc.  FxOutLine: doubles back into the line.
+struct FxOutLine {
+  double2* line;
+  __device__ __forceinline__ void operator()(int idx, fxc v, FxScale sc) const { line[sidx(idx)] = fx_out(v, sc); }
+};
+// Doubles into the line, the band lo < idx < hi (which the caller does not
+// read) left out.
+struct FxOutBand {
+  double2* line;
+  int lo, hi;
+  __device__ __forceinline__ void operator()(int idx, fxc v, FxScale sc) const {
+    if (idx <= lo || idx >= hi) line[sidx(idx)] = fx_out(v, sc);
+  }
+};
+// The integers into the line and their scale into *scale: the caller converts
+// what it reads.
+struct FxOutInt {
+  fxc* line;
+  FxScale* scale;
+  __device__ __forceinline__ void operator()(int idx, fxc v, FxScale sc) const {
+    line[sidx(idx)] = v;
+    if (idx == 0) *scale = sc;
+  }
+};
+
 // The same stage of an FP64 line in fixed point (fx64.cuh).  The first stage
 // (FIRST, l = 1: no twiddles) reads doubles through load and fixes the line's
 // scale, which it leaves in sc; the others read the line's integers.  The
-// last stage writes doubles, the others integers.
-template <int P, int SIGN, bool FIRST, typename Ld>
+// last stage hands its results to out, the others write integers.
+template <int P, int SIGN, bool FIRST, typename Ld, typename Out>
 __device__ __forceinline__ void fx_stage(double2* line, const fxw* __restrict__ tw, const FftStage& s, int n, int tl,
-                                         int TW, Ld load, FxScale& sc, bool last) {
+                                         int TW, Ld load, Out out, FxScale& sc, bool last) {
   constexpr int MAXB = Emax<double2>::value / P;
   const int nb = n / P;
   fxc a[MAXB][P];
@@ -487,7 +514,7 @@ __device__ __forceinline__ void fx_stage(double2* line, const fxw* __restrict__ 
       dftp<P, SIGN>(a[i]);
       if (last) {
 #pragma unroll
-        for (int q = 0; q < P; ++q) line[sidx(ds[i] + q * os)] = fx_out(a[i][q], sc);
+        for (int q = 0; q < P; ++q) out(ds[i] + q * os, a[i][q], sc);
       } else {
         fxc* fl = reinterpret_cast<fxc*>(line);
 #pragma unroll
@@ -497,15 +524,15 @@ __device__ __forceinline__ void fx_stage(double2* line, const fxw* __restrict__ 
   }
   team_sync(TW);
 }
-template <int SIGN, bool FIRST, typename Ld>
+template <int SIGN, bool FIRST, typename Ld, typename Out>
 __device__ __forceinline__ void fx_stage_p(double2* line, const fxw* __restrict__ tw, const FftStage& st, int n, int tl,
-                                           int TW, Ld load, FxScale& sc, bool last) {
+                                           int TW, Ld load, Out out, FxScale& sc, bool last) {
   switch (st.p) {
-    case 8: fx_stage<8, SIGN, FIRST>(line, tw, st, n, tl, TW, load, sc, last); break;
-    case 4: fx_stage<4, SIGN, FIRST>(line, tw, st, n, tl, TW, load, sc, last); break;
-    case 2: fx_stage<2, SIGN, FIRST>(line, tw, st, n, tl, TW, load, sc, last); break;
-    case 3: fx_stage<3, SIGN, FIRST>(line, tw, st, n, tl, TW, load, sc, last); break;
-    default: fx_stage<5, SIGN, FIRST>(line, tw, st, n, tl, TW, load, sc, last); break;
+    case 8: fx_stage<8, SIGN, FIRST>(line, tw, st, n, tl, TW, load, out, sc, last); break;
+    case 4: fx_stage<4, SIGN, FIRST>(line, tw, st, n, tl, TW, load, out, sc, last); break;
+    case 2: fx_stage<2, SIGN, FIRST>(line, tw, st, n, tl, TW, load, out, sc, last); break;
+    case 3: fx_stage<3, SIGN, FIRST>(line, tw, st, n, tl, TW, load, out, sc, last); break;
+    default: fx_stage<5, SIGN, FIRST>(line, tw, st, n, tl, TW, load, out, sc, last); break;
   }
 }
 
@@ -527,18 +554,18 @@ __device__ __forceinline__ void fft_stage_p(C* line, const C* __restrict__ tw, c
 // first(idx), so a caller can form the line on the fly (e.g. the product of
 // two other lines).  All threads of the team call this together; a team with
 // no line passes active=false and still synchronises.
-template <int SIGN, int PATH, typename C, typename First>
+template <int SIGN, int PATH, typename C, typename First, typename Out>
 __device__ __forceinline__ void fft_line_from(C* line, const typename TwOf<C>::type* __restrict__ tw, const FftPlan& pl,
-                                              int tl, bool active, First first) {
+                                              int tl, bool active, First first, Out out) {
   const int n = pl.n;
   const int TW = team_of<C>(pl);
   const int tla = active ? tl : (1 << 20);  // inactive lanes own no butterfly
   if constexpr (std::is_same<C, double2>::value && PATH != kFftLong) {
     if (PATH != kFftAny || n <= kFxMaxLine) {
       FxScale sc;
-      fx_stage_p<SIGN, true>(line, tw, pl.st[0], n, tla, TW, first, sc, pl.nst == 1);
+      fx_stage_p<SIGN, true>(line, tw, pl.st[0], n, tla, TW, first, out, sc, pl.nst == 1);
       for (int s = 1; s < pl.nst; ++s)
-        fx_stage_p<SIGN, false>(line, tw, pl.st[s], n, tla, TW, LineLoad<C>{line}, sc, s + 1 == pl.nst);
+        fx_stage_p<SIGN, false>(line, tw, pl.st[s], n, tla, TW, LineLoad<C>{line}, out, sc, s + 1 == pl.nst);
       return;
     }
   }
@@ -555,9 +582,9 @@ __device__ __forceinline__ void fft_line_from(C* line, const typename TwOf<C>::t
 // Stockham stage of radix 16) and writes it back; thread f then reads row
 // 16 f + q, applies w_256^{f q} and transforms it (the l = 16 stage).  One
 // shared-memory exchange and four warp barriers per line.
-template <int SIGN, typename C, typename First>
+template <int SIGN, typename C, typename First, typename Out>
 __device__ __forceinline__ void fft256_lines(C* base, int ld, int nlines, const C* __restrict__ tw,
-                                             const FftPlan& pl, First first) {
+                                             const FftPlan& pl, First first, Out) {
   const int team = threadIdx.x >> 4;
   const int k = threadIdx.x & 15;
   const int nteams = blockDim.x >> 4;
@@ -597,10 +624,10 @@ __device__ __forceinline__ void fft256_lines(C* base, int ld, int nlines, const 
 
 // The same for FP64 lines in fixed point: 16 of the line's doubles become
 // integers in each thread once the team has agreed on the line's scale, and
-// the second stage's results become doubles on their way to shared memory.
-template <int SIGN, typename First>
+// the second stage hands its results to the line's out.
+template <int SIGN, typename First, typename Out>
 __device__ __forceinline__ void fft256_lines(double2* base, int ld, int nlines, const fxw* __restrict__ tw,
-                                             const FftPlan& pl, First first) {
+                                             const FftPlan& pl, First first, Out outs) {
   const int team = threadIdx.x >> 4;
   const int k = threadIdx.x & 15;
   const int nteams = blockDim.x >> 4;
@@ -639,8 +666,9 @@ __device__ __forceinline__ void fft256_lines(double2* base, int ld, int nlines, 
     }
     __syncwarp();
     if (active) {
+      const auto out = outs(L);
 #pragma unroll
-      for (int s = 0; s < 16; ++s) line[sidx(k + 16 * s)] = fx_out(a[s], sc);
+      for (int s = 0; s < 16; ++s) out(k + 16 * s, a[s], sc);
     }
     __syncwarp();
   }
@@ -673,18 +701,18 @@ template <int PATH> __device__ __forceinline__ int tw_load(const FftPlan& pl) {
 }
 
 // Stages S.. of a compile-time length N on one line; stage 0 reads through first.
-template <int SIGN, int N, int S, typename C, typename First>
+template <int SIGN, int N, int S, typename C, typename First, typename Out>
 __device__ __forceinline__ void fft_ct_stages(C* line, const typename TwOf<C>::type* __restrict__ tw, const FftPlan& pl,
-                                              int tl, int TW, First first, FxScale sc = FxScale{}) {
+                                              int tl, int TW, First first, Out out, FxScale sc = FxScale{}) {
   if constexpr (S < ct_nst(N)) {
     if constexpr (std::is_same<C, double2>::value) {
-      if constexpr (S == 0) fx_stage<ct_radix(N, 0), SIGN, true>(line, tw, pl.st[0], N, tl, TW, first, sc, ct_nst(N) == 1);
-      else fx_stage<ct_radix(N, S), SIGN, false>(line, tw, pl.st[S], N, tl, TW, LineLoad<C>{line}, sc, S + 1 == ct_nst(N));
+      if constexpr (S == 0) fx_stage<ct_radix(N, 0), SIGN, true>(line, tw, pl.st[0], N, tl, TW, first, out, sc, ct_nst(N) == 1);
+      else fx_stage<ct_radix(N, S), SIGN, false>(line, tw, pl.st[S], N, tl, TW, LineLoad<C>{line}, out, sc, S + 1 == ct_nst(N));
     } else {
       if constexpr (S == 0) fft_stage<ct_radix(N, 0), SIGN>(line, tw, pl.st[0], N, tl, TW, first);
       else fft_stage<ct_radix(N, S), SIGN>(line, tw, pl.st[S], N, tl, TW, LineLoad<C>{line});
     }
-    fft_ct_stages<SIGN, N, S + 1>(line, tw, pl, tl, TW, first, sc);
+    fft_ct_stages<SIGN, N, S + 1>(line, tw, pl, tl, TW, first, out, sc);
   }
 }
 
@@ -692,17 +720,18 @@ __device__ __forceinline__ void fft_ct_stages(C* line, const typename TwOf<C>::t
 // base + L*ld; its first stage reads through the loader first(L) returns (a
 // functor idx -> value).  Every thread of the CTA must call this with the
 // same plan.  A length-1 transform is the identity: the inputs are only
-// copied into place.
-template <int SIGN, int PATH = kFftAny, typename C, typename First>
+// copied into place.  Lines transformed in fixed point (kIsFx) hand their
+// results to out(L); the others leave them in the line.
+template <int SIGN, int PATH = kFftAny, typename C, typename First, typename Out>
 __device__ __forceinline__ void fft_lines_from(C* base, int ld, int nlines,
                                                const typename TwOf<C>::type* __restrict__ tw,
-                                               const FftPlan& pl, First first) {
+                                               const FftPlan& pl, First first, Out out) {
   if (pl.n == 1 || pl.nst == 0) {
     for (int L = threadIdx.x; L < nlines; L += blockDim.x) base[L * ld] = first(L)(0);
     return;
   }
   if (PATH == kFft256 || (PATH == kFftAny && pl.tw16_off >= 0)) {
-    fft256_lines<SIGN>(base, ld, nlines, tw, pl, first);
+    fft256_lines<SIGN>(base, ld, nlines, tw, pl, first, out);
     return;
   }
   if (PATH == kFft256) return;
@@ -716,11 +745,22 @@ __device__ __forceinline__ void fft_lines_from(C* base, int ld, int nlines,
     const bool active = L < nlines;
     const int Lc = active ? L : 0;
     if constexpr (ct_length(PATH)) {
-      fft_ct_stages<SIGN, PATH, 0>(base + Lc * ld, tw, pl, active ? tl : (1 << 20), TW, first(Lc));
+      fft_ct_stages<SIGN, PATH, 0>(base + Lc * ld, tw, pl, active ? tl : (1 << 20), TW, first(Lc), out(Lc));
     } else {
-      fft_line_from<SIGN, PATH>(base + Lc * ld, tw, pl, tl, active, first(Lc));
+      fft_line_from<SIGN, PATH>(base + Lc * ld, tw, pl, tl, active, first(Lc), out(Lc));
     }
   }
+}
+
+// As above with the results left in the lines in every form.
+template <int SIGN, int PATH = kFftAny, typename C, typename First>
+__device__ __forceinline__ void fft_lines_from(C* base, int ld, int nlines,
+                                               const typename TwOf<C>::type* __restrict__ tw,
+                                               const FftPlan& pl, First first) {
+  if constexpr (std::is_same<C, double2>::value)
+    fft_lines_from<SIGN, PATH>(base, ld, nlines, tw, pl, first, [&](int L) { return FxOutLine{base + L * ld}; });
+  else
+    fft_lines_from<SIGN, PATH>(base, ld, nlines, tw, pl, first, [](int) { return 0; });
 }
 
 // As fft_lines_from on lines already in place.

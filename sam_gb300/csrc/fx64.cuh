@@ -50,7 +50,13 @@ __device__ __forceinline__ FxSplit fx_split(long long v) {
 __host__ __device__ constexpr FxSplit fx_const(long long v) {
   return FxSplit{(int)((v + 0x80000000ll) >> 32), (int)(uint32_t)(v & 0xffffffffll)};
 }
-__device__ __forceinline__ long long fx_mad(int a, int b, long long c) { return (long long)a * b + c; }
+// (the instruction spelled out: the compiler widens products of such halves
+// to 64 x 64-bit ones, twice the instructions)
+__device__ __forceinline__ long long fx_mad(int a, int b, long long c) {
+  long long r;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+  return r;
+}
 
 // (A 2^32 + C) >> 30 for A the sum of the high products and C the cross terms
 __device__ __forceinline__ long long fx_join(long long A, uint32_t clo) {
@@ -269,8 +275,23 @@ __device__ __forceinline__ long long fx_from(double d, int dsh) {
   const long long s = (long long)((int)hi >> 31);
   return ((long long)m ^ s) - s;
 }
+// sum of (v / 2^(E - 1023))^2 from the same leading bits
+template <int N> __device__ __forceinline__ float fx_l2(const double2* v, int E) {
+  const int base = (E - 127) * (1 << 20);
+  float s = 0.f, t = 0.f;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const float x = __int_as_float(max((__double2hiint(v[i].x) & 0x7fffffff) - base, 0) << 3);
+    const float y = __int_as_float(max((__double2hiint(v[i].y) & 0x7fffffff) - base, 0) << 3);
+    s = fmaf(x, x, s);
+    t = fmaf(y, y, t);
+  }
+  return s + t;
+}
 // The N values of each thread of a team to the line's fixed-point integers.
-template <int N> __device__ __forceinline__ FxScale fx_begin(double2* v, fxc* a, int TW) {
+// With NORM, *norm receives the 2-norm of the line's integers in units of 2^62.
+template <int N, bool NORM = false>
+__device__ __forceinline__ FxScale fx_begin(double2* v, fxc* a, int TW, float* norm = nullptr) {
   const auto umax = [](uint32_t x, uint32_t y) { return max(x, y); };
   uint32_t hm = team_reduce(fx_max_hi<N>(v), TW, umax);
   FxScale sc{0, kFxPlain};
@@ -292,6 +313,9 @@ template <int N> __device__ __forceinline__ FxScale fx_begin(double2* v, fxc* a,
   // L1 < 2^(E - 1023 + g) with room for the sum's own rounding
   int g = (__float_as_int(l1 * 1.0001f) >> 23) - 126;
   if (E == 0) g = 128;  // a line of zeros
+  if constexpr (NORM)
+    *norm = sqrtf(team_reduce(fx_l2<N>(v, E), TW, [](float x, float y) { return x + y; })) *
+            __int_as_float(max(127 - g, 0) << 23);
   if (E == 0x7ff) sc.kind = kFxNaN;
   else if (lift || E + g > 2040) sc.kind = kFxEdge;
   sc.ex = E - 1023 - 62 + g - lift;
@@ -309,10 +333,70 @@ __device__ __forceinline__ double fx_to(long long v, int ex) {
   const int hi = __double2hiint(r);
   return __hiloint2double(hi ? hi + ex * (1 << 20) : 0, __double2loint(r));
 }
-__device__ __forceinline__ double2 fx_out(fxc v, FxScale sc) {
-  if (sc.kind == kFxPlain) return make_double2(fx_to(v.x, sc.ex), fx_to(v.y, sc.ex));
+// The same on the integer pipe, for kernels that the FP64 pipe bounds: the
+// magnitude's leading one moved to bit 63, its top 53 bits rounded to
+// nearest (halves away from zero).
+__device__ __forceinline__ double fx_to_alu(long long v, int ex) {
+  const long long s = v >> 63;
+  const uint64_t m = (uint64_t)((v ^ s) - s);
+  const int lz = __clzll((long long)m);
+  const uint64_t t = m << lz;
+  const uint64_t q = (t >> 11) + ((t >> 10) & 1);  // 2^52 .. 2^53
+  const uint32_t hi = (uint32_t)(q >> 32) + (uint32_t)(1023 + 63 - 1 - lz + ex) * (1u << 20);
+  return m ? __hiloint2double((int)(hi | ((uint32_t)(s >> 32) & 0x80000000u)), (int)(uint32_t)q) : 0.0;
+}
+template <bool ALU = false> __device__ __forceinline__ double2 fx_out(fxc v, FxScale sc) {
+  if (sc.kind == kFxPlain) {
+    if (ALU) return make_double2(fx_to_alu(v.x, sc.ex), fx_to_alu(v.y, sc.ex));
+    return make_double2(fx_to(v.x, sc.ex), fx_to(v.y, sc.ex));
+  }
   if (sc.kind == kFxNaN) return make_double2(__hiloint2double(0x7ff80000, 0), __hiloint2double(0x7ff80000, 0));
   return make_double2(ldexp(__ll2double_rn(v.x), sc.ex), ldexp(__ll2double_rn(v.y), sc.ex));
+}
+
+// A line kept as split integers for products: value = (h 2^32 + l) 2^ex; norm
+// bounds the 2-norm of its integers, in units of 2^62.
+struct FxLine {
+  int ex, kind;
+  float norm;
+  int pad;
+};
+struct __align__(16) FxSplit2 {
+  FxSplit x, y;
+};
+__device__ __forceinline__ FxSplit2 fx_split2(fxc v) { return FxSplit2{fx_split(v.x), fx_split(v.y)}; }
+__device__ __forceinline__ fxc fx_whole(FxSplit2 v) {
+  return fxc{v.x.h * (1ll << 32) + v.x.l, v.y.h * (1ll << 32) + v.y.l};
+}
+
+// The component-wise products of two lines (rhs.f's u_a u_b of two real rows
+// at once) as one line's integers.  By Cauchy and Schwarz the sum of the
+// products' moduli is at most the product of the lines' norms, so the 124-bit
+// products shifted down by r = 62 + ceil(log2(norm_a norm_b)) sum to less
+// than 2^62, the bound a transform needs; each is rounded once.
+struct FxProduct {
+  int s;  // 64 - r: the shift left (or, negative, right) of the products' high words
+  long long half;
+  FxScale sc;
+};
+__device__ __forceinline__ FxProduct fx_product(const FxLine& a, const FxLine& b) {
+  // (norm_a norm_b >= 1/8 for lines scaled by their L1 norms; zero lines any)
+  const int r = max(62 + ((__float_as_int(a.norm * b.norm * 1.001f) >> 23) - 126), 59);
+  FxProduct p;
+  p.s = 64 - r;
+  p.half = p.s >= 0 ? 1ll << (31 - p.s) : 1ll << (-p.s - 1);
+  p.sc.ex = a.ex + b.ex + r;
+  // (room for the exponents of a scaling by 1 / (Nx Ny))
+  p.sc.kind = (a.kind | b.kind) & kFxNaN ? kFxNaN : (p.sc.ex < -960 || p.sc.ex > 940 ? kFxEdge : kFxPlain);
+  return p;
+}
+template <bool LEFT> __device__ __forceinline__ long long fx_mul_line(FxSplit a, FxSplit b, const FxProduct& p) {
+  const long long c = fx_mad(a.l, b.h, fx_mad(a.h, b.l, LEFT ? p.half : 0ll));
+  const long long A = fx_mad(a.h, b.h, c >> 32);
+  if (!LEFT) return (A + p.half) >> -p.s;
+  const uint32_t lo = __funnelshift_l((uint32_t)c, (uint32_t)A, p.s);
+  const uint32_t hi = __funnelshift_l((uint32_t)A, (uint32_t)(A >> 32), p.s);
+  return (long long)(((uint64_t)hi << 32) | lo);
 }
 
 }  // namespace samgpu

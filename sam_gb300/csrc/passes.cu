@@ -46,8 +46,6 @@ void launch_x2z(const double2* in, double2* out, const Grid& g, int nvar, int nx
   if (grid < 1) grid = 1;
   k_x2z<<<grid, kThreads, 0, s>>>(in, out, g, nvar, nx2);
 }
-
-
 SAMGPU_INST(double)
 
 }  // namespace samgpu

@@ -99,7 +99,24 @@ struct YFwdArgs {
   int nvar, tz, ld;
   long long in_kx, in_z, in_n;
   long long out_ky, out_kx, out_n;
+  // FP64 form, resident stage: the first CTA also writes the z-forward pass's
+  // kz table of this stage (ZFwdArgs::kz_tab), dt read on the device
+  double* kz_tab;
+  const DevState* kz_state;
+  double kz_gamma, kz_zeta, kz_vis, kz_pr_inv;
 };
+
+// What a ky row of a z-forward tile contributes to its modes' wave numbers
+// and (FP64 form) integrating factors exp(-nu k^2 dt_fac) = e(kx, ky) e(kz).
+template <typename W> struct EpiRow {
+  W rky, k_sq, ef, et;
+};
+// Shared memory behind the lines of a z-forward tile of ty rows and nf
+// fields (modes 1, 2): the scale of each fixed-point line, the rows' constants.
+template <typename T> constexpr size_t z_fwd_extra(int mode, int nf, int ty) {
+  if (mode == 0) return 0;
+  return (sizeof(T) == 8 ? sizeof(FxScale) * nf * ty : 0) + sizeof(EpiRow<T>) * ty;
+}
 
 template <typename T>
 struct ZFwdArgs {
@@ -126,6 +143,10 @@ struct ZFwdArgs {
   // as products of per-direction tables [2][Mx + My + Mz] (velocity, then
   // temperature with nu / Pr), written by launch_if_tables for this stage
   const dd* ift;
+  // FP64 form, mode 2: rkz(k), then the integrating factors' kz part for the
+  // velocity and for T, written by the stage's y-forward pass (null: formed
+  // per mode)
+  const double* kz_tab;
   T nz_inv;                  // filled by the launcher: 1/Nz
   FastDiv fd_t, fd_m;  // filled by the launcher: ty, Nz_min
 };
@@ -154,7 +175,8 @@ template <typename T> inline void set_smem_limits() {
 }
 // vmax (max_only forms): ints 0..7 hold the per-field maxima (FP32 form: the
 // float bit patterns in ints 0..3; double-float form: 64-bit keys of
-// dd_abs_key in ints 0..7, vkind = 1), int 8 the non-finite flag
+// dd_abs_key in ints 0..7, vkind = 1; FP64 form: bit patterns of doubles,
+// vkind = 2), int 8 the non-finite flag
 void launch_vel_max_finish(const double* partials, int nblk, const Grid& g, DevState* st, int i_cfl, double cfl0,
                            double adv_cfl_limit, cudaStream_t s, const double* pv = nullptr, int npv = 0,
                            int* vmax = nullptr, int vkind = 0);

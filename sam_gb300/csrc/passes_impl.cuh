@@ -1207,10 +1207,26 @@ __device__ __forceinline__ void y_fwd_body(const YFwdArgs<T>& a, const FftPlan* 
   load_twiddles<T>(s_tw, a.tw, tw_load<PATH>(pl));
   const C* src = a.in + (long long)m * a.in_n + (long long)i * a.in_kx + (long long)z0 * a.in_z;
   __syncthreads();
+  if (a.kz_tab && bid == 0) {
+    // the z-forward pass of the same stage, next on the stream, reads
+    // rkz(k), exp(-nu rkz^2 dt_fac) and the same with nu / Pr: one exp per
+    // kz here instead of one per mode there
+    const double vis_f = a.kz_vis * (a.kz_gamma * a.kz_state->dt + a.kz_zeta * a.kz_state->dt);  // sam.f:293-295
+    for (int k = threadIdx.x; k < a.g.mz; k += blockDim.x) {
+      const double rkz = a.g.wave_z * (double)kwave(k, a.g.kz, a.g.mz);
+      a.kz_tab[k] = rkz;
+      a.kz_tab[a.g.mz + k] = exp(-vis_f * (rkz * rkz));
+      a.kz_tab[2 * a.g.mz + k] = exp(-(vis_f * a.kz_pr_inv) * (rkz * rkz));
+    }
+  }
   // the first stage reads its inputs straight from the rows of C (no
   // shared-memory staging); the rows are contiguous in y
-  fft_lines_from<-1, PATH>(s_ln, ld, nl, s_tw, pl,
-                           [&](int L) { return RowLoad<C, COH>{src + (long long)L * a.in_z}; });
+  const auto rows = [&](int L) { return RowLoad<C, COH>{src + (long long)L * a.in_z}; };
+  if constexpr (kIsFx<C, PATH>)
+    fft_lines_from<-1, PATH>(s_ln, ld, nl, s_tw, pl, rows,
+                             [&](int L) { return FxOutBand{s_ln + L * ld, km, ny - km}; });
+  else
+    fft_lines_from<-1, PATH>(s_ln, ld, nl, s_tw, pl, rows);
   __syncthreads();
   C* dst = a.out + (long long)m * a.out_n + (long long)i * a.out_kx + z0;
   store_tile_rows(dst, a.out_ky, s_ln, ld, a.tz, nl, my, [&](int j) { return kpos(j, km, my, ny); });
@@ -1225,10 +1241,12 @@ __device__ __forceinline__ double wexp(double x) { return exp(x); }
 __device__ __forceinline__ float wexp(float x) { return expf(x); }
 
 // Per-launch constants of the epilogue in working type W, formed once per
-// thread: the FP32 form then touches no FP64 arithmetic per mode.
+// CTA: the FP32 form then touches no FP64 arithmetic per mode.
 template <typename W> struct EpiConst {
   W wave_x, wave_y, wave_z, nz_inv, dt_fac1, dt_fac2, mvis_f, mvis_t, bx, bz, lapse, cth, sth;
-  bool same_t, nz_pow2;
+  // 1/Nz: whether the divergence sums are still to be multiplied by it (the
+  // fixed-point lines of a power of two carry it in their exponents)
+  bool same_t, nz_pow2, scale, tilt;
 };
 
 template <typename W, typename T>
@@ -1238,6 +1256,8 @@ __device__ __forceinline__ EpiConst<W> epi_const(const ZFwdArgs<T>& a, double dt
   e.wave_x = (W)a.g.wave_x; e.wave_y = (W)a.g.wave_y; e.wave_z = (W)a.g.wave_z;
   e.nz_inv = (W)a.nz_inv;
   e.nz_pow2 = is_pow2_inv(a.g.nz);
+  e.scale = true;
+  e.tilt = sc.buoy_fac_x != 0.0;
   e.dt_fac1 = (W)(sc.gamma * dt);
   e.dt_fac2 = (W)(sc.zeta * dt);
   const double vis_f = sc.vis * (sc.gamma * dt + sc.zeta * dt);  // sam.f:293-295
@@ -1283,35 +1303,39 @@ __device__ __forceinline__ void epi_load(const ZFwdArgs<T>& a, int i, int j, int
 }
 
 // rhs.f:108-142 for one mode (kx i, ky j, kz k) in working type W, then
-// (mode 2) sam.f:210-221 and 293-314.  ln points at field 0 of this mode in
-// shared memory; field f is at ln[f * fstride].
-template <typename W, typename T>
-__device__ __forceinline__ void epi_mode(const ZFwdArgs<T>& a, const cx_t<T>* ln, int fstride, int i, int j, int k,
-                                         const EpiConst<W>& c, const EpiIn<W>& in) {
+// (mode 2) sam.f:210-221 and 293-314.  val(f) is the transform of field f at
+// this mode, times Nz where c.scale says so.
+template <typename W, typename T, typename Val>
+__device__ __forceinline__ void epi_mode(const ZFwdArgs<T>& a, Val val, int i, int j, int k, const EpiConst<W>& c,
+                                         const EpiRow<W>& row, const EpiIn<W>& in) {
   using C = cx_t<T>;
   const Grid& g = a.g;
   const StageConsts& sc = a.sc;
   const int nf = a.nf;
-  const W rkx = c.wave_x * (W)i;
-  const W rky = c.wave_y * (W)kwave(j, g.ky, g.my);
-  const W rkz = c.wave_z * (W)kwave(k, g.kz, g.mz);
-  const W rk_sq_raw = rkx * rkx + rky * rky + rkz * rkz;
-  const W rk_sq = rk_sq_raw > (W)1.0e-10 ? rk_sq_raw : (W)1.0e-10;
+  const W rkx = c.wave_x * (W)i, rky = row.rky;
+  W rkz;
+  if constexpr (std::is_same<W, double>::value) rkz = a.kz_tab ? a.kz_tab[k] : c.wave_z * (W)kwave(k, g.kz, g.mz);
+  else rkz = c.wave_z * (W)kwave(k, g.kz, g.mz);
+  const W rk_sq_raw = row.k_sq + rkz * rkz;
+  W rk_sq;
+  if constexpr (std::is_same<W, double>::value)  // (compared as integers: both are positive)
+    rk_sq = __double_as_longlong(rk_sq_raw) > __double_as_longlong(1.0e-10) ? rk_sq_raw : 1.0e-10;
+  else rk_sq = rk_sq_raw > (W)1.0e-10 ? rk_sq_raw : (W)1.0e-10;
   W tr[9], ti[9];
 #pragma unroll
   for (int f = 0; f < 9; ++f) {
-    if (f < nf) {
-      const C v = ln[f * fstride];
-      tr[f] = scale_by((W)v.x, c.nz_inv, c.nz_pow2);
-      ti[f] = scale_by((W)v.y, c.nz_inv, c.nz_pow2);
-    } else {
-      tr[f] = (W)0; ti[f] = (W)0;
-    }
+    if (f < nf) val(f, tr[f], ti[f]);
+    else tr[f] = ti[f] = (W)0;
   }
   // -i (a + i b) = b - i a
-  const W s1r = rkx * tr[0] + rky * tr[1] + rkz * tr[3], s1i = rkx * ti[0] + rky * ti[1] + rkz * ti[3];
-  const W s2r = rkx * tr[1] + rky * tr[2] + rkz * tr[4], s2i = rkx * ti[1] + rky * ti[2] + rkz * ti[4];
-  const W s3r = rkx * tr[3] + rky * tr[4] + rkz * tr[5], s3i = rkx * ti[3] + rky * ti[4] + rkz * ti[5];
+  W s1r = rkx * tr[0] + rky * tr[1] + rkz * tr[3], s1i = rkx * ti[0] + rky * ti[1] + rkz * ti[3];
+  W s2r = rkx * tr[1] + rky * tr[2] + rkz * tr[4], s2i = rkx * ti[1] + rky * ti[2] + rkz * ti[4];
+  W s3r = rkx * tr[3] + rky * tr[4] + rkz * tr[5], s3i = rkx * ti[3] + rky * ti[4] + rkz * ti[5];
+  if (c.scale) {
+    s1r = scale_by(s1r, c.nz_inv, c.nz_pow2); s1i = scale_by(s1i, c.nz_inv, c.nz_pow2);
+    s2r = scale_by(s2r, c.nz_inv, c.nz_pow2); s2i = scale_by(s2i, c.nz_inv, c.nz_pow2);
+    s3r = scale_by(s3r, c.nz_inv, c.nz_pow2); s3i = scale_by(s3i, c.nz_inv, c.nz_pow2);
+  }
   W r1r = s1i, r1i = -s1r, r2r = s2i, r2i = -s2r, r3r = s3i, r3i = -s3r, r4r = (W)0, r4i = (W)0;
   if (sc.i_strat) {
     W wr = in.ur[2], wi = in.ui[2];
@@ -1320,16 +1344,33 @@ __device__ __forceinline__ void epi_mode(const ZFwdArgs<T>& a, const cx_t<T>* ln
       wi = c.cth * in.ui[2] - c.sth * in.ui[0];
     }
     const W thr = in.ur[3], thi = in.ui[3];
-    r1r += c.bx * thr; r1i += c.bx * thi;
+    if (c.tilt) {
+      r1r += c.bx * thr; r1i += c.bx * thi;
+    }
     r3r += c.bz * thr; r3i += c.bz * thi;
-    const W s4r = rkx * tr[6] + rky * tr[7] + rkz * tr[8];
-    const W s4i = rkx * ti[6] + rky * ti[7] + rkz * ti[8];
+    W s4r = rkx * tr[6] + rky * tr[7] + rkz * tr[8];
+    W s4i = rkx * ti[6] + rky * ti[7] + rkz * ti[8];
+    if (c.scale) {
+      s4r = scale_by(s4r, c.nz_inv, c.nz_pow2);
+      s4i = scale_by(s4i, c.nz_inv, c.nz_pow2);
+    }
     r4r = s4i - c.lapse * wr;
     r4i = -s4r - c.lapse * wi;
   }
   // p = -i (k . R) / k^2 ;  R -= i k p   (rhs.f:134-139)
   const W qr = rkx * r1r + rky * r2r + rkz * r3r, qi = rkx * r1i + rky * r2i + rkz * r3i;
-  const W pr = qi / rk_sq, pim = -qr / rk_sq;
+  W pr, pim;
+  if constexpr (std::is_same<W, double>::value) {
+    // one reciprocal for both quotients, each corrected by its remainder
+    const double inv = 1.0 / rk_sq;
+    pr = qi * inv;
+    pr = fma(fma(-pr, rk_sq, qi), inv, pr);
+    pim = -qr * inv;
+    pim = fma(fma(-pim, rk_sq, -qr), inv, pim);
+  } else {
+    pr = qi / rk_sq;
+    pim = -qr / rk_sq;
+  }
   // -i rk p = rk * (p.i, -p.r)
   r1r += rkx * pim; r1i -= rkx * pr;
   r2r += rky * pim; r2i -= rky * pr;
@@ -1352,6 +1393,9 @@ __device__ __forceinline__ void epi_mode(const ZFwdArgs<T>& a, const cx_t<T>* ln
     const int oy = g.mx, oz = g.mx + g.my, tw = g.mx + g.my + g.mz;
     ef = tb[i] * tb[oy + j] * tb[oz + k];
     et = c.same_t ? ef : tb[tw + i] * tb[tw + oy + j] * tb[tw + oz + k];
+  } else if (std::is_same<W, double>::value && a.kz_tab) {
+    ef = row.ef * (W)a.kz_tab[g.mz + k];
+    et = c.same_t ? ef : row.et * (W)a.kz_tab[2 * g.mz + k];
   } else {
     ef = wexp(c.mvis_f * rk_sq_raw);
     et = c.same_t ? ef : wexp(c.mvis_t * rk_sq_raw);
@@ -1398,12 +1442,26 @@ __device__ __forceinline__ void z_fwd_body(const ZFwdArgs<T>& a, const FftPlan* 
   const int nl = min(a.ty, my - j0);
   load_twiddles<T>(s_tw, a.tw, tw_load<PATH>(pl));
   // lines of all nf fields for the nl rows of this tile, packed as f * nl + t;
-  // the first stage reads the z-contiguous rows of D straight from memory
+  // the first stage reads the z-contiguous rows of D straight from memory.
+  // Fixed-point lines stay integers, their scales behind the tile's lines: of
+  // Nz results only the Nz_min stored modes are converted, and 1/Nz, where
+  // it is a power of two, costs nothing.
+  constexpr bool FX = kIsFx<C, PATH>;
+  const bool ints = FX && nz > 1 && a.mode != 0;
+  FxScale* s_sc = reinterpret_cast<FxScale*>(s_ln + (size_t)nf * a.ty * ld);
+  EpiRow<T>* s_row = reinterpret_cast<EpiRow<T>*>(s_sc + (std::is_same<T, double>::value ? nf * a.ty : 0));
   __syncthreads();
-  fft_lines_from<-1, PATH>(s_ln, ld, nf * nl, s_tw, pl, [&](int L) {
+  const auto rows = [&](int L) {
     const int f = L / nl, t = L - f * nl;
     return RowLoad<C, COH>{a.in + (long long)f * a.in_n + (long long)i * a.in_kx + (long long)(j0 + t) * a.in_ky};
-  });
+  };
+  if constexpr (FX) {
+    if (ints)
+      fft_lines_from<-1, PATH>(s_ln, ld, nf * nl, s_tw, pl, rows, [&](int L) {
+        return FxOutInt{reinterpret_cast<fxc*>(s_ln + L * ld), s_sc + L};
+      });
+  }
+  if (!ints) fft_lines_from<-1, PATH>(s_ln, ld, nf * nl, s_tw, pl, rows);
   __syncthreads();
   const T nz_inv = a.nz_inv;
   if (a.mode == 0) {
@@ -1411,7 +1469,8 @@ __device__ __forceinline__ void z_fwd_body(const ZFwdArgs<T>& a, const FftPlan* 
       const int r = (int)fdiv(e, a.fd_m), k = e - r * mz;
       const int f = (int)fdiv(r, a.fd_t), t = r - f * a.ty;
       if (t >= nl) continue;
-      C v = s_ln[(f * nl + t) * ld + sidx(kpos(k, km, mz, nz))];
+      const int L = f * nl + t;
+      C v = s_ln[L * ld + sidx(kpos(k, km, mz, nz))];
       v.x *= nz_inv;
       v.y *= nz_inv;
       a.in[(long long)f * a.in_n + (long long)i * a.in_kx + (long long)(j0 + t) * a.in_ky + k] = v;
@@ -1420,11 +1479,33 @@ __device__ __forceinline__ void z_fwd_body(const ZFwdArgs<T>& a, const FftPlan* 
   }
   double dt = 0.0;
   if (a.mode == 2) dt = ldc<COH>(&a.state->dt);
-  // the epilogue constants once per CTA (FP64 arithmetic on one thread)
+  // the epilogue constants once per CTA (FP64 arithmetic on one thread), the
+  // rows' once per row
   __shared__ EpiConst<T> s_cw;
-  if (threadIdx.x == 0) s_cw = epi_const<T>(a, dt);
+  if (threadIdx.x == 0) {
+    EpiConst<T> e = epi_const<T>(a, dt);
+    if (ints && e.nz_pow2) e.scale = false;
+    s_cw = e;
+  }
   __syncthreads();
   const EpiConst<T> cw = s_cw;
+  for (int t = threadIdx.x; t < nl; t += blockDim.x) {
+    EpiRow<T> r;
+    const T rkx = cw.wave_x * (T)i;
+    r.rky = cw.wave_y * (T)kwave(j0 + t, g.ky, my);
+    r.k_sq = rkx * rkx + r.rky * r.rky;
+    r.ef = r.et = (T)1;
+    if constexpr (std::is_same<T, double>::value)
+      if (a.kz_tab) {
+        r.ef = exp(cw.mvis_f * r.k_sq);
+        r.et = cw.same_t ? r.ef : exp(cw.mvis_t * r.k_sq);
+      }
+    s_row[t] = r;
+  }
+  if constexpr (FX)
+    if (!cw.scale)
+      for (int L = threadIdx.x; L < nf * nl; L += blockDim.x) s_sc[L].ex -= 31 - __clz(nz);
+  __syncthreads();
   // two modes per iteration: their global loads are issued together
   for (int e0 = threadIdx.x; e0 < nl * mz; e0 += 2 * blockDim.x) {
     const int e1 = e0 + blockDim.x;
@@ -1438,16 +1519,41 @@ __device__ __forceinline__ void z_fwd_body(const ZFwdArgs<T>& a, const FftPlan* 
       if (h == 1 && !has1) break;
       const int t = h ? t1 : t0, k = h ? k1 : k0, j = j0 + t;
       const C* ln = s_ln + t * ld + sidx(kpos(k, km, mz, nz));
+      const auto val = [&](int f, T& re, T& im) {
+        if constexpr (FX) {
+          if (ints) {
+            // (this loop is bound by the FP64 pipe: convert on the other one)
+            const C v = fx_out<true>(*reinterpret_cast<const fxc*>(ln + f * nl * ld), s_sc[f * nl + t]);
+            re = v.x;
+            im = v.y;
+            return;
+          }
+        }
+        const C v = ln[f * nl * ld];
+        re = v.x;
+        im = v.y;
+      };
       // (the FP32 form treats the mean mode in FP64 below)
-      if (sizeof(T) == 8 || i != 0 || j != 0 || k != 0) epi_mode<T, T>(a, ln, nl * ld, i, j, k, cw, h ? in1 : in0);
+      if (sizeof(T) == 8 || i != 0 || j != 0 || k != 0)
+        epi_mode<T, T>(a, val, i, j, k, cw, s_row[t], h ? in1 : in0);
     }
   }
-  if (sizeof(T) == 4 && i == 0 && j0 == 0 && threadIdx.x == 0) {
-    // the FP32 form keeps the mean (k = 0) mode in FP64; one thread, outside
-    // the per-mode loop so that no FP64 instruction is issued per mode
-    EpiIn<double> ind;
-    epi_load<double>(a, 0, 0, 0, ind);
-    epi_mode<double, T>(a, s_ln + sidx(kpos(0, km, mz, nz)), nl * ld, 0, 0, 0, epi_const<double>(a, dt), ind);
+  if constexpr (sizeof(T) == 4) {
+    if (i == 0 && j0 == 0 && threadIdx.x == 0) {
+      // the FP32 form keeps the mean (k = 0) mode in FP64; one thread, outside
+      // the per-mode loop so that no FP64 instruction is issued per mode
+      EpiIn<double> ind;
+      epi_load<double>(a, 0, 0, 0, ind);
+      const C* ln = s_ln + sidx(kpos(0, km, mz, nz));
+      epi_mode<double, T>(
+          a,
+          [&](int f, double& re, double& im) {
+            const C v = ln[f * nl * ld];
+            re = (double)v.x;
+            im = (double)v.y;
+          },
+          0, 0, 0, epi_const<double>(a, dt), EpiRow<double>{0.0, 0.0, 1.0, 1.0}, ind);
+    }
   }
   if (a.mode == 2 && a.sc.last && bid == 0 && threadIdx.x == 0) {
     // sam.f:318 time = time + dt, once per step (no CTA of this launch reads
@@ -1465,10 +1571,10 @@ __global__ void __launch_bounds__(kThreads, MinBlocks<T, kPassZFwd, PATH>::value
 // vel_max.f:28-49 on the per-CTA partials written by k_x_pass.
 // Parseval sums of vel_max (see launch_parseval): sums of the stored modes'
 // squares, FP64-accurate, per-thread strided order, block tree, fixed launch
-// shape.  The FP32 form (the only user) accumulates the exact squares of its
+// shape.  The FP32 form accumulates the exact squares of its
 // FP32 values in error-free FP32 pairs (about 48 bits: FP64 arithmetic, one
 // instruction per value pair of the 1/64-rate FP64 pipe plus a conversion,
-// made this kernel FP64-bound); the FP64 form would use FP64.
+// made this kernel FP64-bound); the others use FP64 arithmetic.
 __device__ __forceinline__ DF df_add_wsq(DF a, float v, float w) {
   // a + w v^2 with w a power of two (exact scaling of the exact square p + e)
   const float p = v * v;
@@ -1508,7 +1614,16 @@ __device__ __forceinline__ void parseval_body(const cx_t<T>* __restrict__ u, con
       for (int f = 0; f < 4; ++f)
         if (f < g.lu) {
           const cx_t<T> v = u[f * nm + m];
-          const double re = (double)v.x, im = (double)v.y;
+          double re = (double)v.x, im = (double)v.y;
+          if (kx0) {
+            // the physical field takes the real part of the kx = 0 lines
+            // (xy_trans_b.f:28-31): the plane's Hermitian part counts,
+            // (u(ky, kz) + conj u(-ky, -kz)) / 2
+            const int j = (int)m / g.mz, k = (int)m - j * g.mz;
+            const cx_t<T> h = u[f * nm + (long long)(j ? g.my - j : 0) * g.mz + (k ? g.mz - k : 0)];
+            re = 0.5 * (re + (double)h.x);
+            im = 0.5 * (im - (double)h.y);
+          }
           if (kx0) acc0[f] = fma(re, re, fma(im, im, acc0[f]));
           else acc1[f] = fma(re, re, fma(im, im, acc1[f]));
         }
@@ -1600,8 +1715,10 @@ __device__ __forceinline__ void vel_max_finish_body(const double* __restrict__ p
         const double n = (double)g.nx * (double)g.ny * (double)g.nz;
         fin[f][0] = ldc<COH>(pv + (long long)npv * g.lu + f) * n;
         fin[f][1] = red[0] * n;
-        fin[f][2] = vkind ? dd_key_value(ldc<COH>(reinterpret_cast<const unsigned long long*>(vmax) + f))
-                          : (double)__int_as_float(ldc<COH>(vmax + f));
+        const unsigned long long key =
+            vkind ? ldc<COH>(reinterpret_cast<const unsigned long long*>(vmax) + f) : 0ull;
+        fin[f][2] = vkind == 2 ? __longlong_as_double((long long)key)
+                               : (vkind ? dd_key_value(key) : (double)__int_as_float(ldc<COH>(vmax + f)));
         fin[f][3] = (double)ldc<COH>(vmax + 8);
       }
       __syncthreads();

@@ -205,6 +205,7 @@ struct Ctx {
   int partial_blocks = 0;
   double* pv = nullptr;  // vel_max's wave-space sums (FP32 and double-float forms)
   dd* ift = nullptr;     // double-float form: integrating-factor tables of the stage
+  double* kz_tab = nullptr;  // FP64 form: kz wave numbers and integrating factors of the stage (3 Mz)
   DevState* state = nullptr;
   Scratch sc[4];
   // tile choices
@@ -477,15 +478,24 @@ static int run_x_pass(Ctx& c, int in_mode, int out_mode, int nin, const void* in
   if (stats) {
     if (a.max_only) launch_parseval<T>((const cx_t<T>*)c.U, c.g, c.pv, c.stream);
     launch_vel_max_finish(c.partials, nblk, c.g, c.state, c.cfg.i_cfl, c.cfg.cfl0, c.adv_cfl_limit, c.stream,
-                          a.max_only ? c.pv : nullptr, kParsevalBlocks, a.vmax, kIsDD<T> ? 1 : 0);
+                          a.max_only ? c.pv : nullptr, kParsevalBlocks, a.vmax,
+                          kIsDD<T> ? 1 : (std::is_same<T, double>::value ? 2 : 0));
   }
   return 0;
 }
 
 template <typename T>
 static int run_y_fwd(Ctx& c, const void* in, void* out, int nvar, long long in_kx, long long in_z, long long in_n,
-                     long long out_ky, long long out_kx, long long out_n) {
+                     long long out_ky, long long out_kx, long long out_n, const StageConsts* stage = nullptr) {
   YFwdArgs<T> a{};
+  if (stage && std::is_same<T, double>::value) {
+    a.kz_tab = c.kz_tab;
+    a.kz_state = c.state;
+    a.kz_gamma = stage->gamma;
+    a.kz_zeta = stage->zeta;
+    a.kz_vis = stage->vis;
+    a.kz_pr_inv = stage->pr_inv;
+  }
   a.g = c.g;
   a.in = (const cx_t<T>*)in;
   a.out = (cx_t<T>*)out;
@@ -535,12 +545,15 @@ static int run_z_fwd(Ctx& c, ZFwdArgs<T>& a) {
   a.tw = tw_of<T>(c.pz);
   a.ld = line_ld(c.g.nz);
   a.sched = c.sched[4];
-  a.ty = pick_tile(c.pz, c.ty_zf, a.nf, sizeof(cx_t<T>), a.sched);
+  auto bytes = [&](int ty) {
+    return tile_smem(c.pz, ty * a.nf, sizeof(cx_t<T>), a.sched) + z_fwd_extra<T>(a.mode, a.nf, ty);
+  };
+  for (a.ty = c.ty_zf; a.ty > 1 && bytes(a.ty) > kSmemMax;) a.ty /= 2;
   if (kIsDD<T> && a.mode == 2) {
     launch_if_tables(c.state, a.sc, c.g, c.ift, c.stream);
     a.ift = c.ift;
   }
-  const size_t smem = tile_smem(c.pz, a.ty * a.nf, sizeof(cx_t<T>), a.sched);
+  const size_t smem = bytes(a.ty);
   if constexpr (std::is_same<T, float>::value) {
     if (c.rec) {
       ens_record_z_fwd(*c.rec, a, c.pz.d, smem);
@@ -554,8 +567,10 @@ static int run_z_fwd(Ctx& c, ZFwdArgs<T>& a) {
 // One fused RK stage on the resident state (sam.f:169-314).  When ev is
 // given, ev[p] is recorded before pass p and ev[5] after the last pass; when
 // only >= 0, just pass `only` (0..4) runs (used by the autotuner).
+// write_p = 0: the pressure of this stage is not kept (inside whole steps
+// only the last stage's can be read).
 template <typename T>
-static int enqueue_stage(Ctx& c, int nrk, cudaEvent_t* ev = nullptr, int only = -1) {
+static int enqueue_stage(Ctx& c, int nrk, cudaEvent_t* ev, int only, int write_p) {
   const Grid& g = c.g;
   const long long nzmm = (long long)g.mx * g.my * g.mz;
   int rc = 0;
@@ -613,9 +628,10 @@ static int enqueue_stage(Ctx& c, int nrk, cudaEvent_t* ev = nullptr, int only = 
   if (rc) return rc;
   if (ev) cudaEventRecord(ev[3], c.stream);
   // y forward: C -> D(m, kx, ky, z)
+  const StageConsts consts = stage_consts(c, nrk, write_p);
   if (run(3))
     rc = run_y_fwd<T>(c, c.S3, c.S1, g.lr, g.ny, (long long)g.mx * g.ny, (long long)g.nz * g.mx * g.ny, g.nz,
-                      (long long)g.my * g.nz, (long long)g.mx * g.my * g.nz);
+                      (long long)g.my * g.nz, (long long)g.mx * g.my * g.nz, &consts);
   if (rc) return rc;
   if (ev) cudaEventRecord(ev[4], c.stream);
   if (!run(4)) {
@@ -633,16 +649,17 @@ static int enqueue_stage(Ctx& c, int nrk, cudaEvent_t* ev = nullptr, int only = 
   a.p = (cx_t<T>*)c.P;
   a.u_ky = g.mz; a.u_kx = (long long)g.my * g.mz; a.u_n = nzmm;
   a.state = c.state;
-  a.sc = stage_consts(c, nrk, 1);
+  a.sc = consts;
+  if (std::is_same<T, double>::value) a.kz_tab = c.kz_tab;
   rc = run_z_fwd<T>(c, a);
   if (ev) cudaEventRecord(ev[5], c.stream);
   return rc;
 }
 
-static int stage_any(Ctx& c, int nrk, cudaEvent_t* ev = nullptr, int only = -1) {
-  if (c.cfg.precision == 32) return enqueue_stage<float>(c, nrk, ev, only);
-  if (c.cfg.precision == kPrecDD) return enqueue_stage<dd>(c, nrk, ev, only);
-  return enqueue_stage<double>(c, nrk, ev, only);
+static int stage_any(Ctx& c, int nrk, cudaEvent_t* ev = nullptr, int only = -1, int write_p = 1) {
+  if (c.cfg.precision == 32) return enqueue_stage<float>(c, nrk, ev, only, write_p);
+  if (c.cfg.precision == kPrecDD) return enqueue_stage<dd>(c, nrk, ev, only, write_p);
+  return enqueue_stage<double>(c, nrk, ev, only, write_p);
 }
 
 static int check_launch() {
@@ -663,6 +680,7 @@ static void free_ctx(Ctx* c) {
   cudaFree(c->U); cudaFree(c->R); cudaFree(c->P);
   cudaFree(c->S1); cudaFree(c->S2); cudaFree(c->S3);
   cudaFree(c->partials); cudaFree(c->state); cudaFree(c->ou); cudaFree(c->pv); cudaFree(c->ift);
+  cudaFree(c->kz_tab);
   cudaFree(c->les_cds); cudaFree(c->les_phys); cudaFree(c->les_work);
   cudaFree(c->les_feat); cudaFree(c->les_coef);
   cudaFree(c->mlp_p); cudaFree(c->mlp_m); cudaFree(c->mlp_v); cudaFree(c->mlp_g); cudaFree(c->mlp_loss);
@@ -828,6 +846,11 @@ static int init_ctx(const sam_gpu_config* cfg) {
   if ((rc = build_plan(g.nx, c->px)) || (rc = build_plan(g.ny, c->py)) || (rc = build_plan(g.nz, c->pz))) {
     free_ctx(c); g_ctx = nullptr; return rc;
   }
+  // FP64 z-forward tiles that leave room for two CTAs per SM: one CTA's
+  // fixed-point transforms overlap the other's FP64 epilogue (256^3: 2 rows
+  // 0.92 ms, 4 rows, one CTA, 1.09; 128^3: 4 rows, two CTAs, 0.143, 2 rows 0.157)
+  if (cfg->precision == 64)
+    while (c->ty_zf > 1 && tile_smem(c->pz, c->ty_zf * g.lr, sizeof(double2)) > kSmemMax / 2 - 1024) c->ty_zf /= 2;
   cudaError_t e = cudaStreamCreateWithFlags(&c->own, cudaStreamNonBlocking);
   if (e != cudaSuccess) { free_ctx(c); g_ctx = nullptr; return fail(SAM_GPU_ECUDA, "stream: %s", cudaGetErrorString(e)); }
   c->stream = c->own;
@@ -861,6 +884,7 @@ static int init_ctx(const sam_gpu_config* cfg) {
   if (ok) cudaMemset(c->pv, 0, pv_bytes);
   if (ok && cfg->precision == kPrecDD)
     ok = cudaMalloc(&c->ift, sizeof(dd) * 2 * ((size_t)g.mx + g.my + g.mz)) == cudaSuccess;
+  ok = ok && cudaMalloc(&c->kz_tab, sizeof(double) * 3 * (size_t)g.mz) == cudaSuccess;
   if (!ok) { free_ctx(c); g_ctx = nullptr; return fail(SAM_GPU_ECUDA, "device allocation failed"); }
   cudaMemset(c->U, 0, es * g.lu * nzmm);
   cudaMemset(c->R, 0, es * g.lu * nzmm);
@@ -956,7 +980,7 @@ static bool ens_eligible(const Ctx& c) {
 
 static int enqueue_step(Ctx& c) {
   int rc = 0;
-  for (int nrk = 1; nrk <= c.cfg.nrk_max && !rc; ++nrk) rc = stage_any(c, nrk);
+  for (int nrk = 1; nrk <= c.cfg.nrk_max && !rc; ++nrk) rc = stage_any(c, nrk, nullptr, -1, nrk == c.cfg.nrk_max);
   if (!rc && c.ou) {
     if (c.cfg.precision == 32) ou_apply<float>((float2*)c.U, c.g, c.ou, c.state, c.stream);
     else ou_apply<double>((double2*)c.U, c.g, c.ou, c.state, c.stream);
@@ -994,7 +1018,7 @@ int sam_gpu_ensemble_step(int nsteps) {
         if (s + 1 > m.cfg.nrk_max) continue;
         EnsRecorder* r = &E.recs[k * 3 + (size_t)s];
         m.rec = r;
-        const int rc = stage_any(m, s + 1);
+        const int rc = stage_any(m, s + 1, nullptr, -1, s + 1 == m.cfg.nrk_max);
         m.rec = nullptr;
         if (rc) return rc;
         rs.push_back(r);
@@ -1329,7 +1353,7 @@ int sam_gpu_step(int nsteps) {
     cudaGraph_t graph;
     CK(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal));
     int rc = 0;
-    for (int nrk = 1; nrk <= c.cfg.nrk_max && !rc; ++nrk) rc = stage_any(c, nrk);
+    for (int nrk = 1; nrk <= c.cfg.nrk_max && !rc; ++nrk) rc = stage_any(c, nrk, nullptr, -1, nrk == c.cfg.nrk_max);
     if (!rc && c.ou) {
       if (c.cfg.precision == 32) ou_apply<float>((float2*)c.U, c.g, c.ou, c.state, c.stream);
       else ou_apply<double>((double2*)c.U, c.g, c.ou, c.state, c.stream);
