@@ -155,6 +155,9 @@ template <typename T> void launch_z_inv(const ZInvArgs<T>& a, const FftPlan* pl,
 template <typename T> void launch_y_inv(const YInvArgs<T>& a, const FftPlan* pl, size_t smem, cudaStream_t s);
 template <typename T> void launch_x_pass(const XPassArgs<T>& a, const FftPlan* pl, size_t smem, cudaStream_t s);
 template <typename T> int x_pass_blocks(const XPassArgs<T>& a);
+// whether the FP64 x pass of these arguments (max_only given) runs the fused
+// 256-point kernel, which forms vel_max's maxima only
+bool x_fused_fp64(const XPassArgs<double>& a);
 template <typename T> void launch_y_fwd(const YFwdArgs<T>& a, const FftPlan* pl, size_t smem, cudaStream_t s);
 template <typename T> void launch_z_fwd(const ZFwdArgs<T>& a, const FftPlan* pl, size_t smem, cudaStream_t s);
 template <typename T> void smem_limits_zinv(int optin);

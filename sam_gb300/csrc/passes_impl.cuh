@@ -1183,6 +1183,220 @@ __host__ __device__ inline bool x_f256_applies(const XPassArgs<float>& a) {
          a.nin <= 4 && (a.g.lr == 6 || a.g.lr == 9) && (!a.partials || a.max_only) && a.yt >= 2 && a.yt % 2 == 0;
 }
 
+// ------------------------------------------------ x pass, FP64 at Nx = 256
+// The x pass of the plain FP64 step with 256-point x lines (spectral input
+// rows, products out, no subgrid terms) with the physical fields kept in
+// fixed point between the two transforms: the backward transform leaves split
+// integers and each line's scale and norm, a product line is formed as
+// integers (fx_product) and goes straight into its forward transform, and
+// only the stored modes become doubles.  Against the general kernel that takes
+// out, per product line, 512 FP64 products, a conversion to doubles of every
+// physical value and back to integers of every product, and the FP64 sums of
+// the split: the general kernel kept the FP64 pipe 50 % busy and its 16 teams
+// 56 % (9 product lines a round).  A team of 16 threads takes a product line
+// from its factors to HBM by itself, as in k_x_pass_f256; the exchange between
+// the two radix-16 stages goes through half a line (re, then im), so that 16
+// teams' scratch and an 8-row tile's input lines leave room for two CTAs per SM.
+constexpr int kXfx256Threads = 256;
+constexpr int kXfx256Teams = kXfx256Threads / 16;
+__host__ __device__ constexpr size_t x_fx256_smem(int lines) {
+  return sizeof(fxw) * 256 + (size_t)lines * (sizeof(fxc) * kXf256Ld + sizeof(FxLine)) +
+         (size_t)kXfx256Teams * kXf256Ld * sizeof(long long);
+}
+
+template <int V = 0>
+__global__ void __launch_bounds__(kXfx256Threads, 2) k_x_pass_fx256(const __grid_constant__ XPassArgs<double> a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ unsigned long long s_vmax[4];
+  __shared__ int s_bad;
+  constexpr int nx = 256, LD = kXf256Ld;
+  const int ny = a.g.ny, kmx = a.g.kx, mx = a.g.mx;
+  const int Y = a.yt, yp = Y / 2, nl = a.nin * yp;
+  fxw* s_tw = reinterpret_cast<fxw*>(smem_raw);
+  double2* s_in = reinterpret_cast<double2*>(s_tw + 256);
+  FxLine* s_line = reinterpret_cast<FxLine*>(s_in + nl * LD);
+  long long* s_ex = reinterpret_cast<long long*>(s_line + nl);
+  const int nyt = (ny + Y - 1) / Y;
+  const int z = blockIdx.x / nyt;
+  const int y0 = (blockIdx.x - z * nyt) * Y;
+  const int yv = min(Y, ny - y0);
+  const int tid = threadIdx.x;
+  s_tw[tid] = a.tw[tid];
+  if (tid < 4) s_vmax[tid] = 0;
+  if (tid == 4) s_bad = 0;
+  {
+    // zeros in the truncated band (sidx of its ends: one contiguous run)
+    const int b0 = sidx(kmx + 1), nb = sidx(nx - kmx - 1) - b0 + 1;
+    for (int L = tid >> 4; L < nl; L += kXfx256Teams)
+      for (int j = tid & 15; j < nb; j += 16) s_in[L * LD + b0 + j] = make_double2(0.0, 0.0);
+  }
+  {
+    // the stored half spectra, two rows per line (x + i y): a thread takes one
+    // kx of a line at a time and issues the loads of a batch before its stores
+    const int total = nl * mx;
+    struct Pair { double2 x, y; };
+    batched<Pair>(
+        total,
+        [&](int e) {
+          const int L = (int)fdiv(e, a.fd_mx), kx = e - L * mx;
+          const int f = (int)fdiv(L, a.fd_yp), c = L - f * yp;
+          const int ya = y0 + 2 * c;
+          const double2* src = a.in + (long long)f * a.in_n + (long long)z * a.in_z + (long long)ya * a.in_y + kx;
+          Pair q;
+          q.x = ya < ny ? src[0] : make_double2(0.0, 0.0);
+          q.y = ya + 1 < ny ? src[a.in_y] : make_double2(0.0, 0.0);
+          return q;
+        },
+        [&](int e, Pair q) {
+          const int L = (int)fdiv(e, a.fd_mx), kx = e - L * mx;
+          if (kx == 0) {  // xy_trans_b.f:28-31 keeps only the real part of kx = 0
+            q.x.y = 0.0;
+            q.y.y = 0.0;
+          }
+          s_in[L * LD + sidx(kx)] = make_double2(q.x.x - q.y.y, q.x.y + q.y.x);
+          if (kx > 0) s_in[L * LD + sidx(nx - kx)] = make_double2(q.x.x + q.y.y, q.y.x - q.x.y);
+        });
+  }
+  __syncthreads();
+
+  // ---- the backward transforms (xy_trans_b.f:39-60), in place
+  const int team = tid >> 4, k = tid & 15;
+  const unsigned tmask = 0xFFFFu << (tid & 16);
+  const fxw* w = s_tw + k;
+  const int rounds = (nl + kXfx256Teams - 1) / kXfx256Teams;
+  for (int r = 0; r < rounds; ++r) {
+    const int L = r * kXfx256Teams + team;
+    const bool active = L < nl;
+    fxc* line = reinterpret_cast<fxc*>(s_in) + (active ? L : 0) * LD;
+    fxc v[16];
+    FxScale sc;
+    float norm;
+    {
+      double2 d[16];
+#pragma unroll
+      for (int q = 0; q < 16; ++q)
+        d[q] = active ? reinterpret_cast<const double2*>(line)[k + 17 * q] : make_double2(0.0, 0.0);
+      sc = fx_begin<16, true>(d, v, 16, &norm);
+    }
+    if (!active) continue;  // (whole teams; the rest is synchronised per team)
+    dft16<+1>(v);
+    // (the first stage read and writes the thread's own column)
+#pragma unroll
+    for (int s = 0; s < 16; ++s) line[17 * s + k] = v[s];
+    __syncwarp(tmask);
+    v[0] = line[17 * k];
+#pragma unroll
+    for (int q = 1; q < 16; ++q) v[q] = ctw<+1>(line[17 * k + q], w[16 * q]);
+    dft16<+1>(v);
+    __syncwarp(tmask);
+#pragma unroll
+    for (int s = 0; s < 16; ++s) reinterpret_cast<FxSplit2*>(line)[k + 17 * s] = fx_split2(v[s]);
+    // 2-norm of the physical line: sqrt(256) times the spectral one
+    if (k == 0) s_line[L] = FxLine{sc.ex, sc.kind, 16.0f * norm, 0};
+    if (a.partials) {
+      // vel_max (vel_max.f:11-21): max |u| of the line's rows and the
+      // non-finite flag; the sums come from wave space (k_parseval)
+      const int f = (int)fdiv(L, a.fd_yp), c = L - f * yp;
+      unsigned long long m = 0;
+#pragma unroll
+      for (int s = 0; s < 16; ++s) {
+        if (2 * c < yv) m = max(m, (unsigned long long)llabs(v[s].x));
+        if (2 * c + 1 < yv) m = max(m, (unsigned long long)llabs(v[s].y));
+      }
+      // (non-negative doubles compare as their bit patterns)
+      const double2 d = fx_out(fxc{(long long)m, 0}, sc);
+      unsigned long long key = (unsigned long long)__double_as_longlong(d.x);
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) key = max(key, __shfl_xor_sync(tmask, key, o));
+      if (k == 0) {
+        if (key >= 0x7ff0000000000000ull) s_bad = 1;
+        else atomicMax(&s_vmax[f], key);
+      }
+    }
+  }
+  __syncthreads();
+  if (a.partials) {
+    // one atomic per field and CTA (order-independent, so deterministic)
+    if (tid < a.g.lu) atomicMax(reinterpret_cast<unsigned long long*>(a.vmax) + tid, s_vmax[tid]);
+    if (tid == 4 && s_bad) atomicOr(a.vmax + 8, 1);
+  }
+
+  // ---- products (rhs.f:46-60), forward transforms, split, scale, store
+  // C(m, z, kx, y) (xy_trans_f.f:20-37)
+  const bool pow2 = is_pow2_inv(ny);
+  const int shift = 1 + 8 + (31 - __clz(ny));  // log2(2 Nx Ny) for a power of two
+  long long* tx = s_ex + team * LD;
+  const int partner = (tid & 16) | ((16 - k) & 15);
+  const int nq = a.g.lr * yp;
+  for (int q = team; q < nq; q += kXfx256Teams) {
+    const int m = (int)fdiv(q, a.fd_yp), c = q - m * yp;
+    int fa, fb;
+    product_pair(m, fa, fb);
+    const FxProduct p = fx_product(s_line[fa * yp + c], s_line[fb * yp + c]);
+    const FxSplit2* pa = reinterpret_cast<const FxSplit2*>(s_in) + (fa * yp + c) * LD + k;
+    const FxSplit2* pb = reinterpret_cast<const FxSplit2*>(s_in) + (fb * yp + c) * LD + k;
+    fxc v[16];
+    if (p.s >= 0) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const FxSplit2 ea = pa[17 * j], eb = pb[17 * j];
+        v[j] = fxc{fx_mul_line<true>(ea.x, eb.x, p), fx_mul_line<true>(ea.y, eb.y, p)};
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const FxSplit2 ea = pa[17 * j], eb = pb[17 * j];
+        v[j] = fxc{fx_mul_line<false>(ea.x, eb.x, p), fx_mul_line<false>(ea.y, eb.y, p)};
+      }
+    }
+    dft16<-1>(v);
+    __syncwarp(tmask);  // the team's reads of its previous line are done
+#pragma unroll
+    for (int s = 0; s < 16; ++s) tx[17 * s + k] = v[s].x;
+    __syncwarp(tmask);
+#pragma unroll
+    for (int s = 0; s < 16; ++s) v[s].x = tx[17 * k + s];
+    __syncwarp(tmask);
+#pragma unroll
+    for (int s = 0; s < 16; ++s) tx[17 * s + k] = v[s].y;
+    __syncwarp(tmask);
+#pragma unroll
+    for (int s = 0; s < 16; ++s) v[s].y = tx[17 * k + s];
+#pragma unroll
+    for (int s = 1; s < 16; ++s) v[s] = ctw<-1>(v[s], w[16 * s]);
+    dft16<-1>(v);
+    FxScale sc = p.sc;
+    if (pow2) sc.ex -= shift;
+    double2* o = a.out + (long long)z * a.out_z + (long long)m * a.out_n + (long long)k * a.out_kx + y0 + 2 * c;
+    const bool two = 2 * c + 1 < yv, one = 2 * c < yv;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      if (16 * j > kmx) break;
+      // Z(Nx - kx) for kx = k + 16 j, from the partner thread
+      const fxc snd = k == 0 ? v[(16 - j) & 15] : v[15 - j];
+      const fxc z2{__shfl_sync(tmask, snd.x, partner), __shfl_sync(tmask, snd.y, partner)};
+      const fxc z1 = v[j];
+      if (k + 16 * j <= kmx && one) {
+        double2 ve = fx_out(fxc{z1.x + z2.x, z1.y - z2.y}, sc);
+        double2 vo = fx_out(fxc{z1.y + z2.y, z2.x - z1.x}, sc);
+        if (!pow2) {
+          ve.x *= a.fn; ve.y *= a.fn;
+          vo.x *= a.fn; vo.y *= a.fn;
+        }
+        double2* oj = o + (long long)(16 * j) * a.out_kx;
+        oj[0] = ve;
+        if (two) oj[1] = vo;
+      }
+    }
+  }
+}
+
+// whether k_x_pass_fx256 runs this launch (else the general kernel)
+__host__ __device__ inline bool x_fx256_applies(const XPassArgs<double>& a) {
+  return a.g.nx == 256 && a.sched == 0 && a.in_mode == 0 && a.out_mode == 2 && a.les == 0 && a.nin == a.g.lu &&
+         a.nin <= 4 && (a.g.lr == 6 || a.g.lr == 9) && (!a.partials || a.max_only) && a.yt >= 2 && a.yt % 2 == 0;
+}
+
 // --------------------------------------------------------------- y forward
 // Tile: field m, kx column i, planes z0 .. z0+TZ-1.  Output D(m, kx, ky, z)
 // keeps |ky| <= ky_max (xy_trans_f.f:45-52).
@@ -1830,6 +2044,12 @@ void launch_x_pass(const XPassArgs<T>& a0, const FftPlan* pl, size_t smem, cudaS
       return;
     }
   }
+  if constexpr (std::is_same<T, double>::value) {
+    if (x_fused_fp64(a)) {
+      k_x_pass_fx256<><<<x_pass_blocks(a), kXfx256Threads, x_fx256_smem(a.nin * (a.yt / 2)), s>>>(a);
+      return;
+    }
+  }
   with_path<T>(a.g.nx, a.sched, [&](auto p) {
     constexpr int PATH = decltype(p)::value;
     k_x_pass<T, PATH><<<x_pass_blocks(a), x_threads(sizeof(T), PATH == kFft256), smem, s>>>(a, pl);
@@ -1869,6 +2089,7 @@ void smem_limits_yinv(int optin) {
 template <typename T>
 void smem_limits_x(int optin) {
   if constexpr (std::is_same<T, float>::value) allow_dynamic_smem((const void*)k_x_pass_f256<>, optin);
+  if constexpr (std::is_same<T, double>::value) allow_dynamic_smem((const void*)k_x_pass_fx256<>, optin);
   each_path<T>([&](auto p) { allow_dynamic_smem((const void*)k_x_pass<T, decltype(p)::value>, optin); });
 }
 template <typename T>

@@ -460,8 +460,9 @@ static int run_x_pass(Ctx& c, int in_mode, int out_mode, int nin, const void* in
     a.partials = c.partials;
     // the FP32 and double-float forms take vel_max's sums from wave space
     // (Parseval, FP64 arithmetic): the x pass then only forms max |u| and
-    // the NaN check
-    a.max_only = (sizeof(T) == 4 || kIsDD<T>) && in_mode == 0 && in == c.S2;
+    // the NaN check (in FP64 in the fused x pass of 256-point lines)
+    a.max_only = in_mode == 0 && in == c.S2;
+    if constexpr (std::is_same<T, double>::value) a.max_only = a.max_only && x_fused_fp64(a);
     a.vmax = reinterpret_cast<int*>(c.pv + 4 * ((size_t)kParsevalBlocks + 1));
   }
   if constexpr (std::is_same<T, float>::value) {
