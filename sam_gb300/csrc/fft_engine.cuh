@@ -440,28 +440,65 @@ __device__ __forceinline__ void fft_stage(C* line, const C* __restrict__ tw, con
 // What becomes of the results of a fixed-point line: element idx, an integer
 // of scale sc.  FxOutLine: doubles back into the line.
 struct FxOutLine {
+  static constexpr bool kNorm = false;
   double2* line;
   __device__ __forceinline__ void operator()(int idx, fxc v, FxScale sc) const { line[sidx(idx)] = fx_out(v, sc); }
 };
 // Doubles into the line, the band lo < idx < hi (which the caller does not
 // read) left out.
 struct FxOutBand {
+  static constexpr bool kNorm = false;
   double2* line;
   int lo, hi;
   __device__ __forceinline__ void operator()(int idx, fxc v, FxScale sc) const {
     if (idx <= lo || idx >= hi) line[sidx(idx)] = fx_out(v, sc);
   }
 };
-// The integers into the line and their scale into *scale: the caller converts
-// what it reads.
+// The integers into the line and their scale into *scale (the caller converts
+// what it reads), or, with no scale given, doubles as FxOutLine.
 struct FxOutInt {
-  fxc* line;
+  static constexpr bool kNorm = false;
+  double2* line;
   FxScale* scale;
   __device__ __forceinline__ void operator()(int idx, fxc v, FxScale sc) const {
-    line[sidx(idx)] = v;
-    if (idx == 0) *scale = sc;
+    if (scale) {
+      reinterpret_cast<fxc*>(line)[sidx(idx)] = v;
+      if (idx == 0) *scale = sc;
+    } else {
+      line[sidx(idx)] = fx_out(v, sc);
+    }
   }
 };
+// Split integers for products and what fx_product needs to know of the line,
+// or, with no info given, doubles.
+struct FxOutSplit {
+  static constexpr bool kNorm = true;
+  double2* line;
+  FxLine* info;
+  __device__ __forceinline__ void operator()(int idx, fxc v, FxScale sc) const {
+    if (info) {
+      reinterpret_cast<FxSplit2*>(line)[sidx(idx)] = fx_split2(v);
+      if (idx == 0) *info = FxLine{sc.ex, sc.kind, sc.norm};
+    } else {
+      line[sidx(idx)] = fx_out(v, sc);
+    }
+  }
+};
+
+// A first-stage loader that gives integers of a known scale (kInts) instead
+// of doubles: a product line of two lines of split integers.
+struct FxProductLoad {
+  static constexpr bool kInts = true;
+  const FxSplit2 *a, *b;
+  FxProduct p;
+  __device__ __forceinline__ fxc operator()(int idx) const {
+    const FxSplit2 ea = a[sidx(idx)], eb = b[sidx(idx)];
+    return fxc{fx_mul_line(ea.x, eb.x, p), fx_mul_line(ea.y, eb.y, p)};
+  }
+  __device__ __forceinline__ FxScale scale() const { return p.sc; }
+};
+template <typename L, typename = void> struct LoadsInts { static constexpr bool value = false; };
+template <typename L> struct LoadsInts<L, std::enable_if_t<L::kInts>> { static constexpr bool value = true; };
 
 // The same stage of an FP64 line in fixed point (fx64.cuh).  The first stage
 // (FIRST, l = 1: no twiddles) reads doubles through load and fixes the line's
@@ -474,7 +511,18 @@ __device__ __forceinline__ void fx_stage(double2* line, const fxw* __restrict__ 
   const int nb = n / P;
   fxc a[MAXB][P];
   int ds[MAXB];  // where the butterfly's outputs start
-  if constexpr (FIRST) {
+  if constexpr (FIRST && LoadsInts<Ld>::value) {
+    sc = load.scale();
+#pragma unroll
+    for (int i = 0; i < MAXB; ++i) {
+      const int b = tl + i * TW;
+      ds[i] = b;
+      if (b < nb) {
+#pragma unroll
+        for (int q = 0; q < P; ++q) a[i][q] = load(b + s.m * q);
+      }
+    }
+  } else if constexpr (FIRST) {
     double2 v[MAXB][P];
 #pragma unroll
     for (int i = 0; i < MAXB; ++i) {
@@ -487,7 +535,7 @@ __device__ __forceinline__ void fx_stage(double2* line, const fxw* __restrict__ 
         for (int q = 0; q < P; ++q) v[i][q] = load(b + s.m * q);
       }
     }
-    sc = fx_begin<MAXB * P>(&v[0][0], &a[0][0], TW);
+    sc = fx_begin<MAXB * P, Out::kNorm>(&v[0][0], &a[0][0], TW, Out::kNorm ? sqrtf((float)n) : 0.f);
   } else {
     const fxc* fl = reinterpret_cast<const fxc*>(line);
 #pragma unroll
@@ -640,16 +688,23 @@ __device__ __forceinline__ void fft256_lines(double2* base, int ld, int nlines, 
     fxc* fl = reinterpret_cast<fxc*>(line);
     fxc a[16];
     FxScale sc;
-    {
+    const auto ld0 = first(active ? L : 0);
+    const auto out = outs(active ? L : 0);
+    if constexpr (LoadsInts<std::decay_t<decltype(ld0)>>::value) {
+      sc = ld0.scale();
+      if (active) {
+#pragma unroll
+        for (int q = 0; q < 16; ++q) a[q] = ld0(k + 16 * q);
+      }
+    } else {
       double2 v[16];
 #pragma unroll
       for (int q = 0; q < 16; ++q) v[q] = make_double2(0.0, 0.0);
       if (active) {
-        const auto ld0 = first(L);
 #pragma unroll
         for (int q = 0; q < 16; ++q) v[q] = ld0(k + 16 * q);
       }
-      sc = fx_begin<16>(v, a, 16);
+      sc = fx_begin<16, decltype(outs(0))::kNorm>(v, a, 16, 16.f);
     }
     dft16<SIGN>(a);
     __syncwarp();
@@ -666,7 +721,6 @@ __device__ __forceinline__ void fft256_lines(double2* base, int ld, int nlines, 
     }
     __syncwarp();
     if (active) {
-      const auto out = outs(L);
 #pragma unroll
       for (int s = 0; s < 16; ++s) out(k + 16 * s, a[s], sc);
     }
@@ -727,7 +781,8 @@ __device__ __forceinline__ void fft_lines_from(C* base, int ld, int nlines,
                                                const typename TwOf<C>::type* __restrict__ tw,
                                                const FftPlan& pl, First first, Out out) {
   if (pl.n == 1 || pl.nst == 0) {
-    for (int L = threadIdx.x; L < nlines; L += blockDim.x) base[L * ld] = first(L)(0);
+    if constexpr (!LoadsInts<std::decay_t<decltype(first(0))>>::value)  // (x lines only: Nx >= 2)
+      for (int L = threadIdx.x; L < nlines; L += blockDim.x) base[L * ld] = first(L)(0);
     return;
   }
   if (PATH == kFft256 || (PATH == kFftAny && pl.tw16_off >= 0)) {

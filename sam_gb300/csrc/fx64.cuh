@@ -214,9 +214,10 @@ template <int SIGN> __device__ __forceinline__ void dft16(fxc* a) {
 
 // ---------------------------------------------------------------- conversions
 // The scale of a line: value = integer * 2^ex.
-struct FxScale {
+struct __align__(16) FxScale {
   int ex;
-  int kind;  // kFxPlain, or one of the exceptional lines
+  int kind;    // kFxPlain, or one of the exceptional lines
+  float norm;  // 2-norm of the transform's integers in units of 2^62 (where asked for)
 };
 constexpr int kFxPlain = 0;  // every result's exponent stays in the normal range
 constexpr int kFxEdge = 1;   // it may not: results go through ldexp
@@ -289,12 +290,13 @@ template <int N> __device__ __forceinline__ float fx_l2(const double2* v, int E)
   return s + t;
 }
 // The N values of each thread of a team to the line's fixed-point integers.
-// With NORM, *norm receives the 2-norm of the line's integers in units of 2^62.
-template <int N, bool NORM = false>
-__device__ __forceinline__ FxScale fx_begin(double2* v, fxc* a, int TW, float* norm = nullptr) {
+// NORM (lines whose transform becomes a product's factor; root_n = sqrt(n)):
+// with the line's 2-norm, and scaled so that the transform's 2-norm, root_n
+// times the line's, does not pass 2^62 either.
+template <int N, bool NORM> __device__ __forceinline__ FxScale fx_begin(double2* v, fxc* a, int TW, float root_n = 0.f) {
   const auto umax = [](uint32_t x, uint32_t y) { return max(x, y); };
   uint32_t hm = team_reduce(fx_max_hi<N>(v), TW, umax);
-  FxScale sc{0, kFxPlain};
+  FxScale sc{0, kFxPlain, 0.f};
   int lift = 0;
   if (hm < ((uint32_t)kFxTiny << 20) && hm > 0) {
     lift = kFxLift;
@@ -309,13 +311,16 @@ __device__ __forceinline__ FxScale fx_begin(double2* v, fxc* a, int TW, float* n
   }
   if (__any_sync(0xffffffffu, lift)) hm = team_reduce(hm, TW, umax);
   const int E = (int)(hm >> 20);
-  const float l1 = team_reduce(fx_l1<N>(v, E), TW, [](float x, float y) { return x + y; });
-  // L1 < 2^(E - 1023 + g) with room for the sum's own rounding
-  int g = (__float_as_int(l1 * 1.0001f) >> 23) - 126;
+  const auto sum = [](float x, float y) { return x + y; };
+  float bound = team_reduce(fx_l1<N>(v, E), TW, sum), l2 = 0.f;
+  if constexpr (NORM) {
+    l2 = root_n * sqrtf(team_reduce(fx_l2<N>(v, E), TW, sum));
+    bound = fmaxf(bound, l2);
+  }
+  // bound < 2^(E - 1023 + g) with room for the sums' own rounding
+  int g = (__float_as_int(bound * 1.0001f) >> 23) - 126;
   if (E == 0) g = 128;  // a line of zeros
-  if constexpr (NORM)
-    *norm = sqrtf(team_reduce(fx_l2<N>(v, E), TW, [](float x, float y) { return x + y; })) *
-            __int_as_float(max(127 - g, 0) << 23);
+  if constexpr (NORM) sc.norm = l2 * __int_as_float(max(127 - g, 0) << 23);
   if (E == 0x7ff) sc.kind = kFxNaN;
   else if (lift || E + g > 2040) sc.kind = kFxEdge;
   sc.ex = E - 1023 - 62 + g - lift;
@@ -355,11 +360,10 @@ template <bool ALU = false> __device__ __forceinline__ double2 fx_out(fxc v, FxS
 }
 
 // A line kept as split integers for products: value = (h 2^32 + l) 2^ex; norm
-// bounds the 2-norm of its integers, in units of 2^62.
-struct FxLine {
+// <= 1 is the 2-norm of its integers, in units of 2^62.
+struct __align__(16) FxLine {
   int ex, kind;
   float norm;
-  int pad;
 };
 struct __align__(16) FxSplit2 {
   FxSplit x, y;
@@ -375,28 +379,63 @@ __device__ __forceinline__ fxc fx_whole(FxSplit2 v) {
 // products shifted down by r = 62 + ceil(log2(norm_a norm_b)) sum to less
 // than 2^62, the bound a transform needs; each is rounded once.
 struct FxProduct {
-  int s;  // 64 - r: the shift left (or, negative, right) of the products' high words
+  int s;  // 64 - r, at least 1 (norms up to 1) and at most 5 (lines scaled by their L1 norms have norms above 1/3)
   long long half;
   FxScale sc;
 };
 __device__ __forceinline__ FxProduct fx_product(const FxLine& a, const FxLine& b) {
-  // (norm_a norm_b >= 1/8 for lines scaled by their L1 norms; zero lines any)
-  const int r = max(62 + ((__float_as_int(a.norm * b.norm * 1.001f) >> 23) - 126), 59);
+  const int r = min(max(62 + ((__float_as_int(a.norm * b.norm * 1.001f) >> 23) - 126), 59), 63);
   FxProduct p;
   p.s = 64 - r;
-  p.half = p.s >= 0 ? 1ll << (31 - p.s) : 1ll << (-p.s - 1);
+  p.half = 1ll << (31 - p.s);
   p.sc.ex = a.ex + b.ex + r;
+  p.sc.norm = 0.f;
   // (room for the exponents of a scaling by 1 / (Nx Ny))
   p.sc.kind = (a.kind | b.kind) & kFxNaN ? kFxNaN : (p.sc.ex < -960 || p.sc.ex > 940 ? kFxEdge : kFxPlain);
   return p;
 }
-template <bool LEFT> __device__ __forceinline__ long long fx_mul_line(FxSplit a, FxSplit b, const FxProduct& p) {
-  const long long c = fx_mad(a.l, b.h, fx_mad(a.h, b.l, LEFT ? p.half : 0ll));
+__device__ __forceinline__ long long fx_mul_line(FxSplit a, FxSplit b, const FxProduct& p) {
+  const long long c = fx_mad(a.l, b.h, fx_mad(a.h, b.l, p.half));
   const long long A = fx_mad(a.h, b.h, c >> 32);
-  if (!LEFT) return (A + p.half) >> -p.s;
   const uint32_t lo = __funnelshift_l((uint32_t)c, (uint32_t)A, p.s);
   const uint32_t hi = __funnelshift_l((uint32_t)A, (uint32_t)(A >> 32), p.s);
   return (long long)(((uint64_t)hi << 32) | lo);
+}
+// Physical values of a line of n points (elements sidx(0) .. sidx(n - 1)) to
+// split integers below 2^62, by one warp.
+__host__ __device__ __forceinline__ int sidx(int p);
+__device__ __forceinline__ void fx_line_in_place(double2* line, FxLine* info, int n) {
+  const int lane = threadIdx.x & 31;
+  uint32_t hm = 0;
+  for (int x = lane; x < n; x += 32) hm = max(hm, fx_max_hi<1>(line + sidx(x)));
+  hm = __reduce_max_sync(0xffffffffu, hm);
+  const bool lift = hm < ((uint32_t)kFxTiny << 20) && hm > 0;
+  const double f = lift ? __hiloint2double((1023 + kFxLift) << 20, 0) : 1.0;
+  if (lift) {
+    hm = 0;
+    for (int x = lane; x < n; x += 32) {
+      double2 v = line[sidx(x)];
+      v.x *= f;
+      v.y *= f;
+      line[sidx(x)] = v;
+      hm = max(hm, fx_max_hi<1>(&v));
+    }
+    hm = __reduce_max_sync(0xffffffffu, hm);
+  }
+  const int E = (int)(hm >> 20);
+  float l2 = 0.f;
+  for (int x = lane; x < n; x += 32) l2 += fx_l2<1>(line + sidx(x), E);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) l2 += __shfl_xor_sync(0xffffffffu, l2, o);
+  l2 = sqrtf(l2);
+  const int g = E ? (__float_as_int(l2 * 1.0001f) >> 23) - 126 : 128;
+  for (int x = lane; x < n; x += 32) {
+    const double2 v = line[sidx(x)];
+    reinterpret_cast<FxSplit2*>(line)[sidx(x)] = fx_split2(fxc{fx_from(v.x, E + g), fx_from(v.y, E + g)});
+  }
+  if (lane == 0)
+    *info = FxLine{E - 1023 - 62 + g - (lift ? kFxLift : 0), E == 0x7ff ? kFxNaN : kFxPlain,
+                   l2 * __int_as_float(max(127 - g, 0) << 23)};
 }
 
 }  // namespace samgpu

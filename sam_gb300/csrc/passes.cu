@@ -46,10 +46,6 @@ void launch_x2z(const double2* in, double2* out, const Grid& g, int nvar, int nx
   if (grid < 1) grid = 1;
   k_x2z<<<grid, kThreads, 0, s>>>(in, out, g, nvar, nx2);
 }
-bool x_fused_fp64(const XPassArgs<double>& a) {
-  return x_fx256_applies(a) && x_fx256_smem(a.nin * (a.yt / 2)) <= (size_t)smem_optin() - 1024;
-}
-
 SAMGPU_INST(double)
 
 }  // namespace samgpu

@@ -60,6 +60,7 @@ struct XPassArgs {
   // group: product lines transformed per round of out_mode 2 (a multiple of
   // the CTA's teams where it exceeds them), any split of the Lr * Y/2 lines
   int in_mode, out_mode, nin, yt, group, ld;
+  int prod_lines;  // lines of room behind the input lines (products, vel_max's scratch)
   // vel_max partials: max_only = 1 leaves the sums to k_parseval (FP32 form)
   int max_only;
   int* vmax;  // max_only: per-field max |u| (float bit patterns) and the NaN flag, atomically
@@ -111,6 +112,8 @@ struct YFwdArgs {
 template <typename W> struct EpiRow {
   W rky, k_sq, ef, et;
 };
+// (these records follow the 16-byte elements of the lines)
+static_assert(sizeof(FxScale) == 16 && sizeof(FxLine) == 16, "records keep the alignment of what follows them");
 // Shared memory behind the lines of a z-forward tile of ty rows and nf
 // fields (modes 1, 2): the scale of each fixed-point line, the rows' constants.
 template <typename T> constexpr size_t z_fwd_extra(int mode, int nf, int ty) {
@@ -155,9 +158,11 @@ template <typename T> void launch_z_inv(const ZInvArgs<T>& a, const FftPlan* pl,
 template <typename T> void launch_y_inv(const YInvArgs<T>& a, const FftPlan* pl, size_t smem, cudaStream_t s);
 template <typename T> void launch_x_pass(const XPassArgs<T>& a, const FftPlan* pl, size_t smem, cudaStream_t s);
 template <typename T> int x_pass_blocks(const XPassArgs<T>& a);
-// whether the FP64 x pass of these arguments (max_only given) runs the fused
-// 256-point kernel, which forms vel_max's maxima only
-bool x_fused_fp64(const XPassArgs<double>& a);
+// Shared memory of an FP64 x pass with products behind its lines: scale and
+// norm of each of `in` input lines, scale of each of `prod` product lines.
+template <typename T> constexpr size_t x_extra(int out_mode, int in, int prod) {
+  return std::is_same<T, double>::value && out_mode == 2 ? sizeof(FxLine) * in + sizeof(FxScale) * prod : 0;
+}
 template <typename T> void launch_y_fwd(const YFwdArgs<T>& a, const FftPlan* pl, size_t smem, cudaStream_t s);
 template <typename T> void launch_z_fwd(const ZFwdArgs<T>& a, const FftPlan* pl, size_t smem, cudaStream_t s);
 template <typename T> void smem_limits_zinv(int optin);

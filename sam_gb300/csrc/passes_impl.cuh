@@ -503,6 +503,13 @@ __device__ __forceinline__ void x_pass_body(const XPassArgs<T>& a, const FftPlan
   const int Y = a.yt, yp = Y / 2, ld = a.ld;
   const int nin = a.nin;
   C* s_pr = s_in + nin * yp * ld;                // group product lines
+  // FP64 form with products and no subgrid terms: the physical lines are
+  // split integers (ints), their scales and norms behind the lines; the
+  // results of a product line stay integers until they are stored
+  constexpr bool FX = kIsFx<C, PATH>;
+  const bool ints = FX && a.out_mode == 2 && !a.les;
+  FxLine* s_line = reinterpret_cast<FxLine*>(s_pr + (size_t)a.prod_lines * ld);
+  FxScale* s_psc = reinterpret_cast<FxScale*>(s_line + nin * yp);
   // vel_max's reduction scratch shares the product lines' space (it is done
   // before the first product is formed)
   double* s_red = reinterpret_cast<double*>(s_pr);
@@ -588,8 +595,14 @@ __device__ __forceinline__ void x_pass_body(const XPassArgs<T>& a, const FftPlan
           });
     }
     __syncthreads();
-    fft_lines_from<+1, PATH>(s_in, ld, nin * yp, s_tw, pl,
-                       [&](int L) { return BandLoad<C>{s_in + L * ld, kmx, nx - kmx}; });
+    const auto rows = [&](int L) { return BandLoad<C>{s_in + L * ld, kmx, nx - kmx}; };
+    if constexpr (FX) {
+      fft_lines_from<+1, PATH>(s_in, ld, nin * yp, s_tw, pl, rows, [&](int L) {
+        return FxOutSplit{s_in + L * ld, ints ? s_line + L : nullptr};
+      });
+    } else {
+      fft_lines_from<+1, PATH>(s_in, ld, nin * yp, s_tw, pl, rows);
+    }
   } else {
     // physical rows of P(n, z, y, x)
     struct Pair { T x, y; };
@@ -664,6 +677,49 @@ __device__ __forceinline__ void x_pass_body(const XPassArgs<T>& a, const FftPlan
         atomicMax(reinterpret_cast<unsigned long long*>(a.vmax) + f, tm);
         if (f == 0 && tb) atomicOr(a.vmax + 8, 1);
       }
+      __syncthreads();
+    }
+  } else if (std::is_same<T, double>::value && a.partials && a.max_only) {
+    // the FP64 step: max |u| of each line by one warp, as integers where the
+    // line holds them, else as the bit patterns of non-negative doubles, which
+    // compare alike; the sums come from wave space (k_parseval)
+    if constexpr (std::is_same<T, double>::value) {
+      unsigned long long* s_km = reinterpret_cast<unsigned long long*>(s_red);
+      const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+      if (threadIdx.x < 5) s_km[threadIdx.x] = 0ull;
+      __syncthreads();
+      for (int L = w; L < a.g.lu * yp; L += nw) {
+        const int f = (int)fdiv(L, a.fd_yp), c = L - f * yp;
+        const bool ra = y0 + 2 * c < ny, rb = y0 + 2 * c + 1 < ny;
+        unsigned long long m = 0ull;
+        for (int x = lane; x < nx; x += 32) {
+          const C v = s_in[L * ld + sidx(x)];
+          unsigned long long ma, mb;
+          if (ints) {
+            const fxc q = fx_whole(*reinterpret_cast<const FxSplit2*>(&v));
+            ma = (unsigned long long)llabs(q.x);
+            mb = (unsigned long long)llabs(q.y);
+          } else {
+            ma = (unsigned long long)__double_as_longlong(v.x) & 0x7fffffffffffffffull;
+            mb = (unsigned long long)__double_as_longlong(v.y) & 0x7fffffffffffffffull;
+          }
+          if (ra) m = max(m, ma);
+          if (rb) m = max(m, mb);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (lane == 0) {
+          if (ints)
+            m = (unsigned long long)__double_as_longlong(
+                fx_out(fxc{(long long)m, 0}, FxScale{s_line[L].ex, s_line[L].kind, 0.f}).x);
+          if (m >= 0x7ff0000000000000ull) s_km[4] = 1ull;
+          else atomicMax(s_km + f, m);
+        }
+      }
+      __syncthreads();
+      // one atomic per field and CTA (order-independent, so deterministic)
+      if (threadIdx.x < a.g.lu) atomicMax(reinterpret_cast<unsigned long long*>(a.vmax) + threadIdx.x, s_km[threadIdx.x]);
+      if (threadIdx.x == 4 && s_km[4]) atomicOr(a.vmax + 8, 1);
       __syncthreads();
     }
   } else if (a.partials && a.max_only) {
@@ -867,6 +923,12 @@ __device__ __forceinline__ void x_pass_body(const XPassArgs<T>& a, const FftPlan
 
   // ---- outputs
   if (a.out_mode == 3) return;  // statistics only (vel_max.f)
+  if constexpr (FX) {
+    if (ints && a.in_mode != 0) {
+      for (int L = threadIdx.x >> 5; L < nin * yp; L += blockDim.x >> 5) fx_line_in_place(s_in + L * ld, s_line + L, nx);
+      __syncthreads();
+    }
+  }
   if (a.out_mode == 0) {
     // physical rows (xy_trans_b.f:57-59)
     for (int e = threadIdx.x; e < nin * Y * nx; e += blockDim.x) {
@@ -892,15 +954,38 @@ __device__ __forceinline__ void x_pass_body(const XPassArgs<T>& a, const FftPlan
     // out_mode 2 (rhs.f:46-60): the products of the physical lines, formed
     // while the first FFT stage loads them, straight into the product lines
     C* lines = a.out_mode == 1 ? s_in : s_pr;
-    fft_lines_from<-1, PATH>(lines, ld, gl, s_tw, pl, [&](int L) {
-      if (a.out_mode == 1) return ProductLoad<C>{lines + L * ld, nullptr, nullptr};
+    const auto lines_of = [&](int L, int& fa, int& fb) {
       const int q = l0 + L;
       const int m = (int)fdiv(q, a.fd_yp), c = q - m * yp;
-      int fa, fb;
       product_pair(m, fa, fb);
-      const C* gl_ = a.les ? s_in + ((a.g.lu + m) * yp + c) * ld : nullptr;
-      return ProductLoad<C>{s_in + (fa * yp + c) * ld, s_in + (fb * yp + c) * ld, gl_};
-    });
+      fa = fa * yp + c;
+      fb = fb * yp + c;
+      return (a.g.lu + m) * yp + c;  // the line of the product's subgrid term
+    };
+    const auto from_values = [&](int L) {
+      if (a.out_mode == 1) return ProductLoad<C>{lines + L * ld, nullptr, nullptr};
+      int fa, fb;
+      const int fg = lines_of(L, fa, fb);
+      return ProductLoad<C>{s_in + fa * ld, s_in + fb * ld, a.les ? s_in + fg * ld : nullptr};
+    };
+    if constexpr (FX) {
+      if (ints) {
+        const auto from_ints = [&](int L) {
+          int fa, fb;
+          lines_of(L, fa, fb);
+          return FxProductLoad{reinterpret_cast<const FxSplit2*>(s_in + fa * ld),
+                               reinterpret_cast<const FxSplit2*>(s_in + fb * ld), fx_product(s_line[fa], s_line[fb])};
+        };
+        fft_lines_from<-1, PATH>(lines, ld, gl, s_tw, pl, from_ints,
+                                 [&](int L) { return FxOutInt{lines + L * ld, s_psc + L}; });
+      } else {
+        fft_lines_from<-1, PATH>(lines, ld, gl, s_tw, pl, from_values, [&](int L) {
+          return FxOutInt{lines + L * ld, a.out_mode == 2 ? s_psc + L : nullptr};
+        });
+      }
+    } else {
+      fft_lines_from<-1, PATH>(lines, ld, gl, s_tw, pl, from_values);
+    }
     __syncthreads();
     // split the two real transforms, keep kx <= kx_max, scale, store
     // C(m, z, kx, y): a thread keeps one line (the rows y0+2c, y0+2c+1 of
@@ -918,11 +1003,35 @@ __device__ __forceinline__ void x_pass_body(const XPassArgs<T>& a, const FftPlan
           const C* ln = lines + L * ld;
           C* o = a.out + (long long)z * a.out_z + y0 + (long long)m * a.out_n + (long long)lane * a.out_kx + 2 * c;
           const bool two = 2 * c + 1 < yv, one = 2 * c < yv;
+          FxScale sc{};
+          if constexpr (FX)
+            if (a.out_mode == 2) {
+              sc = s_psc[L];
+              if (fn_pow2) sc.ex -= 1 + (31 - __clz(nx)) + (31 - __clz(ny));
+            }
           for (int kx = lane; kx < mx; kx += lanes, o += ostep) {
             const C z1 = ln[sidx(kx)];
             const C z2 = ln[sidx(kx == 0 ? 0 : nx - kx)];
-            const C ve = mk<C>(scale_by(z1.x + z2.x, fn, fn_pow2), scale_by(z1.y - z2.y, fn, fn_pow2));
-            const C vo = mk<C>(scale_by(z1.y + z2.y, fn, fn_pow2), scale_by(z2.x - z1.x, fn, fn_pow2));
+            C ve, vo;
+            bool done = false;
+            if constexpr (FX) {
+              if (a.out_mode == 2) {
+                // the split in integers; 1/(2 Nx Ny) in the exponent where it
+                // is a power of two
+                const fxc i1 = *reinterpret_cast<const fxc*>(&z1), i2 = *reinterpret_cast<const fxc*>(&z2);
+                ve = fx_out(fxc{i1.x + i2.x, i1.y - i2.y}, sc);
+                vo = fx_out(fxc{i1.y + i2.y, i2.x - i1.x}, sc);
+                if (!fn_pow2) {
+                  ve.x *= fn; ve.y *= fn;
+                  vo.x *= fn; vo.y *= fn;
+                }
+                done = true;
+              }
+            }
+            if (!done) {
+              ve = mk<C>(scale_by(z1.x + z2.x, fn, fn_pow2), scale_by(z1.y - z2.y, fn, fn_pow2));
+              vo = mk<C>(scale_by(z1.y + z2.y, fn, fn_pow2), scale_by(z2.x - z1.x, fn, fn_pow2));
+            }
             if (two) {
               if ((reinterpret_cast<uintptr_t>(o) & (2 * sizeof(C) - 1)) == 0) {
                 store_pair(o, ve, vo);
@@ -1270,13 +1379,12 @@ __global__ void __launch_bounds__(kXfx256Threads, 2) k_x_pass_fx256(const __grid
     fxc* line = reinterpret_cast<fxc*>(s_in) + (active ? L : 0) * LD;
     fxc v[16];
     FxScale sc;
-    float norm;
     {
       double2 d[16];
 #pragma unroll
       for (int q = 0; q < 16; ++q)
         d[q] = active ? reinterpret_cast<const double2*>(line)[k + 17 * q] : make_double2(0.0, 0.0);
-      sc = fx_begin<16, true>(d, v, 16, &norm);
+      sc = fx_begin<16, true>(d, v, 16, 16.f);
     }
     if (!active) continue;  // (whole teams; the rest is synchronised per team)
     dft16<+1>(v);
@@ -1291,8 +1399,7 @@ __global__ void __launch_bounds__(kXfx256Threads, 2) k_x_pass_fx256(const __grid
     __syncwarp(tmask);
 #pragma unroll
     for (int s = 0; s < 16; ++s) reinterpret_cast<FxSplit2*>(line)[k + 17 * s] = fx_split2(v[s]);
-    // 2-norm of the physical line: sqrt(256) times the spectral one
-    if (k == 0) s_line[L] = FxLine{sc.ex, sc.kind, 16.0f * norm, 0};
+    if (k == 0) s_line[L] = FxLine{sc.ex, sc.kind, sc.norm};
     if (a.partials) {
       // vel_max (vel_max.f:11-21): max |u| of the line's rows and the
       // non-finite flag; the sums come from wave space (k_parseval)
@@ -1336,18 +1443,10 @@ __global__ void __launch_bounds__(kXfx256Threads, 2) k_x_pass_fx256(const __grid
     const FxSplit2* pa = reinterpret_cast<const FxSplit2*>(s_in) + (fa * yp + c) * LD + k;
     const FxSplit2* pb = reinterpret_cast<const FxSplit2*>(s_in) + (fb * yp + c) * LD + k;
     fxc v[16];
-    if (p.s >= 0) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const FxSplit2 ea = pa[17 * j], eb = pb[17 * j];
-        v[j] = fxc{fx_mul_line<true>(ea.x, eb.x, p), fx_mul_line<true>(ea.y, eb.y, p)};
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const FxSplit2 ea = pa[17 * j], eb = pb[17 * j];
-        v[j] = fxc{fx_mul_line<false>(ea.x, eb.x, p), fx_mul_line<false>(ea.y, eb.y, p)};
-      }
+    for (int j = 0; j < 16; ++j) {
+      const FxSplit2 ea = pa[17 * j], eb = pb[17 * j];
+      v[j] = fxc{fx_mul_line(ea.x, eb.x, p), fx_mul_line(ea.y, eb.y, p)};
     }
     dft16<-1>(v);
     __syncwarp(tmask);  // the team's reads of its previous line are done
@@ -1672,7 +1771,7 @@ __device__ __forceinline__ void z_fwd_body(const ZFwdArgs<T>& a, const FftPlan* 
   if constexpr (FX) {
     if (ints)
       fft_lines_from<-1, PATH>(s_ln, ld, nf * nl, s_tw, pl, rows, [&](int L) {
-        return FxOutInt{reinterpret_cast<fxc*>(s_ln + L * ld), s_sc + L};
+        return FxOutInt{s_ln + L * ld, s_sc + L};
       });
   }
   if (!ints) fft_lines_from<-1, PATH>(s_ln, ld, nf * nl, s_tw, pl, rows);
@@ -2045,8 +2144,9 @@ void launch_x_pass(const XPassArgs<T>& a0, const FftPlan* pl, size_t smem, cudaS
     }
   }
   if constexpr (std::is_same<T, double>::value) {
-    if (x_fused_fp64(a)) {
-      k_x_pass_fx256<><<<x_pass_blocks(a), kXfx256Threads, x_fx256_smem(a.nin * (a.yt / 2)), s>>>(a);
+    const size_t fsm = x_fx256_smem(a.nin * (a.yt / 2));
+    if (x_fx256_applies(a) && fsm <= (size_t)smem_optin() - 1024) {
+      k_x_pass_fx256<><<<x_pass_blocks(a), kXfx256Threads, fsm, s>>>(a);
       return;
     }
   }

@@ -380,6 +380,7 @@ static int x_red_lines(const Ctx& c) {
 template <typename T>
 static int x_tile(Ctx& c, int nin, int out_mode, int& yt, int& grp) {
   const size_t es = sizeof(cx_t<T>);
+  const size_t prod_extra = x_extra<T>(out_mode, 0, 1);
   const int threads = x_threads((int)sizeof(T), x_reg16(c));
   const int team = x_reg16(c) ? 16 : (sizeof(T) == 4 ? c.px.h.team_sp : c.px.h.team);
   const int teams = threads / team > 0 ? threads / team : 1;
@@ -392,12 +393,12 @@ static int x_tile(Ctx& c, int nin, int out_mode, int& yt, int& grp) {
   const size_t rmin = line * (size_t)x_red_lines<T>(c);
   for (yt = c.yt_x;; yt /= 2) {
     const int yp = yt / 2;
-    const size_t base = tile_smem(c.px, nin * yp, es, c.sched[2]);
+    const size_t base = tile_smem(c.px, nin * yp, es, c.sched[2]) + x_extra<T>(out_mode, nin * yp, 0);
     if (out_mode != 2) {
       grp = 0;
       if (base + rmin <= budget) return 0;
     } else if (base + rmin <= budget) {
-      const int fit = (int)((budget - base) / line);
+      const int fit = (int)((budget - base) / (line + prod_extra));
       const int total = c.g.lr * yp;
       grp = std::min(std::min(fit, std::max(c.grp_x, 1) * yp), total);
       if (grp > teams && grp < total) grp -= grp % teams;
@@ -408,8 +409,9 @@ static int x_tile(Ctx& c, int nin, int out_mode, int& yt, int& grp) {
 }
 
 template <typename T>
-static size_t x_smem(Ctx& c, int nin, int yt, int grp) {
-  return tile_smem(c.px, nin * (yt / 2) + std::max(grp, x_red_lines<T>(c)), sizeof(cx_t<T>), c.sched[2]);
+static size_t x_smem(Ctx& c, const XPassArgs<T>& a) {
+  return tile_smem(c.px, a.nin * (a.yt / 2) + a.prod_lines, sizeof(cx_t<T>), c.sched[2]) +
+         x_extra<T>(a.out_mode, a.nin * (a.yt / 2), a.prod_lines);
 }
 
 template <typename T>
@@ -444,6 +446,7 @@ static int run_x_pass(Ctx& c, int in_mode, int out_mode, int nin, const void* in
   a.sched = c.sched[2];
   int rc = x_tile<T>(c, nin, out_mode, a.yt, a.group);
   if (rc) return rc;
+  a.prod_lines = std::max(a.group, x_red_lines<T>(c));
   a.ld = line_ld(c.g.nx);
   a.in_y = in_y; a.in_z = in_z; a.in_n = in_n;
   a.out_kx = out_kx; a.out_z = out_z; a.out_n = out_n;
@@ -458,11 +461,9 @@ static int run_x_pass(Ctx& c, int in_mode, int out_mode, int nin, const void* in
       c.partial_blocks = nblk;
     }
     a.partials = c.partials;
-    // the FP32 and double-float forms take vel_max's sums from wave space
-    // (Parseval, FP64 arithmetic): the x pass then only forms max |u| and
-    // the NaN check (in FP64 in the fused x pass of 256-point lines)
+    // the resident step takes vel_max's sums from wave space (Parseval): the
+    // x pass then only forms max |u| and the NaN check
     a.max_only = in_mode == 0 && in == c.S2;
-    if constexpr (std::is_same<T, double>::value) a.max_only = a.max_only && x_fused_fp64(a);
     a.vmax = reinterpret_cast<int*>(c.pv + 4 * ((size_t)kParsevalBlocks + 1));
   }
   if constexpr (std::is_same<T, float>::value) {
@@ -471,11 +472,11 @@ static int run_x_pass(Ctx& c, int in_mode, int out_mode, int nin, const void* in
       EnsFinishArgs fa{c.partials, nblk, c.g, c.state, c.cfg.i_cfl, c.cfg.cfl0, c.adv_cfl_limit, c.pv,
                        kParsevalBlocks, a.vmax};
       if (stats && !a.max_only) return fail(SAM_GPU_EUNSUPPORTED, "ensemble stage: FP64 vel_max partials");
-      ens_record_x_pass(*c.rec, a, c.px.d, x_smem<T>(c, nin, a.yt, a.group), stats, &pa, &fa);
+      ens_record_x_pass(*c.rec, a, c.px.d, x_smem<T>(c, a), stats, &pa, &fa);
       return 0;
     }
   }
-  launch_x_pass<T>(a, c.px.d, x_smem<T>(c, nin, a.yt, a.group), c.stream);
+  launch_x_pass<T>(a, c.px.d, x_smem<T>(c, a), c.stream);
   if (stats) {
     if (a.max_only) launch_parseval<T>((const cx_t<T>*)c.U, c.g, c.pv, c.stream);
     launch_vel_max_finish(c.partials, nblk, c.g, c.state, c.cfg.i_cfl, c.cfg.cfl0, c.adv_cfl_limit, c.stream,
