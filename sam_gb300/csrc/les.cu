@@ -40,9 +40,9 @@ struct Halo {
   __device__ __forceinline__ long long ninterior() const { return (long long)nx * ny * nz; }
 };
 
-__constant__ int c_ifact[6] = {1, 1, 1, 2, 2, 2};
-__constant__ int c_ip[6] = {0, 1, 2, 0, 1, 0};
-__constant__ int c_jp[6] = {0, 1, 2, 1, 2, 2};
+// index pairs of the tensor's six components, ifact = (1,1,1,2,2,2)
+__device__ constexpr int kIp[6] = {0, 1, 2, 0, 1, 0};
+__device__ constexpr int kJp[6] = {0, 1, 2, 1, 2, 2};
 
 // ---- filter.f:7-42 on one 2-D plane set: 1-4-1 across the three planes of
 // f_bar(Lx,Ly,n_var,3) (halos included), 1-4-1 along y using those halo rows,
@@ -93,9 +93,9 @@ __device__ __forceinline__ void strain(const double* __restrict__ ub, const Halo
 }
 
 __device__ __forceinline__ double smag(const double* s) {
-  double sum = 0.0;
-  for (int q = 0; q < 6; ++q) sum += c_ifact[q] * s[q] * s[q];
-  return sqrt(2.0 * sum);
+  const double d = s[0] * s[0] + s[1] * s[1] + s[2] * s[2];
+  const double o = s[3] * s[3] + s[4] * s[4] + s[5] * s[5];
+  return sqrt(2.0 * (d + 2.0 * o));
 }
 
 // sm.f:77-86: vt = c_smag delta^2 |S| on the interior of the haloed output
@@ -126,52 +126,99 @@ __global__ void k_periodic3(double* __restrict__ f, Halo H) {
 }
 
 // dm.f:99-116: |S|, |S| S_ij and u_bar_i u_bar_j on the interior
-//   q[0..5] = S, q[6..11] = |S| S, q[12..17] = ub_i ub_j, q[18] = |S|
+//   q[0..5] = S, q[6..11] = |S| S, q[12..17] = ub_i ub_j, q[18] = |S| (with vt)
 __global__ void k_dm_fields(const double* __restrict__ ub, double* __restrict__ q, Halo H, double dxi, double dyi,
-                            double dzi) {
+                            double dzi, int with_smag) {
   const long long n = H.ninterior();
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
     const int x = (int)(e % H.nx), y = (int)((e / H.nx) % H.ny), z = (int)(e / ((long long)H.nx * H.ny));
     double s[6];
     strain(ub, H, x, y, z, dxi, dyi, dzi, s);
     const double sm = smag(s);
+    const double u[3] = {ub[e], ub[n + e], ub[2 * n + e]};
+#pragma unroll
     for (int c = 0; c < 6; ++c) {
       q[c * n + e] = s[c];
       q[(6 + c) * n + e] = sm * s[c];
-      q[(12 + c) * n + e] = ub[c_ip[c] * n + e] * ub[c_jp[c] * n + e];
+      q[(12 + c) * n + e] = u[kIp[c]] * u[kJp[c]];
     }
-    q[18 * n + e] = sm;
+    if (with_smag) q[18 * n + e] = sm;
   }
 }
 
-// separable 1-4-1 test filter of one periodic interior field at (x, y, z),
-// summed in filter.f's order: across planes, then along y, then along x
-__device__ __forceinline__ double tfilter(const double* __restrict__ f, const Halo& H, int x, int y, int z) {
-  auto h = [&](int a, int b) {
-    return f[H.in(x + a, y + b, z - 1)] + 4 * f[H.in(x + a, y + b, z)] + f[H.in(x + a, y + b, z + 1)];
-  };
-  auto g = [&](int a) { return h(a, -1) + 4 * h(a, 0) + h(a, 1); };
-  return (1.0 / 216.0) * (g(-1) + 4 * g(0) + g(1));
+// dm.f:122-150: L_ij, M_ij at each interior point, per-CTA sums of
+// ifact L M and ifact M M (fixed order, deterministic).  Bound by the FP64
+// pipe, so the 1-4-1 test filter is taken one direction at a time (across
+// planes, along y, along x: filter.f's order): a CTA does a 32 x 8 tile of
+// one plane, each of the 21 fields in turn through two shared tiles, 2 FP64
+// operations a point and direction (7 a point and field with the tile's halo
+// rows against 27 for the stencil in one step; the dynamic coefficient at
+// 256^3 24 -> 8 ms, with the integer factors no longer converted to FP64 per
+// point).
+constexpr int kDmTx = 32, kDmTy = 8;
+static_assert(kDmTx * kDmTy == kThreads, "one point per thread");
+static long long dm_tiles(int nx, int ny, int nz) {
+  return (long long)((nx + kDmTx - 1) / kDmTx) * ((ny + kDmTy - 1) / kDmTy) * nz;
 }
 
-// dm.f:122-150: L_ij, M_ij at each interior point, per-CTA sums of
-// ifact L M and ifact M M (fixed-order tree, deterministic)
-__global__ void k_dm_lm(const double* __restrict__ ub, const double* __restrict__ q, Halo H, double alpha_sq,
-                        double* __restrict__ part) {
+__global__ void __launch_bounds__(kThreads, 3)
+    k_dm_lm(const double* __restrict__ ub, const double* __restrict__ q, Halo H, double alpha_sq,
+            double* __restrict__ part) {
+  constexpr int HX = kDmTx + 2, HY = kDmTy + 2;
+  __shared__ double s_h[2][HY * HX], s_g[2][kDmTy * HX];
   __shared__ double red[2][kThreads];
   const long long n = H.ninterior();
+  const int tid = threadIdx.x, tx = tid & (kDmTx - 1), ty = tid / kDmTx;
+  const int ntx = (H.nx + kDmTx - 1) / kDmTx, nty = (H.ny + kDmTy - 1) / kDmTy;
+  const long long tiles = (long long)ntx * nty * H.nz;
+  const double inv = 1.0 / 216.0;
   double num = 0.0, den = 0.0;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-    const int x = (int)(e % H.nx), y = (int)((e / H.nx) % H.ny), z = (int)(e / ((long long)H.nx * H.ny));
+  for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
+    const int z = (int)(t / (ntx * nty)), r = (int)(t - (long long)z * (ntx * nty));
+    const int x0 = (r % ntx) * kDmTx, y0 = (r / ntx) * kDmTy;
+    // this thread's points of the tile with halo (at most two), the planes' offsets
+    long long off[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int e = min(tid + i * kThreads, HY * HX - 1);
+      const int xx = (x0 + e % HX - 1 + H.nx) % H.nx, yy = (y0 + e / HX - 1 + H.ny) % H.ny;
+      off[i] = (long long)yy * H.nx + xx;
+    }
+    const long long pl = (long long)H.nx * H.ny;
+    const long long zm = H.wz(z - 1) * pl, zc = z * pl, zp = H.wz(z + 1) * pl;
+    int buf = 0;
+    auto filt = [&](const double* __restrict__ f) {  // 216 times the filtered field at this thread's point
+      double* h = s_h[buf];
+      double* g = s_g[buf];
+      buf ^= 1;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int e = tid + i * kThreads;
+        if (e < HY * HX) h[e] = f[zm + off[i]] + 4 * f[zc + off[i]] + f[zp + off[i]];
+      }
+      __syncthreads();
+      for (int e = tid; e < kDmTy * HX; e += kThreads) g[e] = h[e] + 4 * h[e + HX] + h[e + 2 * HX];
+      __syncthreads();
+      const double* gp = g + ty * HX + tx;
+      return gp[0] + 4 * gp[1] + gp[2];
+    };
     double uh[3], sh[6];
-    for (int c = 0; c < 3; ++c) uh[c] = tfilter(ub + c * n, H, x, y, z);
-    for (int c = 0; c < 6; ++c) sh[c] = tfilter(q + c * n, H, x, y, z);
-    const double smh = smag(sh);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) uh[c] = inv * filt(ub + c * n);
+#pragma unroll
+    for (int c = 0; c < 6; ++c) sh[c] = inv * filt(q + c * n);
+    const double w = alpha_sq * smag(sh);
+    double n2[2] = {0.0, 0.0}, d2[2] = {0.0, 0.0};
+#pragma unroll
     for (int c = 0; c < 6; ++c) {
-      const double M = -tfilter(q + (6 + c) * n, H, x, y, z) + alpha_sq * smh * sh[c];
-      const double L = tfilter(q + (12 + c) * n, H, x, y, z) - uh[c_ip[c]] * uh[c_jp[c]];
-      num += c_ifact[c] * L * M;
-      den += c_ifact[c] * M * M;
+      const double M = w * sh[c] - inv * filt(q + (6 + c) * n);
+      const double L = inv * filt(q + (12 + c) * n) - uh[kIp[c]] * uh[kJp[c]];
+      n2[c / 3] += L * M;
+      d2[c / 3] += M * M;
+    }
+    if (x0 + tx < H.nx && y0 + ty < H.ny) {
+      num += n2[0] + 2 * n2[1];
+      den += d2[0] + 2 * d2[1];
     }
   }
   red[0][threadIdx.x] = num;
@@ -190,15 +237,30 @@ __global__ void k_dm_lm(const double* __restrict__ ub, const double* __restrict_
   }
 }
 
-// dm.f:176 and 183-189: c_delta_sq = -num / (2 den); vt = c_delta_sq |S|
-__global__ void k_dm_finish(const double* __restrict__ part, int nblk, double* __restrict__ cds) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double num = 0.0, den = 0.0;
-    for (int b = 0; b < nblk; ++b) {
-      num += part[2 * b];
-      den += part[2 * b + 1];
+// dm.f:176 and 183-189: c_delta_sq = -num / (2 den); vt = c_delta_sq |S|.
+// clip: the coefficient the coupled closure uses, dm.f's value, or 0 where it
+// is negative (backscatter would make the eddy viscosity negative) or
+// undefined (no strain: 0/0)
+__global__ void k_dm_finish(const double* __restrict__ part, int nblk, double* __restrict__ cds, int clip) {
+  __shared__ double red[2][kThreads];
+  double num = 0.0, den = 0.0;
+  for (int b = threadIdx.x; b < nblk; b += blockDim.x) {
+    num += part[2 * b];
+    den += part[2 * b + 1];
+  }
+  red[0][threadIdx.x] = num;
+  red[1][threadIdx.x] = den;
+  __syncthreads();
+  for (int h = blockDim.x / 2; h > 0; h >>= 1) {
+    if (threadIdx.x < h) {
+      red[0][threadIdx.x] += red[0][threadIdx.x + h];
+      red[1][threadIdx.x] += red[1][threadIdx.x + h];
     }
-    cds[0] = -0.5 * num / den;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    const double v = -0.5 * red[0][0] / red[1][0];
+    cds[0] = clip && !(v > 0.0) ? 0.0 : v;
   }
 }
 
@@ -307,64 +369,56 @@ void les_sm(const double* u, double* ub, double* vt, int nx, int ny, int nz, dou
   k_periodic3<<<grid_of((long long)(nx + 2) * (ny + 2) * (nz + 2)), kThreads, 0, s>>>(vt, H);
 }
 
-int les_dm_blocks(int nx, int ny, int nz) { return grid_of((long long)nx * ny * nz); }
+int les_dm_blocks(int nx, int ny, int nz) {
+  const long long t = dm_tiles(nx, ny, nz);
+  return (int)(t < sm_count() * 12 ? t : sm_count() * 12);
+}
 
 void les_dm(const double* u, double* ub, double* q, double* part, double* cds, double* vt, int nx, int ny, int nz,
             double alpha_sq, double dxi, double dyi, double dzi, cudaStream_t s) {
   const Halo H = halo(nx, ny, nz);
   const long long n = (long long)nx * ny * nz;
-  const int nb = grid_of(n);
+  const int nb = grid_of(n), nt = les_dm_blocks(nx, ny, nz);
   k_ubar<<<nb, kThreads, 0, s>>>(u, ub, H);
-  k_dm_fields<<<nb, kThreads, 0, s>>>(ub, q, H, dxi, dyi, dzi);
-  k_dm_lm<<<nb, kThreads, 0, s>>>(ub, q, H, alpha_sq, part);
-  k_dm_finish<<<1, 32, 0, s>>>(part, nb, cds);
+  k_dm_fields<<<nb, kThreads, 0, s>>>(ub, q, H, dxi, dyi, dzi, 1);
+  k_dm_lm<<<nt, kThreads, 0, s>>>(ub, q, H, alpha_sq, part);
+  k_dm_finish<<<1, kThreads, 0, s>>>(part, nt, cds, 0);
   k_dm_vt<<<nb, kThreads, 0, s>>>(q, cds, vt, H);
   k_periodic3<<<grid_of((long long)(nx + 2) * (ny + 2) * (nz + 2)), kThreads, 0, s>>>(vt, H);
 }
 
-// ---- coupled dynamic closure: the physical velocity P(n, z, y, x) of the
-// x pass (working precision) into dm.f's haloed FP64 layout u(Lx,Ly,Lz,3),
-// halo planes filled with the periodic images (periodicity.f:7-32)
+// ---- coupled dynamic closure: u_bar (sm.f:47-49) straight from the physical
+// velocity P(n, z, y, x) of the x pass (working precision), periodic
 template <typename T>
-__global__ void k_pack_halo(const T* __restrict__ phys, double* __restrict__ uh, Halo H) {
-  const long long vol = H.vol(), tot = 3 * vol;
-  const int lx = H.nx + 2, ly = H.ny + 2;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < tot; e += (long long)gridDim.x * blockDim.x) {
-    const int n = (int)(e / vol);
-    const long long r = e - n * vol;
-    const int i = (int)(r % lx), j = (int)((r / lx) % ly), k = (int)(r / ((long long)lx * ly));
-    uh[e] = (double)phys[(long long)n * H.ninterior() + H.in(i - 1, j - 1, k - 1)];
+__global__ void k_ubar_phys(const T* __restrict__ u, double* __restrict__ ub, Halo H) {
+  const long long n = H.ninterior();
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
+    const int x = (int)(e % H.nx), y = (int)((e / H.nx) % H.ny), z = (int)(e / ((long long)H.nx * H.ny));
+    ub[e] = 0.5 * ((double)u[e] + (double)u[H.in(x - 1, y, z)]);
+    ub[n + e] = 0.5 * ((double)u[n + e] + (double)u[n + H.in(x, y - 1, z)]);
+    ub[2 * n + e] = 0.5 * ((double)u[2 * n + e] + (double)u[2 * n + H.in(x, y, z - 1)]);
   }
 }
 
-// C delta^2 in use: dm.f's value, or 0 where it is negative (backscatter
-// would make the eddy viscosity negative) or undefined (no strain: 0/0)
-__global__ void k_les_clip(const double* __restrict__ raw, double* __restrict__ cds) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    const double v = raw[0];
-    cds[0] = v > 0.0 ? v : 0.0;
-  }
-}
-
+// u_bar (3), the 18 fields of k_dm_fields, partial sums
 size_t les_dynamic_work(int nx, int ny, int nz) {
-  const size_t n = (size_t)nx * ny * nz, vol = (size_t)(nx + 2) * (ny + 2) * (nz + 2);
-  return 4 * vol + 22 * n + 2 * (size_t)les_dm_blocks(nx, ny, nz) + 8;
+  const size_t n = (size_t)nx * ny * nz;
+  return 21 * n + 2 * (size_t)les_dm_blocks(nx, ny, nz);
 }
 
 template <typename T>
 void les_dynamic(const T* phys, double* work, double* cds, int nx, int ny, int nz, double dxi, double dyi,
                  double dzi, cudaStream_t s) {
   const Halo H = halo(nx, ny, nz);
-  const size_t n = (size_t)nx * ny * nz, vol = (size_t)(nx + 2) * (ny + 2) * (nz + 2);
-  double* uh = work;
-  double* vt = uh + 3 * vol;
-  double* ub = vt + vol;
+  const size_t n = (size_t)nx * ny * nz;
+  double* ub = work;
   double* q = ub + 3 * n;
-  double* part = q + 19 * n;
-  double* raw = part + 2 * les_dm_blocks(nx, ny, nz);
-  k_pack_halo<T><<<grid_of(3 * (long long)vol), kThreads, 0, s>>>(phys, uh, H);
-  les_dm(uh, ub, q, part, raw, vt, nx, ny, nz, 4.0, dxi, dyi, dzi, s);
-  k_les_clip<<<1, 32, 0, s>>>(raw, cds);
+  double* part = q + 18 * n;
+  const int nb = grid_of((long long)n), nt = les_dm_blocks(nx, ny, nz);
+  k_ubar_phys<T><<<nb, kThreads, 0, s>>>(phys, ub, H);
+  k_dm_fields<<<nb, kThreads, 0, s>>>(ub, q, H, dxi, dyi, dzi, 0);
+  k_dm_lm<<<nt, kThreads, 0, s>>>(ub, q, H, 4.0, part);
+  k_dm_finish<<<1, kThreads, 0, s>>>(part, nt, cds, 1);
 }
 template void les_dynamic<double>(const double*, double*, double*, int, int, int, double, double, double,
                                   cudaStream_t);
