@@ -486,14 +486,23 @@ struct FxOutSplit {
 };
 
 // A first-stage loader that gives integers of a known scale (kInts) instead
-// of doubles: a product line of two lines of split integers.
+// of doubles: a product line of two lines of split integers, plus the line g
+// of doubles (a subgrid term; may be null).
 struct FxProductLoad {
   static constexpr bool kInts = true;
   const FxSplit2 *a, *b;
+  const double2* g;
   FxProduct p;
   __device__ __forceinline__ fxc operator()(int idx) const {
     const FxSplit2 ea = a[sidx(idx)], eb = b[sidx(idx)];
-    return fxc{fx_mul_line(ea.x, eb.x, p), fx_mul_line(ea.y, eb.y, p)};
+    fxc v{fx_mul_line(ea.x, eb.x, p), fx_mul_line(ea.y, eb.y, p)};
+    if (g) {
+      const double2 d = g[sidx(idx)];
+      const int dsh = p.sc.ex + 1023 + 62;
+      v.x = (v.x >> p.down) + fx_from(d.x, dsh);
+      v.y = (v.y >> p.down) + fx_from(d.y, dsh);
+    }
+    return v;
   }
   __device__ __forceinline__ FxScale scale() const { return p.sc; }
 };

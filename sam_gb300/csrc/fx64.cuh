@@ -378,20 +378,27 @@ __device__ __forceinline__ fxc fx_whole(FxSplit2 v) {
 // products' moduli is at most the product of the lines' norms, so the 124-bit
 // products shifted down by r = 62 + ceil(log2(norm_a norm_b)) sum to less
 // than 2^62, the bound a transform needs; each is rounded once.
+//
+// With a subgrid term (a line of doubles whose moduli sum to less than
+// 2^g.ex) both parts stay below 2^61: r grows by one, and further where the
+// term is the larger part (down).
 struct FxProduct {
   int s;  // 64 - r, at least 1 (norms up to 1) and at most 5 (lines scaled by their L1 norms have norms above 1/3)
+  int down;
   long long half;
   FxScale sc;
 };
-__device__ __forceinline__ FxProduct fx_product(const FxLine& a, const FxLine& b) {
-  const int r = min(max(62 + ((__float_as_int(a.norm * b.norm * 1.001f) >> 23) - 126), 59), 63);
+__device__ __forceinline__ FxProduct fx_product(const FxLine& a, const FxLine& b, const FxLine* g = nullptr) {
+  int r = min(max(62 + ((__float_as_int(a.norm * b.norm * 1.001f) >> 23) - 126), 59), 63);
   FxProduct p;
-  p.s = 64 - r;
-  p.half = 1ll << (31 - p.s);
+  if (g) r = max(r + 1, g->ex - 61 - a.ex - b.ex);
   p.sc.ex = a.ex + b.ex + r;
+  p.down = min(max(r - 63, 0), 63);
+  p.s = 64 - min(r, 63);
+  p.half = 1ll << (31 - p.s);
   p.sc.norm = 0.f;
   // (room for the exponents of a scaling by 1 / (Nx Ny))
-  p.sc.kind = (a.kind | b.kind) & kFxNaN ? kFxNaN : (p.sc.ex < -960 || p.sc.ex > 940 ? kFxEdge : kFxPlain);
+  p.sc.kind = (a.kind | b.kind | (g ? g->kind : 0)) & kFxNaN ? kFxNaN : (p.sc.ex < -960 || p.sc.ex > 940 ? kFxEdge : kFxPlain);
   return p;
 }
 __device__ __forceinline__ long long fx_mul_line(FxSplit a, FxSplit b, const FxProduct& p) {
@@ -401,9 +408,24 @@ __device__ __forceinline__ long long fx_mul_line(FxSplit a, FxSplit b, const FxP
   const uint32_t hi = __funnelshift_l((uint32_t)A, (uint32_t)(A >> 32), p.s);
   return (long long)(((uint64_t)hi << 32) | lo);
 }
+// The exponent bounding the moduli's sum of a line of n doubles (elements
+// sidx(0) .. sidx(n - 1)), by one warp: sum < 2^info->ex.
+__host__ __device__ __forceinline__ int sidx(int p);
+__device__ __forceinline__ void fx_line_bound(const double2* line, FxLine* info, int n) {
+  const int lane = threadIdx.x & 31;
+  uint32_t hm = 0;
+  for (int x = lane; x < n; x += 32) hm = max(hm, fx_max_hi<1>(line + sidx(x)));
+  hm = __reduce_max_sync(0xffffffffu, hm);
+  const int E = (int)(hm >> 20);
+  float l1 = 0.f;
+  for (int x = lane; x < n; x += 32) l1 += fx_l1<1>(line + sidx(x), E);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) l1 += __shfl_xor_sync(0xffffffffu, l1, o);
+  const int g = (__float_as_int(l1 * 1.0001f) >> 23) - 126;
+  if (lane == 0) *info = FxLine{E ? E - 1023 + g : -1100, E == 0x7ff ? kFxNaN : kFxPlain, 0.f};
+}
 // Physical values of a line of n points (elements sidx(0) .. sidx(n - 1)) to
 // split integers below 2^62, by one warp.
-__host__ __device__ __forceinline__ int sidx(int p);
 __device__ __forceinline__ void fx_line_in_place(double2* line, FxLine* info, int n) {
   const int lane = threadIdx.x & 31;
   uint32_t hm = 0;

@@ -503,11 +503,13 @@ __device__ __forceinline__ void x_pass_body(const XPassArgs<T>& a, const FftPlan
   const int Y = a.yt, yp = Y / 2, ld = a.ld;
   const int nin = a.nin;
   C* s_pr = s_in + nin * yp * ld;                // group product lines
-  // FP64 form with products and no subgrid terms: the physical lines are
-  // split integers (ints), their scales and norms behind the lines; the
-  // results of a product line stay integers until they are stored
+  // FP64 form with products: the physical lines of the factors are split
+  // integers (ints), their scales and norms behind the lines (of subgrid
+  // terms, doubles, a bound); the results of a product line stay integers
+  // until they are stored
   constexpr bool FX = kIsFx<C, PATH>;
-  const bool ints = FX && a.out_mode == 2 && !a.les;
+  const bool ints = FX && a.out_mode == 2;
+  const int nfac = a.g.lu * yp;  // lines of factors
   FxLine* s_line = reinterpret_cast<FxLine*>(s_pr + (size_t)a.prod_lines * ld);
   FxScale* s_psc = reinterpret_cast<FxScale*>(s_line + nin * yp);
   // vel_max's reduction scratch shares the product lines' space (it is done
@@ -598,7 +600,7 @@ __device__ __forceinline__ void x_pass_body(const XPassArgs<T>& a, const FftPlan
     const auto rows = [&](int L) { return BandLoad<C>{s_in + L * ld, kmx, nx - kmx}; };
     if constexpr (FX) {
       fft_lines_from<+1, PATH>(s_in, ld, nin * yp, s_tw, pl, rows, [&](int L) {
-        return FxOutSplit{s_in + L * ld, ints ? s_line + L : nullptr};
+        return FxOutSplit{s_in + L * ld, ints && L < nfac ? s_line + L : nullptr};
       });
     } else {
       fft_lines_from<+1, PATH>(s_in, ld, nin * yp, s_tw, pl, rows);
@@ -924,8 +926,11 @@ __device__ __forceinline__ void x_pass_body(const XPassArgs<T>& a, const FftPlan
   // ---- outputs
   if (a.out_mode == 3) return;  // statistics only (vel_max.f)
   if constexpr (FX) {
-    if (ints && a.in_mode != 0) {
-      for (int L = threadIdx.x >> 5; L < nin * yp; L += blockDim.x >> 5) fx_line_in_place(s_in + L * ld, s_line + L, nx);
+    if (ints && (a.in_mode != 0 || a.les)) {
+      for (int L = threadIdx.x >> 5; L < nin * yp; L += blockDim.x >> 5) {
+        if (L >= nfac) fx_line_bound(s_in + L * ld, s_line + L, nx);
+        else if (a.in_mode != 0) fx_line_in_place(s_in + L * ld, s_line + L, nx);
+      }
       __syncthreads();
     }
   }
@@ -972,16 +977,14 @@ __device__ __forceinline__ void x_pass_body(const XPassArgs<T>& a, const FftPlan
       if (ints) {
         const auto from_ints = [&](int L) {
           int fa, fb;
-          lines_of(L, fa, fb);
+          const int fg = lines_of(L, fa, fb);
           return FxProductLoad{reinterpret_cast<const FxSplit2*>(s_in + fa * ld),
-                               reinterpret_cast<const FxSplit2*>(s_in + fb * ld), fx_product(s_line[fa], s_line[fb])};
+                               reinterpret_cast<const FxSplit2*>(s_in + fb * ld), a.les ? s_in + fg * ld : nullptr,
+                               fx_product(s_line[fa], s_line[fb], a.les ? s_line + fg : nullptr)};
         };
-        fft_lines_from<-1, PATH>(lines, ld, gl, s_tw, pl, from_ints,
-                                 [&](int L) { return FxOutInt{lines + L * ld, s_psc + L}; });
+        fft_lines_from<-1, PATH>(lines, ld, gl, s_tw, pl, from_ints, [&](int L) { return FxOutInt{lines + L * ld, s_psc + L}; });
       } else {
-        fft_lines_from<-1, PATH>(lines, ld, gl, s_tw, pl, from_values, [&](int L) {
-          return FxOutInt{lines + L * ld, a.out_mode == 2 ? s_psc + L : nullptr};
-        });
+        fft_lines_from<-1, PATH>(lines, ld, gl, s_tw, pl, from_values);
       }
     } else {
       fft_lines_from<-1, PATH>(lines, ld, gl, s_tw, pl, from_values);
