@@ -763,19 +763,119 @@ template <int PATH> __device__ __forceinline__ int tw_load(const FftPlan& pl) {
   return PATH == kFft256 ? pl.tw_pass : pl.tw_total;
 }
 
-// Stages S.. of a compile-time length N on one line; stage 0 reads through first.
-template <int SIGN, int N, int S, typename C, typename First, typename Out>
-__device__ __forceinline__ void fft_ct_stages(C* line, const typename TwOf<C>::type* __restrict__ tw, const FftPlan& pl,
-                                              int tl, int TW, First first, Out out, FxScale sc = FxScale{}) {
-  if constexpr (S < ct_nst(N)) {
-    if constexpr (std::is_same<C, double2>::value) {
-      if constexpr (S == 0) fx_stage<ct_radix(N, 0), SIGN, true>(line, tw, pl.st[0], N, tl, TW, first, out, sc, ct_nst(N) == 1);
-      else fx_stage<ct_radix(N, S), SIGN, false>(line, tw, pl.st[S], N, tl, TW, LineLoad<C>{line}, out, sc, S + 1 == ct_nst(N));
-    } else {
-      if constexpr (S == 0) fft_stage<ct_radix(N, 0), SIGN>(line, tw, pl.st[0], N, tl, TW, first);
-      else fft_stage<ct_radix(N, S), SIGN>(line, tw, pl.st[S], N, tl, TW, LineLoad<C>{line});
+// Threads of a team for compile-time length n: build_plan's team (a power of
+// two such that no thread holds more than 8 values in any stage).
+__host__ __device__ constexpr int ct_team(int n) {
+  int tw = 1;
+  while (tw * 8 < n) tw *= 2;
+  for (;;) {
+    bool ok = true;
+    for (int s = 0; s < ct_nst(n); ++s) {
+      const int p = ct_radix(n, s);
+      if ((n / p + tw - 1) / tw > 8 / p) ok = false;
     }
-    fft_ct_stages<SIGN, N, S + 1>(line, tw, pl, tl, TW, first, out, sc);
+    if (ok) return tw;
+    tw *= 2;
+  }
+}
+// Stage S of compile-time length N: radix, sub-transform length, what is
+// left, place in the twiddle table (behind the 16 x 16 table of 256).
+template <int N, int S> struct CtStage {
+  static constexpr int P = ct_radix(N, S);
+  static constexpr int len(int s) { return s == 0 ? 1 : len(s - 1) * ct_radix(N, s - 1); }
+  static constexpr int off(int s) { return s == 0 ? (N == 256 ? 256 : 0) : off(s - 1) + len(s - 1) * (ct_radix(N, s - 1) - 1); }
+  static constexpr int L = len(S), M = N / (L * P), OFF = off(S), TW = ct_team(N), NB = N / P;
+  static constexpr int ITER = (NB + TW - 1) / TW;  // butterflies of a thread
+  static constexpr bool FULL = NB % TW == 0;       // every thread has ITER of them
+};
+// sidx(f M P + k + M q) for k < M as sidx at q = 0 plus a constant where the
+// pads between 16 elements fall alike for every f and k
+template <int M, int P> struct CtIndex {
+  static constexpr bool kFold = (16 % M == 0 || M % 16 == 0) && (16 % (M * P) == 0 || (M * P) % 16 == 0);
+  __device__ static __forceinline__ int at(int f, int k, int q) {
+    if (kFold) return sidx(f * M * P + k) + (M * q + ((M * q) >> 4));
+    return sidx(f * M * P + k + M * q);
+  }
+};
+
+// One stage of a compile-time length: everything but the thread's place is a
+// constant.  active: whether the team has a line.
+template <int SIGN, int N, int S, typename C, typename Ld, typename Out>
+__device__ __forceinline__ void ct_stage(C* line, const typename TwOf<C>::type* __restrict__ tw, int tl, bool active,
+                                         Ld load, Out out, FxScale& sc) {
+  using G = CtStage<N, S>;
+  constexpr bool FX = std::is_same<C, double2>::value;
+  using A = std::conditional_t<FX, fxc, C>;
+  constexpr int P = G::P, M = G::M, TW = G::TW, ITER = G::ITER;
+  A a[ITER][P];
+  A* fl = reinterpret_cast<A*>(line);
+  if constexpr (S == 0 && FX && !LoadsInts<Ld>::value) {
+    double2 v[ITER][P];
+#pragma unroll
+    for (int i = 0; i < ITER; ++i)
+#pragma unroll
+      for (int q = 0; q < P; ++q) v[i][q] = make_double2(0.0, 0.0);
+    if (active) {
+#pragma unroll
+      for (int i = 0; i < ITER; ++i) {
+        const int b = tl + i * TW;
+        if (G::FULL || b < G::NB) {
+#pragma unroll
+          for (int q = 0; q < P; ++q) v[i][q] = load(b + M * q);
+        }
+      }
+    }
+    sc = fx_begin<ITER * P, Out::kNorm>(&v[0][0], &a[0][0], TW, Out::kNorm ? sqrtf((float)N) : 0.f);
+  } else if constexpr (S == 0) {
+    if constexpr (FX) sc = load.scale();
+    if (active) {
+#pragma unroll
+      for (int i = 0; i < ITER; ++i) {
+        const int b = tl + i * TW;
+        if (G::FULL || b < G::NB) {
+#pragma unroll
+          for (int q = 0; q < P; ++q) a[i][q] = load(b + M * q);
+        }
+      }
+    }
+  } else if (active) {
+#pragma unroll
+    for (int i = 0; i < ITER; ++i) {
+      const int b = tl + i * TW;
+      if (G::FULL || b < G::NB) {
+        const int f = b / M, k = b - f * M;
+        const auto* w = tw + G::OFF + f * (P - 1);
+        a[i][0] = fl[CtIndex<M, P>::at(f, k, 0)];
+#pragma unroll
+        for (int q = 1; q < P; ++q) a[i][q] = ctw<SIGN>(fl[CtIndex<M, P>::at(f, k, q)], w[q - 1]);
+      }
+    }
+  }
+  team_sync(TW);
+  if (active) {
+#pragma unroll
+    for (int i = 0; i < ITER; ++i) {
+      const int b = tl + i * TW;
+      if (G::FULL || b < G::NB) {
+        dftp<P, SIGN>(a[i]);
+        // outputs b + q N / P
+#pragma unroll
+        for (int q = 0; q < P; ++q) {
+          if constexpr (FX && S + 1 == ct_nst(N)) out(b + q * (N / P), a[i][q], sc);
+          else fl[CtIndex<N / P, P>::at(0, b, q)] = a[i][q];
+        }
+      }
+    }
+  }
+  team_sync(TW);
+}
+template <int SIGN, int N, int S, typename C, typename First, typename Out>
+__device__ __forceinline__ void fft_ct_stages(C* line, const typename TwOf<C>::type* __restrict__ tw, int tl,
+                                              bool active, First first, Out out, FxScale& sc) {
+  if constexpr (S < ct_nst(N)) {
+    if constexpr (S == 0) ct_stage<SIGN, N, S>(line, tw, tl, active, first, out, sc);
+    else ct_stage<SIGN, N, S>(line, tw, tl, active, 0, out, sc);
+    fft_ct_stages<SIGN, N, S + 1>(line, tw, tl, active, first, out, sc);
   }
 }
 
@@ -799,7 +899,7 @@ __device__ __forceinline__ void fft_lines_from(C* base, int ld, int nlines,
     return;
   }
   if (PATH == kFft256) return;
-  const int TW = team_of<C>(pl);
+  const int TW = ct_length(PATH) ? ct_team(ct_length(PATH) ? PATH : 8) : team_of<C>(pl);
   const int nteams = blockDim.x / TW;
   const int team = threadIdx.x / TW;
   const int tl = threadIdx.x - team * TW;
@@ -809,7 +909,8 @@ __device__ __forceinline__ void fft_lines_from(C* base, int ld, int nlines,
     const bool active = L < nlines;
     const int Lc = active ? L : 0;
     if constexpr (ct_length(PATH)) {
-      fft_ct_stages<SIGN, PATH, 0>(base + Lc * ld, tw, pl, active ? tl : (1 << 20), TW, first(Lc), out(Lc));
+      FxScale sc;
+      fft_ct_stages<SIGN, PATH, 0>(base + Lc * ld, tw, tl, active, first(Lc), out(Lc), sc);
     } else {
       fft_line_from<SIGN, PATH>(base + Lc * ld, tw, pl, tl, active, first(Lc), out(Lc));
     }
