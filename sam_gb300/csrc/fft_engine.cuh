@@ -16,7 +16,6 @@
 
 #include <type_traits>
 
-#include "ddfloat.cuh"
 #include "fx64.cuh"
 
 namespace samgpu {
@@ -24,7 +23,6 @@ namespace samgpu {
 template <typename T> struct Cx;
 template <> struct Cx<double> { using type = double2; };
 template <> struct Cx<float> { using type = float2; };
-template <> struct Cx<dd> { using type = ddc; };
 template <typename T> using cx_t = typename Cx<T>::type;
 
 // Type of a transform's twiddles: fixed point for the FP64 form's lines
@@ -32,7 +30,6 @@ template <typename T> using cx_t = typename Cx<T>::type;
 template <typename C> struct TwOf { using type = C; };
 template <> struct TwOf<double2> { using type = fxw; };
 template <typename T> using tw_t = typename TwOf<cx_t<T>>::type;
-static_assert(sizeof(fxw) == sizeof(double2), "a twiddle table's entries have one size");
 
 template <typename C> __device__ __forceinline__ C mk(decltype(C::x) a, decltype(C::x) b) { C r; r.x = a; r.y = b; return r; }
 
@@ -60,103 +57,10 @@ __device__ __forceinline__ float2 csub(float2 a, float2 b) {
   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_pack(a)), "l"(f2_pack(b)));
   return f2_unpack(r);
 }
-// Double-float complex sums with the real and imaginary parts in one packed
-// pair per instruction: the high parts' TwoSum, the low parts' sum and the
-// renormalisation of ddfloat.cuh's operator+, each step on (re, im) at once
-// (the same IEEE operations and results as two scalar pair sums).
-__device__ __forceinline__ unsigned long long f2p(float a, float b) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void f2u(unsigned long long r, float& a, float& b) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r));
-}
-__device__ __forceinline__ unsigned long long f2add(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ unsigned long long f2sub(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-// s + e = H +- K exactly (TwoSum; for the difference with -K folded in), then
-// the low parts' sum L added and the pair renormalised
-template <bool SUB>
-__device__ __forceinline__ ddc dd_cplx_sum(unsigned long long H, unsigned long long K, unsigned long long L) {
-  const unsigned long long s = SUB ? f2sub(H, K) : f2add(H, K);
-  const unsigned long long bb = f2sub(s, H);
-  const unsigned long long t = f2sub(H, f2sub(s, bb));
-  unsigned long long e = SUB ? f2sub(t, f2add(K, bb)) : f2add(t, f2sub(K, bb));
-  e = f2add(e, L);
-  const unsigned long long h = f2add(s, e);
-  const unsigned long long l = f2sub(e, f2sub(h, s));
-  ddc r;
-  f2u(h, r.x.hi, r.y.hi);
-  f2u(l, r.x.lo, r.y.lo);
-  return r;
-}
-__device__ __forceinline__ ddc cadd(ddc a, ddc b) {
-  return dd_cplx_sum<false>(f2p(a.x.hi, a.y.hi), f2p(b.x.hi, b.y.hi),
-                            f2add(f2p(a.x.lo, a.y.lo), f2p(b.x.lo, b.y.lo)));
-}
-__device__ __forceinline__ ddc csub(ddc a, ddc b) {
-  return dd_cplx_sum<true>(f2p(a.x.hi, a.y.hi), f2p(b.x.hi, b.y.hi),
-                           f2sub(f2p(a.x.lo, a.y.lo), f2p(b.x.lo, b.y.lo)));
-}
 // a * w (SIGN=-1) or a * conj(w) (SIGN=+1)
 template <int SIGN, typename C> __device__ __forceinline__ C ctw(C a, C w) {
   if (SIGN < 0) return mk<C>(a.x * w.x - a.y * w.y, a.x * w.y + a.y * w.x);
   return mk<C>(a.x * w.x + a.y * w.y, a.y * w.x - a.x * w.y);
-}
-__device__ __forceinline__ unsigned long long f2mul(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ unsigned long long f2fma(unsigned long long a, unsigned long long b,
-                                                    unsigned long long c) {
-  unsigned long long r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-// Complex double-float product a * (u + i v)-style: the real and imaginary
-// parts as one packed pair each step, lane k = x (0) or y (1):
-//   R_k = ax * U_k + ay * V_k
-// with U = (c1, c3), V = (c2, c4) the caller's coefficient pairs, given as
-// their high and low parts.  The two exact products (FMA TwoProduct, the
-// error terms formed negated from -ax, -ay so no packed negation is needed),
-// a TwoSum of them, the four cross terms and one renormalisation: the
-// operations of dd_mul_sub on both parts at once.
-__device__ __forceinline__ ddc dd_cplx_dot(ddc a, unsigned long long Uh, unsigned long long Ul,
-                                           unsigned long long Vh, unsigned long long Vl) {
-  const unsigned long long Xh = f2p(a.x.hi, a.x.hi), Xl = f2p(a.x.lo, a.x.lo), nXh = f2p(-a.x.hi, -a.x.hi);
-  const unsigned long long Yh = f2p(a.y.hi, a.y.hi), Yl = f2p(a.y.lo, a.y.lo), nYh = f2p(-a.y.hi, -a.y.hi);
-  const unsigned long long P = f2mul(Xh, Uh), Q = f2mul(Yh, Vh);
-  const unsigned long long nEP = f2fma(nXh, Uh, P), nEQ = f2fma(nYh, Vh, Q);  // -(exact error of P, Q)
-  const unsigned long long s = f2add(P, Q);
-  const unsigned long long bb = f2sub(s, P);
-  unsigned long long e = f2add(f2sub(P, f2sub(s, bb)), f2sub(Q, bb));
-  e = f2sub(e, f2add(nEP, nEQ));
-  e = f2fma(Xh, Ul, e);
-  e = f2fma(Xl, Uh, e);
-  e = f2fma(Yh, Vl, e);
-  e = f2fma(Yl, Vh, e);
-  const unsigned long long h = f2add(s, e);
-  const unsigned long long l = f2sub(e, f2sub(h, s));
-  ddc r;
-  f2u(h, r.x.hi, r.y.hi);
-  f2u(l, r.x.lo, r.y.lo);
-  return r;
-}
-// double-float pairs: a * w as a packed pair (SIGN = -1: U = (wx, wy),
-// V = (-wy, wx); SIGN = +1, a * conj(w): U = (wx, -wy), V = (wy, wx))
-template <int SIGN> __device__ __forceinline__ ddc ctw(ddc a, ddc w) {
-  if (SIGN < 0)
-    return dd_cplx_dot(a, f2p(w.x.hi, w.y.hi), f2p(w.x.lo, w.y.lo), f2p(-w.y.hi, w.x.hi), f2p(-w.y.lo, w.x.lo));
-  return dd_cplx_dot(a, f2p(w.x.hi, -w.y.hi), f2p(w.x.lo, -w.y.lo), f2p(w.y.hi, w.x.hi), f2p(w.y.lo, w.x.lo));
 }
 // FP32: the same products with their rounding spelled out (the second
 // product rounded, the first fused with the sum), so every kernel computes
@@ -174,17 +78,12 @@ template <int SIGN, typename C> __device__ __forceinline__ C cmul_si(C a) {
 // Code paths of the line transforms: kFftAny picks at run time (the plan's
 // length); kFft256 compiles only the 16 x 16 register path (n = 256) and
 // kFftGeneric only the Stockham stages with the radix chosen at run time;
-// PATH = n (32, 64, 96, 128, 256, 512) compiles the Stockham stages of that length
-// with their radices fixed at compile time.  A kernel built for one length
+// PATH = n (ct_length) compiles the Stockham stages of that length with their
+// radices and every stride fixed at compile time (ct_plan).  A kernel built for one length
 // thus carries no registers for another path.
-// The FP64 form's lines run in fixed point (fx64.cuh) up to kFxMaxLine points
-// and in FP64 arithmetic beyond (kFftLong): the fixed-point roundings grow as
-// sqrt(n) against the line's norm and pass FP64's own near n = 1000 (2.1
-// against 1.9 in units of 2^-53 for white lines at 1024, 0.9 against 1.8 at
-// 512, 0.55 against 1.6 at 256).
-constexpr int kFftAny = 0, kFft256 = 1, kFftGeneric = 2, kFftLong = 3;
-constexpr int kFxMaxLine = 512;
-template <typename C, int PATH> inline constexpr bool kIsFx = std::is_same<C, double2>::value && PATH != kFftLong;
+constexpr int kFftAny = 0, kFft256 = 1, kFftGeneric = 2;
+// whether lines are transformed in fixed point (fx64.cuh)
+template <typename C> inline constexpr bool kIsFx = std::is_same<C, double2>::value;
 
 struct FftStage {
   int p;       // radix
@@ -198,19 +97,15 @@ struct FftPlan {
   int n;
   int nst;
   int tw_total;
-  int team;     // threads per line in FP64 (at most 8 values per thread)
-  int team_sp;  // threads per line in FP32 (at most 8 values per thread)
+  int team;     // threads per line of the run-time stages (at most 8 values per thread)
   int tw16_off; // n == 256: offset of the 16 x 16 table w_256^{f q} (else -1)
-  int tw_pass;  // twiddles the pass kernels load: the 16 x 16 table (at 0) for n = 256, else all
+  int tw_pass;  // twiddles the pass kernels load: those of the length's own path (at 0), else all
   FftStage st[10];
 };
 
 // Values a thread holds per stage (8 complex: 16 in FP32 spills registers
 // with five radices compiled into each stage loop).
 template <typename C> struct Emax { static constexpr int value = 8; };
-template <typename C> __device__ __forceinline__ int team_of(const FftPlan& pl) {
-  return sizeof(C) <= 8 ? pl.team_sp : pl.team;
-}
 
 __device__ __forceinline__ int div_m(int b, const FftStage& s) { return (int)(((uint32_t)b * s.mmul) >> 21); }
 
@@ -330,10 +225,6 @@ template <typename C, typename T> __device__ __forceinline__ C crot(C v, T cr, T
 __device__ __forceinline__ float2 crot(float2 v, float cr, float si) {
   return make_float2(__fmaf_rn(v.x, cr, -__fmul_rn(v.y, si)), __fmaf_rn(v.x, si, __fmul_rn(v.y, cr)));
 }
-__device__ __forceinline__ ddc crot(ddc v, dd cr, dd si) {
-  return dd_cplx_dot(v, f2p(cr.hi, si.hi), f2p(cr.lo, si.lo), f2p(-si.hi, cr.hi), f2p(-si.lo, cr.lo));
-}
-
 // 16-point DFT in registers as 4 x 4: DFT4 over n1 of x[4 n1 + n2], the
 // twiddles w16^{n2 k1}, DFT4 over n2; output k1 + 4 k2 in place.
 template <int SIGN, typename C> __device__ __forceinline__ void dft16(C* a) {
@@ -370,12 +261,68 @@ template <int SIGN, typename C> __device__ __forceinline__ void dft16(C* a) {
   }
 }
 
+template <int P, int SIGN, typename C> __device__ __forceinline__ void dftp(C* a);
+// times w9^J (exp(SIGN 2 pi i J / 9))
+template <int SIGN, int J> __device__ __forceinline__ float2 rot9(float2 v) {
+  constexpr double c[5] = {1.0, 0.76604444311897803520, 0.17364817766693034885, -0.5, -0.93969262078590838405};
+  constexpr double s[5] = {0.0, 0.64278760968653932632, 0.98480775301220805937, 0.86602540378443864676, 0.34202014332566873304};
+  return crot(v, (float)c[J], SIGN * (float)s[J]);
+}
+// N1 N2 points, coprime, without twiddles (Good and Thomas): input
+// N2 n1 + N1 n2 (mod N) in row n1, column n2, output k in row k mod N1, column
+// k mod N2
+template <int N1, int N2, int SIGN, typename C> __device__ __forceinline__ void dft_coprime(C* a) {
+  constexpr int N = N1 * N2;
+  C t[N1][N2];
+#pragma unroll
+  for (int n2 = 0; n2 < N2; ++n2) {
+    C c[N1];
+#pragma unroll
+    for (int n1 = 0; n1 < N1; ++n1) c[n1] = a[(N2 * n1 + N1 * n2) % N];
+    dftp<N1, SIGN>(c);
+#pragma unroll
+    for (int n1 = 0; n1 < N1; ++n1) t[n1][n2] = c[n1];
+  }
+#pragma unroll
+  for (int n1 = 0; n1 < N1; ++n1) dftp<N2, SIGN>(t[n1]);
+#pragma unroll
+  for (int k = 0; k < N; ++k) a[k] = t[k % N1][k % N2];
+}
+// 9 points as 3 x 3 with the twiddles w9^1, w9^2 (twice) and w9^4
+template <int SIGN, typename C> __device__ __forceinline__ void dft9(C* a) {
+  C b[3][3];
+#pragma unroll
+  for (int n2 = 0; n2 < 3; ++n2) {
+    C c[3] = {a[n2], a[3 + n2], a[6 + n2]};
+    dft3<SIGN>(c);
+#pragma unroll
+    for (int k1 = 0; k1 < 3; ++k1) b[n2][k1] = c[k1];
+  }
+  b[1][1] = rot9<SIGN, 1>(b[1][1]);
+  b[1][2] = rot9<SIGN, 2>(b[1][2]);
+  b[2][1] = rot9<SIGN, 2>(b[2][1]);
+  b[2][2] = rot9<SIGN, 4>(b[2][2]);
+#pragma unroll
+  for (int k1 = 0; k1 < 3; ++k1) {
+    C c[3] = {b[0][k1], b[1][k1], b[2][k1]};
+    dft3<SIGN>(c);
+#pragma unroll
+    for (int k2 = 0; k2 < 3; ++k2) a[k1 + 3 * k2] = c[k2];
+  }
+}
+
 template <int P, int SIGN, typename C> __device__ __forceinline__ void dftp(C* a) {
-  if (P == 2) dft2<SIGN>(a);
-  else if (P == 3) dft3<SIGN>(a);
-  else if (P == 4) dft4<SIGN>(a);
-  else if (P == 5) dft5<SIGN>(a);
-  else dft8<SIGN>(a);
+  if constexpr (P == 2) dft2<SIGN>(a);
+  else if constexpr (P == 3) dft3<SIGN>(a);
+  else if constexpr (P == 4) dft4<SIGN>(a);
+  else if constexpr (P == 5) dft5<SIGN>(a);
+  else if constexpr (P == 6) dft_coprime<2, 3, SIGN>(a);
+  else if constexpr (P == 8) dft8<SIGN>(a);
+  else if constexpr (P == 9) dft9<SIGN>(a);
+  else if constexpr (P == 10) dft_coprime<2, 5, SIGN>(a);
+  else if constexpr (P == 12) dft_coprime<3, 4, SIGN>(a);
+  else if constexpr (P == 15) dft_coprime<3, 5, SIGN>(a);
+  else dft16<SIGN>(a);
 }
 
 // One Stockham stage of radix P on one line held in shared memory.
@@ -558,7 +505,7 @@ __device__ __forceinline__ void fx_stage(double2* line, const fxw* __restrict__ 
         const fxw* w = tw + s.tw_off + f * (P - 1);
         a[i][0] = fl[sidx(src)];
 #pragma unroll
-        for (int q = 1; q < P; ++q) a[i][q] = ctw<SIGN>(fl[sidx(src + s.m * q)], w[q - 1]);
+        for (int q = 1; q < P; ++q) a[i][q] = ctw<SIGN, true>(fl[sidx(src + s.m * q)], w[q - 1]);
       }
     }
   }
@@ -611,26 +558,20 @@ __device__ __forceinline__ void fft_stage_p(C* line, const C* __restrict__ tw, c
 // first(idx), so a caller can form the line on the fly (e.g. the product of
 // two other lines).  All threads of the team call this together; a team with
 // no line passes active=false and still synchronises.
-template <int SIGN, int PATH, typename C, typename First, typename Out>
+template <int SIGN, typename C, typename First, typename Out>
 __device__ __forceinline__ void fft_line_from(C* line, const typename TwOf<C>::type* __restrict__ tw, const FftPlan& pl,
                                               int tl, bool active, First first, Out out) {
   const int n = pl.n;
-  const int TW = team_of<C>(pl);
+  const int TW = pl.team;
   const int tla = active ? tl : (1 << 20);  // inactive lanes own no butterfly
-  if constexpr (std::is_same<C, double2>::value && PATH != kFftLong) {
-    if (PATH != kFftAny || n <= kFxMaxLine) {
-      FxScale sc;
-      fx_stage_p<SIGN, true>(line, tw, pl.st[0], n, tla, TW, first, out, sc, pl.nst == 1);
-      for (int s = 1; s < pl.nst; ++s)
-        fx_stage_p<SIGN, false>(line, tw, pl.st[s], n, tla, TW, LineLoad<C>{line}, out, sc, s + 1 == pl.nst);
-      return;
-    }
-  }
-  if constexpr (!std::is_same<C, double2>::value || PATH == kFftLong || PATH == kFftAny) {
-    // (a table of a length above kFxMaxLine holds FP64 twiddles)
-    const C* w = reinterpret_cast<const C*>(tw);
-    fft_stage_p<SIGN>(line, w, pl.st[0], n, tla, TW, first);
-    for (int s = 1; s < pl.nst; ++s) fft_stage_p<SIGN>(line, w, pl.st[s], n, tla, TW, LineLoad<C>{line});
+  if constexpr (kIsFx<C>) {
+    FxScale sc;
+    fx_stage_p<SIGN, true>(line, tw, pl.st[0], n, tla, TW, first, out, sc, pl.nst == 1);
+    for (int s = 1; s < pl.nst; ++s)
+      fx_stage_p<SIGN, false>(line, tw, pl.st[s], n, tla, TW, LineLoad<C>{line}, out, sc, s + 1 == pl.nst);
+  } else {
+    fft_stage_p<SIGN>(line, tw, pl.st[0], n, tla, TW, first);
+    for (int s = 1; s < pl.nst; ++s) fft_stage_p<SIGN>(line, tw, pl.st[s], n, tla, TW, LineLoad<C>{line});
   }
 }
 
@@ -737,56 +678,99 @@ __device__ __forceinline__ void fft256_lines(double2* base, int ld, int nlines, 
   }
 }
 
-// The s-th radix of the plan for length n (build_plan's order: 8s, then 4,
-// 2, 3, 5) and the number of stages, at compile time.
-__host__ __device__ constexpr int ct_radix(int n, int s) {
-  int r = n, k = 0;
-  while (r % 8 == 0) { if (k == s) return 8; r /= 8; ++k; }
-  while (r % 4 == 0) { if (k == s) return 4; r /= 4; ++k; }
-  while (r % 2 == 0) { if (k == s) return 2; r /= 2; ++k; }
-  while (r % 3 == 0) { if (k == s) return 3; r /= 3; ++k; }
-  while (r % 5 == 0) { if (k == s) return 5; r /= 5; ++k; }
-  return 0;
-}
-__host__ __device__ constexpr int ct_nst(int n) {
-  int s = 0;
-  while (ct_radix(n, s) != 0) ++s;
-  return s;
-}
-// lengths with a compile-time path
+// Lengths with a compile-time path: all 2^a 3^b 5^c from 16 to 256, and 512.
 __host__ __device__ constexpr bool ct_length(int n) {
-  return n == 32 || n == 64 || n == 96 || n == 128 || n == 256 || n == 512;
+  if (n != 512 && (n < 16 || n > 256)) return false;
+  while (n % 2 == 0) n /= 2;
+  while (n % 3 == 0) n /= 3;
+  while (n % 5 == 0) n /= 5;
+  return n == 1;
 }
-// Twiddles a kernel compiled for PATH loads: the 16 x 16 table alone (at the
-// start of the table) for the register path, all of them otherwise.
+// Radices of a compile-time length and the threads of its team.
+struct CtPlan {
+  int nst, r[4], tw;
+};
+// Lines that `threads` threads transform at once: teams of tw <= 32 threads
+// fill a warp without crossing it, wider ones are whole warps.
+__host__ __device__ constexpr int ct_teams(int tw, int threads) {
+  return tw <= 32 ? (threads / 32) * (32 / tw) : threads / tw;
+}
+// Instructions of one butterfly of radix p in fixed point, its loads and
+// stores included, to weigh the splits of a length against each other
+// (counted, not measured: a complex sum 4, a product by a constant 11, a
+// rotation 34).
+__host__ __device__ constexpr int ct_cost(int p, bool first) {
+  const int dft = p == 2 ? 8 : p == 3 ? 56 : p == 4 ? 32 : p == 5 ? 150 : p == 6 ? 136 : p == 8 ? 140 : p == 9 ? 472 :
+                  p == 10 ? 340 : p == 12 ? 320 : p == 15 ? 730 : 490;
+  return dft + 10 * p + (first ? 30 * p : 34 * (p - 1));
+}
+// The cheapest split into two or three radices for any team of 4 to 32
+// threads (8 from n = 48) that hold at most 10 values each: instructions a
+// line, times the share of a warp that its team takes; within 2 % the larger
+// radices first (128: 8 x 8 x 2 before 8 x 4 x 4, FP32 stage 0.142 against
+// 0.156 ms, FP64 0.513 against 0.503).  Fewer, larger radices
+// in fewer threads (16 x 8 in 8 threads for n = 128) execute fewer instructions
+// but leave too few loads in flight: FP32 x pass at 128^3 0.061 against
+// 0.049 ms for 8 x 8 x 2 in 16.  256 and 512 keep the splits of their own paths.
+__host__ __device__ constexpr CtPlan ct_plan(int n) {
+  if (n == 256) return CtPlan{3, {8, 8, 4, 1}, 32};
+  if (n == 512) return CtPlan{3, {8, 8, 8, 1}, 64};
+  constexpr int R[11] = {2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16};
+  CtPlan best{0, {1, 1, 1, 1}, 0};
+  long cost = 0;
+  for (int i = 10; i >= 0; --i)
+    for (int j = 10; j >= 0; --j) {
+      if (n % (R[i] * R[j])) continue;
+      const int c = n / (R[i] * R[j]);
+      bool known = c == 1;
+      for (int k = 0; k < 11; ++k) known = known || c == R[k];
+      if (!known) continue;
+      const int r[3] = {R[i], R[j], c};
+      const int nst = c == 1 ? 2 : 3;
+      for (int tw = n < 48 ? 4 : 8; tw <= 32; ++tw) {
+        long per = 0;
+        bool ok = true;
+        for (int s = 0; s < nst; ++s) {
+          const int it = (n / r[s] + tw - 1) / tw;
+          if (it * r[s] > 10) ok = false;
+          per += (long)it * ct_cost(r[s], s == 0);
+        }
+        if (!ok) continue;
+        const long line = per * 10000 / (32 / tw);
+        if (best.nst == 0 || line * 50 < cost * 49) {
+          cost = line;
+          best = CtPlan{nst, {r[0], r[1], r[2], 1}, tw};
+        }
+      }
+    }
+  return best;
+}
+// Twiddles of the compile-time stages (the first has none).
+__host__ __device__ constexpr int ct_tw_off(int n, int s) {
+  const CtPlan p = ct_plan(n);
+  int off = n == 256 ? 256 + 7 : 0, l = 1;  // (256: behind the 16 x 16 table, the run-time table's stages)
+  for (int i = 0; i < s; ++i) {
+    if (i > 0) off += l * (p.r[i] - 1);
+    l *= p.r[i];
+  }
+  return off;
+}
+// Twiddles that a kernel compiled for PATH loads: the 16 x 16 table alone (at
+// the start of the table) for the register path, the length's own stages'
+// otherwise, all of them for run-time stages.
 template <int PATH> __device__ __forceinline__ int tw_load(const FftPlan& pl) {
-  return PATH == kFft256 ? pl.tw_pass : pl.tw_total;
+  return PATH == 256 ? pl.tw_total : pl.tw_pass;
 }
 
-// Threads of a team for compile-time length n: build_plan's team (a power of
-// two such that no thread holds more than 8 values in any stage).
-__host__ __device__ constexpr int ct_team(int n) {
-  int tw = 1;
-  while (tw * 8 < n) tw *= 2;
-  for (;;) {
-    bool ok = true;
-    for (int s = 0; s < ct_nst(n); ++s) {
-      const int p = ct_radix(n, s);
-      if ((n / p + tw - 1) / tw > 8 / p) ok = false;
-    }
-    if (ok) return tw;
-    tw *= 2;
-  }
-}
 // Stage S of compile-time length N: radix, sub-transform length, what is
-// left, place in the twiddle table (behind the 16 x 16 table of 256).
+// left, place in the twiddle table.
 template <int N, int S> struct CtStage {
-  static constexpr int P = ct_radix(N, S);
-  static constexpr int len(int s) { return s == 0 ? 1 : len(s - 1) * ct_radix(N, s - 1); }
-  static constexpr int off(int s) { return s == 0 ? (N == 256 ? 256 : 0) : off(s - 1) + len(s - 1) * (ct_radix(N, s - 1) - 1); }
-  static constexpr int L = len(S), M = N / (L * P), OFF = off(S), TW = ct_team(N), NB = N / P;
+  static constexpr CtPlan kPlan = ct_plan(N);
+  static constexpr int len(int s) { return s == 0 ? 1 : len(s - 1) * kPlan.r[s - 1]; }
+  static constexpr int P = kPlan.r[S], L = len(S), M = N / (L * P), OFF = ct_tw_off(N, S), TW = kPlan.tw, NB = N / P;
   static constexpr int ITER = (NB + TW - 1) / TW;  // butterflies of a thread
   static constexpr bool FULL = NB % TW == 0;       // every thread has ITER of them
+  static constexpr bool LAST = S + 1 == kPlan.nst;
 };
 // sidx(f M P + k + M q) for k < M as sidx at q = 0 plus a constant where the
 // pads between 16 elements fall alike for every f and k
@@ -798,6 +782,11 @@ template <int M, int P> struct CtIndex {
   }
 };
 
+// a team's barrier: the warp's where teams do not cross warps
+template <int TW> __device__ __forceinline__ void ct_sync() {
+  if constexpr (TW <= 32) __syncwarp();
+  else team_sync(TW);
+}
 // One stage of a compile-time length: everything but the thread's place is a
 // constant.  active: whether the team has a line.
 template <int SIGN, int N, int S, typename C, typename Ld, typename Out>
@@ -851,7 +840,7 @@ __device__ __forceinline__ void ct_stage(C* line, const typename TwOf<C>::type* 
       }
     }
   }
-  team_sync(TW);
+  ct_sync<TW>();
   if (active) {
 #pragma unroll
     for (int i = 0; i < ITER; ++i) {
@@ -861,18 +850,18 @@ __device__ __forceinline__ void ct_stage(C* line, const typename TwOf<C>::type* 
         // outputs b + q N / P
 #pragma unroll
         for (int q = 0; q < P; ++q) {
-          if constexpr (FX && S + 1 == ct_nst(N)) out(b + q * (N / P), a[i][q], sc);
+          if constexpr (FX && G::LAST) out(b + q * (N / P), a[i][q], sc);
           else fl[CtIndex<N / P, P>::at(0, b, q)] = a[i][q];
         }
       }
     }
   }
-  team_sync(TW);
+  ct_sync<TW>();
 }
 template <int SIGN, int N, int S, typename C, typename First, typename Out>
 __device__ __forceinline__ void fft_ct_stages(C* line, const typename TwOf<C>::type* __restrict__ tw, int tl,
                                               bool active, First first, Out out, FxScale& sc) {
-  if constexpr (S < ct_nst(N)) {
+  if constexpr (S < ct_plan(N).nst) {
     if constexpr (S == 0) ct_stage<SIGN, N, S>(line, tw, tl, active, first, out, sc);
     else ct_stage<SIGN, N, S>(line, tw, tl, active, 0, out, sc);
     fft_ct_stages<SIGN, N, S + 1>(line, tw, tl, active, first, out, sc);
@@ -899,20 +888,33 @@ __device__ __forceinline__ void fft_lines_from(C* base, int ld, int nlines,
     return;
   }
   if (PATH == kFft256) return;
-  const int TW = ct_length(PATH) ? ct_team(ct_length(PATH) ? PATH : 8) : team_of<C>(pl);
-  const int nteams = blockDim.x / TW;
-  const int team = threadIdx.x / TW;
-  const int tl = threadIdx.x - team * TW;
-  const int rounds = (nlines + nteams - 1) / nteams;
-  for (int r = 0; r < rounds; ++r) {
-    const int L = r * nteams + team;
-    const bool active = L < nlines;
-    const int Lc = active ? L : 0;
-    if constexpr (ct_length(PATH)) {
+  if constexpr (ct_length(PATH)) {
+    constexpr int TW = ct_plan(PATH).tw, G = TW <= 32 ? 32 / TW : 1;
+    // lanes behind a warp's last whole team follow along without a line
+    const int lane = threadIdx.x & 31;
+    const int sub = TW <= 32 ? lane / TW : 0;
+    const int team = TW <= 32 ? (int)(threadIdx.x >> 5) * G + sub : (int)threadIdx.x / TW;
+    const int tl = TW <= 32 ? lane - sub * TW : (int)threadIdx.x - team * TW;
+    const int nteams = ct_teams(TW, blockDim.x);
+    const int rounds = (nlines + nteams - 1) / nteams;
+    for (int r = 0; r < rounds; ++r) {
+      const int L = r * nteams + team;
+      const bool active = (TW > 32 || sub < G) && L < nlines;
+      const int Lc = active ? L : 0;
       FxScale sc;
       fft_ct_stages<SIGN, PATH, 0>(base + Lc * ld, tw, tl, active, first(Lc), out(Lc), sc);
-    } else {
-      fft_line_from<SIGN, PATH>(base + Lc * ld, tw, pl, tl, active, first(Lc), out(Lc));
+    }
+  } else {
+    const int TW = pl.team;
+    const int nteams = blockDim.x / TW;
+    const int team = threadIdx.x / TW;
+    const int tl = threadIdx.x - team * TW;
+    const int rounds = (nlines + nteams - 1) / nteams;
+    for (int r = 0; r < rounds; ++r) {
+      const int L = r * nteams + team;
+      const bool active = L < nlines;
+      const int Lc = active ? L : 0;
+      fft_line_from<SIGN>(base + Lc * ld, tw, pl, tl, active, first(Lc), out(Lc));
     }
   }
 }

@@ -70,20 +70,24 @@ __device__ __forceinline__ long long fx_mul(FxSplit a, FxSplit w) {
   const long long c = fx_mad(a.l, w.h, fx_mad(a.h, w.l, 1ll << 29));
   return fx_join(fx_mad(a.h, w.h, c >> 32), (uint32_t)c);
 }
+// with LOW, the low halves' products too (the long lines of the run-time
+// path, whose units in the last place are coarser against their norm)
+__device__ __forceinline__ long long fx_low(FxSplit a, FxSplit w) { return (long long)__mulhi(a.l, w.l); }
 // a * u + b * v, rounded once.  |a|, |b| < 2^62 with a^2 + b^2 < 2^124 and
 // u^2 + v^2 <= 1 (or |a| + |b| < 2^62 and |u| + |v| < 1.6) keep the cross
 // terms below 2^63.
-__device__ __forceinline__ long long fx_dot(FxSplit a, FxSplit b, FxSplit u, FxSplit v) {
-  const long long c = fx_mad(b.l, v.h, fx_mad(b.h, v.l, fx_mad(a.l, u.h, fx_mad(a.h, u.l, 1ll << 29))));
+template <bool LOW = false> __device__ __forceinline__ long long fx_dot(FxSplit a, FxSplit b, FxSplit u, FxSplit v) {
+  long long c = fx_mad(b.l, v.h, fx_mad(b.h, v.l, fx_mad(a.l, u.h, fx_mad(a.h, u.l, 1ll << 29))));
+  if (LOW) c += fx_low(a, u) + fx_low(b, v);
   return fx_join(fx_mad(b.h, v.h, fx_mad(a.h, u.h, c >> 32)), (uint32_t)c);
 }
 __device__ __forceinline__ FxSplit fx_neg(FxSplit w) { return FxSplit{-w.h, -w.l}; }
 
 // a * w (SIGN = -1) or a * conj(w) (SIGN = +1)
-template <int SIGN> __device__ __forceinline__ fxc ctw(fxc a, fxw w) {
+template <int SIGN, bool LOW = false> __device__ __forceinline__ fxc ctw(fxc a, fxw w) {
   const FxSplit x = fx_split(a.x), y = fx_split(a.y), u{w.xh, w.xl}, v{w.yh, w.yl}, nv = fx_neg(v);
-  if (SIGN < 0) return fxc{fx_dot(x, y, u, nv), fx_dot(x, y, v, u)};
-  return fxc{fx_dot(x, y, u, v), fx_dot(x, y, nv, u)};
+  if (SIGN < 0) return fxc{fx_dot<LOW>(x, y, u, nv), fx_dot<LOW>(x, y, v, u)};
+  return fxc{fx_dot<LOW>(x, y, u, v), fx_dot<LOW>(x, y, nv, u)};
 }
 // a * (cr + i ci) for constants
 __device__ __forceinline__ fxc fx_rot(fxc a, FxSplit cr, FxSplit ci) {
@@ -92,6 +96,12 @@ __device__ __forceinline__ fxc fx_rot(fxc a, FxSplit cr, FxSplit ci) {
 }
 template <int SIGN> __device__ __forceinline__ fxc cmul_si(fxc a) {
   return SIGN < 0 ? fxc{a.y, -a.x} : fxc{-a.y, a.x};
+}
+// constants of w9^J in units of 2^-62
+constexpr long long kFxC9[5] = {0, 3532756447825785444ll, 800810873071977681ll, 0, -4333567320897763126ll};
+constexpr long long kFxS9[5] = {0, 2964334632409774423ll, 4541624145405292212ll, 0, 1577289512995517789ll};
+template <int SIGN, int J> __device__ __forceinline__ fxc rot9(fxc v) {
+  return fx_rot(v, fx_const(kFxC9[J]), fx_const(SIGN * kFxS9[J]));
 }
 // v / 2, ties to even
 __device__ __forceinline__ long long fx_half(long long v) { return (v + ((v >> 1) & 1)) >> 1; }
@@ -226,9 +236,21 @@ constexpr int kFxNaN = 2;    // the line holds an infinity or a NaN
 // 2^kFxLift before the conversion (subnormals become normal numbers)
 constexpr int kFxTiny = 80, kFxLift = 256;
 
-// Reduction over the TW threads of a team (all threads of the CTA call it);
-// teams wider than a warp go through shared memory.
+// Reduction over the TW threads of a team (all threads of the CTA call it).
+// Teams of up to 32 threads lie within a warp, 32 / TW to a warp; wider ones
+// are whole warps and go through shared memory.
 template <typename V, typename Op> __device__ __forceinline__ V team_reduce(V v, int TW, Op op) {
+  if (TW < 32 && (TW & (TW - 1))) {
+    // not a power of two: folded onto the team's first lane, then broadcast
+    const int lane = threadIdx.x & 31, tl = lane % TW, base = lane - tl;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      if (o >= TW) continue;
+      const V t = __shfl_sync(0xffffffffu, v, (lane + o) & 31);
+      if (tl < o && tl + o < TW && base + tl + o < 32) v = op(v, t);
+    }
+    return __shfl_sync(0xffffffffu, v, base);
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1)
     if (o < TW) v = op(v, __shfl_xor_sync(0xffffffffu, v, o));

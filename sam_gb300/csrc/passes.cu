@@ -1,5 +1,5 @@
-// The FP64 instantiation of the transform passes (passes_impl.cuh) and the
-// precision-independent kernels: vel_max's completion and the x2z layout.
+// The kernels that no length specialises: vel_max's completion and wave-space
+// sums, the x2z layout.
 #include "passes_impl.cuh"
 
 namespace samgpu {
@@ -46,6 +46,5 @@ void launch_x2z(const double2* in, double2* out, const Grid& g, int nvar, int nx
   if (grid < 1) grid = 1;
   k_x2z<<<grid, kThreads, 0, s>>>(in, out, g, nvar, nx2);
 }
-SAMGPU_INST(double)
 
 }  // namespace samgpu

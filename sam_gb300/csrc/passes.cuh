@@ -1,5 +1,5 @@
 // Argument blocks and launchers of the transform passes (passes_impl.cuh,
-// instantiated in passes.cu, passes_f32.cu and passes_dd_*.cu).
+// instantiated in passes.cu and passes_f32.cu).
 // Strides are in complex (or real, for physical arrays) elements.
 #pragma once
 #include "common.cuh"
@@ -142,10 +142,6 @@ struct ZFwdArgs {
   long long u_ky, u_kx, u_n;
   DevState* state;
   StageConsts sc;
-  // double-float form, mode 2: the integrating factor exp(-nu k^2 dt_fac)
-  // as products of per-direction tables [2][Mx + My + Mz] (velocity, then
-  // temperature with nu / Pr), written by launch_if_tables for this stage
-  const dd* ift;
   // FP64 form, mode 2: rkz(k), then the integrating factors' kz part for the
   // velocity and for T, written by the stage's y-forward pass (null: formed
   // per mode)
@@ -154,45 +150,60 @@ struct ZFwdArgs {
   FastDiv fd_t, fd_m;  // filled by the launcher: ty, Nz_min
 };
 
+// A pass's kernels of one precision are compiled in `parts` units (passes_part.cu):
+// length i of the compile-time lengths in unit i % parts, the run-time path in
+// unit 0.
+__host__ __device__ constexpr int path_part(int n, int parts) {
+  if (!ct_length(n)) return 0;
+  int i = 0;
+  for (int m = 16; m < n; ++m) i += ct_length(m);
+  return i % parts;
+}
+template <typename T>
+inline int x_pass_blocks(const XPassArgs<T>& a) {
+  return a.g.nz * ((a.g.ny + a.yt - 1) / a.yt);
+}
+// the launch-time fields of the x pass's and the z-forward pass's argument
+// blocks (fast divisors, scales), shared by the launchers and the ensemble
+// stage recorder
+template <typename T>
+XPassArgs<T> prep_x_pass(const XPassArgs<T>& a0) {
+  XPassArgs<T> a = a0;
+  a.fd_mx = make_fastdiv(a.g.mx);
+  a.fd_yp = make_fastdiv(a.yt / 2);
+  a.fd_nx = make_fastdiv(a.g.nx);
+  a.fd_y = make_fastdiv(a.yt);
+  a.fn = (T)(0.5 / ((double)a.g.nx * (double)a.g.ny));
+  return a;
+}
+template <typename T>
+ZFwdArgs<T> prep_z_fwd(const ZFwdArgs<T>& a0) {
+  ZFwdArgs<T> a = a0;
+  a.fd_t = make_fastdiv(a.ty);
+  a.fd_m = make_fastdiv(a.g.mz);
+  a.nz_inv = (T)(1.0 / (double)a.g.nz);
+  return a;
+}
+
 template <typename T> void launch_z_inv(const ZInvArgs<T>& a, const FftPlan* pl, size_t smem, cudaStream_t s);
 template <typename T> void launch_y_inv(const YInvArgs<T>& a, const FftPlan* pl, size_t smem, cudaStream_t s);
 template <typename T> void launch_x_pass(const XPassArgs<T>& a, const FftPlan* pl, size_t smem, cudaStream_t s);
-template <typename T> int x_pass_blocks(const XPassArgs<T>& a);
+template <typename T> void launch_y_fwd(const YFwdArgs<T>& a, const FftPlan* pl, size_t smem, cudaStream_t s);
+template <typename T> void launch_z_fwd(const ZFwdArgs<T>& a, const FftPlan* pl, size_t smem, cudaStream_t s);
+// loads the pass kernels of precision T for a grid and opts them into the
+// device's largest dynamic shared memory (before anything is captured)
+template <typename T> void set_smem_limits(int nx, int ny, int nz);
 // Shared memory of an FP64 x pass with products behind its lines: scale and
 // norm of each of `in` input lines, scale of each of `prod` product lines.
 template <typename T> constexpr size_t x_extra(int out_mode, int in, int prod) {
   return std::is_same<T, double>::value && out_mode == 2 ? sizeof(FxLine) * in + sizeof(FxScale) * prod : 0;
 }
-template <typename T> void launch_y_fwd(const YFwdArgs<T>& a, const FftPlan* pl, size_t smem, cudaStream_t s);
-template <typename T> void launch_z_fwd(const ZFwdArgs<T>& a, const FftPlan* pl, size_t smem, cudaStream_t s);
-template <typename T> void smem_limits_zinv(int optin);
-template <typename T> void smem_limits_yinv(int optin);
-template <typename T> void smem_limits_x(int optin);
-template <typename T> void smem_limits_yfwd(int optin);
-template <typename T> void smem_limits_zfwd(int optin);
-// every pass of precision T opted into the device's largest dynamic shared memory
-template <typename T> inline void set_smem_limits() {
-  int dev = 0, optin = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  smem_limits_zinv<T>(optin);
-  smem_limits_yinv<T>(optin);
-  smem_limits_x<T>(optin);
-  smem_limits_yfwd<T>(optin);
-  smem_limits_zfwd<T>(optin);
-}
 // vmax (max_only forms): ints 0..7 hold the per-field maxima (FP32 form: the
-// float bit patterns in ints 0..3; double-float form: 64-bit keys of
-// dd_abs_key in ints 0..7, vkind = 1; FP64 form: bit patterns of doubles,
-// vkind = 2), int 8 the non-finite flag
+// float bit patterns in ints 0..3; FP64 form: bit patterns of doubles in ints
+// 0..7, vkind = 1), int 8 the non-finite flag
 void launch_vel_max_finish(const double* partials, int nblk, const Grid& g, DevState* st, int i_cfl, double cfl0,
                            double adv_cfl_limit, cudaStream_t s, const double* pv = nullptr, int npv = 0,
                            int* vmax = nullptr, int vkind = 0);
-// The double-float form's integrating-factor tables of one stage (mode-2
-// z forward): t[w * (Mx + My + Mz) + r] = exp(-nu_w dt_fac k_r^2) for the
-// wave numbers of kx (r < Mx), ky, then kz, with nu_0 = vis and nu_1 =
-// vis / Pr, dt_fac = (gamma + zeta) dt (sam.f:293-297), dt read on the device.
-void launch_if_tables(const DevState* st, const StageConsts& sc, const Grid& g, dd* t, cudaStream_t s);
 constexpr int kVmaxInts = 16;  // the vmax block at the end of pv
 // vel_max's sums from wave space (Parseval), FP64 arithmetic on the state U
 // (Lu fields (kx, ky, kz)): pv[b * Lu + f] = block b's share of

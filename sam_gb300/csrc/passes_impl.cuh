@@ -1,7 +1,6 @@
 // Kernel templates of the five HBM passes (included by the translation
 // units that instantiate them, one per working precision: passes.cu
-// (FP64, plus the precision-independent kernels), passes_f32.cu and
-// passes_dd.cu).
+// (FP64, plus the precision-independent kernels) and passes_f32.cu).
 // The five HBM passes of one RK3 stage and the reference-layout variants of
 // each transform.  Every pass moves a tile of pencils from HBM into shared
 // memory, transforms it there (fft_engine.cuh) and writes it back transposed
@@ -22,6 +21,7 @@
 #include <math.h>
 
 #include <type_traits>
+#include <utility>
 
 #include "common.cuh"
 #include "passes.cuh"
@@ -53,14 +53,7 @@ template <typename T, int K, int PATH = kFft256> struct MinBlocks {
       PATH == kFftGeneric ? (K == kPassX ? 1 : 2) : (K == kPassZFwd ? 2 : (K == kPassX ? 3 : (PATH == kFft256 ? (K == kPassYInv ? 5 : 4) : 3)));
 };
 template <int K, int PATH> struct MinBlocks<double, K, PATH> {
-  static constexpr int value = PATH == kFftGeneric || PATH == kFftLong ? 1 : 2;
-};
-// double-float pairs: the 16 x 16 register path holds 16 complex pairs (64
-// registers) per thread, as in FP64
-// (the z-forward epilogue keeps one CTA: its tiles fill the shared memory of
-// an SM anyway, and two modes' inputs in flight need the registers)
-template <int K, int PATH> struct MinBlocks<dd, K, PATH> {
-  static constexpr int value = PATH == kFftGeneric || K == kPassZFwd ? 1 : 2;
+  static constexpr int value = PATH == kFftGeneric ? 1 : 2;
 };
 template <typename V, typename Get, typename Put>
 __device__ __forceinline__ void batched(int count, Get get, Put put) {
@@ -79,13 +72,6 @@ __device__ __forceinline__ void batched(int count, Get get, Put put) {
   }
 }
 
-// v * s for a constant s of the launch: in the double-float form, when s is
-// a power of two (1/Nz, 1/(2 Nx Ny) on power-of-two grids), two exact FP32
-// products instead of a pair product
-template <typename W> __device__ __forceinline__ W scale_by(W v, W s, bool pow2) { return v * s; }
-template <> __device__ __forceinline__ dd scale_by<dd>(dd v, dd s, bool pow2) {
-  return pow2 ? dd(__fmul_rn(v.hi, s.hi), __fmul_rn(v.lo, s.hi)) : v * s;
-}
 __host__ __device__ inline bool is_pow2_inv(int n) { return n > 0 && (n & (n - 1)) == 0; }
 
 // First-stage loader reading element idx of a row in global memory.
@@ -307,10 +293,6 @@ __device__ __forceinline__ void store_pair(double2* o, double2 a, double2 b) {
   o[0] = a;
   o[1] = b;
 }
-__device__ __forceinline__ void store_pair(ddc* o, ddc a, ddc b) {
-  o[0] = a;
-  o[1] = b;
-}
 
 // First-stage loader of the backward x transform: the stored half spectrum
 // with the truncated band lo < idx < hi read as zero.
@@ -356,7 +338,6 @@ __device__ __forceinline__ DF df_add_sq(DF a, float v) {
 // on 2^20 random operand pairs, every differing result equalled fmaf.)
 __device__ __forceinline__ float pmul(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double pmul(double a, double b) { return a * b; }
-__device__ __forceinline__ dd pmul(dd a, dd b) { return a * b; }
 
 // First-stage loader of the forward x transform: element idx of line a, or,
 // when b is given, of line a times line b component by component (the two
@@ -507,7 +488,7 @@ __device__ __forceinline__ void x_pass_body(const XPassArgs<T>& a, const FftPlan
   // integers (ints), their scales and norms behind the lines (of subgrid
   // terms, doubles, a bound); the results of a product line stay integers
   // until they are stored
-  constexpr bool FX = kIsFx<C, PATH>;
+  constexpr bool FX = kIsFx<C>;
   const bool ints = FX && a.out_mode == 2;
   const int nfac = a.g.lu * yp;  // lines of factors
   FxLine* s_line = reinterpret_cast<FxLine*>(s_pr + (size_t)a.prod_lines * ld);
@@ -630,58 +611,7 @@ __device__ __forceinline__ void x_pass_body(const XPassArgs<T>& a, const FftPlan
   // ---- vel_max partial sums (vel_max.f:11-21), FP64-accurate,
   // deterministic order (FP64 arithmetic in the FP64 form; error-free FP32
   // pairs in the FP32 form, turned into FP64 per warp)
-  if constexpr (kIsDD<T>) {
-    if (a.partials) {
-      // the double-float form: max |u| as order-preserving 64-bit keys of
-      // the pairs (FP32 and integer work only), the non-finite flag; the
-      // sums come from wave space (k_parseval, FP64)
-      unsigned long long km[4] = {0ull, 0ull, 0ull, 0ull};
-      int bad = 0;
-      for (int e = threadIdx.x; e < yp * nx; e += blockDim.x) {
-        const int c = (int)fdiv(e, a.fd_nx), x = e - c * nx;
-        const bool ra = y0 + 2 * c < ny, rb = y0 + 2 * c + 1 < ny;
-#pragma unroll
-        for (int f = 0; f < 4; ++f)
-          if (f < a.g.lu) {
-            const C v = s_in[(f * yp + c) * ld + sidx(x)];
-            if (ra) {
-              km[f] = max(km[f], dd_abs_key(v.x));
-              bad |= !dd_isfinite(v.x);
-            }
-            if (rb) {
-              km[f] = max(km[f], dd_abs_key(v.y));
-              bad |= !dd_isfinite(v.y);
-            }
-          }
-      }
-      for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-        for (int f = 0; f < 4; ++f) km[f] = max(km[f], __shfl_xor_sync(0xffffffffu, km[f], o));
-        bad |= __shfl_xor_sync(0xffffffffu, bad, o);
-      }
-      const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-      unsigned long long* s_km = reinterpret_cast<unsigned long long*>(s_red);
-      int* s_bad = reinterpret_cast<int*>(s_km + 4 * nw);
-      if ((threadIdx.x & 31) == 0) {
-#pragma unroll
-        for (int f = 0; f < 4; ++f) s_km[w * 4 + f] = km[f];
-        s_bad[w] = bad;
-      }
-      __syncthreads();
-      if (threadIdx.x < a.g.lu) {
-        const int f = threadIdx.x;
-        unsigned long long tm = 0ull;
-        int tb = 0;
-        for (int k = 0; k < nw; ++k) {
-          tm = max(tm, s_km[k * 4 + f]);
-          tb |= s_bad[k];
-        }
-        atomicMax(reinterpret_cast<unsigned long long*>(a.vmax) + f, tm);
-        if (f == 0 && tb) atomicOr(a.vmax + 8, 1);
-      }
-      __syncthreads();
-    }
-  } else if (std::is_same<T, double>::value && a.partials && a.max_only) {
+  if (std::is_same<T, double>::value && a.partials && a.max_only) {
     // the FP64 step: max |u| of each line by one warp, as integers where the
     // line holds them, else as the bit patterns of non-negative doubles, which
     // compare alike; the sums come from wave space (k_parseval)
@@ -846,7 +776,6 @@ __device__ __forceinline__ void x_pass_body(const XPassArgs<T>& a, const FftPlan
   // ---- the closure's invariants (out_mode 4): inputs are S (6), dT/dx (3
   // when Lr = 9) and w (3)
   if (a.out_mode == 4) {
-    if constexpr (!kIsDD<T>) {  // (the double-float form has no closure)
     const int lr = a.g.lr;
     const T bz = (T)a.f_bz, n2 = (T)a.f_n2, dsq = (T)a.f_dsq, nu = (T)a.f_nu;
     for (int e = threadIdx.x; e < yp * nx; e += blockDim.x) {
@@ -882,13 +811,11 @@ __device__ __forceinline__ void x_pass_body(const XPassArgs<T>& a, const FftPlan
         store_features(a.feat, ((long long)z * ny + ya + 1) * nx + x, f);
       }
     }
-    }
     return;
   }
 
   // ---- subgrid stress: the gradient lines become -2 nu_t S and -kappa_t dT
   if (a.les) {
-    if constexpr (!kIsDD<T>) {  // (the double-float form has no closure)
     const int lu = a.g.lu, lr = a.g.lr;
     const T cds = a.les == 1 ? (T)a.les_cds[0] : (T)0, prt = (T)a.les_prt_inv;
     for (int e = threadIdx.x; e < yp * nx; e += blockDim.x) {
@@ -918,7 +845,6 @@ __device__ __forceinline__ void x_pass_body(const XPassArgs<T>& a, const FftPlan
 #pragma unroll
       for (int m = 0; m < 9; ++m)
         if (m < lr) s_in[((lu + m) * yp + c) * ld + sidx(x)] = mk<C>(sx[m], sy[m]);
-    }
     }
     __syncthreads();
   }
@@ -1032,8 +958,8 @@ __device__ __forceinline__ void x_pass_body(const XPassArgs<T>& a, const FftPlan
               }
             }
             if (!done) {
-              ve = mk<C>(scale_by(z1.x + z2.x, fn, fn_pow2), scale_by(z1.y - z2.y, fn, fn_pow2));
-              vo = mk<C>(scale_by(z1.y + z2.y, fn, fn_pow2), scale_by(z2.x - z1.x, fn, fn_pow2));
+              ve = mk<C>((z1.x + z2.x) * fn, (z1.y - z2.y) * fn);
+              vo = mk<C>((z1.y + z2.y) * fn, (z2.x - z1.x) * fn);
             }
             if (two) {
               if ((reinterpret_cast<uintptr_t>(o) & (2 * sizeof(C) - 1)) == 0) {
@@ -1538,7 +1464,7 @@ __device__ __forceinline__ void y_fwd_body(const YFwdArgs<T>& a, const FftPlan* 
   // the first stage reads its inputs straight from the rows of C (no
   // shared-memory staging); the rows are contiguous in y
   const auto rows = [&](int L) { return RowLoad<C, COH>{src + (long long)L * a.in_z}; };
-  if constexpr (kIsFx<C, PATH>)
+  if constexpr (kIsFx<C>)
     fft_lines_from<-1, PATH>(s_ln, ld, nl, s_tw, pl, rows,
                              [&](int L) { return FxOutBand{s_ln + L * ld, km, ny - km}; });
   else
@@ -1648,9 +1574,9 @@ __device__ __forceinline__ void epi_mode(const ZFwdArgs<T>& a, Val val, int i, i
   W s2r = rkx * tr[1] + rky * tr[2] + rkz * tr[4], s2i = rkx * ti[1] + rky * ti[2] + rkz * ti[4];
   W s3r = rkx * tr[3] + rky * tr[4] + rkz * tr[5], s3i = rkx * ti[3] + rky * ti[4] + rkz * ti[5];
   if (c.scale) {
-    s1r = scale_by(s1r, c.nz_inv, c.nz_pow2); s1i = scale_by(s1i, c.nz_inv, c.nz_pow2);
-    s2r = scale_by(s2r, c.nz_inv, c.nz_pow2); s2i = scale_by(s2i, c.nz_inv, c.nz_pow2);
-    s3r = scale_by(s3r, c.nz_inv, c.nz_pow2); s3i = scale_by(s3i, c.nz_inv, c.nz_pow2);
+    s1r = s1r * c.nz_inv; s1i = s1i * c.nz_inv;
+    s2r = s2r * c.nz_inv; s2i = s2i * c.nz_inv;
+    s3r = s3r * c.nz_inv; s3i = s3i * c.nz_inv;
   }
   W r1r = s1i, r1i = -s1r, r2r = s2i, r2i = -s2r, r3r = s3i, r3i = -s3r, r4r = (W)0, r4i = (W)0;
   if (sc.i_strat) {
@@ -1667,8 +1593,8 @@ __device__ __forceinline__ void epi_mode(const ZFwdArgs<T>& a, Val val, int i, i
     W s4r = rkx * tr[6] + rky * tr[7] + rkz * tr[8];
     W s4i = rkx * ti[6] + rky * ti[7] + rkz * ti[8];
     if (c.scale) {
-      s4r = scale_by(s4r, c.nz_inv, c.nz_pow2);
-      s4i = scale_by(s4i, c.nz_inv, c.nz_pow2);
+      s4r = s4r * c.nz_inv;
+      s4i = s4i * c.nz_inv;
     }
     r4r = s4i - c.lapse * wr;
     r4i = -s4r - c.lapse * wi;
@@ -1702,14 +1628,7 @@ __device__ __forceinline__ void epi_mode(const ZFwdArgs<T>& a, Val val, int i, i
   }
   const long long uidx = (long long)i * a.u_kx + (long long)j * a.u_ky + k;
   W ef, et;
-  if constexpr (kIsDD<W>) {
-    // exp(-nu_f k^2) = e(kx) e(ky) e(kz), tabulated for this stage in FP64
-    // and rounded to pairs (launch_if_tables)
-    const dd* tb = a.ift;
-    const int oy = g.mx, oz = g.mx + g.my, tw = g.mx + g.my + g.mz;
-    ef = tb[i] * tb[oy + j] * tb[oz + k];
-    et = c.same_t ? ef : tb[tw + i] * tb[tw + oy + j] * tb[tw + oz + k];
-  } else if (std::is_same<W, double>::value && a.kz_tab) {
+  if (std::is_same<W, double>::value && a.kz_tab) {
     ef = row.ef * (W)a.kz_tab[g.mz + k];
     et = c.same_t ? ef : row.et * (W)a.kz_tab[2 * g.mz + k];
   } else {
@@ -1762,7 +1681,7 @@ __device__ __forceinline__ void z_fwd_body(const ZFwdArgs<T>& a, const FftPlan* 
   // Fixed-point lines stay integers, their scales behind the tile's lines: of
   // Nz results only the Nz_min stored modes are converted, and 1/Nz, where
   // it is a power of two, costs nothing.
-  constexpr bool FX = kIsFx<C, PATH>;
+  constexpr bool FX = kIsFx<C>;
   const bool ints = FX && nz > 1 && a.mode != 0;
   FxScale* s_sc = reinterpret_cast<FxScale*>(s_ln + (size_t)nf * a.ty * ld);
   EpiRow<T>* s_row = reinterpret_cast<EpiRow<T>*>(s_sc + (std::is_same<T, double>::value ? nf * a.ty : 0));
@@ -1967,7 +1886,7 @@ void launch_parseval(const cx_t<T>* u, const Grid& g, double* pv, cudaStream_t s
   k_parseval<T><<<kParsevalBlocks, kThreads, 0, s>>>(u, g, pv);
 }
 // vel_max.f:28-49 on the per-CTA partials written by the x pass (or, in the
-// FP32 and double-float forms, on the wave-space sums and the max keys).
+// resident step, on the wave-space sums and the maxima).
 template <bool COH = false>
 __device__ __forceinline__ void vel_max_finish_body(const double* __restrict__ partials, int nblk, const Grid& g,
                                                     DevState* st, int i_cfl, double cfl0, double adv_cfl_limit,
@@ -2033,8 +1952,7 @@ __device__ __forceinline__ void vel_max_finish_body(const double* __restrict__ p
         fin[f][1] = red[0] * n;
         const unsigned long long key =
             vkind ? ldc<COH>(reinterpret_cast<const unsigned long long*>(vmax) + f) : 0ull;
-        fin[f][2] = vkind == 2 ? __longlong_as_double((long long)key)
-                               : (vkind ? dd_key_value(key) : (double)__int_as_float(ldc<COH>(vmax + f)));
+        fin[f][2] = vkind ? __longlong_as_double((long long)key) : (double)__int_as_float(ldc<COH>(vmax + f));
         fin[f][3] = (double)ldc<COH>(vmax + 8);
       }
       __syncthreads();
@@ -2067,110 +1985,87 @@ __device__ __forceinline__ void vel_max_finish_body(const double* __restrict__ p
 }
 
 // ------------------------------------------------------------------ launchers
+// The lengths with a compile-time path (ct_length), by their place in the list.
+constexpr int ct_count() {
+  int c = 0;
+  for (int n = 16; n <= 512; ++n) c += ct_length(n);
+  return c;
+}
+constexpr int kCtCount = ct_count();
+constexpr int ct_nth(int i) {
+  for (int n = 16; n <= 512; ++n)
+    if (ct_length(n) && i-- == 0) return n;
+  return 0;
+}
+template <int PART, int PARTS, bool EVEN, typename F, int... I>
+void with_ct_path(int n, F f, std::integer_sequence<int, I...>) {
+  auto one = [&](auto i) {
+    constexpr int k = decltype(i)::value;
+    if constexpr (k % PARTS == PART && ct_nth(k) != 256 && !(EVEN && ct_nth(k) % 2))
+      if (n == ct_nth(k)) f(std::integral_constant<int, ct_nth(k)>());
+  };
+  (one(std::integral_constant<int, I>()), ...);
+}
 // Calls f with the code path (an integral constant) that lines of length n
-// take in precision T; sched = 1 is the Stockham schedule of length 256.
-template <typename T, typename F> void with_path(int n, int sched, F f) {
-  using std::integral_constant;
-  switch (n) {
-    case 256:
-      if (sched == 1) f(integral_constant<int, 256>());
-      else f(integral_constant<int, kFft256>());
-      return;
-    case 32: f(integral_constant<int, 32>()); return;
-    case 64: f(integral_constant<int, 64>()); return;
-    case 96: f(integral_constant<int, 96>()); return;
-    case 128: f(integral_constant<int, 128>()); return;
-    case 512: f(integral_constant<int, 512>()); return;
-  }
-  if constexpr (std::is_same<T, double>::value) {
-    if (n > kFxMaxLine) {
-      f(integral_constant<int, kFftLong>());
+// take; sched = 1 is the Stockham schedule of length 256.  Lengths of other
+// units are passed over (EVEN: odd ones too, Nx is even).
+template <int PART, int PARTS, bool EVEN = false, typename F> void with_path(int n, int sched, F f) {
+  if constexpr (path_part(256, PARTS) == PART) {
+    if (n == 256) {
+      if (sched == 1) f(std::integral_constant<int, 256>());
+      else f(std::integral_constant<int, kFft256>());
       return;
     }
   }
-  f(integral_constant<int, kFftGeneric>());
-}
-// Calls f with every code path of precision T.
-template <typename T, typename F> void each_path(F f) {
-  for (int n : {32, 64, 96, 128, 256, 512, 17, kFxMaxLine + 1}) with_path<T>(n, 0, f);
-  with_path<T>(256, 1, f);
+  if (ct_length(n)) with_ct_path<PART, PARTS, EVEN>(n, f, std::make_integer_sequence<int, kCtCount>());
+  else if constexpr (PART == 0) f(std::integral_constant<int, kFftGeneric>());
 }
 
-template <typename T>
-void launch_z_inv(const ZInvArgs<T>& a0, const FftPlan* pl, size_t smem, cudaStream_t s) {
-  const ZInvArgs<T> a = a0;
+template <typename T, int PART, int PARTS>
+void launch_z_inv_part(const ZInvArgs<T>& a, const FftPlan* pl, size_t smem, cudaStream_t s) {
   const int grid = a.nvar * a.g.mx * ((a.g.my + a.ty - 1) / a.ty);
-  with_path<T>(a.g.nz, a.sched,
-               [&](auto p) { k_z_inv<T, decltype(p)::value><<<grid, kThreads, smem, s>>>(a, pl); });
+  with_path<PART, PARTS>(a.g.nz, a.sched,
+                         [&](auto p) { k_z_inv<T, decltype(p)::value><<<grid, kThreads, smem, s>>>(a, pl); });
 }
-template <typename T>
-void launch_y_inv(const YInvArgs<T>& a0, const FftPlan* pl, size_t smem, cudaStream_t s) {
-  const YInvArgs<T> a = a0;
+template <typename T, int PART, int PARTS>
+void launch_y_inv_part(const YInvArgs<T>& a, const FftPlan* pl, size_t smem, cudaStream_t s) {
   const int grid = a.nvar * a.g.nz * ((a.g.mx + a.tx - 1) / a.tx);
-  with_path<T>(a.g.ny, a.sched,
-               [&](auto p) { k_y_inv<T, decltype(p)::value><<<grid, kThreads, smem, s>>>(a, pl); });
+  with_path<PART, PARTS>(a.g.ny, a.sched,
+                         [&](auto p) { k_y_inv<T, decltype(p)::value><<<grid, kThreads, smem, s>>>(a, pl); });
 }
-template <typename T>
-int x_pass_blocks(const XPassArgs<T>& a) {
-  return a.g.nz * ((a.g.ny + a.yt - 1) / a.yt);
-}
-// the launch-time fields of the x pass's and the z-forward pass's argument
-// blocks (fast divisors, scales), shared by the launchers and the ensemble
-// stage recorder
-template <typename T>
-XPassArgs<T> prep_x_pass(const XPassArgs<T>& a0) {
-  XPassArgs<T> a = a0;
-  a.fd_mx = make_fastdiv(a.g.mx);
-  a.fd_yp = make_fastdiv(a.yt / 2);
-  a.fd_nx = make_fastdiv(a.g.nx);
-  a.fd_y = make_fastdiv(a.yt);
-  a.fn = (T)(0.5 / ((double)a.g.nx * (double)a.g.ny));
-  return a;
-}
-template <typename T>
-ZFwdArgs<T> prep_z_fwd(const ZFwdArgs<T>& a0) {
-  ZFwdArgs<T> a = a0;
-  a.fd_t = make_fastdiv(a.ty);
-  a.fd_m = make_fastdiv(a.g.mz);
-  a.nz_inv = (T)(1.0 / (double)a.g.nz);
-  return a;
-}
-
-template <typename T>
-void launch_x_pass(const XPassArgs<T>& a0, const FftPlan* pl, size_t smem, cudaStream_t s) {
-  const XPassArgs<T> a = prep_x_pass(a0);
-  if constexpr (std::is_same<T, float>::value) {
-    const size_t fsm = x_f256_smem(a.nin * (a.yt / 2));
-    if (x_f256_applies(a) && fsm <= (size_t)smem_optin()) {
-      k_x_pass_f256<><<<x_pass_blocks(a), kXf256Threads, fsm, s>>>(a);
-      return;
+template <typename T, int PART, int PARTS>
+void launch_x_pass_part(const XPassArgs<T>& a, const FftPlan* pl, size_t smem, cudaStream_t s) {
+  if constexpr (path_part(256, PARTS) == PART) {
+    if constexpr (std::is_same<T, float>::value) {
+      const size_t fsm = x_f256_smem(a.nin * (a.yt / 2));
+      if (x_f256_applies(a) && fsm <= (size_t)smem_optin()) {
+        k_x_pass_f256<><<<x_pass_blocks(a), kXf256Threads, fsm, s>>>(a);
+        return;
+      }
+    } else {
+      const size_t fsm = x_fx256_smem(a.nin * (a.yt / 2));
+      if (x_fx256_applies(a) && fsm <= (size_t)smem_optin() - 1024) {
+        k_x_pass_fx256<><<<x_pass_blocks(a), kXfx256Threads, fsm, s>>>(a);
+        return;
+      }
     }
   }
-  if constexpr (std::is_same<T, double>::value) {
-    const size_t fsm = x_fx256_smem(a.nin * (a.yt / 2));
-    if (x_fx256_applies(a) && fsm <= (size_t)smem_optin() - 1024) {
-      k_x_pass_fx256<><<<x_pass_blocks(a), kXfx256Threads, fsm, s>>>(a);
-      return;
-    }
-  }
-  with_path<T>(a.g.nx, a.sched, [&](auto p) {
+  with_path<PART, PARTS, true>(a.g.nx, a.sched, [&](auto p) {
     constexpr int PATH = decltype(p)::value;
     k_x_pass<T, PATH><<<x_pass_blocks(a), x_threads(sizeof(T), PATH == kFft256), smem, s>>>(a, pl);
   });
 }
-template <typename T>
-void launch_y_fwd(const YFwdArgs<T>& a0, const FftPlan* pl, size_t smem, cudaStream_t s) {
-  const YFwdArgs<T> a = a0;
+template <typename T, int PART, int PARTS>
+void launch_y_fwd_part(const YFwdArgs<T>& a, const FftPlan* pl, size_t smem, cudaStream_t s) {
   const int grid = a.nvar * a.g.mx * ((a.g.nz + a.tz - 1) / a.tz);
-  with_path<T>(a.g.ny, a.sched,
-               [&](auto p) { k_y_fwd<T, decltype(p)::value><<<grid, kThreads, smem, s>>>(a, pl); });
+  with_path<PART, PARTS>(a.g.ny, a.sched,
+                         [&](auto p) { k_y_fwd<T, decltype(p)::value><<<grid, kThreads, smem, s>>>(a, pl); });
 }
-template <typename T>
-void launch_z_fwd(const ZFwdArgs<T>& a0, const FftPlan* pl, size_t smem, cudaStream_t s) {
-  const ZFwdArgs<T> a = prep_z_fwd(a0);
+template <typename T, int PART, int PARTS>
+void launch_z_fwd_part(const ZFwdArgs<T>& a, const FftPlan* pl, size_t smem, cudaStream_t s) {
   const int grid = a.g.mx * ((a.g.my + a.ty - 1) / a.ty);
-  with_path<T>(a.g.nz, a.sched,
-               [&](auto p) { k_z_fwd<T, decltype(p)::value><<<grid, kThreads, smem, s>>>(a, pl); });
+  with_path<PART, PARTS>(a.g.nz, a.sched,
+                         [&](auto p) { k_z_fwd<T, decltype(p)::value><<<grid, kThreads, smem, s>>>(a, pl); });
 }
 static inline void allow_dynamic_smem(const void* fn, int optin) {
   cudaFuncAttributes at;
@@ -2178,49 +2073,34 @@ static inline void allow_dynamic_smem(const void* fn, int optin) {
   cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)at.sharedSizeBytes);
 }
 
-// Opt every pass into the largest dynamic shared memory the device allows
-// (the per-block opt-in limit less the kernel's static shared memory), per
-// group of passes (each group is instantiated in its own translation unit).
-template <typename T>
-void smem_limits_zinv(int optin) {
-  each_path<T>([&](auto p) { allow_dynamic_smem((const void*)k_z_inv<T, decltype(p)::value>, optin); });
+// Load the kernels a pass along length n runs and opt them into the largest
+// dynamic shared memory the device allows (the per-block opt-in limit less the
+// kernel's static shared memory).
+template <int PART, int PARTS, bool EVEN = false, typename F> void each_sched(int n, F f) {
+  with_path<PART, PARTS, EVEN>(n, 0, f);
+  if (n == 256) with_path<PART, PARTS, EVEN>(n, 1, f);
 }
-template <typename T>
-void smem_limits_yinv(int optin) {
-  each_path<T>([&](auto p) { allow_dynamic_smem((const void*)k_y_inv<T, decltype(p)::value>, optin); });
+template <typename T, int PART, int PARTS> void smem_zinv_part(int n, int optin) {
+  each_sched<PART, PARTS>(n, [&](auto p) { allow_dynamic_smem((const void*)k_z_inv<T, decltype(p)::value>, optin); });
 }
-template <typename T>
-void smem_limits_x(int optin) {
-  if constexpr (std::is_same<T, float>::value) allow_dynamic_smem((const void*)k_x_pass_f256<>, optin);
-  if constexpr (std::is_same<T, double>::value) allow_dynamic_smem((const void*)k_x_pass_fx256<>, optin);
-  each_path<T>([&](auto p) { allow_dynamic_smem((const void*)k_x_pass<T, decltype(p)::value>, optin); });
+template <typename T, int PART, int PARTS> void smem_yinv_part(int n, int optin) {
+  each_sched<PART, PARTS>(n, [&](auto p) { allow_dynamic_smem((const void*)k_y_inv<T, decltype(p)::value>, optin); });
 }
-template <typename T>
-void smem_limits_yfwd(int optin) {
-  each_path<T>([&](auto p) { allow_dynamic_smem((const void*)k_y_fwd<T, decltype(p)::value>, optin); });
+template <typename T, int PART, int PARTS> void smem_x_part(int n, int optin) {
+  if constexpr (path_part(256, PARTS) == PART) {
+    if constexpr (std::is_same<T, float>::value) {
+      if (n == 256) allow_dynamic_smem((const void*)k_x_pass_f256<>, optin);
+    } else {
+      if (n == 256) allow_dynamic_smem((const void*)k_x_pass_fx256<>, optin);
+    }
+  }
+  each_sched<PART, PARTS, true>(n, [&](auto p) { allow_dynamic_smem((const void*)k_x_pass<T, decltype(p)::value>, optin); });
 }
-template <typename T>
-void smem_limits_zfwd(int optin) {
-  each_path<T>([&](auto p) { allow_dynamic_smem((const void*)k_z_fwd<T, decltype(p)::value>, optin); });
+template <typename T, int PART, int PARTS> void smem_yfwd_part(int n, int optin) {
+  each_sched<PART, PARTS>(n, [&](auto p) { allow_dynamic_smem((const void*)k_y_fwd<T, decltype(p)::value>, optin); });
 }
-
-#define SAMGPU_INST_ZINV(T)                                                                   \
-  template void launch_z_inv<T>(const ZInvArgs<T>&, const FftPlan*, size_t, cudaStream_t);     \
-  template void smem_limits_zinv<T>(int);
-#define SAMGPU_INST_YINV(T)                                                                   \
-  template void launch_y_inv<T>(const YInvArgs<T>&, const FftPlan*, size_t, cudaStream_t);     \
-  template void smem_limits_yinv<T>(int);
-#define SAMGPU_INST_X(T)                                                                      \
-  template void launch_x_pass<T>(const XPassArgs<T>&, const FftPlan*, size_t, cudaStream_t);   \
-  template int x_pass_blocks<T>(const XPassArgs<T>&);                                          \
-  template void smem_limits_x<T>(int);
-#define SAMGPU_INST_YFWD(T)                                                                   \
-  template void launch_y_fwd<T>(const YFwdArgs<T>&, const FftPlan*, size_t, cudaStream_t);     \
-  template void smem_limits_yfwd<T>(int);
-#define SAMGPU_INST_ZFWD(T)                                                                   \
-  template void launch_z_fwd<T>(const ZFwdArgs<T>&, const FftPlan*, size_t, cudaStream_t);     \
-  template void smem_limits_zfwd<T>(int);
-#define SAMGPU_INST(T) \
-  SAMGPU_INST_ZINV(T) SAMGPU_INST_YINV(T) SAMGPU_INST_X(T) SAMGPU_INST_YFWD(T) SAMGPU_INST_ZFWD(T)
+template <typename T, int PART, int PARTS> void smem_zfwd_part(int n, int optin) {
+  each_sched<PART, PARTS>(n, [&](auto p) { allow_dynamic_smem((const void*)k_z_fwd<T, decltype(p)::value>, optin); });
+}
 
 }  // namespace samgpu

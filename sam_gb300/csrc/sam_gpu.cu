@@ -51,26 +51,12 @@ struct Plan {
   FftPlan* d = nullptr;
   fxw* tw64 = nullptr;
   float2* tw32 = nullptr;
-  ddc* twdd = nullptr;
 };
-
-// the nearest double-float pair to an extended-precision value
-static dd dd_of(long double v) {
-  const float h = (float)v;
-  return dd(h, (float)(v - (long double)h));
-}
 
 // exp(-i a) = (c, sn) as the FP64 form's fixed-point twiddle, in units of
 // 2^-62; a low half of exactly -2^31 (whose negation does not fit) is moved
 // by one unit
-static fxw fxw_of(int n, long double c, long double sn) {
-  if (n > kFxMaxLine) {
-    // the table of a length whose lines run in FP64 arithmetic
-    const double2 d = make_double2((double)c, (double)sn);
-    fxw w;
-    memcpy(&w, &d, sizeof(w));
-    return w;
-  }
+static fxw fxw_of(long double c, long double sn) {
   auto part = [](long double v, int& h, int& l) {
     long long q = llroundl(v * 4611686018427387904.0L);
     if ((uint32_t)q == 0x80000000u) ++q;
@@ -83,8 +69,11 @@ static fxw fxw_of(int n, long double c, long double sn) {
   return w;
 }
 
-// Radices 8, 4, 2, 3, 5 in that order; twiddles w_{l p}^{f q} = exp(-2 pi i
-// f q / (l p)) in long double, rounded once to each working precision.
+// The twiddles w_{l p}^{f q} = exp(-2 pi i f q / (l p)) of the lengths'
+// transforms, in long double, rounded once to each working precision: first
+// the table that the pass kernels of the length load (its compile-time
+// stages, ct_plan; for n = 256 the 16 x 16 table), then the run-time stages'
+// (radices 8, 4, 2, 3, 5 in that order).
 static int build_plan(int n, Plan& P) {
   FftPlan& pl = P.h;
   memset(&pl, 0, sizeof(pl));
@@ -97,8 +86,8 @@ static int build_plan(int n, Plan& P) {
   while (r % 5 == 0) { fac[ns++] = 5; r /= 5; }
   if (r != 1 || ns > 10 || n > 1024) return fail(SAM_GPU_EINVAL, "FFT length %d must be 2^a 3^b 5^c <= 1024", n);
   pl.nst = ns;
-  // team width: a power of two such that no thread holds more than emax
-  // values in any stage (Emax in fft_engine.cuh)
+  // team width of the run-time stages: a power of two such that no thread
+  // holds more than emax values in any stage (Emax in fft_engine.cuh)
   auto team_for = [&](int emax) {
     int TW = 1;
     while (TW * emax < n) TW *= 2;
@@ -113,76 +102,60 @@ static int build_plan(int n, Plan& P) {
     }
   };
   pl.team = team_for(8);
-  pl.team_sp = team_for(8);
   if (pl.team > kThreads) return fail(SAM_GPU_EINVAL, "FFT length %d needs too wide a team", n);
   std::vector<fxw> t64;
   std::vector<float2> t32;
-  std::vector<ddc> tdd;
-  int l = 1, off = 0;
   const long double two_pi = 6.283185307179586476925286766559005768L;
+  auto push = [&](long e, long m) {  // exp(-2 pi i e / m)
+    const long double a = two_pi * (long double)(e % m) / (long double)m;
+    const long double c = cosl(a), sn = -sinl(a);
+    t64.push_back(fxw_of(c, sn));
+    t32.push_back(make_float2((float)c, (float)sn));
+  };
   pl.tw16_off = -1;
   if (n == 256) {
     // the 16 x 16 register path (fft256_lines): w_256^{f q}, f, q in [0, 16),
-    // stored q-major so the 16 threads of a team read 16 consecutive entries;
-    // first in the table, so that kernels compiled for that path load only it
+    // stored q-major so the 16 threads of a team read 16 consecutive entries
     pl.tw16_off = 0;
     for (int q = 0; q < 16; ++q)
-      for (int f = 0; f < 16; ++f) {
-        const long double a = two_pi * (long double)((f * q) % 256) / 256.0L;
-        const long double c = cosl(a), sn = -sinl(a);
-        t64.push_back(fxw_of(n, c, sn));
-        t32.push_back(make_float2((float)c, (float)sn));
-        tdd.push_back(ddc{dd_of(c), dd_of(sn)});
-      }
-    off = 256;
+      for (int f = 0; f < 16; ++f) push((long)f * q, 256);
+  } else if (ct_length(n)) {
+    const CtPlan cp = ct_plan(n);
+    for (int s = 0, l = 1; s < cp.nst; l *= cp.r[s++])
+      for (int f = 0; f < l && s > 0; ++f)
+        for (int q = 1; q < cp.r[s]; ++q) push((long)f * q, (long)l * cp.r[s]);
   }
-  for (int s = 0; s < ns; ++s) {
-    const int p = fac[s];
+  const int head = (int)t64.size();
+  for (int s = 0, l = 1; s < ns; l *= fac[s++]) {
     FftStage& st = pl.st[s];
-    st.p = p;
+    st.p = fac[s];
     st.l = l;
-    st.m = n / (l * p);
-    st.tw_off = off;
+    st.m = n / (l * st.p);
+    st.tw_off = (int)t64.size();
     st.mmul = (uint32_t)(((1u << 21) + (uint32_t)st.m - 1) / (uint32_t)st.m);
     for (int f = 0; f < l; ++f)
-      for (int q = 1; q < p; ++q) {
-        const long e = ((long)f * q) % ((long)l * p);
-        const long double a = two_pi * (long double)e / (long double)(l * p);
-        const long double c = cosl(a), sn = -sinl(a);
-        t64.push_back(fxw_of(n, c, sn));
-        t32.push_back(make_float2((float)c, (float)sn));
-        tdd.push_back(ddc{dd_of(c), dd_of(sn)});
-      }
-    off += l * (p - 1);
-    l *= p;
+      for (int q = 1; q < st.p; ++q) push((long)f * q, (long)l * st.p);
   }
-  pl.tw_total = off;
-  pl.tw_pass = n == 256 ? 256 : off;
-  if (t64.empty()) {
-    t64.push_back(fxw_of(n, 1, 0));
-    t32.push_back(make_float2(1, 0));
-    tdd.push_back(ddc{dd(1), dd(0)});
-  }
+  pl.tw_total = (int)t64.size();
+  pl.tw_pass = ct_length(n) ? head : pl.tw_total;
+  if (t64.empty()) push(0, 1);
   CK(cudaMalloc(&P.d, sizeof(FftPlan)));
   CK(cudaMemcpy(P.d, &pl, sizeof(FftPlan), cudaMemcpyHostToDevice));
   CK(cudaMalloc(&P.tw64, sizeof(fxw) * t64.size()));
   CK(cudaMemcpy(P.tw64, t64.data(), sizeof(fxw) * t64.size(), cudaMemcpyHostToDevice));
   CK(cudaMalloc(&P.tw32, sizeof(float2) * t32.size()));
   CK(cudaMemcpy(P.tw32, t32.data(), sizeof(float2) * t32.size(), cudaMemcpyHostToDevice));
-  CK(cudaMalloc(&P.twdd, sizeof(ddc) * tdd.size()));
-  CK(cudaMemcpy(P.twdd, tdd.data(), sizeof(ddc) * tdd.size(), cudaMemcpyHostToDevice));
   return 0;
 }
 
 static void free_plan(Plan& P) {
-  cudaFree(P.d); cudaFree(P.tw64); cudaFree(P.tw32); cudaFree(P.twdd);
-  P.d = nullptr; P.tw64 = nullptr; P.tw32 = nullptr; P.twdd = nullptr;
+  cudaFree(P.d); cudaFree(P.tw64); cudaFree(P.tw32);
+  P.d = nullptr; P.tw64 = nullptr; P.tw32 = nullptr;
 }
 
 template <typename T> const tw_t<T>* tw_of(const Plan& P);
 template <> const fxw* tw_of<double>(const Plan& P) { return P.tw64; }
 template <> const float2* tw_of<float>(const Plan& P) { return P.tw32; }
-template <> const ddc* tw_of<dd>(const Plan& P) { return P.twdd; }
 
 // -------------------------------------------------------------- the context
 struct Scratch {
@@ -192,6 +165,7 @@ struct Scratch {
 
 struct Ctx {
   sam_gpu_config cfg{};
+  bool plain_only = false;  // precision kPrecDD: the FP64 form's kernels, plain step only
   Grid g{};
   int nx2 = 0, lm = 0, k_cl = 0;
   double gamma[4] = {0, 0, 0, 0}, zeta[4] = {0, 0, 0, 0}, adv_cfl_limit = 1.0;
@@ -203,8 +177,7 @@ struct Ctx {
   void *U = nullptr, *R = nullptr, *P = nullptr, *S1 = nullptr, *S2 = nullptr, *S3 = nullptr;
   double* partials = nullptr;
   int partial_blocks = 0;
-  double* pv = nullptr;  // vel_max's wave-space sums (FP32 and double-float forms)
-  dd* ift = nullptr;     // double-float form: integrating-factor tables of the stage
+  double* pv = nullptr;  // vel_max's wave-space sums
   double* kz_tab = nullptr;  // FP64 form: kz wave numbers and integrating factors of the stage (3 Mz)
   DevState* state = nullptr;
   Scratch sc[4];
@@ -282,11 +255,9 @@ static size_t csize(const Ctx& c) { return c.cfg.precision == 32 ? sizeof(float2
 // values (no-ops in the FP64 form, whose state is the copy).
 static void state_from_fp64(Ctx& c, const double2* src, void* dst, long long n) {
   if (c.cfg.precision == 32) convert_in<float>(src, (float2*)dst, n, c.stream);
-  else if (c.cfg.precision == kPrecDD) convert_in<dd>(src, (ddc*)dst, n, c.stream);
 }
 static void state_to_fp64(Ctx& c, const void* src, double2* dst, long long n) {
   if (c.cfg.precision == 32) convert_out<float>((const float2*)src, dst, n, c.stream);
-  else if (c.cfg.precision == kPrecDD) convert_out<dd>((const ddc*)src, dst, n, c.stream);
 }
 
 static int line_ld(int n) { return line_stride(n); }
@@ -296,6 +267,13 @@ static int line_ld(int n) { return line_stride(n); }
 static size_t tile_smem(const Plan& P, int lines, size_t es, int sched = 0) {
   const int ntw = sched == 1 && P.h.n == 256 ? P.h.tw_total : P.h.tw_pass;
   return es * ((size_t)ntw + (size_t)lines * line_ld(P.h.n)) + 16;
+}
+
+// lines that a CTA of `threads` threads transforms at once
+static int lines_at_once(const Plan& P, int threads, int sched) {
+  if (P.h.n == 256 && sched != 1) return threads / 16;
+  if (ct_length(P.h.n)) return ct_teams(ct_plan(P.h.n).tw, threads);
+  return std::max(threads / P.h.team, 1);
 }
 
 // dynamic shared memory budget of one CTA: the opt-in limit (227 KB on
@@ -382,8 +360,7 @@ static int x_tile(Ctx& c, int nin, int out_mode, int& yt, int& grp) {
   const size_t es = sizeof(cx_t<T>);
   const size_t prod_extra = x_extra<T>(out_mode, 0, 1);
   const int threads = x_threads((int)sizeof(T), x_reg16(c));
-  const int team = x_reg16(c) ? 16 : (sizeof(T) == 4 ? c.px.h.team_sp : c.px.h.team);
-  const int teams = threads / team > 0 ? threads / team : 1;
+  const int teams = lines_at_once(c.px, threads, c.sched[2]);
   // FP32 tiles leave room for three CTAs per SM (72 registers each; two
   // CTAs with 16-row tiles measured slower), FP64 tiles for two (up to 128
   // registers each): the FP64 pipe needs the second CTA's warps to cover its
@@ -406,6 +383,14 @@ static int x_tile(Ctx& c, int nin, int out_mode, int& yt, int& grp) {
     }
     if (yt <= 2) return fail(SAM_GPU_EINVAL, "x pass does not fit in shared memory (Nx=%d)", c.g.nx);
   }
+}
+
+// FP64 z-forward tiles that leave room for two CTAs per SM: one CTA's
+// fixed-point transforms overlap the other's FP64 epilogue (256^3: 2 rows
+// 0.92 ms, 4 rows, one CTA, 1.09; 128^3: 4 rows, two CTAs, 0.143, 2 rows 0.157).
+static void default_tiles(Ctx& c) {
+  if (c.cfg.precision == 64)
+    while (c.ty_zf > 1 && tile_smem(c.pz, c.ty_zf * c.g.lr, sizeof(double2)) > kSmemMax / 2 - 1024) c.ty_zf /= 2;
 }
 
 template <typename T>
@@ -481,7 +466,7 @@ static int run_x_pass(Ctx& c, int in_mode, int out_mode, int nin, const void* in
     if (a.max_only) launch_parseval<T>((const cx_t<T>*)c.U, c.g, c.pv, c.stream);
     launch_vel_max_finish(c.partials, nblk, c.g, c.state, c.cfg.i_cfl, c.cfg.cfl0, c.adv_cfl_limit, c.stream,
                           a.max_only ? c.pv : nullptr, kParsevalBlocks, a.vmax,
-                          kIsDD<T> ? 1 : (std::is_same<T, double>::value ? 2 : 0));
+                          std::is_same<T, double>::value ? 1 : 0);
   }
   return 0;
 }
@@ -551,10 +536,6 @@ static int run_z_fwd(Ctx& c, ZFwdArgs<T>& a) {
     return tile_smem(c.pz, ty * a.nf, sizeof(cx_t<T>), a.sched) + z_fwd_extra<T>(a.mode, a.nf, ty);
   };
   for (a.ty = c.ty_zf; a.ty > 1 && bytes(a.ty) > kSmemMax;) a.ty /= 2;
-  if (kIsDD<T> && a.mode == 2) {
-    launch_if_tables(c.state, a.sc, c.g, c.ift, c.stream);
-    a.ift = c.ift;
-  }
   const size_t smem = bytes(a.ty);
   if constexpr (std::is_same<T, float>::value) {
     if (c.rec) {
@@ -602,15 +583,13 @@ static int enqueue_stage(Ctx& c, int nrk, cudaEvent_t* ev, int only, int write_p
   if (ev) cudaEventRecord(ev[2], c.stream);
   // dynamic closure at nrk = 1 (once per step, like vel_max): the physical
   // velocity, then dm.f's coefficient on it
-  if constexpr (!kIsDD<T>) {  // (the double-float form has no closure)
-    if (run(2) && c.les_model == 2 && nrk == 1) {
-      rc = run_x_pass<T>(c, 0, 0, 3, c.S2, nullptr, g.mx, (long long)g.ny * g.mx, (long long)g.nz * g.ny * g.mx,
-                         nullptr, c.les_phys, 0, 0, 0, g.nx, (long long)g.nx * g.ny, (long long)g.nx * g.ny * g.nz,
-                         false);
-      if (rc) return rc;
-      les_dynamic<T>((const T*)c.les_phys, c.les_work, c.les_cds, g.nx, g.ny, g.nz, c.les_dxi, c.les_dyi, c.les_dzi,
-                     c.stream);
-    }
+  if (run(2) && c.les_model == 2 && nrk == 1) {
+    rc = run_x_pass<T>(c, 0, 0, 3, c.S2, nullptr, g.mx, (long long)g.ny * g.mx, (long long)g.nz * g.ny * g.mx,
+                       nullptr, c.les_phys, 0, 0, 0, g.nx, (long long)g.nx * g.ny, (long long)g.nx * g.ny * g.nz,
+                       false);
+    if (rc) return rc;
+    les_dynamic<T>((const T*)c.les_phys, c.les_work, c.les_cds, g.nx, g.ny, g.nz, c.les_dxi, c.les_dyi, c.les_dzi,
+                   c.stream);
   }
   // learned closure: the invariants of every point, then the network
   if (run(2) && coef_stage) {
@@ -660,7 +639,6 @@ static int enqueue_stage(Ctx& c, int nrk, cudaEvent_t* ev, int only, int write_p
 
 static int stage_any(Ctx& c, int nrk, cudaEvent_t* ev = nullptr, int only = -1, int write_p = 1) {
   if (c.cfg.precision == 32) return enqueue_stage<float>(c, nrk, ev, only, write_p);
-  if (c.cfg.precision == kPrecDD) return enqueue_stage<dd>(c, nrk, ev, only, write_p);
   return enqueue_stage<double>(c, nrk, ev, only, write_p);
 }
 
@@ -681,7 +659,7 @@ static void free_ctx(Ctx* c) {
   free_plan(c->px); free_plan(c->py); free_plan(c->pz);
   cudaFree(c->U); cudaFree(c->R); cudaFree(c->P);
   cudaFree(c->S1); cudaFree(c->S2); cudaFree(c->S3);
-  cudaFree(c->partials); cudaFree(c->state); cudaFree(c->ou); cudaFree(c->pv); cudaFree(c->ift);
+  cudaFree(c->partials); cudaFree(c->state); cudaFree(c->ou); cudaFree(c->pv);
   cudaFree(c->kz_tab);
   cudaFree(c->les_cds); cudaFree(c->les_phys); cudaFree(c->les_work);
   cudaFree(c->les_feat); cudaFree(c->les_coef);
@@ -805,6 +783,10 @@ static int init_ctx(const sam_gpu_config* cfg) {
   if (cfg->nrk_max < 1 || cfg->nrk_max > 3) return fail(SAM_GPU_EINVAL, "nrk_max must be 1, 2 or 3");
   Ctx* c = new Ctx();
   c->cfg = *cfg;
+  if (cfg->precision == kPrecDD) {
+    c->plain_only = true;
+    c->cfg.precision = 64;
+  }
   Grid& g = c->g;
   g.nx = cfg->nx; g.ny = cfg->ny; g.nz = cfg->nz; g.nze = cfg->nz;
   // init.f:49-73
@@ -848,23 +830,19 @@ static int init_ctx(const sam_gpu_config* cfg) {
   if ((rc = build_plan(g.nx, c->px)) || (rc = build_plan(g.ny, c->py)) || (rc = build_plan(g.nz, c->pz))) {
     free_ctx(c); g_ctx = nullptr; return rc;
   }
-  // FP64 z-forward tiles that leave room for two CTAs per SM: one CTA's
-  // fixed-point transforms overlap the other's FP64 epilogue (256^3: 2 rows
-  // 0.92 ms, 4 rows, one CTA, 1.09; 128^3: 4 rows, two CTAs, 0.143, 2 rows 0.157)
-  if (cfg->precision == 64)
-    while (c->ty_zf > 1 && tile_smem(c->pz, c->ty_zf * g.lr, sizeof(double2)) > kSmemMax / 2 - 1024) c->ty_zf /= 2;
-  cudaError_t e = cudaStreamCreateWithFlags(&c->own, cudaStreamNonBlocking);
-  if (e != cudaSuccess) { free_ctx(c); g_ctx = nullptr; return fail(SAM_GPU_ECUDA, "stream: %s", cudaGetErrorString(e)); }
-  c->stream = c->own;
   {
     int dev = 0, optin = 0;
     cudaGetDevice(&dev);
     if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess && optin > 4096)
       kSmemMax = (size_t)optin - 2048;
   }
-  set_smem_limits<double>();
-  set_smem_limits<float>();
-  set_smem_limits<dd>();
+  default_tiles(*c);
+  cudaError_t e = cudaStreamCreateWithFlags(&c->own, cudaStreamNonBlocking);
+  if (e != cudaSuccess) { free_ctx(c); g_ctx = nullptr; return fail(SAM_GPU_ECUDA, "stream: %s", cudaGetErrorString(e)); }
+  c->stream = c->own;
+  // (the per-routine drop-ins compute in FP64 in every form)
+  set_smem_limits<double>(g.nx, g.ny, g.nz);
+  if (c->cfg.precision == 32) set_smem_limits<float>(g.nx, g.ny, g.nz);
   diag_set_smem_limits();
   const size_t es = csize(*c);
   const size_t nzmm = (size_t)g.mx * g.my * g.mz;
@@ -884,8 +862,6 @@ static int init_ctx(const sam_gpu_config* cfg) {
   const size_t pv_bytes = sizeof(double) * 4 * ((size_t)kParsevalBlocks + 1) + sizeof(int) * kVmaxInts;
   ok = ok && cudaMalloc(&c->pv, pv_bytes) == cudaSuccess;
   if (ok) cudaMemset(c->pv, 0, pv_bytes);
-  if (ok && cfg->precision == kPrecDD)
-    ok = cudaMalloc(&c->ift, sizeof(dd) * 2 * ((size_t)g.mx + g.my + g.mz)) == cudaSuccess;
   ok = ok && cudaMalloc(&c->kz_tab, sizeof(double) * 3 * (size_t)g.mz) == cudaSuccess;
   if (!ok) { free_ctx(c); g_ctx = nullptr; return fail(SAM_GPU_ECUDA, "device allocation failed"); }
   cudaMemset(c->U, 0, es * g.lu * nzmm);
@@ -1376,7 +1352,7 @@ int sam_gpu_step(int nsteps) {
 int sam_gpu_set_forcing(unsigned long long seed, double k_f, double sigma, double t_l, int* n_modes) {
   NEED_CTX();
   if (n_modes) *n_modes = 0;
-  if (c.cfg.precision == kPrecDD && k_f > 0.0 && sigma != 0.0)
+  if (c.plain_only && k_f > 0.0 && sigma != 0.0)
     return fail(SAM_GPU_EUNSUPPORTED, "set_forcing: the double-float form runs the plain step only");
   if (c.gexec) { cudaGraphExecDestroy(c.gexec); c.gexec = nullptr; }
   c.graph_stale = 1;
@@ -1405,7 +1381,7 @@ static int mlp_ensure(Ctx& c);
 
 int sam_gpu_set_les(int model, double c_smag, double pr_t) {
   NEED_CTX();
-  if (model != 0 && c.cfg.precision == kPrecDD)
+  if (model != 0 && c.plain_only)
     return fail(SAM_GPU_EUNSUPPORTED, "set_les: the double-float form runs the plain step only");
   if (model < 0 || model > 3)
     return fail(SAM_GPU_EINVAL, "set_les: model %d (0 off, 1 Smagorinsky, 2 dynamic, 3 learned)", model);
@@ -1675,7 +1651,7 @@ int sam_gpu_box_filter(int f, double* out) {
   const Grid& g = c.g;
   if (!out || f < 1 || g.nx % f || g.ny % f || g.nz % f)
     return fail(SAM_GPU_EINVAL, "box_filter: the grid must divide into blocks of %d", f);
-  if (c.cfg.precision == kPrecDD) return fail(SAM_GPU_EUNSUPPORTED, "box_filter: not in the double-float form");
+  if (c.plain_only) return fail(SAM_GPU_EUNSUPPORTED, "box_filter: not in the double-float form");
   return c.cfg.precision == 32 ? box_filter_impl<float>(c, f, out) : box_filter_impl<double>(c, f, out);
 }
 
@@ -1719,7 +1695,7 @@ int sam_gpu_closure_inputs(unsigned short* feat, double* grads) {
   double dsq, dxi, dyi, dzi;
   grid_spacing(c, dxi, dyi, dzi, dsq);
   c.les_dsq = dsq;
-  if (c.cfg.precision == kPrecDD) return fail(SAM_GPU_EUNSUPPORTED, "closure_inputs: not in the double-float form");
+  if (c.plain_only) return fail(SAM_GPU_EUNSUPPORTED, "closure_inputs: not in the double-float form");
   return c.cfg.precision == 32 ? closure_inputs_impl<float>(c, feat, grads)
                                : closure_inputs_impl<double>(c, feat, grads);
 }
@@ -1948,28 +1924,6 @@ int sam_gpu_init_packet(unsigned long long seed, int kx0, int ky0, int kz0, doub
 
 // ------------------------------------------------------------- diagnostics
 
-// The state the diagnostics read: U and R themselves in the FP64 and FP32
-// forms; FP64 copies (scratch 1 and 2) in the double-float form, whose
-// diagnostics then run the FP64 kernels (prec).
-static int diag_state(Ctx& c, bool with_r, void** u, const void** r, int* prec) {
-  *u = c.U;
-  if (r) *r = c.R;
-  *prec = c.cfg.precision;
-  if (c.cfg.precision != kPrecDD) return 0;
-  const long long nm = (long long)c.g.mx * c.g.my * c.g.mz * c.g.lu;
-  int rc;
-  if ((rc = ensure(c.sc[1], (size_t)nm * 16))) return rc;
-  state_to_fp64(c, c.U, (double2*)c.sc[1].p, nm);
-  *u = c.sc[1].p;
-  if (with_r) {
-    if ((rc = ensure(c.sc[2], (size_t)nm * 16))) return rc;
-    state_to_fp64(c, c.R, (double2*)c.sc[2].p, nm);
-    *r = c.sc[2].p;
-  }
-  *prec = 64;
-  return 0;
-}
-
 int sam_gpu_spectra(double* out) {
   NEED_CTX();
   int rc = ensure(c.sc[3], sizeof(double) * ((size_t)5 * c.lm + 8) * 1024);
@@ -1978,12 +1932,8 @@ int sam_gpu_spectra(double* out) {
   if (c.cfg.i_les) {
     if ((rc = sam_gpu_cl_energy(&e_cl))) return rc;
   }
-  void* u;
-  const void* r;
-  int prec;
-  if ((rc = diag_state(c, true, &u, &r, &prec))) return rc;
-  DiagArgs d = diag_args(c.g, c.lm, c.nx2, c.k_cl, c.cfg.vis, c.cfg.i_les, e_cl, prec);
-  diag_spectra(d, u, r, (double*)c.sc[3].p, out, c.stream);
+  DiagArgs d = diag_args(c.g, c.lm, c.nx2, c.k_cl, c.cfg.vis, c.cfg.i_les, e_cl, c.cfg.precision);
+  diag_spectra(d, c.U, c.R, (double*)c.sc[3].p, out, c.stream);
   return sync_stream(c);
 }
 
@@ -1991,11 +1941,8 @@ int sam_gpu_div_check(double* out4) {
   NEED_CTX();
   int rc = ensure(c.sc[3], sizeof(double) * 8 * 1024);
   if (rc) return rc;
-  void* u;
-  int prec;
-  if ((rc = diag_state(c, false, &u, nullptr, &prec))) return rc;
-  DiagArgs d = diag_args(c.g, c.lm, c.nx2, c.k_cl, c.cfg.vis, c.cfg.i_les, 0.0, prec);
-  diag_div_check(d, u, (double*)c.sc[3].p, out4, c.stream);
+  DiagArgs d = diag_args(c.g, c.lm, c.nx2, c.k_cl, c.cfg.vis, c.cfg.i_les, 0.0, c.cfg.precision);
+  diag_div_check(d, c.U, (double*)c.sc[3].p, out4, c.stream);
   return sync_stream(c);
 }
 
@@ -2003,11 +1950,8 @@ int sam_gpu_cl_energy(double* e_cl) {
   NEED_CTX();
   int rc = ensure(c.sc[3], sizeof(double) * 8 * 1024);
   if (rc) return rc;
-  void* u;
-  int prec;
-  if ((rc = diag_state(c, false, &u, nullptr, &prec))) return rc;
-  DiagArgs d = diag_args(c.g, c.lm, c.nx2, c.k_cl, c.cfg.vis, c.cfg.i_les, 0.0, prec);
-  diag_cl_energy(d, u, (double*)c.sc[3].p, e_cl, c.stream);
+  DiagArgs d = diag_args(c.g, c.lm, c.nx2, c.k_cl, c.cfg.vis, c.cfg.i_les, 0.0, c.cfg.precision);
+  diag_cl_energy(d, c.U, (double*)c.sc[3].p, e_cl, c.stream);
   return sync_stream(c);
 }
 
@@ -2018,13 +1962,8 @@ int sam_gpu_force(const double* ek_0, int k_force) {
   int rc = ensure(c.sc[3], sizeof(double) * 64);
   if (rc) return rc;
   CK(cudaMemcpyAsync(c.sc[3].p, ek_0, sizeof(double) * (k_force + 1), cudaMemcpyHostToDevice, c.stream));
-  void* u;
-  int prec;
-  if ((rc = diag_state(c, false, &u, nullptr, &prec))) return rc;
-  DiagArgs d = diag_args(c.g, c.lm, c.nx2, c.k_cl, c.cfg.vis, c.cfg.i_les, 0.0, prec);
-  diag_force(d, u, (const double*)c.sc[3].p, k_force, c.stream);
-  // the double-float form rescaled an FP64 copy: back into the state
-  if (u != c.U) state_from_fp64(c, (const double2*)u, c.U, (long long)c.g.mx * c.g.my * c.g.mz * c.g.lu);
+  DiagArgs d = diag_args(c.g, c.lm, c.nx2, c.k_cl, c.cfg.vis, c.cfg.i_les, 0.0, c.cfg.precision);
+  diag_force(d, c.U, (const double*)c.sc[3].p, k_force, c.stream);
   return sync_stream(c);
 }
 
@@ -2266,7 +2205,7 @@ int sam_gpu_planes(const int* k_xy, int n_xy, const int* j_xz, int n_xz, const i
     if (i_yz[m] < 1 || i_yz[m] > g.nx) return fail(SAM_GPU_EINVAL, "planes: i_yz(%d) = %d outside 1..%d", m + 1, i_yz[m], g.nx);
     sel.i_yz[m] = i_yz[m] - 1;
   }
-  if (c.cfg.precision == kPrecDD) return fail(SAM_GPU_EUNSUPPORTED, "planes: not in the double-float form");
+  if (c.plain_only) return fail(SAM_GPU_EUNSUPPORTED, "planes: not in the double-float form");
   const int rc = c.cfg.precision == 32 ? planes_impl<float>(c, sel, xy, xz, yz, mean)
                                        : planes_impl<double>(c, sel, xy, xz, yz, mean);
   if (rc) return rc;
