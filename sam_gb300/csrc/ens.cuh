@@ -28,6 +28,7 @@ struct EnsParsevalArgs {
   const float2* u;
   Grid g;
   double* pv;
+  int nblk;
 };
 struct EnsFinishArgs {
   const double* partials;
@@ -42,7 +43,7 @@ struct EnsFinishArgs {
 };
 
 // virtual blocks of the wave-space sums per work item
-constexpr int kEnsParsevalChunk = 32;
+constexpr int kEnsParsevalChunk = 8;
 
 // tiles of a transform segment per work item
 constexpr int kEnsChunk = 8;

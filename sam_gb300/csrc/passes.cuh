@@ -108,9 +108,10 @@ struct YFwdArgs {
 };
 
 // What a ky row of a z-forward tile contributes to its modes' wave numbers
-// and (FP64 form) integrating factors exp(-nu k^2 dt_fac) = e(kx, ky) e(kz).
+// and (FP64 form) integrating factors exp(-nu k^2 dt_fac) = e(kx, ky) e(kz), each
+// factor less one and itself, for the velocity and for T.
 template <typename W> struct EpiRow {
-  W rky, k_sq, ef, et;
+  W rky, k_sq, ef[2], et[2];
 };
 // (these records follow the 16-byte elements of the lines)
 static_assert(sizeof(FxScale) == 16 && sizeof(FxLine) == 16, "records keep the alignment of what follows them");
@@ -142,8 +143,8 @@ struct ZFwdArgs {
   long long u_ky, u_kx, u_n;
   DevState* state;
   StageConsts sc;
-  // FP64 form, mode 2: rkz(k), then the integrating factors' kz part for the
-  // velocity and for T, written by the stage's y-forward pass (null: formed
+  // FP64 form, mode 2: rkz(k), then the integrating factors' kz part less one
+  // and itself for the velocity, then for T, written by the stage's y-forward pass (null: formed
   // per mode)
   const double* kz_tab;
   T nz_inv;                  // filled by the launcher: 1/Nz
@@ -208,7 +209,12 @@ constexpr int kVmaxInts = 16;  // the vmax block at the end of pv
 // vel_max's sums from wave space (Parseval), FP64 arithmetic on the state U
 // (Lu fields (kx, ky, kz)): pv[b * Lu + f] = block b's share of
 // sum w |u|^2 (w = 1 for kx = 0, 2 otherwise), pv[npv * Lu + f] = u(0,0,0).
-constexpr int kParsevalBlocks = 152 * 4;
+constexpr int kParsevalBlocks = 152 * 2;  // at most
+// four modes a thread at least (a 32^3 run has 4851)
+inline int parseval_blocks(const Grid& g) {
+  const long long b = ((long long)g.mx * g.my * g.mz + 4 * kThreads - 1) / (4 * kThreads);
+  return (int)(b < kParsevalBlocks ? b : kParsevalBlocks);
+}
 template <typename T> void launch_parseval(const cx_t<T>* u, const Grid& g, double* pv, cudaStream_t s);
 void launch_x2z(const double2* in, double2* out, const Grid& g, int nvar, int nx2, cudaStream_t s);
 

@@ -47,8 +47,8 @@ SAMGPU_ENS_BODY(ens_z_fwd, z_fwd_body, ZFwdArgs)
 __device__ __noinline__ void ens_parseval(const unsigned char* args, int tile) {
   const EnsParsevalArgs& pa = *reinterpret_cast<const EnsParsevalArgs*>(args);
   const int b0 = tile * kEnsParsevalChunk;
-  for (int b = b0; b < b0 + kEnsParsevalChunk && b < kParsevalBlocks; ++b) {
-    parseval_body<float>(pa.u, pa.g, pa.pv, b, kParsevalBlocks);
+  for (int b = b0; b < b0 + kEnsParsevalChunk && b < pa.nblk; ++b) {
+    parseval_body<float>(pa.u, pa.g, pa.pv, b, pa.nblk);
     __syncthreads();
   }
 }
@@ -179,7 +179,7 @@ void ens_record_x_pass(EnsRecorder& r, const XPassArgs<float>& a0, const FftPlan
   push(r, kEnsX, a.g.nx, x_pass_blocks(a), 2, last_of(r, kEnsYInv), -1, smem, a, pl);
   if (stats) {
     const int ix = (int)r.segs.size() - 1;
-    push(r, kEnsParseval, 0, (kParsevalBlocks + kEnsParsevalChunk - 1) / kEnsParsevalChunk, 0, -1, -1, 0, *pa,
+    push(r, kEnsParseval, 0, (pa->nblk + kEnsParsevalChunk - 1) / kEnsParsevalChunk, 0, -1, -1, 0, *pa,
          nullptr);
     const int ip = (int)r.segs.size() - 1;
     push(r, kEnsFinish, 0, 1, 3, ix, ip, 0, *fa, nullptr);

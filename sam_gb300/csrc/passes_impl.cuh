@@ -1451,14 +1451,17 @@ __device__ __forceinline__ void y_fwd_body(const YFwdArgs<T>& a, const FftPlan* 
   __syncthreads();
   if (a.kz_tab && bid == 0) {
     // the z-forward pass of the same stage, next on the stream, reads
-    // rkz(k), exp(-nu rkz^2 dt_fac) and the same with nu / Pr: one exp per
-    // kz here instead of one per mode there
+    // rkz(k), exp(-nu rkz^2 dt_fac) less one and itself, and the same with
+    // nu / Pr: exponentials per kz here instead of one per mode there
     const double vis_f = a.kz_vis * (a.kz_gamma * a.kz_state->dt + a.kz_zeta * a.kz_state->dt);  // sam.f:293-295
     for (int k = threadIdx.x; k < a.g.mz; k += blockDim.x) {
       const double rkz = a.g.wave_z * (double)kwave(k, a.g.kz, a.g.mz);
       a.kz_tab[k] = rkz;
-      a.kz_tab[a.g.mz + k] = exp(-vis_f * (rkz * rkz));
-      a.kz_tab[2 * a.g.mz + k] = exp(-(vis_f * a.kz_pr_inv) * (rkz * rkz));
+      const double xf = -vis_f * (rkz * rkz), xt = -(vis_f * a.kz_pr_inv) * (rkz * rkz);
+      a.kz_tab[a.g.mz + k] = expm1(xf);
+      a.kz_tab[2 * a.g.mz + k] = exp(xf);
+      a.kz_tab[3 * a.g.mz + k] = expm1(xt);
+      a.kz_tab[4 * a.g.mz + k] = exp(xt);
     }
   }
   // the first stage reads its inputs straight from the rows of C (no
@@ -1544,6 +1547,17 @@ __device__ __forceinline__ void epi_load(const ZFwdArgs<T>& a, int i, int j, int
   }
 }
 
+// The product of a row's factor and a kz factor: less one (less1) from their
+// parts less one, or itself from the factors where it is below a half and the
+// difference would lose relative precision.
+template <typename W>
+__device__ __forceinline__ void epi_factor(const W* row, const double* kz, int m, W& e, bool& less1) {
+  const W a = row[0], b = (W)kz[0];
+  e = a + b + a * b;
+  less1 = e > (W)-0.5;
+  if (!less1) e = row[1] * (W)kz[m];
+}
+
 // rhs.f:108-142 for one mode (kx i, ky j, kz k) in working type W, then
 // (mode 2) sam.f:210-221 and 293-314.  val(f) is the transform of field f at
 // this mode, times Nz where c.scale says so.
@@ -1627,10 +1641,18 @@ __device__ __forceinline__ void epi_mode(const ZFwdArgs<T>& a, Val val, int i, i
     return;
   }
   const long long uidx = (long long)i * a.u_kx + (long long)j * a.u_ky + k;
+  // exp(-nu k^2 dt_fac); with tables (FP64 form) less one: a value times
+  // e is then value + value (e - 1), rounded once, unless e is small
   W ef, et;
+  bool less1_f = false, less1_t = false;
   if (std::is_same<W, double>::value && a.kz_tab) {
-    ef = row.ef * (W)a.kz_tab[g.mz + k];
-    et = c.same_t ? ef : row.et * (W)a.kz_tab[2 * g.mz + k];
+    epi_factor(row.ef, a.kz_tab + g.mz + k, g.mz, ef, less1_f);
+    if (c.same_t) {
+      et = ef;
+      less1_t = less1_f;
+    } else {
+      epi_factor(row.et, a.kz_tab + 3 * g.mz + k, g.mz, et, less1_t);
+    }
   } else {
     ef = wexp(c.mvis_f * rk_sq_raw);
     et = c.same_t ? ef : wexp(c.mvis_t * rk_sq_raw);
@@ -1644,8 +1666,15 @@ __device__ __forceinline__ void epi_mode(const ZFwdArgs<T>& a, Val val, int i, i
         ui = ui + c.dt_fac2 * in.ri[f];
       }
       const W vf = f == 3 ? et : ef;  // sam.f:297
-      ur = (ur + c.dt_fac1 * rr[f]) * vf;
-      ui = (ui + c.dt_fac1 * ri[f]) * vf;
+      ur = ur + c.dt_fac1 * rr[f];
+      ui = ui + c.dt_fac1 * ri[f];
+      if (f == 3 ? less1_t : less1_f) {
+        ur = ur + ur * vf;
+        ui = ui + ui * vf;
+      } else {
+        ur = ur * vf;
+        ui = ui * vf;
+      }
       a.u[(long long)f * a.u_n + uidx] = mk<C>((T)ur, (T)ui);
       a.r[(long long)f * a.u_n + uidx] = mk<C>((T)rr[f], (T)ri[f]);
     }
@@ -1729,11 +1758,12 @@ __device__ __forceinline__ void z_fwd_body(const ZFwdArgs<T>& a, const FftPlan* 
     const T rkx = cw.wave_x * (T)i;
     r.rky = cw.wave_y * (T)kwave(j0 + t, g.ky, my);
     r.k_sq = rkx * rkx + r.rky * r.rky;
-    r.ef = r.et = (T)1;
     if constexpr (std::is_same<T, double>::value)
       if (a.kz_tab) {
-        r.ef = exp(cw.mvis_f * r.k_sq);
-        r.et = cw.same_t ? r.ef : exp(cw.mvis_t * r.k_sq);
+        r.ef[0] = expm1(cw.mvis_f * r.k_sq);
+        r.ef[1] = exp(cw.mvis_f * r.k_sq);
+        r.et[0] = cw.same_t ? r.ef[0] : expm1(cw.mvis_t * r.k_sq);
+        r.et[1] = cw.same_t ? r.ef[1] : exp(cw.mvis_t * r.k_sq);
       }
     s_row[t] = r;
   }
@@ -1787,7 +1817,7 @@ __device__ __forceinline__ void z_fwd_body(const ZFwdArgs<T>& a, const FftPlan* 
             re = (double)v.x;
             im = (double)v.y;
           },
-          0, 0, 0, epi_const<double>(a, dt), EpiRow<double>{0.0, 0.0, 1.0, 1.0}, ind);
+          0, 0, 0, epi_const<double>(a, dt), EpiRow<double>{0.0, 0.0, {0.0, 1.0}, {0.0, 1.0}}, ind);
     }
   }
   if (a.mode == 2 && a.sc.last && bid == 0 && threadIdx.x == 0) {
@@ -1820,7 +1850,8 @@ __device__ __forceinline__ DF df_add_wsq(DF a, float v, float w) {
 template <typename T>
 __device__ __forceinline__ void parseval_body(const cx_t<T>* __restrict__ u, const Grid& g, double* __restrict__ pv,
                                               int bid, int nblk) {
-  __shared__ double red[4][kThreads];
+  __shared__ double s_part[4][kThreads / 32];
+  double sum[4];
   const long long nm = (long long)g.mx * g.my * g.mz;
   const int plane = g.my * g.mz;
   if constexpr (sizeof(T) == 4) {
@@ -1838,7 +1869,7 @@ __device__ __forceinline__ void parseval_body(const cx_t<T>* __restrict__ u, con
         }
     }
 #pragma unroll
-    for (int f = 0; f < 4; ++f) red[f][threadIdx.x] = 2.0 * ((double)acc[f].hi + (double)acc[f].lo);
+    for (int f = 0; f < 4; ++f) sum[f] = f < g.lu ? 2.0 * ((double)acc[f].hi + (double)acc[f].lo) : 0.0;
   } else {
     // kx = 0 modes count once, kx > 0 twice (their conjugates): separate sums
     double acc0[4] = {0.0, 0.0, 0.0, 0.0}, acc1[4] = {0.0, 0.0, 0.0, 0.0};
@@ -1864,16 +1895,22 @@ __device__ __forceinline__ void parseval_body(const cx_t<T>* __restrict__ u, con
         }
     }
 #pragma unroll
-    for (int f = 0; f < 4; ++f) red[f][threadIdx.x] = acc0[f] + 2.0 * acc1[f];
+    for (int f = 0; f < 4; ++f) sum[f] = acc0[f] + 2.0 * acc1[f];
+  }
+  // fixed order: within each warp, then the warps in turn (one barrier)
+#pragma unroll
+  for (int f = 0; f < 4; ++f) {
+    if (f >= g.lu) break;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum[f] += __shfl_xor_sync(0xffffffffu, sum[f], o);
+    if ((threadIdx.x & 31) == 0) s_part[f][threadIdx.x >> 5] = sum[f];
   }
   __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s)
-#pragma unroll
-      for (int f = 0; f < 4; ++f) red[f][threadIdx.x] += red[f][threadIdx.x + s];
-    __syncthreads();
+  if (threadIdx.x < g.lu) {
+    double t = 0.0;
+    for (int w = 0; w < (int)blockDim.x / 32; ++w) t += s_part[threadIdx.x][w];
+    pv[(long long)bid * g.lu + threadIdx.x] = t;
   }
-  if (threadIdx.x < g.lu) pv[(long long)bid * g.lu + threadIdx.x] = red[threadIdx.x][0];
   if (bid == 0 && threadIdx.x < g.lu) pv[(long long)nblk * g.lu + threadIdx.x] = (double)u[threadIdx.x * nm].x;
 }
 template <typename T>
@@ -1883,7 +1920,7 @@ __global__ void __launch_bounds__(kThreads) k_parseval(const cx_t<T>* __restrict
 
 template <typename T>
 void launch_parseval(const cx_t<T>* u, const Grid& g, double* pv, cudaStream_t s) {
-  k_parseval<T><<<kParsevalBlocks, kThreads, 0, s>>>(u, g, pv);
+  k_parseval<T><<<parseval_blocks(g), kThreads, 0, s>>>(u, g, pv);
 }
 // vel_max.f:28-49 on the per-CTA partials written by the x pass (or, in the
 // resident step, on the wave-space sums and the maxima).
@@ -1892,7 +1929,6 @@ __device__ __forceinline__ void vel_max_finish_body(const double* __restrict__ p
                                                     DevState* st, int i_cfl, double cfl0, double adv_cfl_limit,
                                                     const double* __restrict__ pv, int npv, int* __restrict__ vmax,
                                                     int vkind) {
-  __shared__ double red[kThreads];
   __shared__ double fin[4][4];
   if (!pv) {
     // a thread reads whole per-CTA records (lu x 4 doubles, contiguous) of
@@ -1936,26 +1972,23 @@ __device__ __forceinline__ void vel_max_finish_body(const double* __restrict__ p
     __syncthreads();
   }
   if (pv) {
-    // sums from wave space: sum u = N u(0,0,0), sum u^2 = N sum w |u|^2
-    for (int f = 0; f < g.lu; ++f) {
+    // sums from wave space: sum u = N u(0,0,0), sum u^2 = N sum w |u|^2; a
+    // warp per field, fixed order
+    const int f = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (f < g.lu) {
       double v = 0.0;
-      for (int b = threadIdx.x; b < npv; b += blockDim.x) v += ldc<COH>(pv + (long long)b * g.lu + f);
-      red[threadIdx.x] = v;
-      __syncthreads();
-      for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-        __syncthreads();
-      }
-      if (threadIdx.x == 0) {
+      for (int b = lane; b < npv; b += 32) v += ldc<COH>(pv + (long long)b * g.lu + f);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane == 0) {
         const double n = (double)g.nx * (double)g.ny * (double)g.nz;
         fin[f][0] = ldc<COH>(pv + (long long)npv * g.lu + f) * n;
-        fin[f][1] = red[0] * n;
+        fin[f][1] = v * n;
         const unsigned long long key =
             vkind ? ldc<COH>(reinterpret_cast<const unsigned long long*>(vmax) + f) : 0ull;
         fin[f][2] = vkind ? __longlong_as_double((long long)key) : (double)__int_as_float(ldc<COH>(vmax + f));
         fin[f][3] = (double)ldc<COH>(vmax + 8);
       }
-      __syncthreads();
     }
     __syncthreads();
     if (threadIdx.x < kVmaxInts) vmax[threadIdx.x] = 0;  // ready for the next step's maxima

@@ -178,7 +178,7 @@ struct Ctx {
   double* partials = nullptr;
   int partial_blocks = 0;
   double* pv = nullptr;  // vel_max's wave-space sums
-  double* kz_tab = nullptr;  // FP64 form: kz wave numbers and integrating factors of the stage (3 Mz)
+  double* kz_tab = nullptr;  // FP64 form: kz wave numbers and integrating factors of the stage (5 Mz)
   DevState* state = nullptr;
   Scratch sc[4];
   // tile choices
@@ -453,9 +453,9 @@ static int run_x_pass(Ctx& c, int in_mode, int out_mode, int nin, const void* in
   }
   if constexpr (std::is_same<T, float>::value) {
     if (c.rec) {
-      EnsParsevalArgs pa{(const float2*)c.U, c.g, c.pv};
+      EnsParsevalArgs pa{(const float2*)c.U, c.g, c.pv, parseval_blocks(c.g)};
       EnsFinishArgs fa{c.partials, nblk, c.g, c.state, c.cfg.i_cfl, c.cfg.cfl0, c.adv_cfl_limit, c.pv,
-                       kParsevalBlocks, a.vmax};
+                       parseval_blocks(c.g), a.vmax};
       if (stats && !a.max_only) return fail(SAM_GPU_EUNSUPPORTED, "ensemble stage: FP64 vel_max partials");
       ens_record_x_pass(*c.rec, a, c.px.d, x_smem<T>(c, a), stats, &pa, &fa);
       return 0;
@@ -465,7 +465,7 @@ static int run_x_pass(Ctx& c, int in_mode, int out_mode, int nin, const void* in
   if (stats) {
     if (a.max_only) launch_parseval<T>((const cx_t<T>*)c.U, c.g, c.pv, c.stream);
     launch_vel_max_finish(c.partials, nblk, c.g, c.state, c.cfg.i_cfl, c.cfg.cfl0, c.adv_cfl_limit, c.stream,
-                          a.max_only ? c.pv : nullptr, kParsevalBlocks, a.vmax,
+                          a.max_only ? c.pv : nullptr, parseval_blocks(c.g), a.vmax,
                           std::is_same<T, double>::value ? 1 : 0);
   }
   return 0;
@@ -862,7 +862,7 @@ static int init_ctx(const sam_gpu_config* cfg) {
   const size_t pv_bytes = sizeof(double) * 4 * ((size_t)kParsevalBlocks + 1) + sizeof(int) * kVmaxInts;
   ok = ok && cudaMalloc(&c->pv, pv_bytes) == cudaSuccess;
   if (ok) cudaMemset(c->pv, 0, pv_bytes);
-  ok = ok && cudaMalloc(&c->kz_tab, sizeof(double) * 3 * (size_t)g.mz) == cudaSuccess;
+  ok = ok && cudaMalloc(&c->kz_tab, sizeof(double) * 5 * (size_t)g.mz) == cudaSuccess;
   if (!ok) { free_ctx(c); g_ctx = nullptr; return fail(SAM_GPU_ECUDA, "device allocation failed"); }
   cudaMemset(c->U, 0, es * g.lu * nzmm);
   cudaMemset(c->R, 0, es * g.lu * nzmm);

@@ -8,6 +8,7 @@ radix-2 transform, whose log2 n levels each round every value once by 0.4 to
 import numpy as np
 import pytest
 
+import oracle as O
 from sam_gb300 import SamGpu
 
 pytestmark = pytest.mark.gpu
@@ -120,4 +121,61 @@ def test_exceptional_lines(gpu_lib, n):
         assert not (np.isfinite(line.real) | np.isfinite(line.imag)).any()
         got[:, 0, 0] = ref[:, 0, 0]
         assert np.array_equal(got, ref)
+    g.close()
+
+
+COMPILED = sorted(2 ** a * 3 ** b * 5 ** c for a in range(9) for b in range(6) for c in range(4)
+                  if 16 <= 2 ** a * 3 ** b * 5 ** c <= 256)
+
+
+@pytest.mark.parametrize("precision, tol", [(64, 1e-13), (32, 1e-5)])
+@pytest.mark.parametrize("axis", ["x", "y", "z"])
+def test_every_compiled_length(gpu_lib, precision, tol, axis):
+    """One resident RK stage on boxes with each length that has compile-time
+    stages along one direction, against the oracle at the bars of the
+    per-routine and the FP32 comparisons (both relative to the largest value)."""
+    for n in COMPILED:
+        if axis == "x" and n % 2:
+            continue
+        d = dict(nx=8, ny=10, nz=12)
+        d["n" + axis] = n
+        cfg = dict(i_strat=1, vis=1e-2, pr=0.7, dt0=0.01, buoy_fac_z=1.0, lapse=1.0, i_cfl=1, cfl0=0.5, **d)
+        g, o = SamGpu(precision=precision, **cfg), O.Oracle(**cfg)
+        u = o.init_random(7)
+        g.upload(u)
+        r = o.wave(o.d.lr)
+        o.stage(u, r, 1)
+        g.stage(1)
+        ug = g.download()
+        m = o.d.nz_min
+        assert np.abs(ug[:m] - u[:m]).max() < tol * np.abs(u[:m]).max(), n
+        so, sg = o.stats(), g.stats()
+        assert abs(sg["dt"] - so["dt"]) < tol * so["dt"], n
+        np.testing.assert_allclose(sg["u_var"][:4], so["u_var"][:4], rtol=max(tol, 1e-12))
+        g.close()
+
+
+@pytest.mark.parametrize("pr", [1.0, 0.4])
+def test_damping_of_single_modes(gpu_lib, pr):
+    """Integrating factors exp(-x), x = nu k^2 dt, from nearly one to far below
+    a half, where the epilogue changes from u + u (e - 1) to u e: no flow, so
+    each mode of T is damped alone.  Bar, per mode and relative to it: the
+    three stages' exponents carry four roundings of relative size 2^-53 each
+    (nu dt, the two parts of k^2, their product), which the exponential turns
+    into 4 x 2^-53, and each stage rounds its factors, their join and the
+    product (four more)."""
+    cfg = dict(nx=24, ny=20, nz=32, i_strat=1, vis=0.5, pr=pr, dt0=0.15, i_cfl=0)
+    g = SamGpu(**cfg)
+    u = g.wave(4)
+    rng = np.random.default_rng(3)
+    m, my, mx = g.nz_min, g.ny_min, g.nx_min
+    u[:m, :, 1:, 3] = rng.standard_normal((m, my, mx - 1)) + 1j * rng.standard_normal((m, my, mx - 1))
+    g.upload(u)
+    g.step(1)
+    got = g.download()
+    k = [np.concatenate([np.arange(0, q // 2 + 1), np.arange(-(q // 2), 0)]) for q in (m, my)]
+    k_sq = k[0][:, None, None] ** 2 + k[1][None, :, None] ** 2 + np.arange(1, mx)[None, None, :] ** 2
+    x = np.longdouble(0.5) / np.longdouble(pr) * np.longdouble(0.15) * k_sq
+    ref = u[:m, :, 1:, 3] * np.exp(-x)
+    assert (np.abs(got[:m, :, 1:, 3] - ref) <= (12 + 4 * x) * 2.0 ** -53 * np.abs(ref)).all()
     g.close()
