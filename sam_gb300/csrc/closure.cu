@@ -740,21 +740,27 @@ __global__ void __launch_bounds__(128, 1)
   }
 }
 
-// grad[p] = sum over CTAs of part[b][p] in CTA order; loss[0] likewise
+// sum over CTAs of part[b][p] in CTA order, sixteen loads in flight
+__device__ __forceinline__ float mlp_part_sum(const float* __restrict__ part, int nblk, int p) {
+  float g = 0.f;
+#pragma unroll 16
+  for (int b = 0; b < nblk; ++b) g += part[(long long)b * (kMlpParams + 1) + p];
+  return g;
+}
+// grad[p] the sum over CTAs; loss[0] likewise
 __global__ void k_mlp_reduce(const float* __restrict__ part, int nblk, float* __restrict__ grad,
                              float* __restrict__ loss) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p > kMlpParams) return;
-  float g = 0.f;
-  for (int b = 0; b < nblk; ++b) g += part[(long long)b * (kMlpParams + 1) + p];
+  const float g = mlp_part_sum(part, nblk, p);
   if (p < kMlpParams) grad[p] = g;
   else loss[0] = g;
 }
 
 long long mlp_partials(long long n) { return ((n + kMlpTile - 1) / kMlpTile) * (kMlpParams + 1); }
 
-void mlp_backward(const __nv_bfloat16* x16, const float2* y, long long n, const MlpDev* dev, const MlpBatch& batch,
-                  float* part, float* grad, float* loss, int* err, bool tensor_cores, cudaStream_t s) {
+int mlp_backward(const __nv_bfloat16* x16, const float2* y, long long n, const MlpDev* dev, const MlpBatch& batch,
+                 float* part, int* err, bool tensor_cores, cudaStream_t s) {
   const long long ntiles = (n + kMlpTile - 1) / kMlpTile;
   int nblk;
   if (tensor_cores) {
@@ -775,28 +781,58 @@ void mlp_backward(const __nv_bfloat16* x16, const float2* y, long long n, const 
     nblk = (int)ntiles;
     k_mlp_bwd<<<nblk, kMlpTile, kBwdSmem, s>>>(x16, y, n, dev, batch.h1, batch.h2, batch.o, part);
   }
-  k_mlp_reduce<<<(kMlpParams + 1 + 255) / 256, 256, 0, s>>>(part, nblk, grad, loss);
+  return nblk;
 }
 
-// Adam (Kingma & Ba 2015): beta1 0.9, beta2 0.999, eps 1e-8, bias-corrected
-__global__ void k_mlp_adam(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
-                           const float* __restrict__ g, float lr_t, float b1, float b2) {
+void mlp_reduce(const float* part, int nblk, float* grad, float* loss, cudaStream_t s) {
+  k_mlp_reduce<<<(kMlpParams + 1 + 127) / 128, 128, 0, s>>>(part, nblk, grad, loss);
+}
+
+// A training step's update in one launch: the gradient's sum over the CTAs (as
+// k_mlp_reduce, the same order), Adam (Kingma & Ba 2015: beta1 0.9, beta2
+// 0.999, eps 1e-8, bias-corrected) and the parameter's place or places in the
+// BF16 device form (k_mlp_pack's).  Three launches and, with the loss kept on
+// the device, one synchronising copy fewer a step: 16 steps of 8192 of 65536
+// points with the data's copies and a forward pass 1.19 -> 0.88 ms.
+__global__ void k_mlp_update(const float* __restrict__ part, int nblk, float* __restrict__ p, float* __restrict__ m,
+                             float* __restrict__ v, float lr_t, float b1, float b2, float* __restrict__ loss,
+                             MlpDev* __restrict__ d) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= kMlpParams) return;
-  const float gi = g[i];
+  if (i > kMlpParams) return;
+  const float gi = mlp_part_sum(part, nblk, i);
+  if (i == kMlpParams) {
+    loss[0] = gi;
+    return;
+  }
   const float mi = b1 * m[i] + (1.f - b1) * gi;
   const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
   m[i] = mi;
   v[i] = vi;
-  p[i] -= lr_t * mi / (sqrtf(vi) + 1e-8f);
+  const float pi = p[i] - lr_t * mi / (sqrtf(vi) + 1e-8f);
+  p[i] = pi;
+  if (i < kMlpOffB1) {
+    d->w1[(i / kMlpIn) * kMlpK1 + i % kMlpIn] = __float2bfloat16_rn(pi);
+  } else if (i < kMlpOffW2) {
+    for (int j = 0; j < 3; ++j) d->w1[(i - kMlpOffB1) * kMlpK1 + kMlpOne + j] = bias_part(pi, j);
+  } else if (i < kMlpOffB2) {
+    const int e = i - kMlpOffW2;
+    d->w2[(e / kMlpH) * kMlpK2 + e % kMlpH] = __float2bfloat16_rn(pi);
+  } else if (i < kMlpOffW3) {
+    for (int j = 0; j < 3; ++j) d->w2[(i - kMlpOffB2) * kMlpK2 + kMlpH + j] = bias_part(pi, j);
+  } else if (i < kMlpOffB3) {
+    const int e = i - kMlpOffW3;
+    d->w3[(e / kMlpH) * kMlpK2 + e % kMlpH] = __float2bfloat16_rn(pi);
+  } else {
+    for (int j = 0; j < 3; ++j) d->w3[(i - kMlpOffB3) * kMlpK2 + kMlpH + j] = bias_part(pi, j);
+  }
 }
 
-void mlp_adam(float* params, float* m, float* v, const float* grad, int step, float lr, MlpDev* dev,
-              cudaStream_t s) {
+void mlp_update(const float* part, int nblk, float* params, float* m, float* v, int step, float lr, float* loss,
+                MlpDev* dev, cudaStream_t s) {
   const double b1 = 0.9, b2 = 0.999;
   const double lr_t = lr * sqrt(1.0 - pow(b2, step)) / (1.0 - pow(b1, step));
-  k_mlp_adam<<<(kMlpParams + 255) / 256, 256, 0, s>>>(params, m, v, grad, (float)lr_t, (float)b1, (float)b2);
-  mlp_pack(params, dev, s);
+  k_mlp_update<<<(kMlpParams + 1 + 127) / 128, 128, 0, s>>>(part, nblk, params, m, v, (float)lr_t, (float)b1,
+                                                           (float)b2, loss, dev);
 }
 
 }  // namespace samgpu

@@ -58,17 +58,18 @@ void mlp_pack(const float* params, MlpDev* dev, cudaStream_t s);
 // launched, or -1 when the tensor map cannot be built (nothing launched).
 int mlp_forward(const __nv_bfloat16* x16, long long n, const MlpDev* dev, float2* coef, const MlpBatch* batch,
                 int* err, cudaStream_t s);
-// Gradient of L = mean over points and both outputs of (C - y)^2, written
-// to grad (kMlpParams floats), and the loss sum into loss[0]; part holds
-// mlp_partials(n) floats.
+// Gradient of L = mean over points and both outputs of (C - y)^2 as partial
+// sums of nblk CTAs (the return value) in part, which holds mlp_partials(n)
+// floats: mlp_reduce writes grad (kMlpParams floats) and the loss sum,
+// mlp_update takes one Adam step on params (m, v moments) and the BF16 form.
 // tensor_cores: the three contractions as tcgen05 MMAs (k_mlp_bwd_tc; err
 // is set on a wait timeout), else the CUDA-core kernel (k_mlp_bwd).
 long long mlp_partials(long long n);
-void mlp_backward(const __nv_bfloat16* x16, const float2* y, long long n, const MlpDev* dev, const MlpBatch& batch,
-                  float* part, float* grad, float* loss, int* err, bool tensor_cores, cudaStream_t s);
-// One Adam step on params (m, v moments), then the BF16 repack.
-void mlp_adam(float* params, float* m, float* v, const float* grad, int step, float lr, MlpDev* dev,
-              cudaStream_t s);
+int mlp_backward(const __nv_bfloat16* x16, const float2* y, long long n, const MlpDev* dev, const MlpBatch& batch,
+                 float* part, int* err, bool tensor_cores, cudaStream_t s);
+void mlp_reduce(const float* part, int nblk, float* grad, float* loss, cudaStream_t s);
+void mlp_update(const float* part, int nblk, float* params, float* m, float* v, int step, float lr, float* loss,
+                MlpDev* dev, cudaStream_t s);
 // FP32 features [n][12] -> BF16 [n][16] (columns 12..14 = 1.0, 15 = 0)
 void mlp_features_bf16(const float* f, __nv_bfloat16* x16, long long n, cudaStream_t s);
 // Self-test of one tensor-core tile: D(128 x 64) = A(128 x 16) B(64 x 16)^T

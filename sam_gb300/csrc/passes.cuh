@@ -209,7 +209,7 @@ constexpr int kVmaxInts = 16;  // the vmax block at the end of pv
 // vel_max's sums from wave space (Parseval), FP64 arithmetic on the state U
 // (Lu fields (kx, ky, kz)): pv[b * Lu + f] = block b's share of
 // sum w |u|^2 (w = 1 for kx = 0, 2 otherwise), pv[npv * Lu + f] = u(0,0,0).
-constexpr int kParsevalBlocks = 152 * 2;  // at most
+constexpr int kParsevalBlocks = 152 * 6;  // at most
 // four modes a thread at least (a 32^3 run has 4851)
 inline int parseval_blocks(const Grid& g) {
   const long long b = ((long long)g.mx * g.my * g.mz + 4 * kThreads - 1) / (4 * kThreads);

@@ -1858,15 +1858,24 @@ __device__ __forceinline__ void parseval_body(const cx_t<T>* __restrict__ u, con
     // kx = 0 modes count once, kx > 0 twice (their conjugates): sum w |u|^2
     // with w = 1/2 for kx = 0 and 1 otherwise, then double
     DF acc[4] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
-    for (long long m = bid * (long long)blockDim.x + threadIdx.x; m < nm;
-         m += (long long)nblk * blockDim.x) {
-      const float w = m < plane ? 0.5f : 1.0f;
+    // (two modes' loads of all fields in flight before the dependent sums)
+    const long long step = (long long)nblk * blockDim.x;
+    for (long long m0 = bid * (long long)blockDim.x + threadIdx.x; m0 < nm; m0 += 2 * step) {
+      cx_t<T> v[2][4];
 #pragma unroll
-      for (int f = 0; f < 4; ++f)
-        if (f < g.lu) {
-          const cx_t<T> v = u[f * nm + m];
-          acc[f] = df_add_wsq(df_add_wsq(acc[f], v.y, w), v.x, w);
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int f = 0; f < 4; ++f) {
+          const long long m = m0 + h * step;
+          v[h][f] = f < g.lu && m < nm ? u[f * nm + m] : mk<cx_t<T>>(0.f, 0.f);
         }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float w = m0 + h * step < plane ? 0.5f : 1.0f;
+#pragma unroll
+        for (int f = 0; f < 4; ++f)
+          if (f < g.lu) acc[f] = df_add_wsq(df_add_wsq(acc[f], v[h][f].y, w), v[h][f].x, w);
+      }
     }
 #pragma unroll
     for (int f = 0; f < 4; ++f) sum[f] = f < g.lu ? 2.0 * ((double)acc[f].hi + (double)acc[f].lo) : 0.0;
@@ -1977,6 +1986,7 @@ __device__ __forceinline__ void vel_max_finish_body(const double* __restrict__ p
     const int f = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (f < g.lu) {
       double v = 0.0;
+#pragma unroll 8
       for (int b = lane; b < npv; b += 32) v += ldc<COH>(pv + (long long)b * g.lu + f);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

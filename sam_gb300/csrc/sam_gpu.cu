@@ -1561,7 +1561,8 @@ int sam_gpu_mlp_grad(const float* feat, const float* target, long long n, float*
   CK(cudaMemcpyAsync(w.y, target, sizeof(float2) * (size_t)n, cudaMemcpyHostToDevice, c.stream));
   if (mlp_forward(x16, n, c.mlp_dev, w.coef, &w.b, c.mlp_err, c.stream) < 0)
     return fail(SAM_GPU_ECUDA, "closure network: no TMA tensor map");
-  mlp_backward(x16, w.y, n, c.mlp_dev, w.b, w.part, c.mlp_g, c.mlp_loss, c.mlp_err, c.mlp_tc_bwd != 0, c.stream);
+  const int nblk = mlp_backward(x16, w.y, n, c.mlp_dev, w.b, w.part, c.mlp_err, c.mlp_tc_bwd != 0, c.stream);
+  mlp_reduce(w.part, nblk, c.mlp_g, c.mlp_loss, c.stream);
   CK(cudaMemcpyAsync(grad, c.mlp_g, sizeof(float) * kMlpParams, cudaMemcpyDeviceToHost, c.stream));
   float ls = 0.f;
   CK(cudaMemcpyAsync(&ls, c.mlp_loss, sizeof(float), cudaMemcpyDeviceToHost, c.stream));
@@ -1595,15 +1596,17 @@ int sam_gpu_mlp_train(const float* feat, const float* target, long long n, int s
   CK(cudaMemcpyAsync(y_all, target, sizeof(float2) * (size_t)n, cudaMemcpyHostToDevice, c.stream));
   const long long nchunks = n / nb;
   std::vector<float> hist((size_t)steps);
+  if ((rc = ensure(c.sc[1], sizeof(float) * (size_t)std::max(steps, 1)))) return rc;  // the losses, read back at the end
+  float* losses = (float*)c.sc[1].p;
   for (int s = 0; s < steps; ++s) {
     const long long off = (s % nchunks) * nb;
     if (mlp_forward(x16 + off * kMlpK1, nb, c.mlp_dev, w.coef, &w.b, c.mlp_err, c.stream) < 0)
       return fail(SAM_GPU_ECUDA, "closure network: no TMA tensor map");
-    mlp_backward(x16 + off * kMlpK1, y_all + off, nb, c.mlp_dev, w.b, w.part, c.mlp_g, c.mlp_loss + 0, c.mlp_err,
-                 c.mlp_tc_bwd != 0, c.stream);
-    mlp_adam(c.mlp_p, c.mlp_m, c.mlp_v, c.mlp_g, ++c.mlp_step, lr, c.mlp_dev, c.stream);
-    if (loss_hist) CK(cudaMemcpyAsync(&hist[s], c.mlp_loss, sizeof(float), cudaMemcpyDeviceToHost, c.stream));
+    const int nblk = mlp_backward(x16 + off * kMlpK1, y_all + off, nb, c.mlp_dev, w.b, w.part, c.mlp_err,
+                                  c.mlp_tc_bwd != 0, c.stream);
+    mlp_update(w.part, nblk, c.mlp_p, c.mlp_m, c.mlp_v, ++c.mlp_step, lr, losses + s, c.mlp_dev, c.stream);
   }
+  if (steps) CK(cudaMemcpyAsync(hist.data(), losses, sizeof(float) * (size_t)steps, cudaMemcpyDeviceToHost, c.stream));
   rc = mlp_check_err(c);
   if (loss_hist)
     for (int s = 0; s < steps; ++s) loss_hist[s] = hist[s] / (2.0f * (float)nb);
