@@ -443,12 +443,7 @@ struct FxProductLoad {
   __device__ __forceinline__ fxc operator()(int idx) const {
     const FxSplit2 ea = a[sidx(idx)], eb = b[sidx(idx)];
     fxc v{fx_mul_line(ea.x, eb.x, p), fx_mul_line(ea.y, eb.y, p)};
-    if (g) {
-      const double2 d = g[sidx(idx)];
-      const int dsh = p.sc.ex + 1023 + 62;
-      v.x = (v.x >> p.down) + fx_from(d.x, dsh);
-      v.y = (v.y >> p.down) + fx_from(d.y, dsh);
-    }
+    if (g) fx_add_term(v, g[sidx(idx)], p);
     return v;
   }
   __device__ __forceinline__ FxScale scale() const { return p.sc; }

@@ -430,6 +430,12 @@ __device__ __forceinline__ long long fx_mul_line(FxSplit a, FxSplit b, const FxP
   const uint32_t hi = __funnelshift_l((uint32_t)A, (uint32_t)(A >> 32), p.s);
   return (long long)(((uint64_t)hi << 32) | lo);
 }
+// a product of fx_mul_line joined with its subgrid term
+__device__ __forceinline__ void fx_add_term(fxc& v, double2 t, const FxProduct& p) {
+  const int dsh = p.sc.ex + 1023 + 62;
+  v.x = (v.x >> p.down) + fx_from(t.x, dsh);
+  v.y = (v.y >> p.down) + fx_from(t.y, dsh);
+}
 // The exponent bounding the moduli's sum of a line of n doubles (elements
 // sidx(0) .. sidx(n - 1)), by one warp: sum < 2^info->ex.
 __host__ __device__ __forceinline__ int sidx(int p);

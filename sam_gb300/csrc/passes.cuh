@@ -88,6 +88,34 @@ struct XPassArgs {
   FastDiv fd_mx, fd_yp, fd_nx, fd_y;  // filled by the launcher
 };
 
+// The fused x passes of 256-point lines (k_x_pass_f256, k_x_pass_fx256): the
+// resident step's form of the pass, with or without a subgrid closure.
+constexpr int kXf256Threads = 288;                  // 18 teams of 16 (two rounds of 9 x 4 product lines)
+constexpr int kXf256Teams = kXf256Threads / 16;
+constexpr int kXf256Ld = 271;                       // line_stride(256)
+static_assert(kXf256Ld == ((256 + (255 >> 4)) | 1), "line stride of a 256-point line");
+__host__ __device__ constexpr size_t x_f256_smem(int lines, bool les) {
+  return sizeof(float2) * (256 + (size_t)(lines + (les ? 0 : kXf256Teams)) * kXf256Ld);
+}
+// 16 or, with a closure, 18 teams (the 18 product lines of a 4-row tile)
+__host__ __device__ constexpr int x_fx256_threads(bool les) { return les ? 288 : 256; }
+__host__ __device__ constexpr size_t x_fx256_smem(int lines, bool les) {
+  return (size_t)lines * (sizeof(fxc) * kXf256Ld + sizeof(FxLine)) +
+         (les ? 0 : sizeof(fxw) * 256 + (size_t)(x_fx256_threads(false) / 16) * kXf256Ld * sizeof(long long));
+}
+template <typename T> inline size_t x_fused_smem(const XPassArgs<T>& a) {
+  const int lines = a.nin * (a.yt / 2);
+  return sizeof(T) == 4 ? x_f256_smem(lines, a.les != 0) : x_fx256_smem(lines, a.les != 0);
+}
+// whether a fused kernel runs this launch (else the general kernel)
+template <typename T> inline bool x_fused(const XPassArgs<T>& a) {
+  return a.g.nx == 256 && a.sched == 0 && a.in_mode == 0 && a.out_mode == 2 &&
+         a.nin == a.g.lu + (a.les ? a.g.lr : 0) && (a.g.lr == 6 || a.g.lr == 9) && (!a.partials || a.max_only) &&
+         a.yt >= 2 && a.yt % 2 == 0 && x_fused_smem(a) + 2048 <= (size_t)smem_optin();
+}
+// rows of a fused tile with a closure: 26 lines, three (FP32) or two CTAs per SM
+constexpr int kXFusedLesRows = 4;
+
 template <typename T>
 struct YFwdArgs {
   Grid g;

@@ -356,38 +356,36 @@ template <typename C> struct ProductLoad {
   }
 };
 
+// |S| = sqrt(2 sum ifact S^2) of the strain in product order.
+template <typename T> __device__ __forceinline__ T strain_norm(const T* s) {
+  const T d = s[0] * s[0] + s[2] * s[2] + s[5] * s[5], o = s[1] * s[1] + s[3] * s[3] + s[4] * s[4];
+  return sqrt((T)2 * ((T)2 * o + d));
+}
+
 // Subgrid stress on one physical point: s[0..5] the strain in product order
 // (S11 S12 S22 S13 S23 S33), s[6..8] dT/dx_a; on return s holds the terms
 // the products receive, -2 nu_t S and -kappa_t dT/dx with
 // nu_t = cds |S|, |S| = sqrt(2 sum ifact S^2), kappa_t = nu_t prt_inv.
 template <typename T>
 __device__ __forceinline__ void sgs_point(T* s, int nf, T cds, T prt_inv) {
-  T sum = (T)0;
+  const T nu2 = (T)-2 * cds * strain_norm(s), kap = (T)0.5 * prt_inv * nu2;
 #pragma unroll
-  for (int m = 0; m < 6; ++m) sum += (m == 1 || m == 3 || m == 4 ? (T)2 : (T)1) * s[m] * s[m];
-  const T nu = cds * sqrt((T)2 * sum);
-  const T nu2 = (T)2 * nu, kap = nu * prt_inv;
-#pragma unroll
-  for (int m = 0; m < 6; ++m) s[m] = -nu2 * s[m];
+  for (int m = 0; m < 6; ++m) s[m] = nu2 * s[m];
 #pragma unroll
   for (int m = 6; m < 9; ++m)
-    if (m < nf) s[m] = -kap * s[m];
+    if (m < nf) s[m] = kap * s[m];
 }
 
 // As sgs_point with per-point coefficients: nu_t = cnu |S|, kappa_t = ckap |S|.
 template <typename T>
 __device__ __forceinline__ void sgs_point_c(T* s, int nf, T cnu, T ckap) {
-  T sum = (T)0;
+  const T sm = strain_norm(s);
+  const T nu2 = (T)-2 * cnu * sm, kap = -ckap * sm;
 #pragma unroll
-  for (int m = 0; m < 6; ++m) sum += (m == 1 || m == 3 || m == 4 ? (T)2 : (T)1) * s[m] * s[m];
-  const T sm = sqrt((T)2 * sum);
-  const T nu = cnu * sm, kap = ckap * sm;
-  const T nu2 = (T)2 * nu;
-#pragma unroll
-  for (int m = 0; m < 6; ++m) s[m] = -nu2 * s[m];
+  for (int m = 0; m < 6; ++m) s[m] = nu2 * s[m];
 #pragma unroll
   for (int m = 6; m < 9; ++m)
-    if (m < nf) s[m] = -kap * s[m];
+    if (m < nf) s[m] = kap * s[m];
 }
 
 // The learned closure's 12 inputs at one point from the strain S (product
@@ -454,6 +452,44 @@ __device__ __forceinline__ void store_features(void* feat, long long pt, const f
   uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(feat) + pt * 16);
   dst[0] = make_uint4(q[0], q[1], q[2], q[3]);
   dst[1] = make_uint4(q[4], q[5], q[6], q[7]);
+}
+
+// The gradient lines (behind the Lu factors) of a tile become the terms the
+// products receive, -2 nu_t S and -kappa_t dT.
+template <typename T>
+__device__ __forceinline__ void sgs_terms(const XPassArgs<T>& a, cx_t<T>* s_in, int ld, int y0, int z) {
+  using C = cx_t<T>;
+  const int nx = a.g.nx, ny = a.g.ny, yp = a.yt / 2;
+  const int lu = a.g.lu, lr = a.g.lr;
+  const T cds = a.les == 1 ? (T)a.les_cds[0] : (T)0, prt = (T)a.les_prt_inv;
+  for (int e = threadIdx.x; e < yp * nx; e += blockDim.x) {
+    const int c = (int)fdiv(e, a.fd_nx), x = e - c * nx;
+    C v[9];
+    T sx[9], sy[9];
+#pragma unroll
+    for (int m = 0; m < 9; ++m)
+      if (m < lr) {
+        v[m] = s_in[((lu + m) * yp + c) * ld + sidx(x)];
+        sx[m] = v[m].x;
+        sy[m] = v[m].y;
+      }
+    if (a.les == 2) {
+      // learned closure: per-point coefficients (rows past Ny are padding)
+      const int ya = min(y0 + 2 * c, ny - 1), yb = min(y0 + 2 * c + 1, ny - 1);
+      const float2 ca = a.les_coef[((long long)z * ny + ya) * nx + x];
+      const float2 cb = a.les_coef[((long long)z * ny + yb) * nx + x];
+      // C delta^2 in the working precision (no FP64 per point in FP32)
+      const T dsq = (T)a.les_dsq;
+      sgs_point_c<T>(sx, lr, (T)ca.x * dsq, (T)ca.y * dsq);
+      sgs_point_c<T>(sy, lr, (T)cb.x * dsq, (T)cb.y * dsq);
+    } else {
+      sgs_point<T>(sx, lr, cds, prt);
+      sgs_point<T>(sy, lr, cds, prt);
+    }
+#pragma unroll
+    for (int m = 0; m < 9; ++m)
+      if (m < lr) s_in[((lu + m) * yp + c) * ld + sidx(x)] = mk<C>(sx[m], sy[m]);
+  }
 }
 
 // ------------------------------------------------------------------ x pass
@@ -816,36 +852,7 @@ __device__ __forceinline__ void x_pass_body(const XPassArgs<T>& a, const FftPlan
 
   // ---- subgrid stress: the gradient lines become -2 nu_t S and -kappa_t dT
   if (a.les) {
-    const int lu = a.g.lu, lr = a.g.lr;
-    const T cds = a.les == 1 ? (T)a.les_cds[0] : (T)0, prt = (T)a.les_prt_inv;
-    for (int e = threadIdx.x; e < yp * nx; e += blockDim.x) {
-      const int c = (int)fdiv(e, a.fd_nx), x = e - c * nx;
-      C v[9];
-      T sx[9], sy[9];
-#pragma unroll
-      for (int m = 0; m < 9; ++m)
-        if (m < lr) {
-          v[m] = s_in[((lu + m) * yp + c) * ld + sidx(x)];
-          sx[m] = v[m].x;
-          sy[m] = v[m].y;
-        }
-      if (a.les == 2) {
-        // learned closure: per-point coefficients (rows past Ny are padding)
-        const int ya = min(y0 + 2 * c, ny - 1), yb = min(y0 + 2 * c + 1, ny - 1);
-        const float2 ca = a.les_coef[((long long)z * ny + ya) * nx + x];
-        const float2 cb = a.les_coef[((long long)z * ny + yb) * nx + x];
-        // C delta^2 in the working precision (no FP64 per point in FP32)
-        const T dsq = (T)a.les_dsq;
-        sgs_point_c<T>(sx, lr, (T)ca.x * dsq, (T)ca.y * dsq);
-        sgs_point_c<T>(sy, lr, (T)cb.x * dsq, (T)cb.y * dsq);
-      } else {
-        sgs_point<T>(sx, lr, cds, prt);
-        sgs_point<T>(sy, lr, cds, prt);
-      }
-#pragma unroll
-      for (int m = 0; m < 9; ++m)
-        if (m < lr) s_in[((lu + m) * yp + c) * ld + sidx(x)] = mk<C>(sx[m], sy[m]);
-    }
+    sgs_terms<T>(a, s_in, ld, y0, z);
     __syncthreads();
   }
 
@@ -1000,17 +1007,13 @@ __global__ void __launch_bounds__(x_threads(sizeof(T), PATH == kFft256), MinBloc
 //    (16 - j) mod 16 for k = 0) and stores the split pair.  Teams synchronise
 //    only among their own 16 threads: the product phase has no CTA barrier
 //    and no separate output loop.
+// With a subgrid closure (LES) the gradient lines join the input lines, and a
+// product's own gradient line, once it is added, is the team's scratch line:
+// 26 lines of a 4-row tile leave room for three CTAs per SM.  The general
+// kernel took 20.5 M instructions a field against 12.5 M here (256^3, learned
+// closure, stage 2: 0.61 -> 0.52 ms).
 // Shared memory: the 16 x 16 twiddles w_256^{k q} at [16 q + k], the Nin *
-// Y/2 input lines, one scratch line per team (vel_max's reduction scratch
-// before the products).
-constexpr int kXf256Threads = 288;                  // 18 teams of 16 (two rounds of 9 x 4 product lines)
-constexpr int kXf256Teams = kXf256Threads / 16;
-constexpr int kXf256Ld = 271;                       // line_stride(256)
-static_assert(kXf256Ld == ((256 + (255 >> 4)) | 1), "line stride of a 256-point line");
-__host__ __device__ constexpr size_t x_f256_smem(int lines) {
-  return sizeof(float2) * (256 + (size_t)(lines + kXf256Teams) * kXf256Ld);
-}
-
+// Y/2 input lines, one scratch line per team (not with LES).
 // the second stage of the 16 x 16 path on a line already in shared memory:
 // thread k reads row 16 k + q, applies w_256^{k q} and transforms it, leaving
 // Z(k + 16 j) in v[j]
@@ -1022,9 +1025,7 @@ __device__ __forceinline__ void f256_rows(float2* v, const float2* line, const f
   dft16<SIGN>(v);
 }
 
-// (a template only so that the translation units including this header
-// share one instantiation)
-template <int V = 0>
+template <bool LES>
 __global__ void __launch_bounds__(kXf256Threads, 3) k_x_pass_f256(const __grid_constant__ XPassArgs<float> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int nx = 256, LD = kXf256Ld;
@@ -1032,7 +1033,10 @@ __global__ void __launch_bounds__(kXf256Threads, 3) k_x_pass_f256(const __grid_c
   float2* s_in = s_tw + 256;
   const int ny = a.g.ny, kmx = a.g.kx, mx = a.g.mx;
   const int Y = a.yt, yp = Y / 2, nl = a.nin * yp;
-  float2* s_pr = s_in + nl * LD;
+  float2* s_pr = s_in + nl * LD;  // (not with LES)
+  constexpr int nw = kXf256Threads / 32;
+  __shared__ float s_mx[4 * nw];
+  __shared__ int s_bad[nw];
   const int nyt = (ny + Y - 1) / Y;
   const int z = blockIdx.x / nyt;
   const int y0 = (blockIdx.x - z * nyt) * Y;
@@ -1135,9 +1139,6 @@ __global__ void __launch_bounds__(kXf256Threads, 3) k_x_pass_f256(const __grid_c
       for (int f = 0; f < 4; ++f) mx4[f] = fmaxf(mx4[f], __shfl_xor_sync(0xffffffffu, mx4[f], o));
       bad |= __shfl_xor_sync(0xffffffffu, bad, o);
     }
-    constexpr int nw = kXf256Threads / 32;
-    float* s_mx = reinterpret_cast<float*>(s_pr);
-    int* s_bad = reinterpret_cast<int*>(s_mx + 4 * nw);
     if ((tid & 31) == 0) {
 #pragma unroll
       for (int f = 0; f < 4; ++f) s_mx[(tid >> 5) * 4 + f] = mx4[f];
@@ -1159,10 +1160,14 @@ __global__ void __launch_bounds__(kXf256Threads, 3) k_x_pass_f256(const __grid_c
     __syncthreads();
   }
 
+  if constexpr (LES) {
+    sgs_terms<float>(a, s_in, LD, y0, z);
+    __syncthreads();
+  }
+
   // ---- products (rhs.f:46-60), forward transforms, split, scale, store
   // C(m, z, kx, y) (xy_trans_f.f:20-37)
   const float fn = a.fn;
-  float2* tline = s_pr + team * LD;
   const int partner = (tid & 16) | ((16 - k) & 15);
   const int nq = a.g.lr * yp;
   for (int q = team; q < nq; q += kXf256Teams) {
@@ -1171,6 +1176,8 @@ __global__ void __launch_bounds__(kXf256Threads, 3) k_x_pass_f256(const __grid_c
     product_pair(m, fa, fb);
     const float2* pa = s_in + (fa * yp + c) * LD + k;
     const float2* pb = s_in + (fb * yp + c) * LD + k;
+    // (with LES the product's gradient line: read here, then overwritten)
+    float2* tline = LES ? s_in + ((a.g.lu + m) * yp + c) * LD : s_pr + team * LD;
     float2 v[16];
     // (scalar products: a packed mul.rn.f32x2 feeding the first stage's
     // packed sums is fused by the compiler into an FMA despite the .rn)
@@ -1178,6 +1185,10 @@ __global__ void __launch_bounds__(kXf256Threads, 3) k_x_pass_f256(const __grid_c
     for (int j = 0; j < 16; ++j) {
       const float2 ea = pa[17 * j], eb = pb[17 * j];
       v[j] = make_float2(pmul(ea.x, eb.x), pmul(ea.y, eb.y));
+      if constexpr (LES) {
+        const float2 eg = tline[k + 17 * j];
+        v[j] = make_float2(v[j].x + eg.x, v[j].y + eg.y);
+      }
     }
     dft16<-1>(v);
     __syncwarp(tmask);  // the team's reads of its previous line are done
@@ -1215,12 +1226,6 @@ __global__ void __launch_bounds__(kXf256Threads, 3) k_x_pass_f256(const __grid_c
   }
 }
 
-// whether k_x_pass_f256 runs this launch (else the general kernel)
-__host__ __device__ inline bool x_f256_applies(const XPassArgs<float>& a) {
-  return a.g.nx == 256 && a.sched == 0 && a.in_mode == 0 && a.out_mode == 2 && a.les == 0 && a.nin == a.g.lu &&
-         a.nin <= 4 && (a.g.lr == 6 || a.g.lr == 9) && (!a.partials || a.max_only) && a.yt >= 2 && a.yt % 2 == 0;
-}
-
 // ------------------------------------------------ x pass, FP64 at Nx = 256
 // The x pass of the plain FP64 step with 256-point x lines (spectral input
 // rows, products out, no subgrid terms) with the physical fields kept in
@@ -1235,37 +1240,41 @@ __host__ __device__ inline bool x_f256_applies(const XPassArgs<float>& a) {
 // from its factors to HBM by itself, as in k_x_pass_f256; the exchange between
 // the two radix-16 stages goes through half a line (re, then im), so that 16
 // teams' scratch and an 8-row tile's input lines leave room for two CTAs per SM.
-constexpr int kXfx256Threads = 256;
-constexpr int kXfx256Teams = kXfx256Threads / 16;
-__host__ __device__ constexpr size_t x_fx256_smem(int lines) {
-  return sizeof(fxw) * 256 + (size_t)lines * (sizeof(fxc) * kXf256Ld + sizeof(FxLine)) +
-         (size_t)kXfx256Teams * kXf256Ld * sizeof(long long);
-}
-
-template <int V = 0>
-__global__ void __launch_bounds__(kXfx256Threads, 2) k_x_pass_fx256(const __grid_constant__ XPassArgs<double> a) {
+//
+// With a subgrid closure (LES) the gradient lines are doubles until the terms
+// are formed, and a product's own gradient line is its team's scratch; the
+// twiddles then stay in memory (L1): 26 lines of a 4-row tile fit an SM twice
+// only without them, and 18 teams take its 18 product lines in one round (16
+// teams 3.28 ms, 2-row tiles with 3 or 4 CTAs per SM 3.53 and 3.61).  The
+// general kernel ran two-row tiles (256^3, dynamic closure, stage 2: 4.30 ->
+// 3.15 ms).  Neither pipe is the bound (FP64 43 %, ALU 39 %): two CTAs whose
+// phases use one or the other overlap in part.
+template <bool LES>
+__global__ void __launch_bounds__(x_fx256_threads(LES), 2) k_x_pass_fx256(const __grid_constant__ XPassArgs<double> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ unsigned long long s_vmax[4];
   __shared__ int s_bad;
-  constexpr int nx = 256, LD = kXf256Ld;
+  constexpr int nx = 256, LD = kXf256Ld, NT = x_fx256_threads(LES), NTEAM = NT / 16;
   const int ny = a.g.ny, kmx = a.g.kx, mx = a.g.mx;
   const int Y = a.yt, yp = Y / 2, nl = a.nin * yp;
-  fxw* s_tw = reinterpret_cast<fxw*>(smem_raw);
-  double2* s_in = reinterpret_cast<double2*>(s_tw + 256);
+  double2* s_in = reinterpret_cast<double2*>(smem_raw);
   FxLine* s_line = reinterpret_cast<FxLine*>(s_in + nl * LD);
-  long long* s_ex = reinterpret_cast<long long*>(s_line + nl);
+  const int nfac = a.g.lu * yp;  // lines of factors
+  // (without LES)
+  fxw* s_tw = reinterpret_cast<fxw*>(s_line + nl);
+  long long* s_ex = reinterpret_cast<long long*>(s_tw + 256);
   const int nyt = (ny + Y - 1) / Y;
   const int z = blockIdx.x / nyt;
   const int y0 = (blockIdx.x - z * nyt) * Y;
   const int yv = min(Y, ny - y0);
   const int tid = threadIdx.x;
-  s_tw[tid] = a.tw[tid];
+  if constexpr (!LES) s_tw[tid] = a.tw[tid];
   if (tid < 4) s_vmax[tid] = 0;
   if (tid == 4) s_bad = 0;
   {
     // zeros in the truncated band (sidx of its ends: one contiguous run)
     const int b0 = sidx(kmx + 1), nb = sidx(nx - kmx - 1) - b0 + 1;
-    for (int L = tid >> 4; L < nl; L += kXfx256Teams)
+    for (int L = tid >> 4; L < nl; L += NTEAM)
       for (int j = tid & 15; j < nb; j += 16) s_in[L * LD + b0 + j] = make_double2(0.0, 0.0);
   }
   {
@@ -1300,10 +1309,10 @@ __global__ void __launch_bounds__(kXfx256Threads, 2) k_x_pass_fx256(const __grid
   // ---- the backward transforms (xy_trans_b.f:39-60), in place
   const int team = tid >> 4, k = tid & 15;
   const unsigned tmask = 0xFFFFu << (tid & 16);
-  const fxw* w = s_tw + k;
-  const int rounds = (nl + kXfx256Teams - 1) / kXfx256Teams;
+  const fxw* __restrict__ w = (LES ? a.tw : s_tw) + k;
+  const int rounds = (nl + NTEAM - 1) / NTEAM;
   for (int r = 0; r < rounds; ++r) {
-    const int L = r * kXfx256Teams + team;
+    const int L = r * NTEAM + team;
     const bool active = L < nl;
     fxc* line = reinterpret_cast<fxc*>(s_in) + (active ? L : 0) * LD;
     fxc v[16];
@@ -1326,6 +1335,11 @@ __global__ void __launch_bounds__(kXfx256Threads, 2) k_x_pass_fx256(const __grid
     for (int q = 1; q < 16; ++q) v[q] = ctw<+1>(line[17 * k + q], w[16 * q]);
     dft16<+1>(v);
     __syncwarp(tmask);
+    if (LES && L >= nfac) {
+#pragma unroll
+      for (int s = 0; s < 16; ++s) reinterpret_cast<double2*>(line)[k + 17 * s] = fx_out<true>(v[s], sc);
+      continue;
+    }
 #pragma unroll
     for (int s = 0; s < 16; ++s) reinterpret_cast<FxSplit2*>(line)[k + 17 * s] = fx_split2(v[s]);
     if (k == 0) s_line[L] = FxLine{sc.ex, sc.kind, sc.norm};
@@ -1357,6 +1371,13 @@ __global__ void __launch_bounds__(kXfx256Threads, 2) k_x_pass_fx256(const __grid
     if (tid == 4 && s_bad) atomicOr(a.vmax + 8, 1);
   }
 
+  if constexpr (LES) {
+    sgs_terms<double>(a, s_in, LD, y0, z);
+    __syncthreads();
+    for (int L = nfac + (tid >> 5); L < nl; L += NT / 32) fx_line_bound(s_in + L * LD, s_line + L, nx);
+    __syncthreads();
+  }
+
   // ---- products (rhs.f:46-60), forward transforms, split, scale, store
   // C(m, z, kx, y) (xy_trans_f.f:20-37)
   const bool pow2 = is_pow2_inv(ny);
@@ -1364,11 +1385,12 @@ __global__ void __launch_bounds__(kXfx256Threads, 2) k_x_pass_fx256(const __grid
   long long* tx = s_ex + team * LD;
   const int partner = (tid & 16) | ((16 - k) & 15);
   const int nq = a.g.lr * yp;
-  for (int q = team; q < nq; q += kXfx256Teams) {
+  for (int q = team; q < nq; q += NTEAM) {
     const int m = (int)fdiv(q, a.fd_yp), c = q - m * yp;
     int fa, fb;
     product_pair(m, fa, fb);
-    const FxProduct p = fx_product(s_line[fa * yp + c], s_line[fb * yp + c]);
+    const int gl = (a.g.lu + m) * yp + c;  // the product's gradient line (LES)
+    const FxProduct p = fx_product(s_line[fa * yp + c], s_line[fb * yp + c], LES ? s_line + gl : nullptr);
     const FxSplit2* pa = reinterpret_cast<const FxSplit2*>(s_in) + (fa * yp + c) * LD + k;
     const FxSplit2* pb = reinterpret_cast<const FxSplit2*>(s_in) + (fb * yp + c) * LD + k;
     fxc v[16];
@@ -1376,20 +1398,31 @@ __global__ void __launch_bounds__(kXfx256Threads, 2) k_x_pass_fx256(const __grid
     for (int j = 0; j < 16; ++j) {
       const FxSplit2 ea = pa[17 * j], eb = pb[17 * j];
       v[j] = fxc{fx_mul_line(ea.x, eb.x, p), fx_mul_line(ea.y, eb.y, p)};
+      if constexpr (LES) fx_add_term(v[j], s_in[gl * LD + k + 17 * j], p);
     }
     dft16<-1>(v);
-    __syncwarp(tmask);  // the team's reads of its previous line are done
+    if constexpr (LES) {
+      fxc* tl = reinterpret_cast<fxc*>(s_in) + gl * LD;
+      // (each thread has read and writes its own column)
 #pragma unroll
-    for (int s = 0; s < 16; ++s) tx[17 * s + k] = v[s].x;
-    __syncwarp(tmask);
+      for (int s = 0; s < 16; ++s) tl[17 * s + k] = v[s];
+      __syncwarp(tmask);
 #pragma unroll
-    for (int s = 0; s < 16; ++s) v[s].x = tx[17 * k + s];
-    __syncwarp(tmask);
+      for (int s = 0; s < 16; ++s) v[s] = tl[17 * k + s];
+    } else {
+      __syncwarp(tmask);  // the team's reads of its previous line are done
 #pragma unroll
-    for (int s = 0; s < 16; ++s) tx[17 * s + k] = v[s].y;
-    __syncwarp(tmask);
+      for (int s = 0; s < 16; ++s) tx[17 * s + k] = v[s].x;
+      __syncwarp(tmask);
 #pragma unroll
-    for (int s = 0; s < 16; ++s) v[s].y = tx[17 * k + s];
+      for (int s = 0; s < 16; ++s) v[s].x = tx[17 * k + s];
+      __syncwarp(tmask);
+#pragma unroll
+      for (int s = 0; s < 16; ++s) tx[17 * s + k] = v[s].y;
+      __syncwarp(tmask);
+#pragma unroll
+      for (int s = 0; s < 16; ++s) v[s].y = tx[17 * k + s];
+    }
 #pragma unroll
     for (int s = 1; s < 16; ++s) v[s] = ctw<-1>(v[s], w[16 * s]);
     dft16<-1>(v);
@@ -1417,12 +1450,6 @@ __global__ void __launch_bounds__(kXfx256Threads, 2) k_x_pass_fx256(const __grid
       }
     }
   }
-}
-
-// whether k_x_pass_fx256 runs this launch (else the general kernel)
-__host__ __device__ inline bool x_fx256_applies(const XPassArgs<double>& a) {
-  return a.g.nx == 256 && a.sched == 0 && a.in_mode == 0 && a.out_mode == 2 && a.les == 0 && a.nin == a.g.lu &&
-         a.nin <= 4 && (a.g.lr == 6 || a.g.lr == 9) && (!a.partials || a.max_only) && a.yt >= 2 && a.yt % 2 == 0;
 }
 
 // --------------------------------------------------------------- y forward
@@ -2079,18 +2106,17 @@ void launch_y_inv_part(const YInvArgs<T>& a, const FftPlan* pl, size_t smem, cud
 template <typename T, int PART, int PARTS>
 void launch_x_pass_part(const XPassArgs<T>& a, const FftPlan* pl, size_t smem, cudaStream_t s) {
   if constexpr (path_part(256, PARTS) == PART) {
-    if constexpr (std::is_same<T, float>::value) {
-      const size_t fsm = x_f256_smem(a.nin * (a.yt / 2));
-      if (x_f256_applies(a) && fsm <= (size_t)smem_optin()) {
-        k_x_pass_f256<><<<x_pass_blocks(a), kXf256Threads, fsm, s>>>(a);
-        return;
+    if (x_fused(a)) {
+      const int blocks = x_pass_blocks(a);
+      const size_t fsm = x_fused_smem(a);
+      if constexpr (std::is_same<T, float>::value) {
+        if (a.les) k_x_pass_f256<true><<<blocks, kXf256Threads, fsm, s>>>(a);
+        else k_x_pass_f256<false><<<blocks, kXf256Threads, fsm, s>>>(a);
+      } else {
+        if (a.les) k_x_pass_fx256<true><<<blocks, x_fx256_threads(true), fsm, s>>>(a);
+        else k_x_pass_fx256<false><<<blocks, x_fx256_threads(false), fsm, s>>>(a);
       }
-    } else {
-      const size_t fsm = x_fx256_smem(a.nin * (a.yt / 2));
-      if (x_fx256_applies(a) && fsm <= (size_t)smem_optin() - 1024) {
-        k_x_pass_fx256<><<<x_pass_blocks(a), kXfx256Threads, fsm, s>>>(a);
-        return;
-      }
+      return;
     }
   }
   with_path<PART, PARTS, true>(a.g.nx, a.sched, [&](auto p) {
@@ -2132,9 +2158,15 @@ template <typename T, int PART, int PARTS> void smem_yinv_part(int n, int optin)
 template <typename T, int PART, int PARTS> void smem_x_part(int n, int optin) {
   if constexpr (path_part(256, PARTS) == PART) {
     if constexpr (std::is_same<T, float>::value) {
-      if (n == 256) allow_dynamic_smem((const void*)k_x_pass_f256<>, optin);
+      if (n == 256) {
+        allow_dynamic_smem((const void*)k_x_pass_f256<false>, optin);
+        allow_dynamic_smem((const void*)k_x_pass_f256<true>, optin);
+      }
     } else {
-      if (n == 256) allow_dynamic_smem((const void*)k_x_pass_fx256<>, optin);
+      if (n == 256) {
+        allow_dynamic_smem((const void*)k_x_pass_fx256<false>, optin);
+        allow_dynamic_smem((const void*)k_x_pass_fx256<true>, optin);
+      }
     }
   }
   each_sched<PART, PARTS, true>(n, [&](auto p) { allow_dynamic_smem((const void*)k_x_pass<T, decltype(p)::value>, optin); });

@@ -429,9 +429,17 @@ static int run_x_pass(Ctx& c, int in_mode, int out_mode, int nin, const void* in
   a.out_mode = out_mode;
   a.nin = nin;
   a.sched = c.sched[2];
-  int rc = x_tile<T>(c, nin, out_mode, a.yt, a.group);
-  if (rc) return rc;
-  a.prod_lines = std::max(a.group, x_red_lines<T>(c));
+  // (a fused closure pass takes its own tile; the general kernel's would be
+  // cut down to two rows by its product lines)
+  a.yt = std::min(c.yt_x, kXFusedLesRows);
+  // the resident step takes vel_max's sums from wave space (Parseval): the
+  // x pass then only forms max |u| and the NaN check
+  a.max_only = stats && in_mode == 0 && in == c.S2;
+  if (!(les && !c.rec && (!stats || a.max_only) && x_fused(a))) {
+    const int rc = x_tile<T>(c, nin, out_mode, a.yt, a.group);
+    if (rc) return rc;
+    a.prod_lines = std::max(a.group, x_red_lines<T>(c));
+  }
   a.ld = line_ld(c.g.nx);
   a.in_y = in_y; a.in_z = in_z; a.in_n = in_n;
   a.out_kx = out_kx; a.out_z = out_z; a.out_n = out_n;
@@ -446,9 +454,6 @@ static int run_x_pass(Ctx& c, int in_mode, int out_mode, int nin, const void* in
       c.partial_blocks = nblk;
     }
     a.partials = c.partials;
-    // the resident step takes vel_max's sums from wave space (Parseval): the
-    // x pass then only forms max |u| and the NaN check
-    a.max_only = in_mode == 0 && in == c.S2;
     a.vmax = reinterpret_cast<int*>(c.pv + 4 * ((size_t)kParsevalBlocks + 1));
   }
   if constexpr (std::is_same<T, float>::value) {

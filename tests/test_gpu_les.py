@@ -3,6 +3,7 @@ on the GPU against the oracle's restatements."""
 import numpy as np
 import pytest
 
+import closure as CL
 import oracle as O
 from sam_gb300 import SamGpu
 
@@ -137,6 +138,41 @@ def test_coupled_closure_stages_and_fp32(gpu_lib):
     u32 = g32.download()
     for n in range(o.d.lu):
         assert relerr(u32[..., n], u[..., n]) <= 2e-5, n
+
+
+@pytest.mark.parametrize("precision,model", [(64, 1), (64, 2), (32, 1), (32, 3)])
+@pytest.mark.parametrize("strat,ny", [(1, 8), (1, 9), (0, 2), (0, 10)])
+def test_closure_on_256_point_lines(gpu_lib, precision, model, strat, ny):
+    """The fused x passes of 256-point lines with a closure (tiles of 4 rows:
+    whole, with one or two rows left, both numbers of products) against
+    the general kernel, which the Stockham schedule takes.  Both add the same
+    terms to the same products; they differ by the rounding of two transforms
+    of 256 points (log2 n + 2 roundings each way at most, all fields of one
+    size), so one stage agrees to 64 roundings of the largest value; the three
+    stages of a step to 256.  The learned closure's network is all zeros here:
+    its coefficient is then the same at every point for both kernels."""
+    cfg = dict(nx=256, ny=ny, nz=8, i_strat=strat, buoy_fac_z=1.0 * strat, lapse=1.0 * strat, vis=1e-4, i_cfl=1, cfl0=0.5)
+    eps = 2.0 ** -53 if precision == 64 else 2.0 ** -24
+    u0 = O.Oracle(**cfg).init_random(7, 0, 1.0, 0, 0.1)
+    out = []
+    for sched in (0, 1):
+        g = SamGpu(precision=precision, **cfg)
+        g.upload(u0)
+        if model == 3:
+            g.mlp_set(np.zeros(CL.N_PARAMS, np.float32))
+        g.set_les(model, c_smag=0.03, pr_t=0.7)
+        g.set_fft_schedule([0, 0, sched, 0, 0])
+        g.stage(1)
+        a = g.download()
+        g.stage(2)
+        g.stage(3)
+        out.append((a, g.download(), g.stats()["dt"]))
+        g.close()
+    (a, b, dt), (ar, br, dtr) = out
+    for n in range(4 if strat else 3):
+        assert relerr(a[..., n], ar[..., n]) <= 64 * eps, n
+        assert relerr(b[..., n], br[..., n]) <= 256 * eps, n
+    assert abs(dt - dtr) <= 64 * eps * dtr
 
 
 def test_closure_off_restores_reference_products(gpu_lib):
