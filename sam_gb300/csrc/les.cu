@@ -17,6 +17,7 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "fx64.cuh"
 #include "les.cuh"
 
 namespace samgpu {
@@ -147,80 +148,162 @@ __global__ void k_dm_fields(const double* __restrict__ ub, double* __restrict__ 
 }
 
 // dm.f:122-150: L_ij, M_ij at each interior point, per-CTA sums of
-// ifact L M and ifact M M (fixed order, deterministic).  Bound by the FP64
-// pipe, so the 1-4-1 test filter is taken one direction at a time (across
-// planes, along y, along x: filter.f's order): a CTA does a 32 x 8 tile of
-// one plane, each of the 21 fields in turn through two shared tiles, 2 FP64
-// operations a point and direction (7 a point and field with the tile's halo
-// rows against 27 for the stencil in one step; the dynamic coefficient at
-// 256^3 24 -> 8 ms, with the integer factors no longer converted to FP64 per
-// point).
-constexpr int kDmTx = 32, kDmTy = 8;
-static_assert(kDmTx * kDmTy == kThreads, "one point per thread");
+// ifact L M and ifact M M (fixed order, deterministic).  The 1-4-1 test filter
+// is taken one direction at a time (across planes, along y, along x: filter.f's
+// order): a CTA does a 32 x 8 x 2 tile, each of the 21 fields in turn.  In FP64
+// that is 7 operations a point and field on the pipe that bounds the kernel
+// (66 cycles each), so the filter runs on integers, as the transforms do: a
+// tile's values of one field under its own power of two (55 bits below its
+// largest value, cut off there: a quarter of an FP64 rounding of it), exact
+// sums, one conversion back.  A tile that holds infinities, NaN, nothing but
+// zeros or numbers near the smallest takes the sums in FP64.  The filtered
+// values stay 216 times too large; the factors are taken out of the sums.
+// Loads of the next field are in flight while this one is filtered.
+// 256^3: 3.2 ms with integers (FP64 pipe 43 %, ALU 48 %), 6.9 in FP64 one
+// direction at a time, 22 with the 27-point stencil.  64 registers (four CTAs
+// per SM, a few spills) against 80 and 128: 3.2, 3.5 and 4.7 ms.
+constexpr int kDmTx = 32, kDmTy = 8, kDmTz = 2;
+static_assert(kDmTx * kDmTy == kThreads, "one column of points per thread");
 static long long dm_tiles(int nx, int ny, int nz) {
-  return (long long)((nx + kDmTx - 1) / kDmTx) * ((ny + kDmTy - 1) / kDmTy) * nz;
+  return (long long)((nx + kDmTx - 1) / kDmTx) * ((ny + kDmTy - 1) / kDmTy) * ((nz + kDmTz - 1) / kDmTz);
 }
+// 1-4-1 sums
+__device__ __forceinline__ double sum141(double a, double b, double c) { return a + 4 * b + c; }
+__device__ __forceinline__ long long sum141(long long a, long long b, long long c) { return a + (b << 2) + c; }
 
-__global__ void __launch_bounds__(kThreads, 3)
+__global__ void __launch_bounds__(kThreads, 4)
     k_dm_lm(const double* __restrict__ ub, const double* __restrict__ q, Halo H, double alpha_sq,
             double* __restrict__ part) {
-  constexpr int HX = kDmTx + 2, HY = kDmTy + 2;
-  __shared__ double s_h[2][HY * HX], s_g[2][kDmTy * HX];
+  constexpr int HX = kDmTx + 2, HY = kDmTy + 2, PZ = kDmTz + 2, NW = kThreads / 32;
+  constexpr int kPts = HY * HX, kRows = kDmTy * HX;
+  __shared__ long long s_h[kDmTz][kPts], s_g[kDmTz][kRows];
+  __shared__ uint32_t s_max[2][NW];
   __shared__ double red[2][kThreads];
-  const long long n = H.ninterior();
+  const long long n = H.ninterior(), pl = (long long)H.nx * H.ny;
   const int tid = threadIdx.x, tx = tid & (kDmTx - 1), ty = tid / kDmTx;
   const int ntx = (H.nx + kDmTx - 1) / kDmTx, nty = (H.ny + kDmTy - 1) / kDmTy;
-  const long long tiles = (long long)ntx * nty * H.nz;
-  const double inv = 1.0 / 216.0;
+  const long long tiles = (long long)ntx * nty * ((H.nz + kDmTz - 1) / kDmTz);
   double num = 0.0, den = 0.0;
   for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
-    const int z = (int)(t / (ntx * nty)), r = (int)(t - (long long)z * (ntx * nty));
+    const int z0 = (int)(t / (ntx * nty)) * kDmTz, r = (int)(t % (ntx * nty));
     const int x0 = (r % ntx) * kDmTx, y0 = (r / ntx) * kDmTy;
     // this thread's points of the tile with halo (at most two), the planes' offsets
-    long long off[2];
+    long long off[2], zo[PZ];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      const int e = min(tid + i * kThreads, HY * HX - 1);
+      const int e = min(tid + i * kThreads, kPts - 1);
       const int xx = (x0 + e % HX - 1 + H.nx) % H.nx, yy = (y0 + e / HX - 1 + H.ny) % H.ny;
       off[i] = (long long)yy * H.nx + xx;
     }
-    const long long pl = (long long)H.nx * H.ny;
-    const long long zm = H.wz(z - 1) * pl, zc = z * pl, zp = H.wz(z + 1) * pl;
-    int buf = 0;
-    auto filt = [&](const double* __restrict__ f) {  // 216 times the filtered field at this thread's point
-      double* h = s_h[buf];
-      double* g = s_g[buf];
-      buf ^= 1;
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int e = tid + i * kThreads;
-        if (e < HY * HX) h[e] = f[zm + off[i]] + 4 * f[zc + off[i]] + f[zp + off[i]];
-      }
-      __syncthreads();
-      for (int e = tid; e < kDmTy * HX; e += kThreads) g[e] = h[e] + 4 * h[e + HX] + h[e + 2 * HX];
-      __syncthreads();
-      const double* gp = g + ty * HX + tx;
-      return gp[0] + 4 * gp[1] + gp[2];
+    for (int p = 0; p < PZ; ++p) zo[p] = (long long)((z0 + p - 1 + H.nz) % H.nz) * pl;
+
+    double v[2][PZ] = {};  // the current field at this thread's points
+    const auto load = [&](const double* __restrict__ f) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        if (tid + i * kThreads < kPts)
+#pragma unroll
+          for (int p = 0; p < PZ; ++p) v[i][p] = f[zo[p] + off[i]];
     };
-    double uh[3], sh[6];
+    const auto largest = [&](int buf) {  // of the loaded field, per warp
+      uint32_t hm = 0;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) uh[c] = inv * filt(ub + c * n);
+      for (int i = 0; i < 2; ++i)
+        if (tid + i * kThreads < kPts)
 #pragma unroll
-    for (int c = 0; c < 6; ++c) sh[c] = inv * filt(q + c * n);
-    const double w = alpha_sq * smag(sh);
-    double n2[2] = {0.0, 0.0}, d2[2] = {0.0, 0.0};
+          for (int p = 0; p < PZ; ++p) hm = max(hm, (uint32_t)__double2hiint(v[i][p]) & 0x7fffffffu);
+      hm = __reduce_max_sync(0xffffffffu, hm);
+      if ((tid & 31) == 0) s_max[buf][tid >> 5] = hm;
+    };
+    int buf = 0;
+    __syncthreads();  // (the last tile's reads are done)
+    load(ub);
+    largest(buf);
+    __syncthreads();
+    // 216 times the loaded field, filtered, at this thread's points; loads the next field
+    const auto filt = [&](const double* __restrict__ next, double* out) {
+      uint32_t hm = s_max[buf][0];
+#pragma unroll
+      for (int w = 1; w < NW; ++w) hm = max(hm, s_max[buf][w]);
+      const int E = (int)(hm >> 20);
+      buf ^= 1;
+      const bool fx = E >= 64 && E < 0x7ff;  // |v| < 2^(E - 1022)
+      const auto planes = [&](auto conv) {
+        using V = decltype(conv(0.0));
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int e = tid + i * kThreads;
+          if (e >= kPts) break;
+          V c[PZ];
+#pragma unroll
+          for (int p = 0; p < PZ; ++p) c[p] = conv(v[i][p]);
+#pragma unroll
+          for (int p = 0; p < kDmTz; ++p) reinterpret_cast<V*>(s_h[p])[e] = sum141(c[p], c[p + 1], c[p + 2]);
+        }
+        __syncthreads();
+        if (next) load(next);
+#pragma unroll
+        for (int p = 0; p < kDmTz; ++p)
+          for (int e = tid; e < kRows; e += kThreads) {
+            const V* h = reinterpret_cast<const V*>(s_h[p]) + e;
+            reinterpret_cast<V*>(s_g[p])[e] = sum141(h[0], h[HX], h[2 * HX]);
+          }
+        if (next) largest(buf);
+        __syncthreads();
+      };
+      if (fx) {
+        planes([&](double d) { return fx_from(d, E + 8); });  // integers below 2^55, their sums below 2^63
+#pragma unroll
+        for (int p = 0; p < kDmTz; ++p) {
+          const long long* g = s_g[p] + ty * HX + tx;
+          out[p] = fx_to_alu(sum141(g[0], g[1], g[2]), E + 8 - 1085);
+        }
+      } else {
+        planes([](double d) { return d; });
+#pragma unroll
+        for (int p = 0; p < kDmTz; ++p) {
+          const double* g = reinterpret_cast<const double*>(s_g[p]) + ty * HX + tx;
+          out[p] = sum141(g[0], g[1], g[2]);
+        }
+      }
+    };
+    double uh[3][kDmTz], sh[6][kDmTz], w[kDmTz];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) filt(c < 2 ? ub + (c + 1) * n : q, uh[c]);
+#pragma unroll
+    for (int c = 0; c < 6; ++c) filt(q + (c < 5 ? c + 1 : 6) * n, sh[c]);
+#pragma unroll
+    for (int p = 0; p < kDmTz; ++p) {
+      double m[6];
+#pragma unroll
+      for (int c = 0; c < 6; ++c) m[c] = sh[c][p];
+      w[p] = alpha_sq / 216.0 * smag(m);
+    }
+    double n2[2][kDmTz] = {}, d2[2][kDmTz] = {};
 #pragma unroll
     for (int c = 0; c < 6; ++c) {
-      const double M = w * sh[c] - inv * filt(q + (6 + c) * n);
-      const double L = inv * filt(q + (12 + c) * n) - uh[kIp[c]] * uh[kJp[c]];
-      n2[c / 3] += L * M;
-      d2[c / 3] += M * M;
+      double a[kDmTz], b[kDmTz];
+      filt(q + (12 + c) * n, a);                    // |S| S_c
+      filt(c < 5 ? q + (7 + c) * n : nullptr, b);   // u_i u_j
+#pragma unroll
+      for (int p = 0; p < kDmTz; ++p) {
+        const double M = w[p] * sh[c][p] - a[p];                             // 216 M
+        const double L = 216.0 * b[p] - uh[kIp[c]][p] * uh[kJp[c]][p];       // 216^2 L
+        n2[c / 3][p] += L * M;
+        d2[c / 3][p] += M * M;
+      }
     }
-    if (x0 + tx < H.nx && y0 + ty < H.ny) {
-      num += n2[0] + 2 * n2[1];
-      den += d2[0] + 2 * d2[1];
-    }
+    if (x0 + tx < H.nx && y0 + ty < H.ny)
+#pragma unroll
+      for (int p = 0; p < kDmTz; ++p)
+        if (z0 + p < H.nz) {
+          num += n2[0][p] + 2 * n2[1][p];
+          den += d2[0][p] + 2 * d2[1][p];
+        }
   }
+  num *= 1.0 / (216.0 * 216.0 * 216.0);
+  den *= 1.0 / (216.0 * 216.0);
   red[0][threadIdx.x] = num;
   red[1][threadIdx.x] = den;
   __syncthreads();

@@ -69,6 +69,33 @@ def test_dynamic_smagorinsky(gpu_lib, dims):
     assert relerr(vt_g, vt_o) < 1e-12
 
 
+@pytest.mark.parametrize("dims", [(8, 5, 3), (40, 9, 15), (64, 16, 2)])
+def test_dynamic_coefficient_of_scaled_and_local_fields(gpu_lib, dims):
+    """The test filter runs on integers under a power of two per tile (32 x 8 x
+    2 points) and in FP64 where a tile has none to offer.  Powers of two leave
+    every rounding of both where it is, so the coefficient does not change by
+    a bit; a field that is zero but for one corner, and tiles cut by the box,
+    against the oracle at the per-routine bar; NaN stays NaN."""
+    nx, ny, nz = dims
+    cfg = dict(nx=nx, ny=ny, nz=nz, xl=1.0, yl=1.3, zl=0.7)
+    g, o = SamGpu(**cfg), O.Oracle(**cfg)
+    u = velocity(nx, ny, nz, 2)
+    c = g.dm(u)[1]
+    assert abs(c - o.dm(u)[1]) <= 1e-12 * abs(c)
+    for k in (-60, -1, 7, 60):
+        assert g.dm(u * 2.0 ** k)[1] == c, k
+    for tiny in (0.0, 1e-300):  # below 2^-959 the sums are taken in FP64
+        v = u * tiny
+        v[1:4, 1:4, 1:3] = u[1:4, 1:4, 1:3]
+        for n in range(3):
+            v[..., n] = periodic_fill(v[..., n].copy())
+        cv, co = g.dm(v)[1], o.dm(v)[1]
+        assert abs(cv - co) <= 1e-12 * abs(co), tiny
+    w = u.copy(order="F")
+    w[2, 2, 2, 1] = np.nan
+    assert np.isnan(g.dm(w)[1])
+
+
 @pytest.mark.parametrize("i_remove", [0, 1])
 def test_get_mean(gpu_lib, i_remove):
     cfg = dict(nx=16, ny=12, nz=40, i_strat=1, buoy_fac_z=1.0, lapse=1.0)
