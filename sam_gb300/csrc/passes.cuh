@@ -6,6 +6,25 @@
 
 namespace samgpu {
 
+// The gradient fields of a subgrid closure behind the Lu factors: the strain
+// S11 S12 S22 S13 S23 S33, with buoyancy the three parts of grad T, and for
+// the learned closure's invariants the three of the vorticity.  k_z enters
+// S13, S23, S33, dT/dz and the first two parts of the vorticity.
+__host__ __device__ inline bool derive_in_y(int n, int lu, int lr) {
+  const int m = n - lu;
+  return m >= 0 && (m < 3 || (m >= 6 && m < lr && m < 8) || m == lr + 2);
+}
+// field of the j-th line the z pass takes, and the number of lines for nvar fields
+__host__ __device__ inline int derive_z_field(int j, int lu, int lr) {
+  const int t = lr > 6 ? 1 : 0, m = j - lu;
+  return m < 0 ? j : lu + (m < 3 ? 3 + m : (m < 3 + t ? 8 : lr + m - 3 - t));
+}
+inline int derive_z_lines(int nvar, int lu, int lr) {
+  int k = 0;
+  for (int n = 0; n < nvar; ++n) k += !derive_in_y(n, lu, lr);
+  return k;
+}
+
 template <typename T>
 struct ZInvArgs {
   Grid g;
@@ -16,9 +35,9 @@ struct ZInvArgs {
   cx_t<T>* out;        // A(n, z, kx, ky)
   const tw_t<T>* tw;   // twiddles of the Nz plan
   int nvar, ty, ld;
-  // derive = 1: fields n >= Lu of the launch are the subgrid gradient fields
-  // m = n - Lu formed from the velocity (and T) rows while loading: S_ab for
-  // the six velocity products, dT/dx_a for the three buoyancy products
+  // derive = 1: fields n >= Lu are gradient fields formed from the velocity
+  // (and T) rows while loading; the launch has those that k_z enters
+  // (derive_z_field), the y pass forms the others
   int derive;
   long long in_ky, in_kx, in_n;
   long long out_kx, out_z, out_n;
@@ -34,6 +53,7 @@ struct YInvArgs {
   cx_t<T>* out;       // B(n, z, y, kx)
   const tw_t<T>* tw;
   int nvar, tx, ld, in_full;
+  int derive;  // 1: gradient fields without k_z (derive_in_y) are formed while loading
   long long in_kx, in_z, in_n;
   long long out_y, out_z, out_n;
 };

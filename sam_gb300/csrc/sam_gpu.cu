@@ -296,7 +296,7 @@ static int run_z_inv(Ctx& c, const void* in, void* out, int nvar, long long in_k
   a.in = (const cx_t<T>*)in;
   a.out = (cx_t<T>*)out;
   a.tw = tw_of<T>(c.pz);
-  a.nvar = nvar;
+  a.nvar = derive ? derive_z_lines(nvar, c.g.lu, c.g.lr) : nvar;
   a.sched = c.sched[0];
   a.ty = pick_tile(c.pz, c.ty_zi, 1, sizeof(cx_t<T>), a.sched);
   a.ld = line_ld(c.g.nz);
@@ -315,8 +315,9 @@ static int run_z_inv(Ctx& c, const void* in, void* out, int nvar, long long in_k
 
 template <typename T>
 static int run_y_inv(Ctx& c, const void* in, void* out, int nvar, int in_full, long long in_kx, long long in_z,
-                     long long in_n, long long out_y, long long out_z, long long out_n) {
+                     long long in_n, long long out_y, long long out_z, long long out_n, int derive = 0) {
   YInvArgs<T> a{};
+  a.derive = derive;
   a.g = c.g;
   a.in = (const cx_t<T>*)in;
   a.out = (cx_t<T>*)out;
@@ -583,7 +584,7 @@ static int enqueue_stage(Ctx& c, int nrk, cudaEvent_t* ev, int only, int write_p
   // y inverse: A -> B(n, z, y, kx)
   if (run(1))
     rc = run_y_inv<T>(c, c.S1, c.S2, ninv, 0, g.my, (long long)g.mx * g.my, (long long)g.nz * g.mx * g.my, g.mx,
-                      (long long)g.ny * g.mx, (long long)g.nz * g.ny * g.mx);
+                      (long long)g.ny * g.mx, (long long)g.nz * g.ny * g.mx, les ? 1 : 0);
   if (rc) return rc;
   if (ev) cudaEventRecord(ev[2], c.stream);
   // dynamic closure at nrk = 1 (once per step, like vel_max): the physical
@@ -1681,7 +1682,7 @@ static int closure_inputs_impl(Ctx& c, unsigned short* feat, double* grads) {
                          (long long)g.mx * g.my, (long long)g.nz * g.mx * g.my, 1)))
     return rc;
   if ((rc = run_y_inv<T>(c, c.sc[1].p, c.sc[2].p, nf, 0, g.my, (long long)g.mx * g.my,
-                         (long long)g.nz * g.mx * g.my, g.mx, (long long)g.ny * g.mx, bn)))
+                         (long long)g.nz * g.mx * g.my, g.mx, (long long)g.ny * g.mx, bn, 1)))
     return rc;
   const cx_t<T>* gin = (const cx_t<T>*)c.sc[2].p + g.lu * bn;
   if ((rc = run_x_pass<T>(c, 0, 0, ng, gin, nullptr, g.mx, (long long)g.ny * g.mx, bn, nullptr, c.sc[0].p, 0, 0, 0,
