@@ -45,9 +45,9 @@ typedef struct sam_gpu_config {
   int rot_sav;        /* 1 for the tilted-box wave, i_prob = 4 (sam.f:176-185) */
   int i_les;          /* Chollet-Lesieur spectra (spectra.f:21) */
   int precision;      /* 64: FP64 drop-in; 48 (SAM_GPU_PREC_DD): the resident step
-                         in double-float pairs on the FP32 pipe (about 48
-                         significand bits; plain step only: no LES, forcing,
-                         planes); 32: FP32 bulk with FP64 reductions.  The
+                         to at least 48 significand bits (the FP64 kernels
+                         run it; plain step only: no LES, forcing, planes);
+                         32: FP32 bulk with FP64 reductions.  The
                          per-routine drop-ins always compute in FP64. */
   double xl, yl, zl;  /* box */
   double vis, pr;     /* viscosity, Prandtl number */

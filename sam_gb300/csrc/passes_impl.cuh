@@ -1,6 +1,6 @@
-// Kernel templates of the five HBM passes (included by the translation
-// units that instantiate them, one per working precision: passes.cu
-// (FP64, plus the precision-independent kernels) and passes_f32.cu).
+// Kernel templates of the five HBM passes (instantiated by passes_part.cu, a
+// translation unit per pass, precision and share of the compiled lengths, and
+// by passes_ens.cu).
 // The five HBM passes of one RK3 stage and the reference-layout variants of
 // each transform.  Every pass moves a tile of pencils from HBM into shared
 // memory, transforms it there (fft_engine.cuh) and writes it back transposed
@@ -44,7 +44,8 @@ constexpr int kBatch = 8;
 // threads) without spills; the compile-time Stockham transposes (lengths 32-512)
 // spilled 40-110 bytes at 64 and keep three CTAs (80 registers; 128^3 y
 // forward 10 % faster); the FP32 z_fwd epilogue spills below 128 and keeps
-// two (three measured slower); FP64 CTAs are bound by the FP64 pipe.
+// two (three measured slower).  FP64 lines are 64-bit integers, two registers
+// each: 128 registers (two CTAs) hold a radix-16 butterfly, 80 (three) spill.
 // The run-time-radix path (kFftGeneric, lengths without a compile-time
 // path) needs more registers: one x pass CTA per SM, two of the others.
 enum PassKind { kPassZInv, kPassYInv, kPassX, kPassYFwd, kPassZFwd };

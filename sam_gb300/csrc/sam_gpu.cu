@@ -364,8 +364,8 @@ static int x_tile(Ctx& c, int nin, int out_mode, int& yt, int& grp) {
   const int teams = lines_at_once(c.px, threads, c.sched[2]);
   // FP32 tiles leave room for three CTAs per SM (72 registers each; two
   // CTAs with 16-row tiles measured slower), FP64 tiles for two (up to 128
-  // registers each): the FP64 pipe needs the second CTA's warps to cover its
-  // dependency latency
+  // registers each): one CTA's barriers and loads pass under the other's
+  // integer butterflies
   const size_t budget = sizeof(T) == 4 ? kSmemMax / 3 - 1024 : kSmemMax / 2 - 1024;
   const size_t line = es * (size_t)line_ld(c.g.nx);
   const size_t rmin = line * (size_t)x_red_lines<T>(c);
@@ -785,7 +785,7 @@ static int init_ctx(const sam_gpu_config* cfg) {
   if (cfg->nx < 2 || cfg->nx % 2 || cfg->ny < 1 || cfg->nz < 1)
     return fail(SAM_GPU_EINVAL, "grid %d x %d x %d: Nx must be even and >= 2", cfg->nx, cfg->ny, cfg->nz);
   if (cfg->precision != 64 && cfg->precision != 32 && cfg->precision != kPrecDD)
-    return fail(SAM_GPU_EINVAL, "precision must be 64, 48 (double-float pairs) or 32");
+    return fail(SAM_GPU_EINVAL, "precision must be 64, 48 or 32");
   if (cfg->nrk_max < 1 || cfg->nrk_max > 3) return fail(SAM_GPU_EINVAL, "nrk_max must be 1, 2 or 3");
   Ctx* c = new Ctx();
   c->cfg = *cfg;
@@ -1359,7 +1359,7 @@ int sam_gpu_set_forcing(unsigned long long seed, double k_f, double sigma, doubl
   NEED_CTX();
   if (n_modes) *n_modes = 0;
   if (c.plain_only && k_f > 0.0 && sigma != 0.0)
-    return fail(SAM_GPU_EUNSUPPORTED, "set_forcing: the double-float form runs the plain step only");
+    return fail(SAM_GPU_EUNSUPPORTED, "set_forcing: the 48-bit form runs the plain step only");
   if (c.gexec) { cudaGraphExecDestroy(c.gexec); c.gexec = nullptr; }
   c.graph_stale = 1;
   if (k_f <= 0.0 || sigma == 0.0) {
@@ -1388,7 +1388,7 @@ static int mlp_ensure(Ctx& c);
 int sam_gpu_set_les(int model, double c_smag, double pr_t) {
   NEED_CTX();
   if (model != 0 && c.plain_only)
-    return fail(SAM_GPU_EUNSUPPORTED, "set_les: the double-float form runs the plain step only");
+    return fail(SAM_GPU_EUNSUPPORTED, "set_les: the 48-bit form runs the plain step only");
   if (model < 0 || model > 3)
     return fail(SAM_GPU_EINVAL, "set_les: model %d (0 off, 1 Smagorinsky, 2 dynamic, 3 learned)", model);
   if (!(pr_t > 0.0)) return fail(SAM_GPU_EINVAL, "set_les: turbulent Prandtl number must be > 0");
@@ -1660,7 +1660,7 @@ int sam_gpu_box_filter(int f, double* out) {
   const Grid& g = c.g;
   if (!out || f < 1 || g.nx % f || g.ny % f || g.nz % f)
     return fail(SAM_GPU_EINVAL, "box_filter: the grid must divide into blocks of %d", f);
-  if (c.plain_only) return fail(SAM_GPU_EUNSUPPORTED, "box_filter: not in the double-float form");
+  if (c.plain_only) return fail(SAM_GPU_EUNSUPPORTED, "box_filter: not in the 48-bit form");
   return c.cfg.precision == 32 ? box_filter_impl<float>(c, f, out) : box_filter_impl<double>(c, f, out);
 }
 
@@ -1704,7 +1704,7 @@ int sam_gpu_closure_inputs(unsigned short* feat, double* grads) {
   double dsq, dxi, dyi, dzi;
   grid_spacing(c, dxi, dyi, dzi, dsq);
   c.les_dsq = dsq;
-  if (c.plain_only) return fail(SAM_GPU_EUNSUPPORTED, "closure_inputs: not in the double-float form");
+  if (c.plain_only) return fail(SAM_GPU_EUNSUPPORTED, "closure_inputs: not in the 48-bit form");
   return c.cfg.precision == 32 ? closure_inputs_impl<float>(c, feat, grads)
                                : closure_inputs_impl<double>(c, feat, grads);
 }
@@ -2214,7 +2214,7 @@ int sam_gpu_planes(const int* k_xy, int n_xy, const int* j_xz, int n_xz, const i
     if (i_yz[m] < 1 || i_yz[m] > g.nx) return fail(SAM_GPU_EINVAL, "planes: i_yz(%d) = %d outside 1..%d", m + 1, i_yz[m], g.nx);
     sel.i_yz[m] = i_yz[m] - 1;
   }
-  if (c.plain_only) return fail(SAM_GPU_EUNSUPPORTED, "planes: not in the double-float form");
+  if (c.plain_only) return fail(SAM_GPU_EUNSUPPORTED, "planes: not in the 48-bit form");
   const int rc = c.cfg.precision == 32 ? planes_impl<float>(c, sel, xy, xz, yz, mean)
                                        : planes_impl<double>(c, sel, xy, xz, yz, mean);
   if (rc) return rc;
