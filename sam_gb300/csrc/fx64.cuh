@@ -372,9 +372,15 @@ __device__ __forceinline__ double fx_to_alu(long long v, int ex) {
   const uint32_t hi = (uint32_t)(q >> 32) + (uint32_t)(1023 + 63 - 1 - lz + ex) * (1u << 20);
   return m ? __hiloint2double((int)(hi | ((uint32_t)(s >> 32) & 0x80000000u)), (int)(uint32_t)q) : 0.0;
 }
-template <bool ALU = false> __device__ __forceinline__ double2 fx_out(fxc v, FxScale sc) {
+// The parts' conversions: both on the FP64 pipe where the integer pipes are the
+// bound (the transposes: 2-8 % slower otherwise), or, where a phase of the
+// kernel does little else, one on each (x pass stores at 128^3 0.232 -> 0.220 ms,
+// both on the integer pipe 0.222; at 256^3 1.074 -> 1.037, with a closure 3.08 ->
+// 2.85, both on the integer pipe 3.09; z forward 0.863 -> 0.856).
+enum FxConv { kFxOnFp64, kFxOnBoth };
+template <FxConv CONV = kFxOnFp64> __device__ __forceinline__ double2 fx_out(fxc v, FxScale sc) {
   if (sc.kind == kFxPlain) {
-    if (ALU) return make_double2(fx_to_alu(v.x, sc.ex), fx_to_alu(v.y, sc.ex));
+    if (CONV == kFxOnBoth) return make_double2(fx_to(v.x, sc.ex), fx_to_alu(v.y, sc.ex));
     return make_double2(fx_to(v.x, sc.ex), fx_to(v.y, sc.ex));
   }
   if (sc.kind == kFxNaN) return make_double2(__hiloint2double(0x7ff80000, 0), __hiloint2double(0x7ff80000, 0));

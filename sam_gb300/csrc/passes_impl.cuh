@@ -1002,8 +1002,8 @@ __device__ __forceinline__ void x_pass_body(const XPassArgs<T>& a, const FftPlan
                 // the split in integers; 1/(2 Nx Ny) in the exponent where it
                 // is a power of two
                 const fxc i1 = *reinterpret_cast<const fxc*>(&z1), i2 = *reinterpret_cast<const fxc*>(&z2);
-                ve = fx_out(fxc{i1.x + i2.x, i1.y - i2.y}, sc);
-                vo = fx_out(fxc{i1.y + i2.y, i2.x - i1.x}, sc);
+                ve = fx_out<kFxOnBoth>(fxc{i1.x + i2.x, i1.y - i2.y}, sc);
+                vo = fx_out<kFxOnBoth>(fxc{i1.y + i2.y, i2.x - i1.x}, sc);
                 if (!fn_pow2) {
                   ve.x *= fn; ve.y *= fn;
                   vo.x *= fn; vo.y *= fn;
@@ -1292,9 +1292,9 @@ __global__ void __launch_bounds__(kXf256Threads, 3) k_x_pass_f256(const __grid_c
 // are formed, and a product's own gradient line is its team's scratch; the
 // twiddles then stay in memory (L1): 26 lines of a 4-row tile fit an SM twice
 // only without them, and 18 teams take its 18 product lines in one round (16
-// teams 3.28 ms, 2-row tiles with 3 or 4 CTAs per SM 3.53 and 3.61).  The
+// teams 4 % slower, 2-row tiles with 3 or 4 CTAs per SM 12 and 14 %).  The
 // general kernel ran two-row tiles (256^3, dynamic closure, stage 2: 4.30 ->
-// 3.15 ms).  Neither pipe is the bound (FP64 43 %, ALU 39 %): two CTAs whose
+// 2.85 ms).  Neither pipe is the bound (FP64 43 %, ALU 39 %): two CTAs whose
 // phases use one or the other overlap in part.
 template <bool LES>
 __global__ void __launch_bounds__(x_fx256_threads(LES), 2) k_x_pass_fx256(const __grid_constant__ XPassArgs<double> a) {
@@ -1384,7 +1384,7 @@ __global__ void __launch_bounds__(x_fx256_threads(LES), 2) k_x_pass_fx256(const 
     __syncwarp(tmask);
     if (LES && L >= nfac) {
 #pragma unroll
-      for (int s = 0; s < 16; ++s) reinterpret_cast<double2*>(line)[k + 17 * s] = fx_out<true>(v[s], sc);
+      for (int s = 0; s < 16; ++s) reinterpret_cast<double2*>(line)[k + 17 * s] = fx_out(v[s], sc);
       continue;
     }
 #pragma unroll
@@ -1485,8 +1485,8 @@ __global__ void __launch_bounds__(x_fx256_threads(LES), 2) k_x_pass_fx256(const 
       const fxc z2{__shfl_sync(tmask, snd.x, partner), __shfl_sync(tmask, snd.y, partner)};
       const fxc z1 = v[j];
       if (k + 16 * j <= kmx && one) {
-        double2 ve = fx_out(fxc{z1.x + z2.x, z1.y - z2.y}, sc);
-        double2 vo = fx_out(fxc{z1.y + z2.y, z2.x - z1.x}, sc);
+        double2 ve = fx_out<kFxOnBoth>(fxc{z1.x + z2.x, z1.y - z2.y}, sc);
+        double2 vo = fx_out<kFxOnBoth>(fxc{z1.y + z2.y, z2.x - z1.x}, sc);
         if (!pow2) {
           ve.x *= a.fn; ve.y *= a.fn;
           vo.x *= a.fn; vo.y *= a.fn;
@@ -1861,8 +1861,8 @@ __device__ __forceinline__ void z_fwd_body(const ZFwdArgs<T>& a, const FftPlan* 
       const auto val = [&](int f, T& re, T& im) {
         if constexpr (FX) {
           if (ints) {
-            // (this loop is bound by the FP64 pipe: convert on the other one)
-            const C v = fx_out<true>(*reinterpret_cast<const fxc*>(ln + f * nl * ld), s_sc[f * nl + t]);
+            // (this loop is bound by the FP64 pipe)
+            const C v = fx_out<kFxOnBoth>(*reinterpret_cast<const fxc*>(ln + f * nl * ld), s_sc[f * nl + t]);
             re = v.x;
             im = v.y;
             return;
