@@ -929,6 +929,107 @@ __device__ __forceinline__ void x_pass_body(const XPassArgs<T>& a, const FftPlan
   }
   const T fn = a.fn;  // 1/(Nx Ny) (xy_trans_f.f:20) and the 1/2 of the split
   const bool fn_pow2 = is_pow2_inv(nx) && is_pow2_inv(ny);
+  // The split of two real transforms at one kx <= kx_max (rows y0+2c and
+  // y0+2c+1), scaled and stored to C(m, z, kx, y) at o; sc is the line's scale
+  // with the power of two of 1/(2 Nx Ny) where it is one (product lines in
+  // fixed point).
+  const auto store_mode = [&](const C* ln, int kx, FxScale sc, C* o, bool two, bool one) {
+    const C z1 = ln[sidx(kx)];
+    const C z2 = ln[sidx(kx == 0 ? 0 : nx - kx)];
+    C ve, vo;
+    bool done = false;
+    if constexpr (FX) {
+      if (a.out_mode == 2) {
+        // the split in integers; 1/(2 Nx Ny) in the exponent where it
+        // is a power of two
+        const fxc i1 = *reinterpret_cast<const fxc*>(&z1), i2 = *reinterpret_cast<const fxc*>(&z2);
+        ve = fx_out<kFxOnBoth>(fxc{i1.x + i2.x, i1.y - i2.y}, sc);
+        vo = fx_out<kFxOnBoth>(fxc{i1.y + i2.y, i2.x - i1.x}, sc);
+        if (!fn_pow2) {
+          ve.x *= fn; ve.y *= fn;
+          vo.x *= fn; vo.y *= fn;
+        }
+        done = true;
+      }
+    }
+    if (!done) {
+      ve = mk<C>((z1.x + z2.x) * fn, (z1.y - z2.y) * fn);
+      vo = mk<C>((z1.y + z2.y) * fn, (z2.x - z1.x) * fn);
+    }
+    if (two) {
+      if ((reinterpret_cast<uintptr_t>(o) & (2 * sizeof(C) - 1)) == 0) {
+        store_pair(o, ve, vo);
+      } else {  // odd Ny: the pair straddles a vector boundary
+        o[0] = ve;
+        o[1] = vo;
+      }
+    } else if (one) {
+      o[0] = ve;
+    }
+  };
+  const auto out_scale = [&](FxScale sc) {
+    if (fn_pow2) sc.ex -= 1 + (31 - __clz(nx)) + (31 - __clz(ny));
+    return sc;
+  };
+  // product line q = m * Y/2 + c (rhs.f:46-60): its factors' lines, and the line
+  // of its subgrid term
+  const auto lines_of = [&](int q, int& fa, int& fb) {
+    const int m = (int)fdiv(q, a.fd_yp), c = q - m * yp;
+    product_pair(m, fa, fb);
+    fa = fa * yp + c;
+    fb = fb * yp + c;
+    return (a.g.lu + m) * yp + c;
+  };
+  const auto product_values = [&](int q) {
+    int fa, fb;
+    const int fg = lines_of(q, fa, fb);
+    return ProductLoad<C>{s_in + fa * ld, s_in + fb * ld, a.les ? s_in + fg * ld : nullptr};
+  };
+  const auto product_ints = [&](int q) {
+    int fa, fb;
+    const int fg = lines_of(q, fa, fb);
+    return FxProductLoad{reinterpret_cast<const FxSplit2*>(s_in + fa * ld),
+                         reinterpret_cast<const FxSplit2*>(s_in + fb * ld),
+                         a.les ? reinterpret_cast<const double2*>(s_in + fg * ld) : nullptr,
+                         fx_product(s_line[fa], s_line[fb], a.les ? s_line + fg : nullptr)};
+  };
+  // FP64 lines of a compiled length whose team is (part of) a warp: the team
+  // takes a product line from its factors to HBM, in a scratch line of its own
+  // and without a barrier of the CTA, so that the integer butterflies of some
+  // warps pass under the conversions and stores of others (8-row tiles, stage 2:
+  // 128^3 0.220 -> 0.180 ms, 64^3 0.033 -> 0.030, 120 x 135 x 162 0.366 ->
+  // 0.329).  In FP32 a team's stores fill half sectors (128^3 0.049 -> 0.056):
+  // its lines go through the rounds below.
+  if constexpr (FX && ct_length(PATH)) {
+    constexpr int TW = ct_plan(PATH).tw;
+    if constexpr (TW <= 32) {
+      if (ints) {
+        constexpr int G = 32 / TW;
+        const int lane = threadIdx.x & 31, sub = lane / TW, tl = lane - sub * TW;
+        const int team = (int)(threadIdx.x >> 5) * G + sub;
+        const int slots = min(ct_teams(TW, blockDim.x), a.group), total = a.g.lr * yp;
+        const int rounds = (total + slots - 1) / slots;
+        for (int r = 0; r < rounds; ++r) {
+          const int q = r * slots + team;
+          const bool active = sub < G && team < slots && q < total;
+          const int qc = active ? q : 0, slot = active ? team : 0;
+          C* line = s_pr + slot * ld;
+          FxScale sc;
+          fft_ct_stages<-1, PATH, 0>(line, s_tw, tl, active, product_ints(qc), FxOutInt{line, s_psc + slot}, sc);
+          __syncwarp();
+          if (active) {
+            const int m = (int)fdiv(q, a.fd_yp), c = q - m * yp;
+            C* o = a.out + (long long)z * a.out_z + y0 + (long long)m * a.out_n + (long long)tl * a.out_kx + 2 * c;
+            const bool two = 2 * c + 1 < yv, one = 2 * c < yv;
+            sc = out_scale(s_psc[slot]);
+            for (int kx = tl; kx < mx; kx += TW, o += (long long)TW * a.out_kx) store_mode(line, kx, sc, o, two, one);
+          }
+          __syncwarp();
+        }
+        return;
+      }
+    }
+  }
   // output line q = m * Y/2 + c: pair c of output field m.  out_mode 1
   // transforms the input lines in place, all at once; out_mode 2 forms the
   // products `group` lines at a time (group >= 1 by construction)
@@ -939,30 +1040,12 @@ __device__ __forceinline__ void x_pass_body(const XPassArgs<T>& a, const FftPlan
     // out_mode 2 (rhs.f:46-60): the products of the physical lines, formed
     // while the first FFT stage loads them, straight into the product lines
     C* lines = a.out_mode == 1 ? s_in : s_pr;
-    const auto lines_of = [&](int L, int& fa, int& fb) {
-      const int q = l0 + L;
-      const int m = (int)fdiv(q, a.fd_yp), c = q - m * yp;
-      product_pair(m, fa, fb);
-      fa = fa * yp + c;
-      fb = fb * yp + c;
-      return (a.g.lu + m) * yp + c;  // the line of the product's subgrid term
-    };
     const auto from_values = [&](int L) {
-      if (a.out_mode == 1) return ProductLoad<C>{lines + L * ld, nullptr, nullptr};
-      int fa, fb;
-      const int fg = lines_of(L, fa, fb);
-      return ProductLoad<C>{s_in + fa * ld, s_in + fb * ld, a.les ? s_in + fg * ld : nullptr};
+      return a.out_mode == 1 ? ProductLoad<C>{lines + L * ld, nullptr, nullptr} : product_values(l0 + L);
     };
     if constexpr (FX) {
       if (ints) {
-        const auto from_ints = [&](int L) {
-          int fa, fb;
-          const int fg = lines_of(L, fa, fb);
-          return FxProductLoad{reinterpret_cast<const FxSplit2*>(s_in + fa * ld),
-                               reinterpret_cast<const FxSplit2*>(s_in + fb * ld), a.les ? s_in + fg * ld : nullptr,
-                               fx_product(s_line[fa], s_line[fb], a.les ? s_line + fg : nullptr)};
-        };
-        fft_lines_from<-1, PATH>(lines, ld, gl, s_tw, pl, from_ints, [&](int L) { return FxOutInt{lines + L * ld, s_psc + L}; });
+        fft_lines_from<-1, PATH>(lines, ld, gl, s_tw, pl, [&](int L) { return product_ints(l0 + L); }, [&](int L) { return FxOutInt{lines + L * ld, s_psc + L}; });
       } else {
         fft_lines_from<-1, PATH>(lines, ld, gl, s_tw, pl, from_values);
       }
@@ -989,42 +1072,10 @@ __device__ __forceinline__ void x_pass_body(const XPassArgs<T>& a, const FftPlan
           FxScale sc{};
           if constexpr (FX)
             if (a.out_mode == 2) {
-              sc = s_psc[L];
-              if (fn_pow2) sc.ex -= 1 + (31 - __clz(nx)) + (31 - __clz(ny));
+              sc = out_scale(s_psc[L]);
             }
           for (int kx = lane; kx < mx; kx += lanes, o += ostep) {
-            const C z1 = ln[sidx(kx)];
-            const C z2 = ln[sidx(kx == 0 ? 0 : nx - kx)];
-            C ve, vo;
-            bool done = false;
-            if constexpr (FX) {
-              if (a.out_mode == 2) {
-                // the split in integers; 1/(2 Nx Ny) in the exponent where it
-                // is a power of two
-                const fxc i1 = *reinterpret_cast<const fxc*>(&z1), i2 = *reinterpret_cast<const fxc*>(&z2);
-                ve = fx_out<kFxOnBoth>(fxc{i1.x + i2.x, i1.y - i2.y}, sc);
-                vo = fx_out<kFxOnBoth>(fxc{i1.y + i2.y, i2.x - i1.x}, sc);
-                if (!fn_pow2) {
-                  ve.x *= fn; ve.y *= fn;
-                  vo.x *= fn; vo.y *= fn;
-                }
-                done = true;
-              }
-            }
-            if (!done) {
-              ve = mk<C>((z1.x + z2.x) * fn, (z1.y - z2.y) * fn);
-              vo = mk<C>((z1.y + z2.y) * fn, (z2.x - z1.x) * fn);
-            }
-            if (two) {
-              if ((reinterpret_cast<uintptr_t>(o) & (2 * sizeof(C) - 1)) == 0) {
-                store_pair(o, ve, vo);
-              } else {  // odd Ny: the pair straddles a vector boundary
-                o[0] = ve;
-                o[1] = vo;
-              }
-            } else if (one) {
-              o[0] = ve;
-            }
+            store_mode(ln, kx, sc, o, two, one);
           }
         }
     }
