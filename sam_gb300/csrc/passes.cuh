@@ -136,6 +136,14 @@ template <typename T> inline bool x_fused(const XPassArgs<T>& a) {
 // rows of a fused tile with a closure: 26 lines, three (FP32) or two CTAs per SM
 constexpr int kXFusedLesRows = 4;
 
+// The tables of a stage's integrating factors (FP64 resident step): 5 Mz
+// doubles per kz, then, aligned, four per row (kx, ky).
+__host__ __device__ inline size_t z_row_off(const Grid& g) { return (5 * (size_t)g.mz + 3) / 4 * 4; }
+template <typename D> __host__ __device__ inline auto z_row_tab(D* kz_tab, const Grid& g) {
+  using V = typename std::conditional<std::is_const<D>::value, const double4, double4>::type;
+  return reinterpret_cast<V*>(kz_tab + z_row_off(g));
+}
+
 template <typename T>
 struct YFwdArgs {
   Grid g;

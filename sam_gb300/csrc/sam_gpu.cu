@@ -178,7 +178,7 @@ struct Ctx {
   double* partials = nullptr;
   int partial_blocks = 0;
   double* pv = nullptr;  // vel_max's wave-space sums
-  double* kz_tab = nullptr;  // FP64 form: kz wave numbers and integrating factors of the stage (5 Mz)
+  double* kz_tab = nullptr;  // FP64 form: kz wave numbers and integrating factors of the stage (z_row_tab)
   DevState* state = nullptr;
   Scratch sc[4];
   // tile choices
@@ -875,7 +875,7 @@ static int init_ctx(const sam_gpu_config* cfg) {
   const size_t pv_bytes = sizeof(double) * 4 * ((size_t)kParsevalBlocks + 1) + sizeof(int) * kVmaxInts;
   ok = ok && cudaMalloc(&c->pv, pv_bytes) == cudaSuccess;
   if (ok) cudaMemset(c->pv, 0, pv_bytes);
-  ok = ok && cudaMalloc(&c->kz_tab, sizeof(double) * 5 * (size_t)g.mz) == cudaSuccess;
+  ok = ok && cudaMalloc(&c->kz_tab, sizeof(double) * (z_row_off(g) + 4 * (size_t)g.mx * g.my)) == cudaSuccess;
   if (!ok) { free_ctx(c); g_ctx = nullptr; return fail(SAM_GPU_ECUDA, "device allocation failed"); }
   cudaMemset(c->U, 0, es * g.lu * nzmm);
   cudaMemset(c->R, 0, es * g.lu * nzmm);
