@@ -139,8 +139,11 @@ constexpr int kXFusedLesRows = 4;
 // The tables of a stage's integrating factors (FP64 resident step): 5 Mz
 // doubles per kz, then, aligned, four per row (kx, ky).
 __host__ __device__ inline size_t z_row_off(const Grid& g) { return (5 * (size_t)g.mz + 3) / 4 * 4; }
+struct __align__(16) RowFactors {
+  double ef[2], et[2];  // exp(-nu k^2 dt_fac) less one and itself, and with nu / Pr
+};
 template <typename D> __host__ __device__ inline auto z_row_tab(D* kz_tab, const Grid& g) {
-  using V = typename std::conditional<std::is_const<D>::value, const double4, double4>::type;
+  using V = typename std::conditional<std::is_const<D>::value, const RowFactors, RowFactors>::type;
   return reinterpret_cast<V*>(kz_tab + z_row_off(g));
 }
 

@@ -1583,13 +1583,13 @@ __device__ __forceinline__ void y_fwd_body(const YFwdArgs<T>& a, const FftPlan* 
     // 0.0266 at 64^3 instead of 0.0246)
     const double vis_f = a.kz_vis * (a.kz_gamma * a.kz_state->dt + a.kz_zeta * a.kz_state->dt);  // sam.f:293-295
     const double rkx = a.g.wave_x * (double)i;
-    double4* rows = z_row_tab(a.kz_tab, a.g) + (long long)i * my;
+    RowFactors* rows = z_row_tab(a.kz_tab, a.g) + (long long)i * my;
     for (int j = threadIdx.x; j < my; j += blockDim.x) {
       const double rky = a.g.wave_y * (double)kwave(j, a.g.ky, my), k_sq = rkx * rkx + rky * rky;
       const double xf = -vis_f * k_sq, xt = -(vis_f * a.kz_pr_inv) * k_sq;
       const double ef0 = expm1(xf), ef1 = exp(xf);
       const bool same = a.kz_pr_inv == 1.0;
-      rows[j] = make_double4(ef0, ef1, same ? ef0 : expm1(xt), same ? ef1 : exp(xt));
+      rows[j] = RowFactors{{ef0, ef1}, {same ? ef0 : expm1(xt), same ? ef1 : exp(xt)}};
     }
     for (int k = threadIdx.x; i == 0 && k < a.g.mz; k += blockDim.x) {
       const double rkz = a.g.wave_z * (double)kwave(k, a.g.kz, a.g.mz);
@@ -1897,11 +1897,11 @@ __device__ __forceinline__ void z_fwd_body(const ZFwdArgs<T>& a, const FftPlan* 
     r.k_sq = rkx * rkx + r.rky * r.rky;
     if constexpr (std::is_same<T, double>::value)
       if (a.kz_tab) {
-        const double4 e = z_row_tab(a.kz_tab, g)[(long long)i * my + j0 + t];
-        r.ef[0] = e.x;
-        r.ef[1] = e.y;
-        r.et[0] = e.z;
-        r.et[1] = e.w;
+        const RowFactors e = z_row_tab(a.kz_tab, g)[(long long)i * my + j0 + t];
+        r.ef[0] = e.ef[0];
+        r.ef[1] = e.ef[1];
+        r.et[0] = e.et[0];
+        r.et[1] = e.et[1];
       }
     s_row[t] = r;
   }

@@ -179,3 +179,24 @@ def test_damping_of_single_modes(gpu_lib, pr):
     ref = u[:m, :, 1:, 3] * np.exp(-x)
     assert (np.abs(got[:m, :, 1:, 3] - ref) <= (12 + 4 * x) * 2.0 ** -53 * np.abs(ref)).all()
     g.close()
+
+
+@pytest.mark.parametrize("nx, ny", [(16, 9), (64, 32), (90, 27), (128, 16), (250, 12)])
+@pytest.mark.parametrize("les", [0, 1])
+def test_product_lines_do_not_depend_on_the_tile(gpu_lib, nx, ny, les):
+    """A product line is formed, transformed and stored by one team whatever
+    the tile's rows and the scratch lines (fewer than the teams, or one for
+    each): the same bits, tiles cut by Ny and an odd last row included."""
+    ref = None
+    for rows, group in ((8, 9), (2, 1), (4, 2), (16, 9), (16, 1)):
+        g = SamGpu(nx=nx, ny=ny, nz=8, i_strat=1, vis=1e-3, dt0=0.01, buoy_fac_z=1.0, lapse=1.0, i_cfl=1, cfl0=0.5)
+        g.init_random(3)
+        if les:
+            g.set_les(1, c_smag=0.03, pr_t=0.7)
+        g.set_tiles(x_rows=rows, x_group=group)
+        g.step(2)
+        got = g.download(), np.array([g.stats()["dt"]])
+        ref = ref or got
+        for a, b in zip(got, ref):
+            assert np.array_equal(a, b), (rows, group)
+        g.close()
