@@ -527,7 +527,7 @@ def run_probe(args):
 
 
 def run_parity_curve(args):
-    """Error of the GPU forms (FP64, double-float, FP32 bulk) against the
+    """Error of the GPU forms (FP64, 48 bits, FP32 bulk) against the
     oracle versus step count on the 128^3 stratified decaying-turbulence
     configuration (N = 1, Pr = 1,
     nu = 1/800, k^4 exp(-2 (k/4)^2) start at rms 1 with theta at 0.1, CFL
@@ -604,7 +604,7 @@ def main():
     ap.add_argument("--impl", default="gb300", choices=["gb300", "reference"])
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-fp32", action="store_true")
-    ap.add_argument("--no-dd", action="store_true", help="skip the double-float form")
+    ap.add_argument("--no-dd", action="store_true", help="skip the 48-bit form")
     ap.add_argument("--no-les", action="store_true")
     ap.add_argument("--no-ensemble", action="store_true")
     ap.add_argument("--grid", type=int, default=256, help="N of the N^3 box (profiling of smaller cases)")
