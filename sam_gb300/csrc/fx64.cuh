@@ -429,8 +429,11 @@ __device__ __forceinline__ FxProduct fx_product(const FxLine& a, const FxLine& b
   p.sc.kind = (a.kind | b.kind | (g ? g->kind : 0)) & kFxNaN ? kFxNaN : (p.sc.ex < -960 || p.sc.ex > 940 ? kFxEdge : kFxPlain);
   return p;
 }
+// (with the low halves' product, up to 2^(62 - r) units: where a and b are the
+// same field it is a square, and without it every product came out low, the
+// mean of u u over 256 points by 0.5 x 2^-53 and over 1024 by 2.7 x 2^-53)
 __device__ __forceinline__ long long fx_mul_line(FxSplit a, FxSplit b, const FxProduct& p) {
-  const long long c = fx_mad(a.l, b.h, fx_mad(a.h, b.l, p.half));
+  const long long c = fx_mad(a.l, b.h, fx_mad(a.h, b.l, p.half + fx_low(a, b)));
   const long long A = fx_mad(a.h, b.h, c >> 32);
   const uint32_t lo = __funnelshift_l((uint32_t)c, (uint32_t)A, p.s);
   const uint32_t hi = __funnelshift_l((uint32_t)A, (uint32_t)(A >> 32), p.s);
