@@ -486,7 +486,7 @@ __device__ __forceinline__ void fx_stage(double2* line, const fxw* __restrict__ 
         for (int q = 0; q < P; ++q) v[i][q] = load(b + s.m * q);
       }
     }
-    sc = fx_begin<MAXB * P, Out::kNorm>(&v[0][0], &a[0][0], TW, Out::kNorm ? sqrtf((float)n) : 0.f);
+    sc = fx_begin<MAXB * P, Out::kNorm, true>(&v[0][0], &a[0][0], TW, Out::kNorm ? sqrtf((float)n) : 0.f);
   } else {
     const fxc* fl = reinterpret_cast<const fxc*>(line);
 #pragma unroll
