@@ -471,40 +471,5 @@ __device__ __forceinline__ void fx_line_bound(const double2* line, FxLine* info,
   const int g = (__float_as_int(l1 * 1.0001f) >> 23) - 126;
   if (lane == 0) *info = FxLine{E ? E - 1023 + g : -1100, E == 0x7ff ? kFxNaN : kFxPlain, 0.f};
 }
-// Physical values of a line of n points (elements sidx(0) .. sidx(n - 1)) to
-// split integers below 2^62, by one warp.
-__device__ __forceinline__ void fx_line_in_place(double2* line, FxLine* info, int n) {
-  const int lane = threadIdx.x & 31;
-  uint32_t hm = 0;
-  for (int x = lane; x < n; x += 32) hm = max(hm, fx_max_hi<1>(line + sidx(x)));
-  hm = __reduce_max_sync(0xffffffffu, hm);
-  const bool lift = hm < ((uint32_t)kFxTiny << 20) && hm > 0;
-  const double f = lift ? __hiloint2double((1023 + kFxLift) << 20, 0) : 1.0;
-  if (lift) {
-    hm = 0;
-    for (int x = lane; x < n; x += 32) {
-      double2 v = line[sidx(x)];
-      v.x *= f;
-      v.y *= f;
-      line[sidx(x)] = v;
-      hm = max(hm, fx_max_hi<1>(&v));
-    }
-    hm = __reduce_max_sync(0xffffffffu, hm);
-  }
-  const int E = (int)(hm >> 20);
-  float l2 = 0.f;
-  for (int x = lane; x < n; x += 32) l2 += fx_l2<1>(line + sidx(x), E);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) l2 += __shfl_xor_sync(0xffffffffu, l2, o);
-  l2 = sqrtf(l2);
-  const int g = E ? (__float_as_int(l2 * 1.0001f) >> 23) - 126 : 128;
-  for (int x = lane; x < n; x += 32) {
-    const double2 v = line[sidx(x)];
-    reinterpret_cast<FxSplit2*>(line)[sidx(x)] = fx_split2(fxc{fx_from(v.x, E + g), fx_from(v.y, E + g)});
-  }
-  if (lane == 0)
-    *info = FxLine{E - 1023 - 62 + g - (lift ? kFxLift : 0), E == 0x7ff ? kFxNaN : kFxPlain,
-                   l2 * __int_as_float(max(127 - g, 0) << 23)};
-}
 
 }  // namespace samgpu

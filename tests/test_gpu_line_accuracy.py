@@ -113,3 +113,22 @@ def test_rhs_of_long_lines_against_fp64(gpu_lib, n, axis):
         fp64 = rhs(g, [inverse(g, u[:g.nz_min, ..., f]) for f in range(3)], np.float64)
         assert distance(got, ref) <= 1.25 * distance(fp64, ref), slope
     g.close()
+
+
+@pytest.mark.parametrize("n", [12, 64, 250, 256, 320, 512])
+def test_rhs_of_given_fields_keeps_small_products(gpu_lib, n):
+    """sam_gpu_rhs on physical arrays where u is 1e-18 of itself wherever v is
+    not zero: r_1 at kx = 0 is -i ky times the mean of u v over x, a product of
+    normal numbers that FP64 keeps to its last bits beside u u of order one.
+    Bar as above."""
+    g = SamGpu(nx=n, ny=10, nz=10)
+    rng = np.random.default_rng(n)
+    uu = g.phys(g.lr)
+    uu[..., :2] = rng.standard_normal(uu.shape[:3] + (2,))
+    uu[: n // 2, ..., 1] = 0.0
+    uu[n // 2:, ..., 0] *= 1e-18
+    p = [uu[..., f].transpose(2, 1, 0).copy() for f in range(3)]
+    got = g.rhs(uu)[:g.nz_min, 1:, 0, 0]
+    ref, fp64 = (rhs(g, p, real)[0][:, 1:, 0] for real in (LD, np.float64))
+    assert distance([got], [ref]) <= 1.25 * distance([fp64], [ref])
+    g.close()
