@@ -82,6 +82,14 @@ inline int smem_optin() {
   }
   return cache[dev];
 }
+// Opts a kernel into the largest dynamic shared memory the device allows: the
+// per-block opt-in limit less the kernel's static shared memory (a request for
+// all of it is refused and leaves the kernel at 48 KB).
+inline void allow_dynamic_smem(const void* fn, int optin) {
+  cudaFuncAttributes at;
+  if (cudaFuncGetAttributes(&at, fn) != cudaSuccess) return;
+  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)at.sharedSizeBytes);
+}
 
 // Records the message returned by sam_gpu_error_string(); returns code.
 int set_error(int code, const char* msg);

@@ -361,9 +361,8 @@ double diag_fp64_peak(cudaStream_t s) {
 }
 
 void diag_set_smem_limits() {
-  cudaFuncSetAttribute(k_deriv, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-  cudaFuncSetAttribute(k_spectra<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-  cudaFuncSetAttribute(k_spectra<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+  for (const void* fn : {(const void*)k_deriv, (const void*)k_spectra<double>, (const void*)k_spectra<float>})
+    allow_dynamic_smem(fn, smem_optin());
 }
 
 void diag_spectra(const DiagArgs& d, const void* u, const void* r, double* scratch, double* host_out, cudaStream_t s) {

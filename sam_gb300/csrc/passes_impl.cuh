@@ -2251,15 +2251,8 @@ void launch_z_fwd_part(const ZFwdArgs<T>& a, const FftPlan* pl, size_t smem, cud
   with_path<PART, PARTS>(a.g.nz, a.sched,
                          [&](auto p) { k_z_fwd<T, decltype(p)::value><<<grid, kThreads, smem, s>>>(a, pl); });
 }
-static inline void allow_dynamic_smem(const void* fn, int optin) {
-  cudaFuncAttributes at;
-  if (cudaFuncGetAttributes(&at, fn) != cudaSuccess) return;
-  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)at.sharedSizeBytes);
-}
-
 // Load the kernels a pass along length n runs and opt them into the largest
-// dynamic shared memory the device allows (the per-block opt-in limit less the
-// kernel's static shared memory).
+// dynamic shared memory the device allows.
 template <int PART, int PARTS, bool EVEN = false, typename F> void each_sched(int n, F f) {
   with_path<PART, PARTS, EVEN>(n, 0, f);
   if (n == 256) with_path<PART, PARTS, EVEN>(n, 1, f);
