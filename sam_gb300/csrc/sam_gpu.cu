@@ -369,7 +369,7 @@ static int x_tile(Ctx& c, int nin, int out_mode, int& yt, int& grp) {
   const size_t budget = sizeof(T) == 4 ? kSmemMax / 3 - 1024 : kSmemMax / 2 - 1024;
   const size_t line = es * (size_t)line_ld(c.g.nx);
   const size_t rmin = line * (size_t)x_red_lines<T>(c);
-  for (yt = c.yt_x;; yt /= 2) {
+  for (yt = c.yt_x;; yt = std::max(yt / 4 * 2, 2)) {  // (row pairs: even)
     const int yp = yt / 2;
     const size_t base = tile_smem(c.px, nin * yp, es, c.sched[2]) + x_extra<T>(out_mode, nin * yp, 0);
     if (out_mode != 2) {
