@@ -401,7 +401,11 @@ void diag_deriv(const Grid& g, int dir, const FftPlan* dplan, const fxw* tw, con
   const int ld = line_stride(n);
   const int nrows = dir == 0 ? g.ny : g.nx;
   const int pairs = (nrows + 1) / 2;
+  // pairs a CTA: as few as give every SM one (a plane is small, and its FP64
+  // conversions and products are bound by the FP64 pipe of the SMs that do
+  // them: with the copies, 32 x 32 45 -> 38 us, 192 x 192 74 -> 63)
   int per = 8;
+  while (per > 1 && per * sm_count() > pairs) per /= 2;
   while (per > 1 && sizeof(double2) * ((size_t)hplan.tw_total + (size_t)per * ld) > 200 * 1024) per /= 2;
   const size_t sm = sizeof(double2) * ((size_t)hplan.tw_total + (size_t)per * ld) + 16;
   const int grid = (pairs + per - 1) / per;
