@@ -159,8 +159,8 @@ struct YFwdArgs {
   int nvar, tz, ld;
   long long in_kx, in_z, in_n;
   long long out_ky, out_kx, out_n;
-  // FP64 form, resident stage: the first CTA also writes the z-forward pass's
-  // kz table of this stage (ZFwdArgs::kz_tab), dt read on the device
+  // FP64 form, resident stage: Mx more CTAs write the z-forward pass's tables of
+  // this stage (ZFwdArgs::kz_tab, RowFactors), dt read on the device
   double* kz_tab;
   const DevState* kz_state;
   double kz_gamma, kz_zeta, kz_vis, kz_pr_inv;

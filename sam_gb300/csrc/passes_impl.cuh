@@ -1578,33 +1578,6 @@ __device__ __forceinline__ void y_fwd_body(const YFwdArgs<T>& a, const FftPlan* 
   load_twiddles<T>(s_tw, a.tw, tw_load<PATH>(pl));
   const C* src = a.in + (long long)m * a.in_n + (long long)i * a.in_kx + (long long)z0 * a.in_z;
   __syncthreads();
-  if (a.kz_tab && m == 0 && zt == 0) {
-    // the z-forward pass of the same stage, next on the stream, reads
-    // rkz(k), exp(-nu rkz^2 dt_fac) less one and itself, and the same with
-    // nu / Pr, and the four exponentials of each (kx, ky): per kz and per row
-    // here instead of per mode there (the rows' in z_fwd's own CTAs, by one
-    // warp while the others waited: z_fwd 0.861 ms at 256^3 instead of 0.834,
-    // 0.0266 at 64^3 instead of 0.0246)
-    const double vis_f = a.kz_vis * (a.kz_gamma * a.kz_state->dt + a.kz_zeta * a.kz_state->dt);  // sam.f:293-295
-    const double rkx = a.g.wave_x * (double)i;
-    RowFactors* rows = z_row_tab(a.kz_tab, a.g) + (long long)i * my;
-    for (int j = threadIdx.x; j < my; j += blockDim.x) {
-      const double rky = a.g.wave_y * (double)kwave(j, a.g.ky, my), k_sq = rkx * rkx + rky * rky;
-      const double xf = -vis_f * k_sq, xt = -(vis_f * a.kz_pr_inv) * k_sq;
-      const double ef0 = expm1(xf), ef1 = exp(xf);
-      const bool same = a.kz_pr_inv == 1.0;
-      rows[j] = RowFactors{{ef0, ef1}, {same ? ef0 : expm1(xt), same ? ef1 : exp(xt)}};
-    }
-    for (int k = threadIdx.x; i == 0 && k < a.g.mz; k += blockDim.x) {
-      const double rkz = a.g.wave_z * (double)kwave(k, a.g.kz, a.g.mz);
-      a.kz_tab[k] = rkz;
-      const double xf = -vis_f * (rkz * rkz), xt = -(vis_f * a.kz_pr_inv) * (rkz * rkz);
-      a.kz_tab[a.g.mz + k] = expm1(xf);
-      a.kz_tab[2 * a.g.mz + k] = exp(xf);
-      a.kz_tab[3 * a.g.mz + k] = expm1(xt);
-      a.kz_tab[4 * a.g.mz + k] = exp(xt);
-    }
-  }
   // the first stage reads its inputs straight from the rows of C (no
   // shared-memory staging); the rows are contiguous in y
   const auto rows = [&](int L) { return RowLoad<C, COH>{src + (long long)L * a.in_z}; };
@@ -1617,10 +1590,51 @@ __device__ __forceinline__ void y_fwd_body(const YFwdArgs<T>& a, const FftPlan* 
   C* dst = a.out + (long long)m * a.out_n + (long long)i * a.out_kx + z0;
   store_tile_rows(dst, a.out_ky, s_ln, ld, a.tz, nl, my, [&](int j) { return kpos(j, km, my, ny); });
 }
+// The tables of a stage's integrating factors, by Mx CTAs ahead of a
+// y-forward pass's own (ZFwdArgs::kz_tab, RowFactors), for the z-forward pass
+// next on the stream: rkz(k), exp(-nu rkz^2 dt_fac) less one and itself, and
+// the same with nu / Pr, and the four exponentials of each (kx, ky): per kz and
+// per row here instead of per mode there (the rows' in z_fwd's own CTAs, by one
+// warp while the others waited: z_fwd 0.861 ms at 256^3 instead of 0.834, 0.0266
+// at 64^3 instead of 0.0246).  In CTAs of their own, because the exponentials
+// take a CTA that has lines to transform as well some 4 us longer, a third of
+// the pass on a small grid.
+template <typename T> __device__ __forceinline__ void stage_factors(const YFwdArgs<T>& a, int i) {
+  const int my = a.g.my, mz = a.g.mz;
+  const double vis_f = a.kz_vis * (a.kz_gamma * a.kz_state->dt + a.kz_zeta * a.kz_state->dt);  // sam.f:293-295
+  const double rkx = a.g.wave_x * (double)i;
+  RowFactors* rows = z_row_tab(a.kz_tab, a.g) + (long long)i * my;
+  for (int j = threadIdx.x; j < my; j += blockDim.x) {
+    const double rky = a.g.wave_y * (double)kwave(j, a.g.ky, my), k_sq = rkx * rkx + rky * rky;
+    const double xf = -vis_f * k_sq, xt = -(vis_f * a.kz_pr_inv) * k_sq;
+    const double ef0 = expm1(xf), ef1 = exp(xf);
+    const bool same = a.kz_pr_inv == 1.0;
+    rows[j] = RowFactors{{ef0, ef1}, {same ? ef0 : expm1(xt), same ? ef1 : exp(xt)}};
+  }
+  for (int k = threadIdx.x; i == 0 && k < mz; k += blockDim.x) {
+    const double rkz = a.g.wave_z * (double)kwave(k, a.g.kz, mz);
+    a.kz_tab[k] = rkz;
+    const double xf = -vis_f * (rkz * rkz), xt = -(vis_f * a.kz_pr_inv) * (rkz * rkz);
+    a.kz_tab[mz + k] = expm1(xf);
+    a.kz_tab[2 * mz + k] = exp(xf);
+    a.kz_tab[3 * mz + k] = expm1(xt);
+    a.kz_tab[4 * mz + k] = exp(xt);
+  }
+}
 template <typename T, int PATH>
 __global__ void __launch_bounds__(kThreads, MinBlocks<T, kPassYFwd, PATH>::value)
     k_y_fwd(const __grid_constant__ YFwdArgs<T> a, const FftPlan* __restrict__ gpl) {
-  y_fwd_body<T, PATH>(a, gpl, blockIdx.x);
+  int first = 0;
+  if constexpr (std::is_same<T, double>::value) {
+    if (a.kz_tab) {
+      first = a.g.mx;
+      if ((int)blockIdx.x < first) {
+        stage_factors(a, blockIdx.x);
+        return;
+      }
+    }
+  }
+  y_fwd_body<T, PATH>(a, gpl, blockIdx.x - first);
 }
 
 __device__ __forceinline__ double wexp(double x) { return exp(x); }
@@ -2241,7 +2255,7 @@ void launch_x_pass_part(const XPassArgs<T>& a, const FftPlan* pl, size_t smem, c
 }
 template <typename T, int PART, int PARTS>
 void launch_y_fwd_part(const YFwdArgs<T>& a, const FftPlan* pl, size_t smem, cudaStream_t s) {
-  const int grid = a.nvar * a.g.mx * ((a.g.nz + a.tz - 1) / a.tz);
+  const int grid = a.nvar * a.g.mx * ((a.g.nz + a.tz - 1) / a.tz) + (a.kz_tab ? a.g.mx : 0);
   with_path<PART, PARTS>(a.g.ny, a.sched,
                          [&](auto p) { k_y_fwd<T, decltype(p)::value><<<grid, kThreads, smem, s>>>(a, pl); });
 }
