@@ -216,7 +216,7 @@ struct ZFwdArgs {
 __host__ __device__ constexpr int path_part(int n, int parts) {
   if (!ct_length(n)) return 0;
   int i = 0;
-  for (int m = 16; m < n; ++m) i += ct_length(m);
+  for (int m = 8; m < n; ++m) i += ct_length(m);
   return i % parts;
 }
 template <typename T>

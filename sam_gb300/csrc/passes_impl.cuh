@@ -2187,12 +2187,12 @@ __device__ __forceinline__ void vel_max_finish_body(const double* __restrict__ p
 // The lengths with a compile-time path (ct_length), by their place in the list.
 constexpr int ct_count() {
   int c = 0;
-  for (int n = 16; n <= 512; ++n) c += ct_length(n);
+  for (int n = 8; n <= 512; ++n) c += ct_length(n);
   return c;
 }
 constexpr int kCtCount = ct_count();
 constexpr int ct_nth(int i) {
-  for (int n = 16; n <= 512; ++n)
+  for (int n = 8; n <= 512; ++n)
     if (ct_length(n) && i-- == 0) return n;
   return 0;
 }
