@@ -77,11 +77,12 @@ template <int SIGN, typename C> __device__ __forceinline__ C cmul_si(C a) {
 
 // Code paths of the line transforms: kFftAny picks at run time (the plan's
 // length); kFft256 compiles only the 16 x 16 register path (n = 256) and
-// kFftGeneric only the Stockham stages with the radix chosen at run time;
+// kFftGeneric only the Stockham stages with the radix chosen at run time
+// (kFftLong the same under another register budget);
 // PATH = n (ct_length) compiles the Stockham stages of that length with their
 // radices and every stride fixed at compile time (ct_plan).  A kernel built for one length
 // thus carries no registers for another path.
-constexpr int kFftAny = 0, kFft256 = 1, kFftGeneric = 2;
+constexpr int kFftAny = 0, kFft256 = 1, kFftGeneric = 2, kFftLong = 3;
 // whether lines are transformed in fixed point (fx64.cuh)
 template <typename C> inline constexpr bool kIsFx = std::is_same<C, double2>::value;
 

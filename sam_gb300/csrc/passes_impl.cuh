@@ -46,16 +46,26 @@ constexpr int kBatch = 8;
 // forward 10 % faster); the FP32 z_fwd epilogue spills below 128 and keeps
 // two (three measured slower).  FP64 lines are 64-bit integers, two registers
 // each: 128 registers (two CTAs) hold a radix-16 butterfly, 80 (three) spill.
-// The run-time-radix path (kFftGeneric, lengths without a compile-time
-// path) needs more registers: one x pass CTA per SM, two of the others.
+// The run-time-radix path (kFftGeneric, lengths without a compile-time path)
+// needs more registers: in FP32 one x pass CTA per SM, two of the others; in
+// FP64 see two_ctas_upto.
 enum PassKind { kPassZInv, kPassYInv, kPassX, kPassYFwd, kPassZFwd };
 template <typename T, int K, int PATH = kFft256> struct MinBlocks {
   static constexpr int value =
       PATH == kFftGeneric ? (K == kPassX ? 1 : 2) : (K == kPassZFwd ? 2 : (K == kPassX ? 3 : (PATH == kFft256 ? (K == kPassYInv ? 5 : 4) : 3)));
 };
 template <int K, int PATH> struct MinBlocks<double, K, PATH> {
-  static constexpr int value = PATH == kFftGeneric ? 1 : 2;
+  static constexpr int value = PATH == kFftLong ? 1 : 2;
 };
+// The longest lines of which two tiles share an SM (y and z inverse, y forward:
+// 16 lines; z forward: 9; the x pass cuts its tiles to that).  Up to there the
+// FP64 form's run-time path keeps to 128 registers, so that two CTAs do
+// (288^3, a step: 47.8 -> 38.3 ms, 384^3 101 -> 79; x pass of 1024 points 1.35
+// -> 1.08 ms); beyond, spilled values would cost y and z passes of 400 points
+// 13 % (kFftLong: all 255 registers).
+template <typename T, int K> constexpr int two_ctas_upto() {
+  return std::is_same<T, float>::value || K == kPassX ? 1024 : (K == kPassZFwd ? 640 : 384);
+}
 template <typename V, typename Get, typename Put>
 __device__ __forceinline__ void batched(int count, Get get, Put put) {
   for (int base = threadIdx.x; base < count; base += kBatch * blockDim.x) {
@@ -2206,9 +2216,9 @@ void with_ct_path(int n, F f, std::integer_sequence<int, I...>) {
   (one(std::integral_constant<int, I>()), ...);
 }
 // Calls f with the code path (an integral constant) that lines of length n
-// take; sched = 1 is the Stockham schedule of length 256.  Lengths of other
-// units are passed over (EVEN: odd ones too, Nx is even).
-template <int PART, int PARTS, bool EVEN = false, typename F> void with_path(int n, int sched, F f) {
+// take in pass K; sched = 1 is the Stockham schedule of length 256.  Lengths of
+// other units are passed over (in the x pass odd ones too, Nx is even).
+template <typename T, int K, int PART, int PARTS, typename F> void with_path(int n, int sched, F f) {
   if constexpr (path_part(256, PARTS) == PART) {
     if (n == 256) {
       if (sched == 1) f(std::integral_constant<int, 256>());
@@ -2216,20 +2226,25 @@ template <int PART, int PARTS, bool EVEN = false, typename F> void with_path(int
       return;
     }
   }
-  if (ct_length(n)) with_ct_path<PART, PARTS, EVEN>(n, f, std::make_integer_sequence<int, kCtCount>());
-  else if constexpr (PART == 0) f(std::integral_constant<int, kFftGeneric>());
+  if (ct_length(n)) {
+    with_ct_path<PART, PARTS, K == kPassX>(n, f, std::make_integer_sequence<int, kCtCount>());
+  } else if constexpr (PART == 0) {
+    constexpr int upto = two_ctas_upto<T, K>();
+    if (n <= upto) f(std::integral_constant<int, kFftGeneric>());
+    else if constexpr (upto < 1024) f(std::integral_constant<int, kFftLong>());
+  }
 }
 
 template <typename T, int PART, int PARTS>
 void launch_z_inv_part(const ZInvArgs<T>& a, const FftPlan* pl, size_t smem, cudaStream_t s) {
   const int grid = a.nvar * a.g.mx * ((a.g.my + a.ty - 1) / a.ty);
-  with_path<PART, PARTS>(a.g.nz, a.sched,
+  with_path<T, kPassZInv, PART, PARTS>(a.g.nz, a.sched,
                          [&](auto p) { k_z_inv<T, decltype(p)::value><<<grid, kThreads, smem, s>>>(a, pl); });
 }
 template <typename T, int PART, int PARTS>
 void launch_y_inv_part(const YInvArgs<T>& a, const FftPlan* pl, size_t smem, cudaStream_t s) {
   const int grid = a.nvar * a.g.nz * ((a.g.mx + a.tx - 1) / a.tx);
-  with_path<PART, PARTS>(a.g.ny, a.sched,
+  with_path<T, kPassYInv, PART, PARTS>(a.g.ny, a.sched,
                          [&](auto p) { k_y_inv<T, decltype(p)::value><<<grid, kThreads, smem, s>>>(a, pl); });
 }
 template <typename T, int PART, int PARTS>
@@ -2248,7 +2263,7 @@ void launch_x_pass_part(const XPassArgs<T>& a, const FftPlan* pl, size_t smem, c
       return;
     }
   }
-  with_path<PART, PARTS, true>(a.g.nx, a.sched, [&](auto p) {
+  with_path<T, kPassX, PART, PARTS>(a.g.nx, a.sched, [&](auto p) {
     constexpr int PATH = decltype(p)::value;
     k_x_pass<T, PATH><<<x_pass_blocks(a), x_threads(sizeof(T), PATH == kFft256), smem, s>>>(a, pl);
   });
@@ -2256,26 +2271,26 @@ void launch_x_pass_part(const XPassArgs<T>& a, const FftPlan* pl, size_t smem, c
 template <typename T, int PART, int PARTS>
 void launch_y_fwd_part(const YFwdArgs<T>& a, const FftPlan* pl, size_t smem, cudaStream_t s) {
   const int grid = a.nvar * a.g.mx * ((a.g.nz + a.tz - 1) / a.tz) + (a.kz_tab ? a.g.mx : 0);
-  with_path<PART, PARTS>(a.g.ny, a.sched,
+  with_path<T, kPassYFwd, PART, PARTS>(a.g.ny, a.sched,
                          [&](auto p) { k_y_fwd<T, decltype(p)::value><<<grid, kThreads, smem, s>>>(a, pl); });
 }
 template <typename T, int PART, int PARTS>
 void launch_z_fwd_part(const ZFwdArgs<T>& a, const FftPlan* pl, size_t smem, cudaStream_t s) {
   const int grid = a.g.mx * ((a.g.my + a.ty - 1) / a.ty);
-  with_path<PART, PARTS>(a.g.nz, a.sched,
+  with_path<T, kPassZFwd, PART, PARTS>(a.g.nz, a.sched,
                          [&](auto p) { k_z_fwd<T, decltype(p)::value><<<grid, kThreads, smem, s>>>(a, pl); });
 }
 // Load the kernels a pass along length n runs and opt them into the largest
 // dynamic shared memory the device allows.
-template <int PART, int PARTS, bool EVEN = false, typename F> void each_sched(int n, F f) {
-  with_path<PART, PARTS, EVEN>(n, 0, f);
-  if (n == 256) with_path<PART, PARTS, EVEN>(n, 1, f);
+template <typename T, int K, int PART, int PARTS, typename F> void each_sched(int n, F f) {
+  with_path<T, K, PART, PARTS>(n, 0, f);
+  if (n == 256) with_path<T, K, PART, PARTS>(n, 1, f);
 }
 template <typename T, int PART, int PARTS> void smem_zinv_part(int n, int optin) {
-  each_sched<PART, PARTS>(n, [&](auto p) { allow_dynamic_smem((const void*)k_z_inv<T, decltype(p)::value>, optin); });
+  each_sched<T, kPassZInv, PART, PARTS>(n, [&](auto p) { allow_dynamic_smem((const void*)k_z_inv<T, decltype(p)::value>, optin); });
 }
 template <typename T, int PART, int PARTS> void smem_yinv_part(int n, int optin) {
-  each_sched<PART, PARTS>(n, [&](auto p) { allow_dynamic_smem((const void*)k_y_inv<T, decltype(p)::value>, optin); });
+  each_sched<T, kPassYInv, PART, PARTS>(n, [&](auto p) { allow_dynamic_smem((const void*)k_y_inv<T, decltype(p)::value>, optin); });
 }
 template <typename T, int PART, int PARTS> void smem_x_part(int n, int optin) {
   if constexpr (path_part(256, PARTS) == PART) {
@@ -2291,13 +2306,13 @@ template <typename T, int PART, int PARTS> void smem_x_part(int n, int optin) {
       }
     }
   }
-  each_sched<PART, PARTS, true>(n, [&](auto p) { allow_dynamic_smem((const void*)k_x_pass<T, decltype(p)::value>, optin); });
+  each_sched<T, kPassX, PART, PARTS>(n, [&](auto p) { allow_dynamic_smem((const void*)k_x_pass<T, decltype(p)::value>, optin); });
 }
 template <typename T, int PART, int PARTS> void smem_yfwd_part(int n, int optin) {
-  each_sched<PART, PARTS>(n, [&](auto p) { allow_dynamic_smem((const void*)k_y_fwd<T, decltype(p)::value>, optin); });
+  each_sched<T, kPassYFwd, PART, PARTS>(n, [&](auto p) { allow_dynamic_smem((const void*)k_y_fwd<T, decltype(p)::value>, optin); });
 }
 template <typename T, int PART, int PARTS> void smem_zfwd_part(int n, int optin) {
-  each_sched<PART, PARTS>(n, [&](auto p) { allow_dynamic_smem((const void*)k_z_fwd<T, decltype(p)::value>, optin); });
+  each_sched<T, kPassZFwd, PART, PARTS>(n, [&](auto p) { allow_dynamic_smem((const void*)k_z_fwd<T, decltype(p)::value>, optin); });
 }
 
 }  // namespace samgpu
