@@ -1425,14 +1425,17 @@ int sam_gpu_set_les(int model, double c_smag, double pr_t) {
       CK(cudaMalloc(&c.les_phys, (es / 2) * 3 * (size_t)g.nx * g.ny * g.nz));
       CK(cudaMalloc(&c.les_work, sizeof(double) * les_dynamic_work(g.nx, g.ny, g.nz)));
     }
-    if (model == 3 && !c.les_feat) {
+    if (model == 3) {
       const size_t np = (size_t)g.nx * g.ny * g.nz;
       int rc = mlp_ensure(c);
       if (rc) return rc;
-      CK(cudaMalloc(&c.les_feat, 32 * np));
-      CK(cudaMalloc(&c.les_coef, sizeof(float2) * np));
-      // zero until the first stage 1 forms them (no subgrid terms before)
-      CK(cudaMemsetAsync(c.les_coef, 0, sizeof(float2) * np, c.stream));
+      // (closure_inputs may have allocated the invariants before)
+      if (!c.les_feat) CK(cudaMalloc(&c.les_feat, 32 * np));
+      if (!c.les_coef) {
+        CK(cudaMalloc(&c.les_coef, sizeof(float2) * np));
+        // zero until the first stage 1 forms them (no subgrid terms before)
+        CK(cudaMemsetAsync(c.les_coef, 0, sizeof(float2) * np, c.stream));
+      }
     }
   }
   double dsq;
