@@ -458,6 +458,7 @@ static int run_x_pass(Ctx& c, int in_mode, int out_mode, int nin, const void* in
     if (nblk > c.partial_blocks) {
       cudaFree(c.partials);
       c.partials = nullptr;
+      c.partial_blocks = 0;
       CK(cudaMalloc(&c.partials, sizeof(double) * 4 * 4 * (size_t)nblk));
       c.partial_blocks = nblk;
     }
@@ -1410,16 +1411,20 @@ int sam_gpu_set_les(int model, double c_smag, double pr_t) {
     const int nf = g.lu + g.lr + (model == 3 ? 3 : 0);
     const size_t s1 = (size_t)nf * g.mx * g.my * g.nz;
     const size_t s2 = (size_t)nf * g.nz * g.ny * g.mx;
-    if (c.s1_elems < s1) {
-      cudaFree(c.S1); c.S1 = nullptr; c.s1_elems = 0;
-      CK(cudaMalloc(&c.S1, es * s1));
-      c.s1_elems = s1;
-    }
-    if (c.s2_elems < s2) {
-      cudaFree(c.S2); c.S2 = nullptr; c.s2_elems = 0;
-      CK(cudaMalloc(&c.S2, es * s2));
-      c.s2_elems = s2;
-    }
+    // (the old buffers stay in use until there are new ones: a failed allocation
+    // leaves the solver as it was)
+    auto grow = [&](void*& p, size_t& have, size_t want) {
+      void* q = nullptr;
+      if (have >= want) return cudaSuccess;
+      const cudaError_t e = cudaMalloc(&q, es * want);
+      if (e != cudaSuccess) return e;
+      cudaFree(p);
+      p = q;
+      have = want;
+      return cudaSuccess;
+    };
+    CK(grow(c.S1, c.s1_elems, s1));
+    CK(grow(c.S2, c.s2_elems, s2));
     if (!c.les_cds) CK(cudaMalloc(&c.les_cds, sizeof(double)));
     if (model == 2 && !c.les_work) {
       CK(cudaMalloc(&c.les_phys, (es / 2) * 3 * (size_t)g.nx * g.ny * g.nz));
