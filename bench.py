@@ -800,8 +800,8 @@ def main():
                 "algorithmic_bytes_per_launch": xb,
                 "traffic": tr.get("bytes_per_launch") if tr else None,
                 "peak_source": "MEASURED_PEAKS.json hbm_gbs (measured)" if "hbm_gbs" in peaks else "fallback",
-                "note": "the FP64 transforms run as 64-bit fixed point on the integer pipes, which bound them "
-                        "(counters at 256^3 in profiles/x_pass_256_ncu.md); the rate of FP64 arithmetic no longer does",
+                "note": "the FP64 transforms run as 64-bit fixed point on the integer pipes, which bound them; "
+                        "the rate of FP64 arithmetic no longer does",
                 "fp64_equivalent": {"achieved": alu, "unit": "TFLOP/s", "flops_per_launch": x_pass_flops(),
                                     "fp64_fma_peak": fp64_peak,
                                     "peak_source": "FP64 FMA peak measured live in this run (DFMA loop)"},
@@ -817,8 +817,7 @@ def main():
                             "achieved": a32, "peak": hbm_peak, "unit": "GB/s", "frac": a32 / hbm_peak,
                             "traffic": tr32.get("bytes_per_launch") if tr32 else None,
                             "algorithmic_bytes_per_launch": xb32, "ms": x32_ms,
-                            "note": "bound by shared-memory traffic and latency: counters at 256^3 in "
-                                    "profiles/x_pass_f256_fp32_256_ncu.md"}
+                            "note": "bound by shared-memory traffic and latency"}
     if ddf is not None:
         xd_ms = ddf.pop("_x_ms")
         ad = x_pass_bytes(w=8) / (xd_ms / 1e3) / 1e9

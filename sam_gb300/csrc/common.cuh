@@ -50,8 +50,8 @@ constexpr int kThreads = 256;
 // sam_gpu_config.precision of the form that asks for about 48 significand
 // bits in the plain step (SAM_GPU_PREC_DD in sam_gpu.h).  It runs the FP64
 // form's kernels: fixed-point lines carry more bits than pairs of FP32 numbers
-// did and are faster (256^3 stage 2: 2.83 against 3.36 ms, 128^3 0.51 against
-// 0.53, 120x135x162 1.54 against 1.66).
+// did and are faster but on the smallest grids (a step: 256^3 8.5 against 10.3
+// ms, 128^3 1.35 against 1.59, 384^3 79 against 85; 32^3 141 against 131 us).
 constexpr int kPrecDD = 48;
 
 // Streaming multiprocessors of the current device (looked up once per

@@ -1,10 +1,17 @@
 // Batched mixed-radix FFT engine for sm_103a: lines of length n <= 1024 held
-// in shared memory, each line transformed by a team of TW threads (TW a power
-// of two, TW >= n/8; teams wider than a warp synchronise on a named barrier).
-// A stage of radix p (2, 3, 4, 5, 8) is a self-sorting Stockham step done in
-// place: every thread first loads all of its butterfly inputs (at most 8
-// complex values) into registers, the team synchronises, then the thread
-// computes and writes its outputs.  The plan is read from shared memory.
+// in shared memory, each line transformed by a team of threads.  A stage is a
+// self-sorting Stockham step done in place: every thread first loads all of its
+// butterfly inputs into registers, the team synchronises, then the thread
+// computes and writes its outputs.
+//  - Lengths of 8 to 256, and 512: radices (2 to 16), teams (of any width up to
+//    a warp, packed into warps; 64 threads at 512) and every index but the
+//    thread's place are fixed at compile time (ct_plan); at most 10 values a
+//    thread.
+//  - 256 points besides as 16 x 16 in registers (fft256_lines).
+//  - The rest: radices 2, 3, 4, 5 and 8 read from the plan in shared memory,
+//    teams of a power of two >= n / 8 threads (wider ones than a warp
+//    synchronise on a named barrier), at most 8 values a thread.
+// FP64 lines are integers under one scale while they are transformed (fx64.cuh).
 //
 // Conventions are FFTPACK's (the reference's fft.f): unnormalised transforms,
 // SIGN = -1 is cfftf (exp(-i ...)), SIGN = +1 is cfftb (exp(+i ...)).

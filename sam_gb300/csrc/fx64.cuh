@@ -5,16 +5,17 @@
 // (measured).  The transforms of the FP64 form therefore run in 64-bit fixed
 // point on the integer pipes: a line's doubles become integers under one
 // scale for the whole line, every butterfly sum is exact, every twiddle
-// product is rounded once at the line's last bit, and the results are
-// converted back to doubles.
+// product is off by a unit or two of the line's last place at most (below),
+// and the results are converted back to doubles.
 //
 // Scale: with L1 = sum (|re| + |im|) over the line, every partial sum and
 // every result of a discrete Fourier transform is at most L1 in modulus, so
 // the line is scaled to L1 < 2^62 and nothing can overflow.  A unit in the
 // last place is then at most 2^-61 L1 <= 2^-61 sqrt(2 n) |x|_2: about 2^-57
-// of the line's norm at n = 256, which leaves room for the roundings of the
-// twiddle products below the 2^-53 of FP64 arithmetic
-// (tests/test_gpu_fixed_point.py compares both with extended precision).
+// of the line's norm at n = 256 and 2^-55.5 at n = 1024, which leaves room for
+// the roundings of the twiddle products below the 2^-53 of FP64 arithmetic
+// (tests/test_gpu_fixed_point.py and test_gpu_line_accuracy.py compare both
+// with extended precision).
 //
 // Exceptional lines: a line holding an infinity or a NaN gives NaN
 // throughout; lines whose largest value is so small or so large that the
@@ -50,8 +51,7 @@ __device__ __forceinline__ FxSplit fx_split(long long v) {
 __host__ __device__ constexpr FxSplit fx_const(long long v) {
   return FxSplit{(int)((v + 0x80000000ll) >> 32), (int)(uint32_t)(v & 0xffffffffll)};
 }
-// (the instruction spelled out: the compiler widens products of such halves
-// to 64 x 64-bit ones, twice the instructions)
+// (the instruction spelled out, so that it is the one intended)
 __device__ __forceinline__ long long fx_mad(int a, int b, long long c) {
   long long r;
   asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
@@ -64,16 +64,20 @@ __device__ __forceinline__ long long fx_join(long long A, uint32_t clo) {
   const uint32_t hi = __funnelshift_l((uint32_t)A, (uint32_t)(A >> 32), 2);
   return (long long)(((uint64_t)hi << 32) | lo);
 }
-// a * w, w in units of 2^-62, |w| <= 1: rounded to the nearest unit (the low
-// halves' product, below 2^-32 of a unit, is left out)
+// a * w, w in units of 2^-62, |w| <= 1: within 1.5 units (half of one by
+// rounding, up to one by the low halves' product, which is left out)
 __device__ __forceinline__ long long fx_mul(FxSplit a, FxSplit w) {
   const long long c = fx_mad(a.l, w.h, fx_mad(a.h, w.l, 1ll << 29));
   return fx_join(fx_mad(a.h, w.h, c >> 32), (uint32_t)c);
 }
-// with LOW, the low halves' products too (the long lines of the run-time
-// path, whose units in the last place are coarser against their norm)
+// the low halves' product, in units of the cross terms: added in products of
+// fields (fx_mul_line), and with LOW in the twiddle products of the run-time
+// path's long lines, whose units in the last place are coarser against their
+// norm
 __device__ __forceinline__ long long fx_low(FxSplit a, FxSplit w) { return (long long)__mulhi(a.l, w.l); }
-// a * u + b * v, rounded once.  |a|, |b| < 2^62 with a^2 + b^2 < 2^124 and
+// a * u + b * v, rounded once with LOW, else within 2.5 units.  (Without LOW a
+// transform of 256 points is 0.35 x 2^-53 off instead of 0.31, of 512 0.80
+// instead of 0.74: FP64 arithmetic 1.6-1.8.)  |a|, |b| < 2^62 with a^2 + b^2 < 2^124 and
 // u^2 + v^2 <= 1 (or |a| + |b| < 2^62 and |u| + |v| < 1.6) keep the cross
 // terms below 2^63.
 template <bool LOW = false> __device__ __forceinline__ long long fx_dot(FxSplit a, FxSplit b, FxSplit u, FxSplit v) {
@@ -415,7 +419,8 @@ __device__ __forceinline__ fxc fx_whole(FxSplit2 v) {
 // at once) as one line's integers.  By Cauchy and Schwarz the sum of the
 // products' moduli is at most the product of the lines' norms, so the 124-bit
 // products shifted down by r = 62 + ceil(log2(norm_a norm_b)) sum to less
-// than 2^62, the bound a transform needs; each is rounded once.
+// than 2^62, the bound a transform needs; each is rounded once (all four
+// products of halves are formed).
 //
 // With a subgrid term (a line of doubles whose moduli sum to less than
 // 2^g.ex) both parts stay below 2^61: r grows by one, and further where the

@@ -1,5 +1,5 @@
 // Argument blocks and launchers of the transform passes (passes_impl.cuh,
-// instantiated in passes.cu and passes_f32.cu).
+// instantiated in passes_part.cu and passes_ens.cu).
 // Strides are in complex (or real, for physical arrays) elements.
 #pragma once
 #include "common.cuh"

@@ -1,7 +1,7 @@
 // The ensemble's persistent stage kernel and its recorder (ens.cuh): the
 // FP32 pass bodies of passes_impl.cuh, instantiated with L2-coherent loads
-// for the transform lengths that have a compile-time FFT path (32, 64, 96,
-// 128), run as work items drawn from one ticket counter.
+// for the transform lengths 32, 64, 96 and 128, run as work items drawn from
+// one ticket counter.
 #include <algorithm>
 #include <cstring>
 

@@ -38,14 +38,20 @@ __device__ __forceinline__ void load_twiddles(tw_t<T>* s_tw, const tw_t<T>* __re
 constexpr int kBatch = 8;
 
 // Resident CTAs per SM each kernel's register budget is sized for (measured
-// at 256^3): in FP32 the transpose passes of the 16 x 16 register path fit
+// at 256^3): in FP32 the transpose passes of the 16 x 16 register path have
 // 64 registers (four CTAs; the y inverse 48 with five, 5 % faster; the y
 // forward at six measured 12 % slower) and the x pass 72 (three CTAs of 288
-// threads) without spills; the compile-time Stockham transposes (lengths 32-512)
-// spilled 40-110 bytes at 64 and keep three CTAs (80 registers; 128^3 y
-// forward 10 % faster); the FP32 z_fwd epilogue spills below 128 and keeps
-// two (three measured slower).  FP64 lines are 64-bit integers, two registers
-// each: 128 registers (two CTAs) hold a radix-16 butterfly, 80 (three) spill.
+// threads); the compile-time Stockham transposes spilled 40-110 bytes at 64 and
+// have three CTAs (80 registers; 128^3 y forward 10 % faster); the FP32 z_fwd
+// epilogue spills below 128 and has two (three measured slower).  FP64 lines
+// are 64-bit integers, two registers each: 128 registers (two CTAs) hold a
+// radix-16 butterfly, 80 (three) spill.  About half of the kernels spill
+// (ptxas -v: 239 of 472): the forward transposes little (FP64 y at most 190
+// bytes at compiled lengths), the inverse ones, whose gradient fields of the
+// closures are two more copies of the transform, 120-170 at 128 and 256
+// points and up to 1116 at lengths with a factor of 125 (FP32 y inverse of 256
+// points 260), without the plain step having become slower by it (256^3 FP32 y
+// inverse 0.067 ms with and without).
 // The run-time-radix path (kFftGeneric, lengths without a compile-time path)
 // needs more registers: in FP32 one x pass CTA per SM, two of the others; in
 // FP64 see two_ctas_upto.
@@ -85,7 +91,6 @@ __device__ __forceinline__ void batched(int count, Get get, Put put) {
 
 __host__ __device__ inline bool is_pow2_inv(int n) { return n > 0 && (n & (n - 1)) == 0; }
 
-// First-stage loader reading element idx of a row in global memory.
 // Store phase of the transposes: line t (t < nl) of a tile of `tile` lines
 // in shared memory goes to dst[r * ostride + t] for output rows r < nr,
 // taking its element at line position pos(r).  A thread keeps one line and
@@ -114,6 +119,7 @@ template <bool COH, typename V> __device__ __forceinline__ V ldc(const V* p) {
   else return *p;
 }
 
+// First-stage loader reading element idx of a row in global memory.
 template <typename C, bool COH = false> struct RowLoad {
   const C* __restrict__ row;
   __device__ __forceinline__ C operator()(int idx) const { return ldc<COH>(row + idx); }
