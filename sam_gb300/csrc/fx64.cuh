@@ -5,8 +5,8 @@
 // (measured).  The transforms of the FP64 form therefore run in 64-bit fixed
 // point on the integer pipes: a line's doubles become integers under one
 // scale for the whole line, every butterfly sum is exact, every twiddle
-// product is off by a unit or two of the line's last place at most (below),
-// and the results are converted back to doubles.
+// product is off by 2.5 units of the line's last place at most (below), and the
+// results are converted back to doubles.
 //
 // Scale: with L1 = sum (|re| + |im|) over the line, every partial sum and
 // every result of a discrete Fourier transform is at most L1 in modulus, so
